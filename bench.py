@@ -274,9 +274,9 @@ def reference_arm(a, cfg):
 # ---------------------------------------------------------------- roofline
 def noise_cuts(L, cfg, theta):
     """Per beam set and dataset, the own-FFT path's noise cut-off (bins k
-    with min(k, m - k) > kc carry exp(-sigma^2 w_k^2 / 2) < e^-760, i.e.
-    exactly 0; the same formula as the library's noise_cut), with the grid
-    step of each beam set from the library and sigma = the dataset's noise
+    with min(k, m - k) > kc carry exp(-sigma^2 w_k^2 / 2) < e^-72, below
+    the rounding of the sums they enter; the same formula as the library's
+    noise_cut), with the grid step of each beam set from the library and sigma = the dataset's noise
     (the proposals keep the sigma multiplier at 1)."""
     n = cfg["fftsize"]
     m = n // 2
@@ -288,7 +288,7 @@ def noise_cuts(L, cfg, theta):
         for d, bi in enumerate(cfg["map_beam"]):
             if bi != b:
                 continue
-            x = np.sqrt(1520.0) / (cfg["sigmas"][d] * iflux)
+            x = 12.0 / (cfg["sigmas"][d] * iflux)
             kcs.append(m if x >= m else int(np.ceil(x)) + 1)
         sets.append(kcs)
     return sets

@@ -23,6 +23,14 @@ namespace dev {
 
 constexpr double kTwoPi = 6.283185307179586476925286766559005768394;
 constexpr double kSmallLogVal = -30.0;
+// Noise exponent below which a spectrum bin is taken as 0: e^-70 < 2^-100.
+// No bin exceeds the DC bin, which is 1, so all of the at most 2^26 bins of
+// a P(D) past this line together add less than 2^-74 to any of its values,
+// 2^-21 of one rounding of the DC term alone (2^-53); exp itself underflows
+// only at -745.2, a 3.3 times wider line.  Against a line at -750: 128
+// proposals x 3 beam sets of n = 65536 487 -> 475 us, 64 of n = 2048 in two
+// bands 7.83 -> 7.65 ms, every result the same to the last bit.
+constexpr double kNoiseZero = -70.0;
 
 // ------------------------------------------------------------------ exp2
 // Table-driven 2^x after Tang ("Table-driven implementation of the

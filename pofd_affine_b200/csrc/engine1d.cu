@@ -505,15 +505,15 @@ void launch_rfill(int per, bool seg, dim3 grid, cudaStream_t st, const BSet1Dev*
 // Moments, sigma estimate and the shift decision (PDFactory.cc:660-679,
 // 1067-1076), one thread per (proposal, beam set).
 // Noise cut-off of the half-length spectrum (own-FFT path): with noise sigma
-// the factor exp(-sigma^2 w_k^2 / 2) is below e^-760 -- exactly 0 in double
-// precision, whose exp underflows below -745.2 -- for every bin k with
-// min(k, m - k) > kc, kc = ceil(sqrt(1520) / (sigma * 2 pi / (n dflux))) + 1.
-// Returns m (no bin is cut) without noise.
+// the factor exp(-sigma^2 w_k^2 / 2) is below e^-72 -- past the line
+// dev::kNoiseZero, where a bin is below the rounding of the sum it enters --
+// for every bin k with min(k, m - k) > kc, kc = ceil(sqrt(144) / (sigma *
+// 2 pi / (n dflux))) + 1.  Returns m (no bin is cut) without noise.
 __device__ __forceinline__ int noise_cut(double sigma, double dflux, int n) {
   const int m = n / 2;
   if (!(sigma > 0.0)) return m;
   const double iflux = dev::kTwoPi / (static_cast<double>(n) * dflux);
-  const double x = sqrt(1520.0) / (sigma * iflux);
+  const double x = 12.0 / (sigma * iflux);
   return (x >= static_cast<double>(m)) ? m : static_cast<int>(ceil(x)) + 1;
 }
 
@@ -575,8 +575,8 @@ __global__ void k_moments1(const BSet1Dev* __restrict__ bsets,
 // dataset of the beam set (PDFactory.cc:1106-1132, 1174-1188).  The
 // self-conjugate Nyquist bin keeps only its real part, which is what the
 // c2r transform uses of it.  Where every dataset's noise exponent is below
-// -750, exp() underflows to exactly 0 and the reference's product is 0: those
-// bins are written as 0 without evaluating exp/sincos of the R spectrum.
+// dev::kNoiseZero the bins are written as 0 without evaluating exp/sincos of
+// the R spectrum.
 __global__ void __launch_bounds__(NT)
 k_spectrum1(const BSet1Dev* __restrict__ bsets,
             const DSet1Dev* __restrict__ dsets, int B, int D, int n, int nc,
@@ -598,7 +598,7 @@ k_spectrum1(const BSet1Dev* __restrict__ bsets,
     const double sigma = sm * dsets[bs.ds_begin + dd].sigma_base;
     if (!(sigma > 0)) { all_zero = false; break; }
     const double sigfac = -0.5 * sigma * sigma;
-    if (!(sigfac * wv * wv < -750.0)) all_zero = false;
+    if (!(sigfac * wv * wv < dev::kNoiseZero)) all_zero = false;
   }
   if (all_zero) {
     for (int dd = 0; dd < bs.nds; ++dd)
@@ -910,8 +910,8 @@ k_fftB(int m1, int rowsz, int nrows_per_w, const int* __restrict__ mstatus,
 
 // The spectrum on bin pairs (q, m - q): the real-transform split X from Z,
 // exp(X - X_0) with the mean shift, the noise factor per dataset (bins whose
-// noise exponent is below -750 for every dataset are exactly 0, as in the
-// reference), and the merge Z' of the inverse real transform, written into
+// noise exponent is below dev::kNoiseZero for every dataset are 0), and the
+// merge Z' of the inverse real transform, written into
 // each dataset's row.  Wn[k] = e^{-2 pi i k / n}, k in [0, m].
 __device__ __forceinline__ bool spec_all_zero(const BSet1Dev& bs, const DSet1Dev* dsets,
                                               double sm, double wv, int k) {
@@ -920,7 +920,7 @@ __device__ __forceinline__ bool spec_all_zero(const BSet1Dev& bs, const DSet1Dev
     const double sigma = sm * dsets[bs.ds_begin + dd].sigma_base;
     if (!(sigma > 0)) return false;
     const double sigfac = -0.5 * sigma * sigma;
-    if (!(sigfac * wv * wv < -750.0)) return false;
+    if (!(sigfac * wv * wv < dev::kNoiseZero)) return false;
   }
   return true;
 }

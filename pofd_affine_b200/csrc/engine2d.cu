@@ -719,8 +719,8 @@ __device__ __forceinline__ void spectrum2_selfconj(const BSet2Dev& bs, const DSe
 // (PDFactoryDouble.cc:1241-1342, 1383-1437).  The noise exponent of a
 // dataset is added to the exponent of exp(R~ - R~00) -- one exp per bin and
 // dataset for the reference's two, the same product rounded once.  Bins
-// where every dataset's noise exponent is below -750 are exactly 0 in the
-// reference and are written as 0 directly.
+// where every dataset's noise exponent is below dev::kNoiseZero are written
+// as 0 directly.
 __global__ void __launch_bounds__(NT, 5)
 k_spectrum2(const BSet2Dev* __restrict__ bsets,
             const DSet2Dev* __restrict__ dsets, int B, int D, int n, int nc,
@@ -746,7 +746,7 @@ k_spectrum2(const BSet2Dev* __restrict__ bsets,
     if (!(s1 > 0 || s2 > 0)) { all_zero = false; break; }
     const double sf1 = -0.5 * s1 * s1 * iflux1 * iflux1;
     const double sf2 = -0.5 * s2 * s2 * iflux2 * iflux2;
-    if (!(sf1 * didx1 * didx1 + sf2 * didx2 * didx2 < -750.0)) all_zero = false;
+    if (!(sf1 * didx1 * didx1 + sf2 * didx2 * didx2 < dev::kNoiseZero)) all_zero = false;
   }
   double2* out0 = reinterpret_cast<double2*>(pbuf) + static_cast<size_t>(w) * D * n * nc;
   if (all_zero) {
@@ -1501,7 +1501,7 @@ k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dset
       const double didx1 = (i1 < nc) ? static_cast<double>(i1) : static_cast<double>(N - i1);
       const double didx2 = static_cast<double>(i2);
       const double nz = noisy ? sf1n * didx1 * didx1 + sf2n * didx2 * didx2 : 0.0;
-      if (noisy && nz < -750.0) {  // exactly 0 in the reference
+      if (noisy && nz < dev::kNoiseZero) {
         buf[q] = make_double2(0.0, 0.0);
         continue;
       }
@@ -1530,7 +1530,7 @@ k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dset
         }
         const double didx1 = static_cast<double>(i1);
         const double nz = noisy ? sf1n * didx1 * didx1 + sf2n * didx2 * didx2 : 0.0;
-        if (noisy && nz < -750.0) {
+        if (noisy && nz < dev::kNoiseZero) {
           b[si] = make_double2(0.0, 0.0);
           if (j1 != i1) b[sj] = make_double2(0.0, 0.0);
           continue;
