@@ -938,7 +938,7 @@ int pofd_like2_profile(pofd_like2* L, unsigned nprop, const float* theta,
     need(L && theta && stage_ms && nstages, "null argument");
     need(reps > 0, "reps must be > 0");
     L->eng->profile_stages(nprop, theta, npar, reps, stage_ms);
-    *nstages = pofd::Engine2::kNumStages;
+    *nstages = L->eng->num_stages();
     return POFD_OK;
   });
 }

@@ -1288,6 +1288,671 @@ __global__ void k_reduce2(const BSet2Dev* __restrict__ bsets,
   logl[w] = (st == 0) ? LogLike : qnan;
 }
 
+// ------------------------------------------------------------------
+// Transforms of FFT mode 1 (n a power of two in [512, 4096]): the R grid,
+// its row transforms, the columns with the spectrum between their two
+// transforms, and the inverse row transforms with the marginal sums of the
+// P(D), in three kernels with one intermediate array.
+//
+//   k_rowfwd2   R of a few rows (straight into registers, never stored),
+//               their forward row DFTs, columns 0 .. kc of the result
+//   k_colspec2  per column: forward DFT, spectrum, inverse DFT, in place
+//   k_rowinv2   inverse row DFTs of columns 0 .. kc, the P(D) rows and the
+//               marginal sums
+//
+// kc is the noise cut-off in band 2: with noise sigma every bin of a column
+// k2 > kc lies past dev::kNoiseZero, so those columns are neither computed,
+// stored nor read (kc = 427 of 1024 at n = 2048, 2.8 mJy).  The intermediate
+// array is kept by columns, [k2][row], so that the column kernel, which
+// reads and writes it whole, streams; the row kernels take several rows at
+// a time and touch it in contiguous pieces of 2 G rows (64 bytes at n =
+// 2048).
+//
+// One DFT, n = 16 M, M = 16 M3, runs on M threads with 16 values each: with
+// input j = n1 M + u, u = m M3 + s and output k = k1 + 16 k2 + 256 k3,
+//   stage 1: 16-point register DFTs over n1, times W_n^{u k1};
+//   stage 2: 16-point register DFTs over m, times W_M^{s k2};
+//   stage 3: M3-point register DFTs over s;
+// thread u holds (k1, s) = (u / M3, u % M3) in stage 2 and the outputs of
+// p = k1 + 16 k2 = u, u + M, ... in stage 3.  The two exchanges go through
+// shared memory, pitched so that neither side has bank conflicts.  A column
+// goes back through the same stages transposed.  Twiddle powers come from
+// four table entries per thread and stage (W^x, W^2x, W^4x, W^8x, made in
+// long double), the other eleven by one product each: a table of all of
+// them would cost as much shared memory traffic again as the exchanges.
+template <int N>
+struct Fft2 {
+  static constexpr int M = N / 16, M3 = N / 256;
+  static constexpr int PITCH = M + M3;        // of the first exchange, [k1][u]
+  static constexpr int SL = 256 * (M3 + 1);   // slots per DFT: [p][s], one pad
+  static constexpr int PP = 16 / M3;          // stage-3 DFTs per thread
+};
+
+template <int S>
+__device__ __forceinline__ void tw16(double2* v, const double2* __restrict__ T) {
+  double2 w1 = __ldg(T), w2 = __ldg(T + 1), w4 = __ldg(T + 2), w8 = __ldg(T + 3);
+  if (S > 0) {
+    w1.y = -w1.y;
+    w2.y = -w2.y;
+    w4.y = -w4.y;
+    w8.y = -w8.y;
+  }
+  const double2 w3 = fft::cmul(w1, w2);
+  v[1] = fft::cmul(v[1], w1);
+  v[2] = fft::cmul(v[2], w2);
+  v[3] = fft::cmul(v[3], w3);
+  v[4] = fft::cmul(v[4], w4);
+  v[8] = fft::cmul(v[8], w8);
+  v[9] = fft::cmul(v[9], fft::cmul(w1, w8));
+  v[10] = fft::cmul(v[10], fft::cmul(w2, w8));
+  v[11] = fft::cmul(v[11], fft::cmul(w3, w8));
+  const double2 w5 = fft::cmul(w1, w4), w6 = fft::cmul(w2, w4), w7 = fft::cmul(w3, w4);
+  v[5] = fft::cmul(v[5], w5);
+  v[6] = fft::cmul(v[6], w6);
+  v[7] = fft::cmul(v[7], w7);
+  v[12] = fft::cmul(v[12], fft::cmul(w4, w8));
+  v[13] = fft::cmul(v[13], fft::cmul(w5, w8));
+  v[14] = fft::cmul(v[14], fft::cmul(w6, w8));
+  v[15] = fft::cmul(v[15], fft::cmul(w7, w8));
+}
+
+// Stages 1 and 2: v[n1] = input n1 M + u of the thread; leaves the stage-3
+// inputs in the slots b[p (M3 + 1) + s].
+template <int N, int S>
+__device__ __forceinline__ void fft2_head(double2* v, double2* b, int u,
+                                          const double2* __restrict__ TW) {
+  using F = Fft2<N>;
+  fft::dft<16, S>(v);
+  tw16<S>(v, TW + 4 * u);
+#pragma unroll
+  for (int k1 = 0; k1 < 16; ++k1) b[k1 * F::PITCH + u] = v[k1];
+  __syncthreads();
+  const int k1 = u / F::M3, s = u % F::M3;
+#pragma unroll
+  for (int m = 0; m < 16; ++m) v[m] = b[k1 * F::PITCH + m * F::M3 + s];
+  fft::dft<16, S>(v);
+  tw16<S>(v, TW + 64 * s);
+  __syncthreads();
+#pragma unroll
+  for (int k2 = 0; k2 < 16; ++k2) b[(k1 + 16 * k2) * (F::M3 + 1) + s] = v[k2];
+  __syncthreads();
+}
+
+// The transposed stages 2 and 1 of the inverse, from the slots to v[n1] =
+// output n1 M + u.
+template <int N>
+__device__ __forceinline__ void fft2_tail_inv(double2* v, double2* b, int u,
+                                              const double2* __restrict__ TW) {
+  using F = Fft2<N>;
+  const int k1 = u / F::M3, s = u % F::M3;
+#pragma unroll
+  for (int k2 = 0; k2 < 16; ++k2) v[k2] = b[(k1 + 16 * k2) * (F::M3 + 1) + s];
+  tw16<1>(v, TW + 64 * s);
+  fft::dft<16, 1>(v);
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < 16; ++m) b[k1 * F::PITCH + m * F::M3 + s] = v[m];
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = b[j * F::PITCH + u];
+  tw16<1>(v, TW + 4 * u);
+  fft::dft<16, 1>(v);
+}
+
+// 32 bytes in one store (both values' cells adjoin and are 32-byte aligned)
+__device__ __forceinline__ void st32(double2* p, double2 a, double2 b) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};"
+               :
+               : "l"(p), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y)
+               : "memory");
+}
+__device__ __forceinline__ void ld32(const double2* p, double2& a, double2& b) {
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y)
+               : "l"(p)
+               : "memory");
+}
+
+// Threads, DFTs (pairs of rows) and rows per block of the row kernels.
+template <int N>
+struct RowCfg {
+  static constexpr int M = N / 16;
+  static constexpr int T = N <= 512 ? 128 : 256;
+  static constexpr int G = T / M;
+  static constexpr int ROWS = 2 * G;
+};
+inline int rowcfg_rows(int n) { return n <= 1024 ? 8 : (n == 2048 ? 4 : 2); }
+inline size_t rowfwd_smem(int n) {
+  return static_cast<size_t>(rowcfg_rows(n) / 2) * 256 * (n / 256 + 1) * sizeof(double2);
+}
+constexpr int RI_ROWS = 32;  // P(D) rows per block of k_rowinv2 (>= 2 G)
+inline size_t rowinv_smem(int n) {
+  return rowfwd_smem(n) + static_cast<size_t>(rowcfg_rows(n) / 2) * n * sizeof(double);
+}
+// columns per block of k_colspec2
+template <int N>
+struct ColCfg {
+  static constexpr int M = N / 16;
+  static constexpr int T = M < 128 ? 128 : M;
+  static constexpr int C = T / M;
+};
+inline int colcfg_cols(int n) { return n >= 2048 ? 1 : 2048 / n; }
+inline size_t colspec_smem(int n, bool several) {
+  return static_cast<size_t>(colcfg_cols(n)) * 256 * (n / 256 + 1) * sizeof(double2) *
+         (several ? 2 : 1);
+}
+
+// Last column of the half spectrum with a bin inside the noise line (n / 2
+// without noise in band 2).
+__device__ __forceinline__ int noise_cut2(double sigma1, double sigma2, double dflux2, int n) {
+  const int h = n / 2;
+  if (!(sigma1 > 0 || sigma2 > 0)) return h;
+  const double iflux2 = dev::kTwoPi / (static_cast<double>(n) * dflux2);
+  const double x = 12.0 / (fabs(sigma2) * iflux2);  // sqrt(2 * 72): past kNoiseZero
+  return (x >= static_cast<double>(h)) ? h : static_cast<int>(x) + 1;
+}
+
+// The edge cells of row 0 (band-1 edge integral, the double integral at
+// [0, 0]; times dflux1*dflux2) before the row transforms, and the noise
+// cut-offs of each dataset and of each beam set (the widest of its
+// datasets).
+__global__ void __launch_bounds__(NT)
+k_redge0_2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dsets, int B, int D,
+           int n, int edge, int nedge, int ngr, const int* __restrict__ mstatus,
+           const double* __restrict__ sigmult, const double* __restrict__ epart,
+           double* __restrict__ row0, int* __restrict__ kcset, int* __restrict__ kcds) {
+  __shared__ double shr[32];
+  const int wb = blockIdx.y;
+  const int w = wb / B, b = wb - w * B;
+  if (mstatus[w] != 0) return;
+  const BSet2Dev& bs = bsets[b];
+  const double fluxfac = bs.dflux1 * bs.dflux2;
+  const int ncol = n + nedge;
+  const double* ep = epart + static_cast<size_t>(wb) * ngr * ncol;
+  const int j = blockIdx.x * NT + threadIdx.x;
+  if (j >= 1 && j < n) {
+    double c = 0.0;
+    if (edge)
+      for (int g = 0; g < ngr; ++g) c += ep[static_cast<size_t>(g) * ncol + j];
+    row0[static_cast<size_t>(wb) * n + j] = edge ? c * bs.iRxnorm * fluxfac : 0.0;
+  }
+  if (blockIdx.x != 0) return;
+  double r00 = 0.0;
+  if (edge) {
+    for (int jj = threadIdx.x; jj < nedge; jj += NT) {
+      double c = 0.0;
+      for (int g = 0; g < ngr; ++g) c += ep[static_cast<size_t>(g) * ncol + n + jj];
+      r00 += (jj == 0 || jj == nedge - 1) ? 0.5 * c : c;
+    }
+    r00 = dev::block_sum<NT>(r00, shr) * bs.iR00norm;
+  }
+  if (threadIdx.x == 0) {
+    row0[static_cast<size_t>(wb) * n] = edge ? r00 * fluxfac : 0.0;
+    const double sm1 = sigmult[2 * w], sm2 = sigmult[2 * w + 1];
+    int kmax = 0;
+    for (int dd = 0; dd < bs.nds; ++dd) {
+      const int d = bs.ds_begin + dd;
+      const int kc = noise_cut2(sm1 * dsets[d].sb1, sm2 * dsets[d].sb2, bs.dflux2, n);
+      kcds[static_cast<size_t>(w) * D + d] = kc;
+      kmax = max(kmax, kc);
+    }
+    kcset[wb] = kmax;
+  }
+}
+
+// R and its forward row transforms.  A block takes groups of ROWS = 2 G rows,
+// each pair of rows on M threads; a thread evaluates R at its 16 columns u,
+// u + M, ... of both rows (the colour terms as in k_rgrid2, read once per
+// thread for its 16 columns) straight into the 16 inputs of its first DFT,
+// the two rows as real and imaginary part.  Of the result Z the two rows'
+// spectra X0 = (Z_k + conj Z_{n-k}) / 2, X1 = (Z_k - conj Z_{n-k}) / 2i go out
+// for k <= kc.  Block partials of the trapezoid moments of getRStats
+// (PDFactoryDouble.cc:593-722) and of the DC bin: rpart[wb][block][5].
+template <int N>
+__global__ void __launch_bounds__(RowCfg<N>::T, 512 / RowCfg<N>::T)
+k_rowfwd2(const BSet2Dev* __restrict__ bsets, int B, int D, int edge, int gpb,
+          const int* __restrict__ mstatus, const double* __restrict__ rw,
+          const int2* __restrict__ rcnt, const double* __restrict__ row0,
+          const double* __restrict__ redge, const int* __restrict__ kcset,
+          double2* __restrict__ ybuf, double* __restrict__ rpart,
+          const double2* __restrict__ TW) {
+  using F = Fft2<N>;
+  using R = RowCfg<N>;
+  constexpr int M = F::M, M3 = F::M3, G = R::G, T = R::T;
+  constexpr int nc = N / 2 + 1;
+  extern __shared__ double2 fsm[];  // [G][SL]
+  __shared__ double shr[32];
+  __shared__ dev::Exp2Table e2;
+  const int wb = blockIdx.y;
+  const int w = wb / B, bsi = wb - w * B;
+  if (mstatus[w] != 0) return;
+  e2.load();
+  __syncthreads();
+  const BSet2Dev& bs = bsets[bsi];
+  const int t = threadIdx.x, g = t / M, u = t % M;
+  double2* b = fsm + g * F::SL;
+  const int nrows = bs.nrows, ts3 = 3 * bs.Ts;
+  const double fluxfac = bs.dflux1 * bs.dflux2;
+  const double* __restrict__ colinv = bs.colinv + u;
+  const double* __restrict__ collog = bs.collog + u;
+  const double* __restrict__ cflux2 = bs.rflux2 + u;
+  const int kc = kcset[wb];
+  double2* Y = ybuf + (static_cast<size_t>(w) * D + bs.ds_begin) * N * nc;
+  unsigned cpos = 0, cneg = 0, czero = 0;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    if (colinv[q * M] == 0.0) czero |= 1u << q;
+    else if (bs.colsgn[q * M + u]) cneg |= 1u << q;
+    else cpos |= 1u << q;
+  }
+  const unsigned hsm = (bs.hassign[0] ? 1u : 0u) | (bs.hassign[1] ? 2u : 0u) |
+                       (bs.hassign[2] ? 4u : 0u) | (bs.hassign[3] ? 8u : 0u);
+  double m1 = 0.0, v1 = 0.0, m2 = 0.0, v2 = 0.0, r0 = 0.0;
+  for (int gi = 0; gi < gpb; ++gi) {
+    const int rbase = (blockIdx.x * gpb + gi) * R::ROWS;
+    if (rbase >= N) break;
+    double2 v[16];
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      const int r = rbase + 2 * g + h;
+      double acc[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) acc[q] = 0.0;
+      if (r == 0) {
+        const double* e0 = row0 + static_cast<size_t>(wb) * N + u;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) acc[q] = e0[q * M];
+      } else {
+        const int sgn1 = bs.rowsgn[r];
+        if (sgn1 >= 0) {
+          const size_t ri = static_cast<size_t>(wb) * nrows + r;
+          const int2 nt = rcnt[ri];
+          const double* __restrict__ L = rw + ri * ts3;
+          double lf2[16];  // read again per row: not held through the DFT
+#pragma unroll
+          for (int q = 0; q < 16; ++q) lf2[q] = collog[q * M];
+#pragma unroll 1
+          for (int fs = 0; fs < 2; ++fs) {
+            const unsigned cols = fs ? cneg : cpos;
+            if (!cols || !((hsm >> (sgn1 + fs)) & 1u)) continue;
+            const double* __restrict__ Tm = fs ? L + 3 * nt.x : L;
+            const int cnt = fs ? nt.y : nt.x;
+            if ((cols | czero) == 0xffffu) {  // every column of this sign
+              for (int k = 0; k < cnt; ++k) {
+                const double c0 = __ldg(Tm + 3 * k), c1 = __ldg(Tm + 3 * k + 1),
+                             c2 = __ldg(Tm + 3 * k + 2);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                  const double d = lf2[q] - c1;
+                  acc[q] += c0 * dev::exp2_tab(d * d * c2, e2.t);
+                }
+              }
+            } else {
+              for (int k = 0; k < cnt; ++k) {
+                const double c0 = __ldg(Tm + 3 * k), c1 = __ldg(Tm + 3 * k + 1),
+                             c2 = __ldg(Tm + 3 * k + 2);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                  if (!((cols >> q) & 1u)) continue;
+                  const double d = lf2[q] - c1;
+                  acc[q] += c0 * dev::exp2_tab(d * d * c2, e2.t);
+                }
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) acc[q] = acc[q] * colinv[q * M] * fluxfac;
+        if (u == 0) acc[0] = edge ? redge[static_cast<size_t>(wb) * (2 * N + 1) + N + r] * fluxfac : 0.0;
+      }
+      // moment sums of the row; the first and last column weigh a half
+      double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        double a = acc[q];
+        if ((q == 0 && u == 0) || (q == 15 && u == M - 1)) a *= 0.5;
+        const double cf = cflux2[q * M];
+        const double ca = cf * a;
+        s0 += a;
+        s1 += ca;
+        s2 += cf * ca;
+      }
+      const double wr = (r == 0 || r == N - 1) ? 0.5 : 1.0, cf1 = bs.rowflux[r];
+      s0 *= wr;
+      m1 += cf1 * s0;
+      v1 += cf1 * cf1 * s0;
+      m2 += wr * s1;
+      v2 += wr * s2;
+      // the first row waits in the thread's own slots of the exchange
+      double* keep = reinterpret_cast<double*>(b) + u;
+      if (h == 0) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) keep[q * M] = acc[q];
+      } else {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = make_double2(keep[q * M], acc[q]);
+      }
+    }
+    __syncthreads();
+    fft2_head<N, -1>(v, b, u, TW);
+#pragma unroll
+    for (int pp = 0; pp < F::PP; ++pp) {
+      double2* s = b + (pp * M + u) * (M3 + 1);
+      double2 z[M3];
+#pragma unroll
+      for (int i = 0; i < M3; ++i) z[i] = s[i];
+      fft::dft<M3, -1>(z);
+#pragma unroll
+      for (int i = 0; i < M3; ++i) s[i] = z[i];
+    }
+    __syncthreads();
+    for (int k = t; k <= kc; k += T) {
+      const int kn = (N - k) & (N - 1);
+      const int pk = (k & 255) * (M3 + 1) + (k >> 8), pn = (kn & 255) * (M3 + 1) + (kn >> 8);
+      double2* o = Y + static_cast<size_t>(k) * N + rbase;
+#pragma unroll
+      for (int gg = 0; gg < G; ++gg) {
+        const double2 a = fsm[gg * F::SL + pk], c = fsm[gg * F::SL + pn];
+        const double2 x0 = make_double2(0.5 * (a.x + c.x), 0.5 * (a.y - c.y));
+        const double2 x1 = make_double2(0.5 * (a.y + c.y), 0.5 * (c.x - a.x));
+        st32(o + 2 * gg, x0, x1);
+        if (k == 0) r0 += x0.x + x1.x;
+      }
+    }
+    __syncthreads();
+  }
+  m1 = dev::block_sum<T>(m1, shr);
+  v1 = dev::block_sum<T>(v1, shr);
+  m2 = dev::block_sum<T>(m2, shr);
+  v2 = dev::block_sum<T>(v2, shr);
+  if (t == 0) {
+    double* o = rpart + (static_cast<size_t>(wb) * gridDim.x + blockIdx.x) * 5;
+    o[0] = m1; o[1] = v1; o[2] = m2; o[3] = v2; o[4] = r0;
+  }
+}
+
+// Moments, shift decisions (PDFactoryDouble.cc:560-585, 1198-1213) and the
+// DC bin R~00 from the row kernel's partials; one block per proposal and
+// beam set.
+__global__ void __launch_bounds__(NT)
+k_rmom2(const BSet2Dev* __restrict__ bsets, int B, int nparts, const int* __restrict__ mstatus,
+        const double* __restrict__ rpart, double* __restrict__ mom, double* __restrict__ r0buf) {
+  __shared__ double shr[32];
+  const int wb = blockIdx.x;
+  const int w = wb / B;
+  if (mstatus[w] != 0) return;
+  const BSet2Dev& bs = bsets[wb - w * B];
+  const double* p = rpart + static_cast<size_t>(wb) * nparts * 5;
+  double a[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int k = threadIdx.x; k < nparts; k += NT)
+#pragma unroll
+    for (int i = 0; i < 5; ++i) a[i] += p[5 * k + i];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) a[i] = dev::block_sum<NT>(a[i], shr);
+  if (threadIdx.x == 0) {
+    const double s1 = sqrt(a[1]), s2 = sqrt(a[3]);
+    const bool d1 = (s1 > bs.dflux1) && (fabs(a[0]) > bs.dflux1);
+    const bool d2 = (s2 > bs.dflux2) && (fabs(a[2]) > bs.dflux2);
+    double* o = mom + static_cast<size_t>(wb) * 8;
+    o[0] = a[0]; o[1] = a[2]; o[2] = a[1]; o[3] = a[3];
+    o[4] = d1 ? -a[0] : 0.0; o[5] = d2 ? -a[2] : 0.0;
+    o[6] = d1 ? 1.0 : 0.0; o[7] = d2 ? 1.0 : 0.0;
+    r0buf[wb] = a[4];
+  }
+}
+
+// exp(R~ - R~00) with the shifts and one dataset's noise at one bin (the
+// work of k_spectrum2, same formulas).
+struct Spec2 {
+  double r0, sf1, sf2, s1n, s2n;
+  bool sh1, sh2, noisy;
+  template <int N>
+  __device__ __forceinline__ double2 bin(double2 X, int i1, int i2) const {
+    const double d1 = static_cast<double>((i1 <= N / 2) ? i1 : N - i1);
+    const double d2 = static_cast<double>(i2);
+    const double nz = noisy ? s1n * d1 * d1 + s2n * d2 * d2 : 0.0;
+    if (noisy && nz < dev::kNoiseZero) return make_double2(0.0, 0.0);
+    double ival = X.y;
+    if (sh1) ival -= (i1 <= N / 2) ? sf1 * d1 : -sf1 * d1;
+    if (sh2) ival -= sf2 * d2;
+    double sn, cs;
+    sincos(ival, &sn, &cs);
+    const double ep = exp((X.x - r0) + nz);
+    return make_double2(ep * cs, ep * sn);
+  }
+  // a bin of a self-conjugate column (i2 = 0 or n/2), Xm its mirror's value:
+  // the Hermitian part, or the real part where the row is its own mirror
+  template <int N>
+  __device__ __forceinline__ double2 bin_self(double2 X, double2 Xm, int i1, int i2) const {
+    if (i1 == 0 && i2 == 0) return make_double2(1.0, 0.0);
+    const int j1 = (N - i1) & (N - 1);
+    const double2 p = bin<N>(X, i1, i2);
+    if (j1 == i1) return make_double2(p.x, 0.0);
+    const double2 q = bin<N>(Xm, j1, i2);
+    return make_double2(0.5 * (p.x + q.x), 0.5 * (p.y - q.y));
+  }
+};
+
+// The columns: forward DFT, spectrum, inverse DFT, once per dataset of the
+// beam set; in place for the set's first dataset, the others' columns into
+// their own arrays.  The stage-3 outputs of the forward DFT stay in
+// registers through the spectrum into the first stage of the inverse.  A
+// warp's lanes hold 32 consecutive rows there, so that bins past the noise
+// line cost whole warps nothing.  M threads per column and four blocks of
+// 128 threads per SM: one block's loads, barriers and stores overlap the
+// others' arithmetic.
+template <int N>
+__global__ void __launch_bounds__(ColCfg<N>::T, N == 4096 ? 2 : 4)
+k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dsets, int B,
+           int D, const int* __restrict__ mstatus, const double* __restrict__ sigmult,
+           const double* __restrict__ mom, const double* __restrict__ r0buf,
+           const int* __restrict__ kcset, const int* __restrict__ kcds,
+           double2* __restrict__ ybuf, const double2* __restrict__ TW) {
+  using F = Fft2<N>;
+  constexpr int M = F::M, M3 = F::M3, C = ColCfg<N>::C;
+  constexpr int nc = N / 2 + 1;
+  extern __shared__ double2 csm[];  // [C][SL], with several datasets twice
+  const int wb = blockIdx.y;
+  const int w = wb / B, bsi = wb - w * B;
+  if (mstatus[w] != 0) return;
+  const int c0 = blockIdx.x * C;
+  const int kc = kcset[wb];
+  if (c0 > kc) return;
+  const int t = threadIdx.x, u = t % M;
+  const int i2 = c0 + t / M;
+  const BSet2Dev& bs = bsets[bsi];
+  const double iflux1 = dev::kTwoPi / (static_cast<double>(N) * bs.dflux1);
+  const double iflux2 = dev::kTwoPi / (static_cast<double>(N) * bs.dflux2);
+  const double* mo = mom + static_cast<size_t>(wb) * 8;
+  Spec2 sp;
+  sp.r0 = r0buf[wb];
+  sp.sf1 = mo[4] * iflux1;
+  sp.sf2 = mo[5] * iflux2;
+  sp.sh1 = mo[6] != 0.0;
+  sp.sh2 = mo[7] != 0.0;
+  double2* b = csm + (t / M) * F::SL;
+  const bool several = bs.nds > 1;
+  double2* zs = several ? b + C * F::SL : b;  // the column's spectrum, kept
+  const bool live = i2 <= kc;
+  // blocks with a self-conjugate column, or with several datasets, pass the
+  // spectrum through shared memory
+  const bool staged = several || c0 == 0 || (c0 <= N / 2 && N / 2 < c0 + C);
+  const bool self = i2 == 0 || i2 == N / 2;
+  double2 v[16];
+  double2* Yc = ybuf + (static_cast<size_t>(w) * D + bs.ds_begin) * N * nc +
+                static_cast<size_t>(i2) * N + u;
+#pragma unroll
+  for (int n1 = 0; n1 < 16; ++n1) v[n1] = live ? Yc[n1 * M] : make_double2(0.0, 0.0);
+  fft2_head<N, -1>(v, b, u, TW);
+  if (staged) {
+#pragma unroll 1
+    for (int pp = 0; pp < F::PP; ++pp) {
+      const int p = pp * M + u;
+      double2 z[M3];
+#pragma unroll
+      for (int i = 0; i < M3; ++i) z[i] = b[p * (M3 + 1) + i];
+      fft::dft<M3, -1>(z);
+#pragma unroll
+      for (int i = 0; i < M3; ++i) zs[p * (M3 + 1) + i] = z[i];
+    }
+    __syncthreads();
+  }
+  for (int dd = 0; dd < bs.nds; ++dd) {
+    const int d = bs.ds_begin + dd;
+    const int kd = kcds[static_cast<size_t>(w) * D + d];
+    if (c0 > kd) continue;
+    const double s1 = sigmult[2 * w] * dsets[d].sb1, s2 = sigmult[2 * w + 1] * dsets[d].sb2;
+    sp.noisy = (s1 > 0 || s2 > 0);
+    sp.s1n = -0.5 * s1 * s1 * iflux1 * iflux1;
+    sp.s2n = -0.5 * s2 * s2 * iflux2 * iflux2;
+    double2* oc = ybuf + (static_cast<size_t>(w) * D + d) * N * nc + static_cast<size_t>(i2) * N + u;
+    if (staged) {
+      // the bins wait in the thread's own places of the output column, since
+      // a mirror's value may still be read from the slots
+#pragma unroll 1
+      for (int j = 0; j < 16; ++j) {
+        const int p = (j / M3) * M + u, k3 = j % M3;
+        const int i1 = p + 256 * k3, j1 = (N - i1) & (N - 1);
+        const double2 X = zs[p * (M3 + 1) + k3];
+        if (i2 > kd) continue;
+        oc[j * M] = self ? sp.bin_self<N>(X, zs[(j1 & 255) * (M3 + 1) + (j1 >> 8)], i1, i2)
+                         : sp.bin<N>(X, i1, i2);
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int pp = 0; pp < F::PP; ++pp) {
+      const int p = pp * M + u;
+      double2 z[M3];
+      if (staged) {
+#pragma unroll
+        for (int i = 0; i < M3; ++i)
+          z[i] = (i2 <= kd) ? oc[(pp * M3 + i) * M] : make_double2(0.0, 0.0);
+      } else {
+#pragma unroll
+        for (int i = 0; i < M3; ++i) z[i] = b[p * (M3 + 1) + i];
+        fft::dft<M3, -1>(z);
+#pragma unroll
+        for (int i = 0; i < M3; ++i) z[i] = sp.bin<N>(z[i], p + 256 * i, i2);
+      }
+      fft::dft<M3, 1>(z);
+#pragma unroll
+      for (int i = 0; i < M3; ++i) b[p * (M3 + 1) + i] = z[i];
+    }
+    __syncthreads();
+    fft2_tail_inv<N>(v, b, u, TW);
+    if (i2 <= kd) {
+#pragma unroll
+      for (int n1 = 0; n1 < 16; ++n1) oc[n1 * M] = v[n1];
+    }
+    __syncthreads();
+  }
+}
+
+// Inverse row transforms of one dataset's columns 0 .. kc, two rows as the
+// real and imaginary part of one DFT, with the marginal sums of the clipped
+// P(D): a block takes RI_ROWS rows, G pairs at a time, and keeps the column
+// sums of its rows in shared memory (each column of a pair's rows belongs to
+// one thread).  P(D) rows go out at pitch `pitch`.
+template <int N>
+__global__ void __launch_bounds__(RowCfg<N>::T, 512 / RowCfg<N>::T)
+k_rowinv2(int D, const int* __restrict__ mstatus, const int* __restrict__ kcds,
+          const double2* __restrict__ ybuf, int pitch, double* __restrict__ pbuf,
+          double* __restrict__ rowpart, double* __restrict__ colpart,
+          const double2* __restrict__ TW) {
+  using F = Fft2<N>;
+  using R = RowCfg<N>;
+  constexpr int M = F::M, M3 = F::M3, G = R::G, T = R::T;
+  constexpr int nc = N / 2 + 1, H = N / 2;
+  constexpr int WP = M / 32;  // warps per pair
+  extern __shared__ double2 fsm[];  // [G][SL], then column sums [G][N]
+  __shared__ double rsum[RI_ROWS][WP];
+  const int wd = blockIdx.y;
+  if (mstatus[wd / D] != 0) return;
+  const int t = threadIdx.x, g = t / M, u = t % M;
+  double2* b = fsm + g * F::SL;
+  double* csum = reinterpret_cast<double*>(fsm + G * F::SL);
+  double* cs = csum + g * N;
+  const int kc = kcds[wd];
+  const double2* Y = ybuf + static_cast<size_t>(wd) * N * nc;
+  const int rblk = blockIdx.x * RI_ROWS;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) cs[(j / M3) * M + u + 256 * (j % M3)] = 0.0;
+#pragma unroll 1
+  for (int it = 0; it < RI_ROWS / R::ROWS; ++it) {
+    const int rbase = rblk + it * R::ROWS;
+    // columns k and n - k of the G pairs, W = X0 + i X1
+    for (int k = t; k <= kc; k += T) {
+      const double2* s = Y + static_cast<size_t>(k) * N + rbase;
+      double2 x0[G], x1[G];
+#pragma unroll
+      for (int gg = 0; gg < G; ++gg) ld32(s + 2 * gg, x0[gg], x1[gg]);
+#pragma unroll
+      for (int gg = 0; gg < G; ++gg) {
+        double2* o = fsm + gg * F::SL;
+        if (k == 0 || k == H) {  // the imaginary parts of these are not used
+          o[k] = make_double2(x0[gg].x, x1[gg].x);
+        } else {
+          o[k] = make_double2(x0[gg].x - x1[gg].y, x0[gg].y + x1[gg].x);
+          o[N - k] = make_double2(x0[gg].x + x1[gg].y, x1[gg].x - x0[gg].y);
+        }
+      }
+    }
+    __syncthreads();
+    double2 v[16];
+#pragma unroll
+    for (int n1 = 0; n1 < 16; ++n1) {
+      const int i = n1 * M + u;
+      v[n1] = (min(i, N - i) <= kc) ? b[i] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    fft2_head<N, 1>(v, b, u, TW);
+    double s0 = 0.0, s1 = 0.0;
+    double* p0 = pbuf + (static_cast<size_t>(wd) * N + rbase + 2 * g) * pitch;
+    double* p1 = p0 + pitch;
+#pragma unroll
+    for (int pp = 0; pp < F::PP; ++pp) {
+      const int p = pp * M + u;
+      double2 z[M3];
+#pragma unroll
+      for (int i = 0; i < M3; ++i) z[i] = b[p * (M3 + 1) + i];
+      fft::dft<M3, 1>(z);
+#pragma unroll
+      for (int i = 0; i < M3; ++i) {
+        const int j = p + 256 * i;
+        p0[j] = z[i].x;
+        p1[j] = z[i].y;
+        const double a0 = clip0(z[i].x), a1 = clip0(z[i].y);
+        s0 += a0;
+        s1 += a1;
+        cs[j] += a0 + a1;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    }
+    if ((t & 31) == 0) {
+      const int r = it * R::ROWS + 2 * g;
+      rsum[r][u >> 5] = s0;
+      rsum[r + 1][u >> 5] = s1;
+    }
+    __syncthreads();
+  }
+  for (int j = t; j < N; j += T) {
+    double a = csum[j];
+#pragma unroll
+    for (int gg = 1; gg < G; ++gg) a += csum[gg * N + j];
+    colpart[(static_cast<size_t>(wd) * gridDim.x + blockIdx.x) * N + j] = a;
+  }
+  if (t < RI_ROWS) {
+    double a = rsum[t][0];
+#pragma unroll
+    for (int k = 1; k < WP; ++k) a += rsum[t][k];
+    rowpart[static_cast<size_t>(wd) * N + rblk + t] = a;
+  }
+}
+
 // Bonus integrals and the band-1 slope penalty of each proposal's model,
 // one block per proposal.  numberCountsDoubleLogNormal::splineInt(a, b)
 // (numberCountsDoubleLogNormal.cc:1549-1631) integrates
@@ -1299,277 +1964,6 @@ __global__ void k_reduce2(const BSet2Dev* __restrict__ bsets,
 // an invalid model; the penalty is differenceRegularize of the band-1 knots
 // (numberCountsDoubleLogNormal.cc:2154-2173) before the factor alpha.
 // fill_at >= 0 stores the four integrals as floats at theta[w][fill_at..].
-// ------------------------------------------------------------------
-// Column transforms fused with the spectrum (FFT mode 1).  After batched 1D
-// row transforms of the R grid (cuFFT D2Z on its n rows), the row-
-// transformed grid Y[i1][i2] (n x nc, row stride nc) goes down its columns
-// here: each block takes C = 256 / M adjacent columns (M = n / 16 threads
-// per column) into shared memory, runs the forward n-point DFT of every
-// column, forms per bin exp(R~ - R~00) with the shifts and one dataset's
-// noise (the work of k_spectrum2, same formulas), runs the inverse column
-// DFT and writes the columns of that dataset's half spectrum, which batched
-// 1D Z2D row transforms then take to the P(D).  So the spectrum costs no
-// HBM round trip of its own and the column passes of both 2D transforms
-// read and write the grid once.
-//
-// Column DFT, n = 16 M, M = 16 M3 (n in [512, 4096]): with n = n1 M + u,
-// u = m M3 + s and k = k1 + 16 (k2 + 16 k3),
-//   stage 1: 16-point register DFTs over n1, times W_n^{u k1};
-//   stage 2: 16-point register DFTs over m, times W_M^{s k2};
-//   stage 3: M3-point register DFTs over s.
-// The forward output stays in the stage-3 slots, position
-// (16 k1 + k2)(M3 + 1) + k3 (a padded stride, free of bank conflicts); the
-// spectrum works slot by slot, and the inverse runs the transposed stages
-// in reverse order (M3-point DFTs over k3, twiddle W_M^{-s k2}, 16-point
-// DFTs over k2, twiddle W_n^{-u k1}, 16-point DFTs over k1), which read
-// those slots and end in natural order.  Twiddles W_n^j, j < n, come from
-// two shared tables H[j >> 5] L[j & 31] built on the host in long double.
-constexpr int CS_THREADS = 256;
-
-__host__ __device__ constexpr int cs_slots(int n) { return 256 * (n / 256 + 1); }
-inline size_t colspec_smem(int n) {
-  const int C = CS_THREADS / (n / 16);
-  return (static_cast<size_t>(C) * cs_slots(n) + n / 32 + 32) * sizeof(double2);
-}
-
-template <int S>
-__device__ __forceinline__ double2 cs_tw(const double2* H, const double2* L, int j) {
-  const double2 h = H[j >> 5];
-  const int lo = j & 31;
-  const double2 w = lo ? fft::cmul(h, L[lo]) : h;
-  return (S < 0) ? w : make_double2(w.x, -w.y);
-}
-
-// forward column DFT of the C columns in buf (natural order in, stage-3
-// slots out)
-template <int N>
-__device__ __forceinline__ void cs_forward(double2* buf, const double2* H, const double2* L,
-                                           int c, int u) {
-  constexpr int M = N / 16, M3 = N / 256, SL = cs_slots(N), PP = 16 / M3;
-  double2* b = buf + c * SL;
-  double2 v[16];
-#pragma unroll
-  for (int n1 = 0; n1 < 16; ++n1) v[n1] = b[n1 * M + u];
-  fft::dft<16, -1>(v);
-#pragma unroll
-  for (int k1 = 1; k1 < 16; ++k1)
-    if (u) v[k1] = fft::cmul(v[k1], cs_tw<-1>(H, L, u * k1));
-  __syncthreads();
-#pragma unroll
-  for (int k1 = 0; k1 < 16; ++k1) b[k1 * M + u] = v[k1];
-  __syncthreads();
-  {
-    const int k1 = u / M3, s = u % M3;
-#pragma unroll
-    for (int m = 0; m < 16; ++m) v[m] = b[k1 * M + m * M3 + s];
-    fft::dft<16, -1>(v);
-#pragma unroll
-    for (int k2 = 1; k2 < 16; ++k2)
-      if (s) v[k2] = fft::cmul(v[k2], cs_tw<-1>(H, L, 16 * s * k2));
-    __syncthreads();
-#pragma unroll
-    for (int k2 = 0; k2 < 16; ++k2) b[(k1 * 16 + k2) * (M3 + 1) + s] = v[k2];
-    __syncthreads();
-  }
-#pragma unroll
-  for (int pp = 0; pp < PP; ++pp) {
-    const int pr = pp * M + u;
-    double2 z[M3];
-#pragma unroll
-    for (int s2 = 0; s2 < M3; ++s2) z[s2] = b[pr * (M3 + 1) + s2];
-    fft::dft<M3, -1>(z);
-#pragma unroll
-    for (int k3 = 0; k3 < M3; ++k3) b[pr * (M3 + 1) + k3] = z[k3];
-  }
-  __syncthreads();
-}
-
-// inverse column DFT: stage-3 slots in, natural order out (into b[i1])
-template <int N>
-__device__ __forceinline__ void cs_inverse(double2* buf, const double2* H, const double2* L,
-                                           int c, int u) {
-  constexpr int M = N / 16, M3 = N / 256, SL = cs_slots(N), PP = 16 / M3;
-  double2* b = buf + c * SL;
-#pragma unroll
-  for (int pp = 0; pp < PP; ++pp) {
-    const int pr = pp * M + u;
-    const int k2 = pr & 15;
-    double2 z[M3];
-#pragma unroll
-    for (int k3 = 0; k3 < M3; ++k3) z[k3] = b[pr * (M3 + 1) + k3];
-    fft::dft<M3, 1>(z);
-#pragma unroll
-    for (int s2 = 0; s2 < M3; ++s2)
-      b[pr * (M3 + 1) + s2] = (s2 * k2) ? fft::cmul(z[s2], cs_tw<1>(H, L, 16 * s2 * k2)) : z[s2];
-  }
-  __syncthreads();
-  double2 v[16];
-  {
-    const int k1 = u / M3, s = u % M3;
-#pragma unroll
-    for (int k2 = 0; k2 < 16; ++k2) v[k2] = b[(k1 * 16 + k2) * (M3 + 1) + s];
-    fft::dft<16, 1>(v);
-    __syncthreads();
-    // Z_{k1}[m M3 + s], times W_n^{-u' k1} for u' = m M3 + s
-#pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int up = m * M3 + s;
-      b[k1 * M + up] = (up * k1) ? fft::cmul(v[m], cs_tw<1>(H, L, up * k1)) : v[m];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int k1 = 0; k1 < 16; ++k1) v[k1] = b[k1 * M + u];
-  fft::dft<16, 1>(v);
-  __syncthreads();
-#pragma unroll
-  for (int n1 = 0; n1 < 16; ++n1) b[n1 * M + u] = v[n1];
-  __syncthreads();
-}
-
-// Sum of the row-transformed grid's column 0 over the rows: R~00 (the DC
-// bin of the 2D transform), one block per (proposal, beam set).
-__global__ void __launch_bounds__(NT)
-k_r0sum2(int n, int nc, const int* __restrict__ mstatus, int B,
-         const double* __restrict__ rbuf, double* __restrict__ r0) {
-  __shared__ double shr[32];
-  const int wb = blockIdx.x;
-  if (mstatus[wb / B] != 0) return;
-  const double2* Y = reinterpret_cast<const double2*>(rbuf) + static_cast<size_t>(wb) * n * nc;
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += NT) acc += Y[static_cast<size_t>(i) * nc].x;
-  acc = dev::block_sum<NT>(acc, shr);
-  if (threadIdx.x == 0) r0[wb] = acc;
-}
-
-template <int N>
-__global__ void __launch_bounds__(CS_THREADS, 2)
-k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dsets, int B,
-           int D, const int* __restrict__ mstatus, const double* __restrict__ sigmult,
-           const double* __restrict__ mom, const double* __restrict__ r0buf,
-           const double* __restrict__ rbuf, double* __restrict__ pbuf,
-           const double2* __restrict__ WH, const double2* __restrict__ WL) {
-  constexpr int M = N / 16, M3 = N / 256, SL = cs_slots(N);
-  constexpr int C = CS_THREADS / M;
-  constexpr int nc = N / 2 + 1;
-  extern __shared__ double2 csm[];
-  double2* buf = csm;                 // [C][SL]
-  double2* Hs = csm + C * SL;         // N / 32
-  double2* Ls = Hs + N / 32;          // 32
-  const int wb = blockIdx.y;
-  const int w = wb / B, bsi = wb - w * B;
-  if (mstatus[w] != 0) return;
-  const int t = threadIdx.x;
-  for (int i = t; i < N / 32 + 32; i += CS_THREADS)
-    Hs[i] = (i < N / 32) ? WH[i] : WL[i - N / 32];
-  const int c0 = blockIdx.x * C;      // first column of the block
-  const int c = t / M, u = t % M;
-  const BSet2Dev& bs = bsets[bsi];
-  const double2* Y = reinterpret_cast<const double2*>(rbuf) + static_cast<size_t>(wb) * N * nc;
-  const double iflux1 = dev::kTwoPi / (static_cast<double>(N) * bs.dflux1);
-  const double iflux2 = dev::kTwoPi / (static_cast<double>(N) * bs.dflux2);
-  const double sm1 = sigmult[2 * w], sm2 = sigmult[2 * w + 1];
-  const double* mo = mom + static_cast<size_t>(wb) * 8;
-  const double r0 = r0buf[wb];
-  const double sf1 = mo[4] * iflux1, sf2 = mo[5] * iflux2;
-  const bool sh1 = mo[6] != 0.0, sh2 = mo[7] != 0.0;
-  for (int dd = 0; dd < bs.nds; ++dd) {
-    const int d = bs.ds_begin + dd;
-    const DSet2Dev& ds = dsets[d];
-    // load the C columns (a warp covers 32 / C rows of C adjacent columns)
-    for (int e = t; e < C * N; e += CS_THREADS) {
-      const int i1 = e / C, cc = e % C;
-      const int i2 = c0 + cc;
-      buf[cc * SL + i1] = (i2 < nc) ? Y[static_cast<size_t>(i1) * nc + i2] : make_double2(0.0, 0.0);
-    }
-    __syncthreads();
-    cs_forward<N>(buf, Hs, Ls, c, u);
-    // spectrum, slot by slot and in place; the self-conjugate columns
-    // (i2 = 0 and n/2) go by mirror pairs (i1, n - i1), each pair owned by
-    // one thread: their Hermitian parts are conjugates of each other
-    const double s1 = sm1 * ds.sb1, s2 = sm2 * ds.sb2;
-    const bool noisy = (s1 > 0 || s2 > 0);
-    const double sf1n = -0.5 * s1 * s1 * iflux1 * iflux1;
-    const double sf2n = -0.5 * s2 * s2 * iflux2 * iflux2;
-#pragma unroll 4
-    for (int q = t; q < C * SL; q += CS_THREADS) {
-      const int cc = q / SL, pos = q % SL;
-      const int pr = pos / (M3 + 1), k3 = pos % (M3 + 1);
-      const int i2 = c0 + cc;
-      if (k3 == M3 || i2 >= nc || i2 == 0 || i2 == N / 2) continue;
-      const int i1 = (pr >> 4) + 16 * ((pr & 15) + 16 * k3);
-      const double didx1 = (i1 < nc) ? static_cast<double>(i1) : static_cast<double>(N - i1);
-      const double didx2 = static_cast<double>(i2);
-      const double nz = noisy ? sf1n * didx1 * didx1 + sf2n * didx2 * didx2 : 0.0;
-      if (noisy && nz < dev::kNoiseZero) {
-        buf[q] = make_double2(0.0, 0.0);
-        continue;
-      }
-      const double2 X = buf[q];
-      double ival = X.y;
-      if (sh1) ival -= (i1 < nc) ? sf1 * static_cast<double>(i1) : -sf1 * static_cast<double>(N - i1);
-      if (sh2) ival -= sf2 * static_cast<double>(i2);
-      double sn, cs;
-      sincos(ival, &sn, &cs);
-      const double ep = exp((X.x - r0) + nz);
-      buf[q] = make_double2(ep * cs, ep * sn);
-    }
-    for (int cc = 0; cc < C; ++cc) {
-      const int i2 = c0 + cc;
-      if (i2 != 0 && i2 != N / 2) continue;
-      double2* b = buf + cc * SL;
-      const double didx2 = static_cast<double>(i2);
-#pragma unroll 1
-      for (int i1 = t; i1 <= N / 2; i1 += CS_THREADS) {
-        const int j1 = (N - i1) % N;
-        const int si = ((i1 & 15) * 16 + ((i1 >> 4) & 15)) * (M3 + 1) + (i1 >> 8);
-        const int sj = ((j1 & 15) * 16 + ((j1 >> 4) & 15)) * (M3 + 1) + (j1 >> 8);
-        if (i1 == 0 && i2 == 0) {
-          b[si] = make_double2(1.0, 0.0);
-          continue;
-        }
-        const double didx1 = static_cast<double>(i1);
-        const double nz = noisy ? sf1n * didx1 * didx1 + sf2n * didx2 * didx2 : 0.0;
-        if (noisy && nz < dev::kNoiseZero) {
-          b[si] = make_double2(0.0, 0.0);
-          if (j1 != i1) b[sj] = make_double2(0.0, 0.0);
-          continue;
-        }
-        const double2 X = b[si];
-        double ival = X.y;
-        if (sh1) ival -= sf1 * static_cast<double>(i1);
-        if (sh2) ival -= sf2 * didx2;
-        double sn, cs;
-        sincos(ival, &sn, &cs);
-        const double ep = exp((X.x - r0) + nz);
-        if (j1 == i1) {
-          b[si] = make_double2(ep * cs, 0.0);
-        } else {
-          const double2 Xq = b[sj];
-          double iq = Xq.y;
-          if (sh1) iq -= -sf1 * static_cast<double>(N - j1);
-          if (sh2) iq -= sf2 * didx2;
-          double sq, cq;
-          sincos(iq, &sq, &cq);
-          const double eq = exp((Xq.x - r0) + nz);
-          const double2 o = make_double2(0.5 * (ep * cs + eq * cq), 0.5 * (ep * sn - eq * sq));
-          b[si] = o;
-          b[sj] = make_double2(o.x, -o.y);
-        }
-      }
-    }
-    __syncthreads();
-    cs_inverse<N>(buf, Hs, Ls, c, u);
-    double2* Pd = reinterpret_cast<double2*>(pbuf) + (static_cast<size_t>(w) * D + d) * N * nc;
-    for (int e = t; e < C * N; e += CS_THREADS) {
-      const int i1 = e / C, cc = e % C;
-      const int i2 = c0 + cc;
-      if (i2 < nc) Pd[static_cast<size_t>(i1) * nc + i2] = buf[cc * SL + i1];
-    }
-    __syncthreads();
-  }
-}
-
 constexpr int kBonus2Threads = 256;
 __global__ void __launch_bounds__(kBonus2Threads)
 k_bonus2(Model2Dev m, float* theta, int npar, double logfac,
@@ -1916,8 +2310,7 @@ void Engine2::free_static() {
   static_allocs_.clear();
   d_bsets_ = nullptr;
   d_dsets_ = nullptr;
-  d_cwh_ = nullptr;
-  d_cwl_ = nullptr;
+  d_ctw_ = nullptr;
   colspec_ = false;
   static_ok_ = false;
 }
@@ -2130,7 +2523,7 @@ void Engine2::free_work() {
                   ws_.rpart, ws_.redge, ws_.epart, ws_.fpart, ws_.mom, ws_.pbuf, ws_.rowpart,
                   ws_.colpart, ws_.pinfo, ws_.gpart, ws_.pdout,
                   ws_.theta_in, ws_.logl, ws_.status, ws_.bonus, ws_.bcnt,
-                  ws_.bstatus, ws_.bsig, ws_.r0};
+                  ws_.bstatus, ws_.bsig, ws_.r0, ws_.row0, ws_.kcset, ws_.kcds};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (ws_.h_theta) cudaFreeHost(ws_.h_theta);
@@ -2165,7 +2558,11 @@ void Engine2::reserve(unsigned P) {
   ws_.bsig = dal<double>(2 * static_cast<size_t>(P));
   ws_.rw = dal<double>(static_cast<size_t>(P) * B_ * nrows * Tmax_ * 3);
   ws_.rcnt = dal<int2>(static_cast<size_t>(P) * B_ * nrows);
-  ws_.rbuf = dal<double>(static_cast<size_t>(P) * B_ * n * nc2);
+  ws_.rrows = rbuf_rows();
+  ws_.rbuf = dal<double>(static_cast<size_t>(P) * ws_.rrows * n * nc2);
+  ws_.row0 = dal<double>(static_cast<size_t>(P) * B_ * n);
+  ws_.kcset = dal<int>(static_cast<size_t>(P) * B_);
+  ws_.kcds = dal<int>(static_cast<size_t>(P) * D_);
   ws_.rpart = dal<double>(static_cast<size_t>(P) * B_ * gx_ * gy_ * 4);
   ws_.redge = dal<double>(static_cast<size_t>(P) * B_ * (2 * n + 1));
   const size_t ngr = edge_ ? (nedge_ + ER_MIN - 1) / ER_MIN : 0;
@@ -2186,36 +2583,42 @@ void Engine2::reserve(unsigned P) {
                           static_cast<int>(3 * 8192 * sizeof(double))), "attr");
 }
 
-// Twiddle tables and kernel attributes of FFT mode 1 where the size allows.
+// Twiddle table and kernel attributes of FFT mode 1 where the size allows.
 void Engine2::setup_colspec() {
   const unsigned n = n_;
   colspec_ = fft_mode_ == 1 && (n == 512 || n == 1024 || n == 2048 || n == 4096);
   if (!colspec_) return;
-  if (!d_cwh_) {
-    std::vector<double2> wh(n / 32), wl(32);
+  if (!d_ctw_) {
+    // W_n^{u 2^i}, u < n / 16, i < 4 (the second stage's W_{n/16}^s is row 16 s)
+    std::vector<double2> tw(n / 4);
     const long double tau = 6.283185307179586476925286766559005768L;
-    for (unsigned h = 0; h < n / 32; ++h) {
-      const long double a = -tau * static_cast<long double>(32 * h) / static_cast<long double>(n);
-      wh[h] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
-    }
-    for (unsigned l = 0; l < 32; ++l) {
-      const long double a = -tau * static_cast<long double>(l) / static_cast<long double>(n);
-      wl[l] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
-    }
-    d_cwh_ = dal<double2>(wh.size());
-    d_cwl_ = dal<double2>(wl.size());
-    static_allocs_.push_back(d_cwh_);
-    static_allocs_.push_back(d_cwl_);
-    ck(cudaMemcpy(d_cwh_, wh.data(), wh.size() * sizeof(double2), cudaMemcpyHostToDevice), "upload");
-    ck(cudaMemcpy(d_cwl_, wl.data(), wl.size() * sizeof(double2), cudaMemcpyHostToDevice), "upload");
+    for (unsigned u = 0; u < n / 16; ++u)
+      for (unsigned i = 0; i < 4; ++i) {
+        const unsigned e = (u << i) % n;
+        const long double a = -tau * static_cast<long double>(e) / static_cast<long double>(n);
+        tw[4 * u + i] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
+      }
+    d_ctw_ = dal<double2>(tw.size());
+    static_allocs_.push_back(d_ctw_);
+    ck(cudaMemcpy(d_ctw_, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice), "upload");
   }
-  const int sm = static_cast<int>(colspec_smem(static_cast<int>(n)));
+#define POFD_ATTR2(NN)                                                                       \
+  {                                                                                          \
+    const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;                            \
+    ck(cudaFuncSetAttribute(k_rowfwd2<NN>, dyn, static_cast<int>(rowfwd_smem(NN))), "attr"); \
+    ck(cudaFuncSetAttribute(k_rowinv2<NN>, dyn, static_cast<int>(rowinv_smem(NN))), "attr"); \
+    ck(cudaFuncSetAttribute(k_colspec2<NN>, dyn, static_cast<int>(colspec_smem(NN, true))),  \
+       "attr");                                                                              \
+    const auto pref = cudaFuncAttributePreferredSharedMemoryCarveout;                        \
+    ck(cudaFuncSetAttribute(k_rowinv2<NN>, pref, cudaSharedmemCarveoutMaxShared), "attr");   \
+  }
   switch (n) {
-    case 512: ck(cudaFuncSetAttribute(k_colspec2<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr"); break;
-    case 1024: ck(cudaFuncSetAttribute(k_colspec2<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr"); break;
-    case 2048: ck(cudaFuncSetAttribute(k_colspec2<2048>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr"); break;
-    default: ck(cudaFuncSetAttribute(k_colspec2<4096>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr"); break;
+    case 512: POFD_ATTR2(512) break;
+    case 1024: POFD_ATTR2(1024) break;
+    case 2048: POFD_ATTR2(2048) break;
+    default: POFD_ATTR2(4096) break;
   }
+#undef POFD_ATTR2
 }
 
 void Engine2::drop_plans() {
@@ -2235,6 +2638,11 @@ void Engine2::set_fft_mode(int mode) {
   drop_plans();
   if (static_ok_) setup_colspec();
   else colspec_ = false;
+  if (ws_.rbuf && ws_.rrows < rbuf_rows()) {  // the modes keep different grids in rbuf
+    const unsigned P = ws_.P;
+    free_work();
+    reserve(P);
+  }
 }
 
 double Engine2::time_sequence(unsigned nprop, const float* theta, unsigned npar, int reps) {
@@ -2323,21 +2731,11 @@ void Engine2::set_reference_sums(bool on) {
 
 void Engine2::ensure_plans(unsigned nprop) {
   auto it = plans_.find(nprop);
-  if (it != plans_.end() && it->second.fwd) return;
+  if (it != plans_.end() && (it->second.fwd || colspec_)) return;
   Plans pl;
   int nn[2] = {static_cast<int>(n_), static_cast<int>(n_)};
   const int nc = static_cast<int>(n_) / 2 + 1;
-  if (colspec_) {
-    // 1D row transforms of every (proposal, beam set) or (proposal, dataset)
-    // grid: n rows each, padded real rows of 2 nc doubles / nc complex
-    int n1[1] = {nn[0]};
-    int ie[1] = {2 * nc}, oe[1] = {nc};
-    bool grew = fftwork_.make(&pl.fwd, 1, n1, ie, 2 * nc, oe, nc, CUFFT_D2Z,
-                              static_cast<int>(nprop * B_ * n_));
-    int ie2[1] = {nc}, oe2[1] = {2 * nc};
-    grew |= fftwork_.make(&pl.inv, 1, n1, ie2, nc, oe2, 2 * nc, CUFFT_Z2D,
-                          static_cast<int>(nprop * D_ * n_));
-    if (grew) drop_graphs();
+  if (colspec_) {  // the row and column kernels need no cuFFT plans
     plans_[nprop] = pl;
     return;
   }
@@ -2376,26 +2774,10 @@ void Engine2::launch_all(unsigned nprop, const float* theta, unsigned npar,
                                              ws_.mstatus, ws_.cnt, ws_.rw, ws_.rcnt);
   }
   mark(2);
-  const int rb = tune_.rgrid_rows;
-  const unsigned gy = static_cast<unsigned>((n - 1 + rb - 1) / rb);
-  const unsigned gxg = static_cast<unsigned>((n + RG_COLS - 1) / RG_COLS);
-  switch (rb) {
-    case 2:
-      k_rgrid2<2><<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, ws_.mstatus, ws_.rw,
-                                                       ws_.rcnt, ws_.rbuf, ws_.rpart);
-      break;
-    case 8:
-      k_rgrid2<8><<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, ws_.mstatus, ws_.rw,
-                                                       ws_.rcnt, ws_.rbuf, ws_.rpart);
-      break;
-    default:
-      k_rgrid2<4><<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, ws_.mstatus, ws_.rw,
-                                                       ws_.rcnt, ws_.rbuf, ws_.rpart);
-  }
-  mark(3);
   const int er = tune_.edge_rows;
   const int ngr = (ne + er - 1) / er;
-  if (edge_) {
+  auto edges = [&] {
+    if (!edge_) return;
     const unsigned gxe = static_cast<unsigned>((n + ne + RG_COLS - 1) / RG_COLS);
     switch (er) {
       case 4:
@@ -2412,9 +2794,67 @@ void Engine2::launch_all(unsigned nprop, const float* theta, unsigned npar,
     }
     k_ry2<<<dim3((n - 1 + RY_ROWS - 1) / RY_ROWS, P * B), NT, 0, st>>>(
         d_bsets_, B, n, ne, ws_.mstatus, ws_.rw, ws_.rcnt, ws_.redge);
+  };
+  const int pitch = static_cast<int>(ppitch());  // of a P(D) row
+  int nct = static_cast<int>(nct_), s = 2;       // marginal column tiles; stage
+  if (colspec_ && !r_only) {
+    edges();
+    k_redge0_2<<<dim3((n + NT - 1) / NT, P * B), NT, 0, st>>>(
+        d_bsets_, d_dsets_, B, D, n, edge_ ? 1 : 0, ne, ngr, ws_.mstatus, ws_.sigmult, ws_.epart,
+        ws_.row0, ws_.kcset, ws_.kcds);
+    mark(3);
+    // groups of rows per block: the tuning's rows per block, at least one
+    const int rows = rowcfg_rows(n), gpb = std::max(1, tune_.rgrid_rows / rows);
+    const int nblk = (n / rows + gpb - 1) / gpb;
+    double2* Y = reinterpret_cast<double2*>(ws_.rbuf);
+    bool several = false;
+    for (const auto& bs : h_bsets_) several = several || bs.nds > 1;
+#define POFD_ROWS2(NN)                                                                          \
+  {                                                                                             \
+    k_rowfwd2<NN><<<dim3(nblk, P * B), RowCfg<NN>::T, rowfwd_smem(NN), st>>>(                   \
+        d_bsets_, B, D, edge_ ? 1 : 0, gpb, ws_.mstatus, ws_.rw, ws_.rcnt, ws_.row0, ws_.redge, \
+        ws_.kcset, Y, ws_.rpart, d_ctw_);                                                       \
+    mark(4);                                                                                    \
+    k_rmom2<<<P * B, NT, 0, st>>>(d_bsets_, B, nblk, ws_.mstatus, ws_.rpart, ws_.mom, ws_.r0);  \
+    mark(5);                                                                                    \
+    k_colspec2<NN><<<dim3((nc + ColCfg<NN>::C - 1) / ColCfg<NN>::C, P * B), ColCfg<NN>::T,      \
+                     colspec_smem(NN, several), st>>>(d_bsets_, d_dsets_, B, D, ws_.mstatus,    \
+                                                      ws_.sigmult, ws_.mom, ws_.r0, ws_.kcset,  \
+                                                      ws_.kcds, Y, d_ctw_);                     \
+    mark(6);                                                                                    \
+    k_rowinv2<NN><<<dim3(n / RI_ROWS, P * D), RowCfg<NN>::T, rowinv_smem(NN), st>>>(            \
+        D, ws_.mstatus, ws_.kcds, Y, pitch, ws_.pbuf, ws_.rowpart, ws_.colpart, d_ctw_);        \
   }
-  mark(4);
-  {
+    switch (n) {
+      case 512: POFD_ROWS2(512) break;
+      case 1024: POFD_ROWS2(1024) break;
+      case 2048: POFD_ROWS2(2048) break;
+      case 4096: POFD_ROWS2(4096) break;
+      default: throw Error(POFD_E_ARG, "row and column transforms: unsupported size");
+    }
+#undef POFD_ROWS2
+    nct = 1;
+    s = 7;
+  } else {
+    const int rb = tune_.rgrid_rows;
+    const unsigned gy = static_cast<unsigned>((n - 1 + rb - 1) / rb);
+    const unsigned gxg = static_cast<unsigned>((n + RG_COLS - 1) / RG_COLS);
+    switch (rb) {
+      case 2:
+        k_rgrid2<2><<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, ws_.mstatus, ws_.rw,
+                                                         ws_.rcnt, ws_.rbuf, ws_.rpart);
+        break;
+      case 8:
+        k_rgrid2<8><<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, ws_.mstatus, ws_.rw,
+                                                         ws_.rcnt, ws_.rbuf, ws_.rpart);
+        break;
+      default:
+        k_rgrid2<4><<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, ws_.mstatus, ws_.rw,
+                                                         ws_.rcnt, ws_.rbuf, ws_.rpart);
+    }
+    mark(3);
+    edges();
+    mark(4);
     const int nfp = (n + NT - 1) / NT;
     k_rfinish2<<<dim3(nfp, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, edge_ ? 1 : 0, ne, ngr,
                                                 static_cast<int>(gxg * gy), ws_.mstatus,
@@ -2422,62 +2862,44 @@ void Engine2::launch_all(unsigned nprop, const float* theta, unsigned npar,
                                                 ws_.fpart);
     k_rfinal2<<<P * B, NT, 0, st>>>(d_bsets_, B, n, nc2, edge_ ? 1 : 0, ne, ngr, nfp,
                                     ws_.mstatus, ws_.epart, ws_.fpart, ws_.rbuf, ws_.mom);
-  }
-  mark(5);
-  if (r_only) {
-    ck(cudaGetLastError(), "kernel launch");
-    return;
-  }
-  fk(cufftSetStream(pl.fwd, st), "cufftSetStream");
-  fk(cufftExecD2Z(pl.fwd, ws_.rbuf, reinterpret_cast<cufftDoubleComplex*>(ws_.rbuf)),
-     colspec_ ? "cufftExecD2Z rows" : "cufftExecD2Z 2D");
-  mark(6);
-  if (colspec_) {
-    k_r0sum2<<<P * B, NT, 0, st>>>(n, nc, ws_.mstatus, B, ws_.rbuf, ws_.r0);
-    const int C = CS_THREADS / (n / 16);
-    const dim3 g((nc + C - 1) / C, P * B);
-    const size_t sm = colspec_smem(n);
-#define POFD_CS(NN)                                                                        \
-  k_colspec2<NN><<<g, CS_THREADS, sm, st>>>(d_bsets_, d_dsets_, B, D, ws_.mstatus,          \
-                                             ws_.sigmult, ws_.mom, ws_.r0, ws_.rbuf, ws_.pbuf, \
-                                             d_cwh_, d_cwl_)
-    switch (n) {
-      case 512: POFD_CS(512); break;
-      case 1024: POFD_CS(1024); break;
-      case 2048: POFD_CS(2048); break;
-      case 4096: POFD_CS(4096); break;
-      default: throw Error(POFD_E_ARG, "column transform: unsupported size");
+    mark(5);
+    if (r_only) {
+      ck(cudaGetLastError(), "kernel launch");
+      return;
     }
-#undef POFD_CS
-  } else {
+    fk(cufftSetStream(pl.fwd, st), "cufftSetStream");
+    fk(cufftExecD2Z(pl.fwd, ws_.rbuf, reinterpret_cast<cufftDoubleComplex*>(ws_.rbuf)),
+       "cufftExecD2Z 2D");
+    mark(6);
     const unsigned gs = static_cast<unsigned>((static_cast<size_t>(n) * nc + NT - 1) / NT);
     k_spectrum2<<<dim3(gs, P * B), NT, 0, st>>>(d_bsets_, d_dsets_, B, D, n, nc, ws_.mstatus,
                                                 ws_.sigmult, ws_.mom, ws_.rbuf, ws_.pbuf);
+    mark(7);
+    fk(cufftSetStream(pl.inv, st), "cufftSetStream");
+    fk(cufftExecZ2D(pl.inv, reinterpret_cast<cufftDoubleComplex*>(ws_.pbuf), ws_.pbuf),
+       "cufftExecZ2D 2D");
+    mark(8);
+    k_pscan2<<<dim3(nct_, nrt_, P * D), NT, 0, st>>>(D, n, nc2, ws_.mstatus, ws_.pbuf,
+                                                      ws_.rowpart, ws_.colpart);
+    s = 9;
   }
-  mark(7);
-  fk(cufftSetStream(pl.inv, st), "cufftSetStream");
-  fk(cufftExecZ2D(pl.inv, reinterpret_cast<cufftDoubleComplex*>(ws_.pbuf), ws_.pbuf),
-     colspec_ ? "cufftExecZ2D rows" : "cufftExecZ2D 2D");
-  mark(8);
-  k_pscan2<<<dim3(nct_, nrt_, P * D), NT, 0, st>>>(D, n, nc2, ws_.mstatus, ws_.pbuf,
-                                                    ws_.rowpart, ws_.colpart);
-  mark(9);
+  mark(s);
   k_psplit2<<<P * D, SNT, 3 * static_cast<size_t>(n) * sizeof(double), st>>>(
-      d_bsets_, d_dsets_, B, D, n, nc2, static_cast<int>(nct_), static_cast<int>(nrt_),
+      d_bsets_, d_dsets_, B, D, n, pitch, nct, static_cast<int>(nrt_),
       ws_.mstatus, ws_.sigmult, ws_.mom, ws_.pbuf, ws_.rowpart, ws_.colpart, ws_.pinfo);
   if (refsum_)
     k_pseq2<<<P * D, NT, static_cast<size_t>(n) * sizeof(double), st>>>(
-        d_bsets_, d_dsets_, D, n, nc2, ws_.mstatus, ws_.pbuf, ws_.pinfo);
-  mark(10);
-  k_pgather2<<<dim3(gchunks_, P * D), NT, 0, st>>>(d_bsets_, d_dsets_, D, n, nc2,
+        d_bsets_, d_dsets_, D, n, pitch, ws_.mstatus, ws_.pbuf, ws_.pinfo);
+  mark(s + 1);
+  k_pgather2<<<dim3(gchunks_, P * D), NT, 0, st>>>(d_bsets_, d_dsets_, D, n, pitch,
                                                     static_cast<int>(gchunks_), ws_.mstatus,
                                                     ws_.pbuf, ws_.pinfo, ws_.gpart);
-  mark(11);
+  mark(s + 2);
   k_reduce2<<<(P + 127) / 128, 128, 0, st>>>(d_bsets_, d_dsets_, B, D, P,
                                             static_cast<int>(gchunks_), std::log(2.0),
                                             ws_.mstatus, ws_.sigmult, ws_.pinfo,
                                             ws_.gpart, prior_, ws_.bonus, logl, status);
-  mark(12);
+  mark(s + 3);
   ck(cudaGetLastError(), "kernel launch");
 }
 
@@ -2684,10 +3106,10 @@ int Engine2::pd_host(int bs, int ds, const float* theta, unsigned npar,
     info16[12] = info.sg1pos; info16[13] = info.sg1neg; info16[14] = info.sg2pos; info16[15] = info.sg2neg;
   }
   if (info.status != 0) return info.status;
-  const size_t n = n_, nc2 = 2 * (n / 2 + 1);
+  const size_t n = n_;
   const unsigned blocks = static_cast<unsigned>((n * n + 255) / 256);
-  k_pdwrite2<<<blocks, 256, 0, stream_>>>(ws_.pbuf + static_cast<size_t>(d) * n * nc2,
-                                          static_cast<int>(n), static_cast<int>(nc2), info.s1,
+  k_pdwrite2<<<blocks, 256, 0, stream_>>>(ws_.pbuf + static_cast<size_t>(d) * n * ppitch(),
+                                          static_cast<int>(n), static_cast<int>(ppitch()), info.s1,
                                           info.s2, info.itot, setlog ? 1 : 0, ws_.pdout);
   ck(cudaGetLastError(), "pdwrite2");
   ck(cudaMemcpyAsync(pd_out, ws_.pdout, n * n * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H pd");
@@ -2729,13 +3151,14 @@ void Engine2::profile_stages(unsigned nprop, const float* theta, unsigned npar,
   std::vector<double> lls(nprop);
   std::vector<int> sts(nprop);
   eval_host(nprop, theta, npar, lls.data(), sts.data());
+  const int ns = num_stages();
   cudaEvent_t ev[kNumStages + 1];
   for (auto& e : ev) ck(cudaEventCreate(&e), "event create");
-  for (int k = 0; k < kNumStages; ++k) stage_ms[k] = 0.0;
+  for (int k = 0; k < ns; ++k) stage_ms[k] = 0.0;
   for (int r = 0; r < reps; ++r) {
     launch_all(nprop, ws_.theta_in, npar, ws_.logl, ws_.status, stream_, ev);
     ck(cudaStreamSynchronize(stream_), "synchronize");
-    for (int k = 0; k < kNumStages; ++k) {
+    for (int k = 0; k < ns; ++k) {
       float ms = 0.f;
       ck(cudaEventElapsedTime(&ms, ev[k], ev[k + 1]), "elapsed");
       stage_ms[k] += ms / reps;
@@ -2753,12 +3176,11 @@ const char* Engine2::stage_name(int i) {
 }
 
 const char* Engine2::stage_name_now(int i) const {
-  static const char* names[kNumStages] = {
-      "k_model2", "k_rows2", "k_rgrid2", "k_redge2+k_ry2", "k_rfinish2+k_rfinal2",
-      "cufft_d2z_rows", "k_r0sum2+k_colspec2", "cufft_z2d_rows", "k_pscan2", "k_psplit2",
-      "k_pgather2", "k_reduce2"};
+  static const char* names[] = {
+      "k_model2", "k_rows2", "k_redge2+k_ry2+k_redge0_2", "k_rowfwd2", "k_rmom2",
+      "k_colspec2", "k_rowinv2", "k_psplit2", "k_pgather2", "k_reduce2"};
   if (!colspec_) return stage_name(i);
-  return (i >= 0 && i < kNumStages) ? names[i] : "";
+  return (i >= 0 && i < num_stages()) ? names[i] : "";
 }
 
 }  // namespace pofd

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 #include <cufft.h>
 
+#include <algorithm>
 #include <map>
 #include <vector>
 
@@ -143,10 +144,11 @@ class Engine2 {
   void profile_stages(unsigned nprop, const float* theta, unsigned npar,
                       int reps, double* stage_ms);
   static const char* stage_name(int i);
+  int num_stages() const { return colspec_ ? 10 : kNumStages; }
   // the stage names of the FFT mode in use
   const char* stage_name_now(int i) const;
   int kernels_per_eval() const {
-    return (edge_ ? 12 : 10) + (colspec_ ? 1 : 0) + (prior_.needs_bonus() ? 1 : 0) +
+    return (edge_ ? 12 : 10) + (prior_.needs_bonus() ? 1 : 0) +
            (refsum_ ? 1 : 0);
   }
   // Reference-order normalisation and means (k_pseq2 after the split
@@ -166,10 +168,9 @@ class Engine2 {
   }
   void set_tuning(const Tune2& t);
   bool reference_sums() const { return refsum_; }
-  // 0: batched 2D cuFFT transforms with k_spectrum2 between them; 1: batched
-  // 1D cuFFT row transforms around this library's fused column-transform +
-  // spectrum kernel (k_colspec2), where n is a power of two in [512, 4096]
-  // (mode 0 otherwise).
+  // 0: batched 2D cuFFT transforms with k_spectrum2 between them; 1: this
+  // library's row and column kernels (k_rowfwd2, k_colspec2, k_rowinv2),
+  // where n is a power of two in [512, 4096] (mode 0 otherwise).
   void set_fft_mode(int mode);
   int fft_mode() const { return fft_mode_; }
   // the fused column path is (or, before the first evaluation, will be) used
@@ -254,14 +255,16 @@ class Engine2 {
   std::map<unsigned, Plans> plans_;
   FftWorkArea fftwork_;
   void setup_colspec();
+  unsigned rbuf_rows() const { return colspec_ ? D_ : B_; }
+  // row pitch of the P(D) in pbuf
+  size_t ppitch() const { return colspec_ ? n_ : 2 * (static_cast<size_t>(n_) / 2 + 1); }
   void drop_plans();
   int fft_mode_ = 1;
   bool colspec_ = false;
   bool refsum_ = false;
   Tune2 tune_;
   double time_sequence(unsigned nprop, const float* theta, unsigned npar, int reps);
-  double2* d_cwh_ = nullptr;  // e^{-2 pi i 32 h / n}, h < n / 32
-  double2* d_cwl_ = nullptr;  // e^{-2 pi i l / n}, l < 32
+  double2* d_ctw_ = nullptr;  // e^{-2 pi i u 2^i / n}, u < n / 16, i < 4
   Prior2 prior_;
   const double* d_qu_ = nullptr;
   const double* d_qs_ = nullptr;
@@ -275,14 +278,21 @@ class Engine2 {
     double* sigmult = nullptr;  // [P][2]
     double* rw = nullptr;       // [P][B][nrows][T][3] compacted row terms
     int2* rcnt = nullptr;       // [P][B][nrows] (positive, negative) term counts
-    double* rbuf = nullptr;     // [P][B][n][2nc]
+    double* rbuf = nullptr;     // [P][rrows][n][2nc]: the R grid and its spectrum
+                                // (FFT mode 0), or the columns [P][D][nc][n]
+                                // of the transforms (mode 1)
+    unsigned rrows = 0;         // rbuf_rows() it was made for
+    double* row0 = nullptr;     // [P][B][n] edge cells of row 0 (mode 1)
+    int* kcset = nullptr;       // [P][B] noise cut-off columns (mode 1)
+    int* kcds = nullptr;        // [P][D]
     double* rpart = nullptr;    // [P][B][gy][gx][4]
     double* redge = nullptr;    // [P][B][2n+1]: Ry at [n, 2n)
     double* epart = nullptr;    // [P][B][edge row groups][n + nedge]
     double* mom = nullptr;      // [P][B][8]
     double* r0 = nullptr;       // [P][B] R~00 (FFT mode 1)
     double* fpart = nullptr;    // [P][B][n/256][4] edge-cell moment partials
-    double* pbuf = nullptr;     // [P][D][n][2nc]
+    double* pbuf = nullptr;     // [P][D][n][2nc] spectrum and P(D) (mode 0);
+                                // P(D) at pitch n (mode 1)
     double* rowpart = nullptr;  // [P][D][n][nct]
     double* colpart = nullptr;  // [P][D][nrt][n]
     PDInfo2* pinfo = nullptr;   // [P][D]
