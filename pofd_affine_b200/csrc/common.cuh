@@ -67,6 +67,54 @@ __device__ __forceinline__ double exp2_tab(double x, const double* __restrict__ 
   return (x < -1022.0) ? 0.0 : s;
 }
 
+// 2^(-t^2 / 64), the colour terms' Gaussian: the same method with the square
+// folded in.  t^2 = -(64 k + j) - r with |r| <= 1/2 comes out of two fused
+// products of t (the second gives r with one rounding), so a term takes 11
+// FP64 instructions where squaring, scaling and exp2_tab take 13.  The table
+// has 64 entries, 2^(j/64), each stored for the 16 lanes of a half warp: lane
+// l reads column l, so that no lookup has a bank conflict (with one copy of
+// a 256-entry table the conflicts were a third of the lookups' wavefronts).
+// The Taylor series of 2^(r/64) runs to r^5 (truncation < 4e-17).  |t| is
+// capped at sqrt(64 * 1022) with an integer minimum: beyond it the result is
+// 2^-1022, which like 0 never changes the sums it enters (t must not be NaN).
+struct GaussTable {
+  double t[64 * 16];
+  __device__ __forceinline__ void load() {
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+      const double v = exp2(static_cast<double>(i >> 2) / 64.0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) t[4 * i + k] = v;
+    }
+  }
+  __device__ __forceinline__ const double* lane() const { return t + (threadIdx.x & 15); }
+};
+
+// Its constants, the shifter 1.5 * 2^52 and (ln 2 / 64)^m / m!, m = 5 .. 1,
+// opaque to the compiler so that they stay in registers over a block's rows
+// instead of being made again for every term.
+struct GaussC {
+  double sh = 6755399441055744.0, c5 = 1.2417843701716925e-12, c4 = 5.7328516886404020e-10,
+         c3 = 2.1173137155464776e-07, c2 = 5.8649049550561700e-05, c1 = 1.0830424696249145e-02;
+  __device__ __forceinline__ GaussC() {
+    asm volatile("" : "+d"(sh), "+d"(c5), "+d"(c4), "+d"(c3), "+d"(c2), "+d"(c1));
+  }
+};
+
+__device__ __forceinline__ double exp2_gauss(double t, const double* __restrict__ tab,
+                                             const GaussC& g) {
+  t = __hiloint2double(min(__double2hiint(t) & 0x7fffffff, 0x406ff800), __double2loint(t));
+  const double q = fma(-t, t, g.sh);
+  const double nd = q - g.sh;
+  const int n = __double2loint(q);
+  const double r = fma(-t, t, -nd);
+  double p = fma(g.c5, r, g.c4);
+  p = fma(p, r, g.c3);
+  p = fma(p, r, g.c2);
+  p = fma(p, r, g.c1);
+  p = fma(p, r, 1.0);
+  const double v = p * tab[(n & 63) * 16];
+  return __hiloint2double(__double2hiint(v) + ((n & ~63) << 14), __double2loint(v));
+}
 
 // -------------------------------------------------------------- reductions
 template <int NT>

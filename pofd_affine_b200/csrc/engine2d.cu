@@ -16,7 +16,7 @@
 //
 // HBM layout (P proposals, B beam sets, D datasets, n grid, nc = n/2+1,
 // T terms per row slot):
-//   rw    [P][B][n + nedge][T][3]  per-row colour terms (c0, c1, c2)
+//   rw    [P][B][n + nedge][T][3]  per-row colour terms (c0, a, b)
 //   rbuf  [P][B][n][2nc]           R grid (x dflux1 dflux2), then its 2D
 //                                  spectrum in place
 //   pbuf  [P][D][n][2nc]           per-dataset spectrum, then the P(D)
@@ -34,7 +34,7 @@ namespace pofd {
 namespace {
 
 constexpr int NT = 256;
-constexpr int RB_MIN = 2;    // fewest R-grid rows per block (sizes the partials)
+constexpr int RB_MIN = 4;    // fewest R-grid rows per block (sizes the partials)
 constexpr int RTILE = 32;    // P(D) rows per scan block
 constexpr int GCH = 1024;    // data bins per gather block
 constexpr int KMAX = Engine2::KMAX;
@@ -189,12 +189,15 @@ __device__ __forceinline__ double curve_at(const double* x, const double* s,
 }
 
 // One colour term of a row (numberCountsDoubleLogNormal.cc:1883-1963):
-// c0 = weight * counts / sigma * prefac (0: the term is skipped), c1 =
-// log f1 + offset - log(beam1/beam2), c2 = -1/(2 ln2 sigma^2).
+// c0 = weight * counts / sigma * prefac (0: the term is skipped) and the
+// Gaussian exp(-(log f2 - c1)^2 / (2 sigma^2)), c1 = log f1 + offset -
+// log(beam1/beam2), as 2^(-(a log f2 + b)^2 / 64): a = sqrt(32 / ln2) / sigma,
+// b = -a c1.  Returns (c0, a, b).
 __device__ __forceinline__ double3 row_term(const BSet2Dev& bs, const Model2Dev& m,
                                             const double* __restrict__ cs, int r, int sgn,
-                                            int j, double ilog2toe, const double* tab) {
-  double c0 = 0.0, c1 = 0.0, c2 = 0.0;
+                                            int j, const double* tab) {
+  constexpr double kSqrt32OverLn2 = 6.7945744023041525;
+  double c0 = 0.0, a = 0.0, b = 0.0;
   const Sign2Dev& sg = bs.sg[sgn];
   const double f1val = fabs(bs.rowflux[r]);
   if (f1val < sg.maxf1) {
@@ -207,25 +210,29 @@ __device__ __forceinline__ double3 row_term(const BSet2Dev& bs, const Model2Dev&
             1.0 / curve_at(m.sk, cs + 4 * KMAX, m.ns, f1prod, true, m.min_sigma);
         if (sg.ishist) c0 = sg.w[j] * ieta1 * isigma * cts * bs.prefac;
         else c0 = cts * ieta1 * isigma * bs.prefac;
-        c1 = bs.rowlog[r] + curve_at(m.ok, cs + 8 * KMAX, m.no, f1prod, false, 0.0) -
-             sg.logratio[j];
-        c2 = -0.5 * isigma * isigma * ilog2toe;
+        const double c1 = bs.rowlog[r] +
+                          curve_at(m.ok, cs + 8 * KMAX, m.no, f1prod, false, 0.0) -
+                          sg.logratio[j];
+        a = kSqrt32OverLn2 * isigma;
+        b = -a * c1;
+        // an infinite or undefined Gaussian makes R undefined
+        if (!isfinite(a) || !isfinite(b)) c0 = __longlong_as_double(0x7ff8000000000000LL);
       }
     }
   }
-  return make_double3(c0, c1, c2);
+  return make_double3(c0, a, b);
 }
 
 // Per-row colour terms, one warp per row: the row's terms of the positive
 // band-2 sign component, then those of the negative one, each list with
-// its zero terms dropped and its order kept, written as (c0, c1, c2)
+// its zero terms dropped and its order kept, written as (c0, a, b)
 // triples at rw[row][0 .. npos + nneg); rcnt[row] = (npos, nneg).  The R
 // grid kernels read these lists directly (the same values for every lane
 // of a warp), with no per-block staging.
 constexpr int ROWS_PER_BLOCK = NT / 32;
 __global__ void __launch_bounds__(NT)
 k_rows2(const BSet2Dev* __restrict__ bsets, Model2Dev m, int B,
-        double ilog2toe, const int* __restrict__ mstatus,
+        const int* __restrict__ mstatus,
         const double* __restrict__ cnt, double* __restrict__ rw,
         int2* __restrict__ rcnt) {
   __shared__ dev::Exp2Table e2;
@@ -254,7 +261,7 @@ k_rows2(const BSet2Dev* __restrict__ bsets, Model2Dev m, int B,
     for (int kb = k0; kb < k1; kb += 32) {
       const int k = kb + lane;
       double3 t = make_double3(0.0, 0.0, 0.0);
-      if (k < k1) t = row_term(bs, m, cs, r, sgn, k - k0, ilog2toe, e2.t);
+      if (k < k1) t = row_term(bs, m, cs, r, sgn, k - k0, e2.t);
       const bool keep = (k < k1) && t.x != 0.0;
       const unsigned bal = __ballot_sync(0xffffffffu, keep);
       if (keep) {
@@ -271,143 +278,251 @@ k_rows2(const BSet2Dev* __restrict__ bsets, Model2Dev m, int B,
   if (lane == 0) rcnt[static_cast<size_t>(wb) * bs.nrows + r] = make_int2(npos, nneg);
 }
 
-// Main R grid, rows 1..n-1 x columns 1..n-1 (row 0 and column 0 are the
-// edge cells), times dflux1*dflux2, with block partial sums of the
-// trapezoid moments of getRStats (PDFactoryDouble.cc:593-722).  A block
-// covers RG_COLS = RG_CPT * NT columns and RB rows; thread t owns columns
-// base + t + NT q (q < RG_CPT: each store of a warp stays coalesced) and
-// reads their flux constants once.  Per row the sign, the term counts and
-// the list address are read once per thread, and each colour term's
-// (c0, c1, c2) once for all the thread's columns of that term's band-2 sign
-// component: the terms of a cell are summed in the list's order
-// (numberCountsDoubleLogNormal.cc:1972-2002), the columns giving the
-// independent exp2 chains.
-constexpr int RG_CPT = 4;
-constexpr int RG_COLS = RG_CPT * NT;
-template <int RB>
-__global__ void __launch_bounds__(NT, 4)
-k_rgrid2(const BSet2Dev* __restrict__ bsets, int B, int n, int nc2,
-         const int* __restrict__ mstatus, const double* __restrict__ rw,
-         const int2* __restrict__ rcnt, double* __restrict__ rbuf,
-         double* __restrict__ rpart) {
-  __shared__ double shr[32];
-  const int wb = blockIdx.z;
-  const int w = wb / B, b = wb - w * B;
-  if (mstatus[w] != 0) return;
-  __shared__ dev::Exp2Table e2;
-  e2.load();
-  __syncthreads();
-  const BSet2Dev& bs = bsets[b];
-  const int nrows = bs.nrows, ts3 = 3 * bs.Ts;
-  const int* __restrict__ rowsgn = bs.rowsgn;
-  const double* __restrict__ rowflux = bs.rowflux;
-  const int j0 = blockIdx.x * RG_COLS + threadIdx.x;
-  double if2[RG_CPT], lf2[RG_CPT], cf2[RG_CPT];
-  unsigned cpos = 0, cneg = 0;  // columns (bits q) in each band-2 sign component
+// The colour terms of a block's rows first, first + step, ... (below last) in
+// shared memory: signs, counts and, where they fit, the terms themselves, so
+// that no row waits for three dependent reads of its own.
+constexpr int ST_ROWS = 32;    // most rows per block
+constexpr int ST_TERMS = 448;  // colour terms that fit
+struct RowStage {
+  double term[3 * ST_TERMS];
+  double flux[ST_ROWS];
+  int2 cnt[ST_ROWS];
+  int sgn[ST_ROWS], off[ST_ROWS + 1];
+  // ends in a barrier; true when the terms fitted
+  __device__ __forceinline__ bool load(const BSet2Dev& bs, int wb, int first, int step, int count,
+                                       int last, const double* __restrict__ rw,
+                                       const int2* __restrict__ rcnt) {
+    const int t = threadIdx.x;
+    const size_t row0 = static_cast<size_t>(wb) * bs.nrows;
+    if (t < count) {
+      const int r = first + t * step;
+      const int s = (r < last) ? bs.rowsgn[r] : -1;
+      sgn[t] = s;
+      cnt[t] = (s >= 0) ? rcnt[row0 + r] : make_int2(0, 0);
+      flux[t] = (r < last) ? bs.rowflux[r] : 0.0;
+    }
+    __syncthreads();
+    if (t <= count) {
+      int o = 0;
+      for (int i = 0; i < t; ++i) o += cnt[i].x + cnt[i].y;
+      off[t] = o;
+    }
+    __syncthreads();
+    const bool fit = off[count] <= ST_TERMS;
+    if (fit)
+      for (int i = t >> 5; i < count; i += NT / 32) {  // a warp per row
+        const double* L = rw + (row0 + first + i * step) * (3 * bs.Ts);
+        const int c3 = 3 * (off[i + 1] - off[i]);
+        for (int k = t & 31; k < c3; k += 32) term[3 * off[i] + k] = L[k];
+      }
+    __syncthreads();
+    return fit;
+  }
+};
+
+// Columns of a thread (bits q) in each band-2 sign component.
+struct ColMask {
+  unsigned pos = 0, neg = 0;
+};
+
+// The colour terms of one row at a thread's C columns, summed in the list's
+// order (numberCountsDoubleLogNormal.cc:1972-2002), the columns giving the
+// independent exp2 chains.  Rows with terms of either band-2 sign, or
+// columns of both, take each sign component in turn.
+template <int C>
+__device__ __forceinline__ void row_sum(const double* L, int2 nt, int sgn1, unsigned hsm,
+                                        ColMask m, const double* lf2,
+                                        const double* __restrict__ tab, const dev::GaussC& gc,
+                                        double* acc) {
+#pragma unroll 1
+  for (int fs = 0; fs < 2; ++fs) {
+    const unsigned cols = fs ? m.neg : m.pos;
+    if (!cols || !((hsm >> (sgn1 + fs)) & 1u)) continue;
+    const double* T = fs ? L + 3 * nt.x : L;
+    const int cnt = fs ? nt.y : nt.x;
+#pragma unroll 1
+    for (int k = 0; k < cnt; ++k) {
+      const double c0 = T[3 * k], ta = T[3 * k + 1], tb = T[3 * k + 2];
 #pragma unroll
-  for (int q = 0; q < RG_CPT; ++q) {
-    const int j = j0 + q * NT;
-    if2[q] = 0.0;
-    lf2[q] = 0.0;
-    cf2[q] = 0.0;
-    if (j >= 1 && j < n) {
-      if2[q] = bs.colinv[j];
-      lf2[q] = bs.collog[j];
-      cf2[q] = bs.rflux2[j];
-      if (if2[q] != 0.0) {
-        if (bs.colsgn[j]) cneg |= 1u << q;
-        else cpos |= 1u << q;
+      for (int q = 0; q < C; ++q) {
+        if (!((cols >> q) & 1u)) continue;
+        acc[q] += c0 * dev::exp2_gauss(fma(ta, lf2[q], tb), tab, gc);
       }
     }
   }
-  const unsigned hsm = (bs.hassign[0] ? 1u : 0u) | (bs.hassign[1] ? 2u : 0u) |
-                       (bs.hassign[2] ? 4u : 0u) | (bs.hassign[3] ? 8u : 0u);
+}
+// The same where only the positive components exist and no column is
+// negative (a column of flux 0 is multiplied by 0 afterwards), from the
+// staged terms T: nothing but the terms.
+template <int C>
+__device__ __forceinline__ void row_sum_pos(const double* T, int cnt, const double* lf2,
+                                            const double* __restrict__ tab, const dev::GaussC& gc,
+                                            double* acc) {
+#pragma unroll 1
+  for (int k = 0; k < cnt; ++k, T += 3) {
+    const double c0 = T[0], ta = T[1], tb = T[2];
+#pragma unroll
+    for (int q = 0; q < C; ++q)
+      acc[q] += c0 * dev::exp2_gauss(fma(ta, lf2[q], tb), tab, gc);
+  }
+}
+__device__ __forceinline__ unsigned sign_mask(const BSet2Dev& bs) {
+  return (bs.hassign[0] ? 1u : 0u) | (bs.hassign[1] ? 2u : 0u) | (bs.hassign[2] ? 4u : 0u) |
+         (bs.hassign[3] ? 8u : 0u);
+}
+
+// Main R grid, rows 1..n-1 x columns 1..n-1 (row 0 and column 0 are the
+// edge cells), times dflux1*dflux2, with block partial sums of the
+// trapezoid moments of getRStats (PDFactoryDouble.cc:593-722) and of R.  A
+// block covers RG_COLS = RG_CPT * NT columns and nrb rows, gridDim.y apart
+// (faint rows have up to ten times the terms of bright ones: every block
+// gets its share); thread t owns columns base + t + NT q (q < RG_CPT: each
+// store of a warp stays coalesced) and reads their flux constants once.
+// Bound by issue: ~20 instructions, 11 of them FP64, a term and column, and
+// a row's own overhead, since most rows have one to three terms.
+constexpr int RG_CPT = 4;
+constexpr int RG_COLS = RG_CPT * NT;
+__global__ void __launch_bounds__(NT, 3)
+k_rgrid2(const BSet2Dev* __restrict__ bsets, int B, int n, int pitch, int nrb,
+         const int* __restrict__ mstatus, const double* __restrict__ rw,
+         const int2* __restrict__ rcnt, double* __restrict__ rgrid,
+         double* __restrict__ rpart) {
+  __shared__ double shr[32];
+  __shared__ dev::GaussTable gt;
+  __shared__ RowStage st;
+  const int wb = blockIdx.z;
+  const int w = wb / B, b = wb - w * B;
+  if (mstatus[w] != 0) return;
+  const BSet2Dev& bs = bsets[b];
+  const int t = threadIdx.x;
+  const int r0 = 1 + blockIdx.y, step = gridDim.y;
+  gt.load();
+  const bool staged = st.load(bs, wb, r0, step, nrb, n, rw, rcnt);
+  const double* __restrict__ tab = gt.lane();
+  const dev::GaussC gc;
+  const int j0 = blockIdx.x * RG_COLS + t;
   const double fluxfac = bs.dflux1 * bs.dflux2;
-  double m1 = 0.0, v1 = 0.0, m2 = 0.0, v2 = 0.0;
-  for (int rr = 0; rr < RB; ++rr) {
-    const int r = 1 + blockIdx.y * RB + rr;
-    if (r >= n) break;
-    const int sgn1 = rowsgn[r];
-    const size_t ri = static_cast<size_t>(wb) * nrows + r;
+  double ifl[RG_CPT], lf2[RG_CPT], csum[RG_CPT];
+  ColMask m;
+#pragma unroll
+  for (int q = 0; q < RG_CPT; ++q) {
+    const int j = j0 + q * NT;
+    ifl[q] = 0.0;
+    lf2[q] = 0.0;
+    csum[q] = 0.0;
+    if (j >= 1 && j < n) {
+      const double ci = bs.colinv[j];
+      lf2[q] = bs.collog[j];
+      if (ci != 0.0) {
+        ifl[q] = ci * fluxfac;
+        if (bs.colsgn[j]) m.neg |= 1u << q;
+        else m.pos |= 1u << q;
+      }
+    }
+  }
+  const unsigned hsm = sign_mask(bs);
+  // whole tiles of non-negative columns, one sign component, staged terms
+  const bool plain = __syncthreads_and(staged && hsm == 1u && m.neg == 0u) &&
+                     (blockIdx.x + 1) * RG_COLS <= static_cast<unsigned>(n);
+  const int qlast = (n - 1 - j0) % NT == 0 ? (n - 1 - j0) / NT : -1;  // owns column n - 1
+  double m1 = 0.0, v1 = 0.0, m0 = 0.0;
+  double* Rp = rgrid + (static_cast<size_t>(wb) * n + r0) * pitch + j0;
+  const size_t rstep = static_cast<size_t>(step) * pitch;
+  const int rows = min(nrb, (n - r0 + step - 1) / step);
+  for (int rr = 0; rr < rows; ++rr, Rp += rstep) {
     double acc[RG_CPT];
 #pragma unroll
     for (int q = 0; q < RG_CPT; ++q) acc[q] = 0.0;
-    if (sgn1 >= 0) {
-      const int2 nt = rcnt[ri];
-      const double* __restrict__ L = rw + ri * ts3;
+    if (plain) {
+      const int o = st.off[rr];
+      row_sum_pos<RG_CPT>(st.term + 3 * o, st.off[rr + 1] - o, lf2, tab, gc, acc);
 #pragma unroll
-      for (int fs = 0; fs < 2; ++fs) {
-        const unsigned cols = fs ? cneg : cpos;
-        if (!cols || !((hsm >> (sgn1 + fs)) & 1u)) continue;
-        const double* __restrict__ T = fs ? L + 3 * nt.x : L;
-        const int cnt = fs ? nt.y : nt.x;
-        for (int k = 0; k < cnt; ++k) {
-          const double c0 = __ldg(T + 3 * k), c1 = __ldg(T + 3 * k + 1),
-                       c2 = __ldg(T + 3 * k + 2);
+      for (int q = 0; q < RG_CPT; ++q) {
+        acc[q] *= ifl[q];
+        Rp[q * NT] = acc[q];  // (column 0 is an edge cell, filled later)
+      }
+    } else {
+      const int sgn1 = st.sgn[rr];
+      if (sgn1 >= 0) {
+        const double* L = staged ? st.term + 3 * st.off[rr]
+                                 : rw + (static_cast<size_t>(wb) * bs.nrows + r0 + rr * step) *
+                                            (3 * bs.Ts);
+        row_sum<RG_CPT>(L, st.cnt[rr], sgn1, hsm, m, lf2, tab, gc, acc);
+      }
 #pragma unroll
-          for (int q = 0; q < RG_CPT; ++q) {
-            if (!((cols >> q) & 1u)) continue;
-            const double t = lf2[q] - c1;
-            acc[q] += c0 * dev::exp2_tab(t * t * c2, e2.t);
-          }
-        }
+      for (int q = 0; q < RG_CPT; ++q) {
+        acc[q] *= ifl[q];
+        if (j0 + q * NT < n) Rp[q * NT] = acc[q];
       }
     }
-    const double cf1 = rowflux[r];
-    const double rw1 = (r == n - 1) ? 0.5 : 1.0;
-    double* Rrow = rbuf + (static_cast<size_t>(wb) * n + r) * nc2;
+    // the last row and the last column weigh a half in the moments
+    const double rw1 = (r0 + rr * step == n - 1) ? 0.5 : 1.0;
+    double s0 = 0.0;
 #pragma unroll
     for (int q = 0; q < RG_CPT; ++q) {
-      const int j = j0 + q * NT;
-      if (j < 1 || j >= n) continue;
-      const double R = acc[q] * if2[q] * fluxfac;
-      Rrow[j] = R;
-      const double cR = rw1 * R;
-      const double wc = (j == n - 1) ? 0.5 : 1.0;
-      const double p1 = wc * cf1 * cR;
-      const double p2 = wc * cf2[q] * cR;
-      m1 += p1;
-      v1 += cf1 * p1;
-      m2 += p2;
-      v2 += cf2[q] * p2;
+      csum[q] = fma(rw1, acc[q], csum[q]);
+      s0 += acc[q];
     }
+    m0 += s0;
+    if (qlast >= 0) {
+#pragma unroll
+      for (int q = 0; q < RG_CPT; ++q)
+        if (q == qlast) s0 -= 0.5 * acc[q];
+    }
+    const double cf1 = st.flux[rr];
+    s0 *= rw1 * cf1;
+    m1 += s0;
+    v1 = fma(cf1, s0, v1);
+  }
+  double m2 = 0.0, v2 = 0.0;
+#pragma unroll
+  for (int q = 0; q < RG_CPT; ++q) {
+    const int j = j0 + q * NT;
+    if (j < 1 || j >= n) continue;
+    const double cf2 = bs.rflux2[j];
+    const double p2 = ((j == n - 1) ? 0.5 : 1.0) * cf2 * csum[q];
+    m2 += p2;
+    v2 += cf2 * p2;
   }
   m1 = dev::block_sum<NT>(m1, shr);
   v1 = dev::block_sum<NT>(v1, shr);
   m2 = dev::block_sum<NT>(m2, shr);
   v2 = dev::block_sum<NT>(v2, shr);
-  if (threadIdx.x == 0) {
-    double* o = rpart + ((static_cast<size_t>(wb) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * 4;
-    o[0] = m1; o[1] = v1; o[2] = m2; o[3] = v2;
+  m0 = dev::block_sum<NT>(m0, shr);
+  if (t == 0) {
+    double* o = rpart + ((static_cast<size_t>(wb) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * 5;
+    o[0] = m1; o[1] = v1; o[2] = m2; o[3] = v2; o[4] = m0;
   }
 }
 
 // Edge rows (band-1 fluxes below the first grid step) against every main and
 // edge column, weighted by the log-trapezoid factors of the band-1 edge
 // integral (PDFactoryDouble.cc:426-514).  One block per (tile of RG_COLS
-// columns, group of ER edge rows, proposal x beam set), the columns spread
-// over the threads as in k_rgrid2 so that each row's terms are read once per
-// thread for its RG_CPT columns; the group partials are summed in
+// columns, group of er edge rows, proposal x beam set), the columns spread
+// over the threads as in k_rgrid2 and the group's rows gridDim.y apart (the
+// terms sit in the brightest of them); the group partials are summed in
 // k_rfinish2 into Rx (main columns) and the double integral r[0,0] (edge
 // columns).
 constexpr int ER_MIN = 4;    // fewest edge rows per group (sizes the partials)
-template <int ER>
-__global__ void __launch_bounds__(NT, 4)
-k_redge2(const BSet2Dev* __restrict__ bsets, int B, int n, int nedge,
+__global__ void __launch_bounds__(NT, 3)
+k_redge2(const BSet2Dev* __restrict__ bsets, int B, int n, int nedge, int er,
          const int* __restrict__ mstatus, const double* __restrict__ rw,
          const int2* __restrict__ rcnt, double* __restrict__ epart) {
+  __shared__ dev::GaussTable gt;
+  __shared__ RowStage st;
   const int wb = blockIdx.z;
   const int w = wb / B, b = wb - w * B;
   if (mstatus[w] != 0) return;
-  __shared__ dev::Exp2Table e2;
-  e2.load();
-  __syncthreads();
   const BSet2Dev& bs = bsets[b];
+  const int i0 = blockIdx.y, step = gridDim.y;
+  gt.load();
+  const bool staged = st.load(bs, wb, n + i0, step, er, n + nedge, rw, rcnt);
+  const double* __restrict__ tab = gt.lane();
+  const dev::GaussC gc;
   const int ncol = n + nedge;
-  const int nrows = bs.nrows, ts3 = 3 * bs.Ts;
   const int j0 = blockIdx.x * RG_COLS + threadIdx.x;
   double if2[RG_CPT], lf2[RG_CPT], acc[RG_CPT];
-  unsigned cpos = 0, cneg = 0;
+  ColMask m;
 #pragma unroll
   for (int q = 0; q < RG_CPT; ++q) {
     const int j = j0 + q * NT;
@@ -418,42 +533,30 @@ k_redge2(const BSet2Dev* __restrict__ bsets, int B, int n, int nedge,
       if2[q] = bs.colinv[j];
       lf2[q] = bs.collog[j];
       if (if2[q] != 0.0) {
-        if (bs.colsgn[j]) cneg |= 1u << q;
-        else cpos |= 1u << q;
+        if (bs.colsgn[j]) m.neg |= 1u << q;
+        else m.pos |= 1u << q;
       }
     }
   }
-  const unsigned hsm = (bs.hassign[0] ? 1u : 0u) | (bs.hassign[1] ? 2u : 0u) |
-                       (bs.hassign[2] ? 4u : 0u) | (bs.hassign[3] ? 8u : 0u);
-  for (int rr = 0; rr < ER; ++rr) {
-    const int i = blockIdx.y * ER + rr;
+  const unsigned hsm = sign_mask(bs);
+  const bool plain = __syncthreads_and(staged && hsm == 1u && m.neg == 0u);
+  for (int rr = 0; rr < er; ++rr) {
+    const int i = i0 + rr * step;
     if (i >= nedge) break;
-    const int r = n + i;
-    const int sgn1 = bs.rowsgn[r];
-    if (sgn1 < 0) continue;
-    const size_t ri = static_cast<size_t>(wb) * nrows + r;
-    const int2 nt = rcnt[ri];
-    const double* __restrict__ L = rw + ri * ts3;
-    const double wr = ((i == 0 || i == nedge - 1) ? 0.5 : 1.0) * bs.e1[i];
+    const int sgn1 = st.sgn[rr];
+    if (sgn1 < 0 || st.off[rr + 1] == st.off[rr]) continue;
     double rs[RG_CPT];
 #pragma unroll
     for (int q = 0; q < RG_CPT; ++q) rs[q] = 0.0;
-#pragma unroll
-    for (int fs = 0; fs < 2; ++fs) {
-      const unsigned cols = fs ? cneg : cpos;
-      if (!cols || !((hsm >> (sgn1 + fs)) & 1u)) continue;
-      const double* __restrict__ T = fs ? L + 3 * nt.x : L;
-      const int cnt = fs ? nt.y : nt.x;
-      for (int k = 0; k < cnt; ++k) {
-        const double a0 = __ldg(T + 3 * k), a1 = __ldg(T + 3 * k + 1), a2 = __ldg(T + 3 * k + 2);
-#pragma unroll
-        for (int q = 0; q < RG_CPT; ++q) {
-          if (!((cols >> q) & 1u)) continue;
-          const double t = lf2[q] - a1;
-          rs[q] += a0 * dev::exp2_tab(t * t * a2, e2.t);
-        }
-      }
+    if (plain) {
+      const int o = st.off[rr];
+      row_sum_pos<RG_CPT>(st.term + 3 * o, st.off[rr + 1] - o, lf2, tab, gc, rs);
+    } else {
+      const double* L = staged ? st.term + 3 * st.off[rr]
+                               : rw + (static_cast<size_t>(wb) * bs.nrows + n + i) * (3 * bs.Ts);
+      row_sum<RG_CPT>(L, st.cnt[rr], sgn1, hsm, m, lf2, tab, gc, rs);
     }
+    const double wr = ((i == 0 || i == nedge - 1) ? 0.5 : 1.0) * bs.e1[i];
 #pragma unroll
     for (int q = 0; q < RG_CPT; ++q) acc[q] += wr * (rs[q] * if2[q]);
   }
@@ -464,89 +567,84 @@ k_redge2(const BSet2Dev* __restrict__ bsets, int B, int n, int nedge,
   }
 }
 
-// Edge integral along band 2 for column 0 (PDFactoryDouble.cc:518-550):
-// one warp per main row (NT / 32 rows per block, so that the exp2 table is
-// built once for several rows), each lane taking edge columns lane, lane +
-// 32, ...: the row's sign, term counts and each term's (c0, c1, c2) are read
-// once per lane for all its columns of one band-2 sign component; a warp
-// reduction gives the row's sum.
-constexpr int RY_ROWS = NT / 32;
+// Edge integral along band 2 for column 0 (PDFactoryDouble.cc:518-550): a
+// block takes nrb main rows (gridDim.x apart), each of its warps every
+// eighth of them, with the lane's edge columns lane, lane + 32, ... and their
+// constants held over the rows; a warp reduction gives a row's sum.
 constexpr int RY_CPL = 8;  // edge columns per lane held at once
-__global__ void __launch_bounds__(NT, 4)
-k_ry2(const BSet2Dev* __restrict__ bsets, int B, int n, int nedge,
+__global__ void __launch_bounds__(NT, 3)
+k_ry2(const BSet2Dev* __restrict__ bsets, int B, int n, int nedge, int nrb,
       const int* __restrict__ mstatus, const double* __restrict__ rw,
       const int2* __restrict__ rcnt, double* __restrict__ redge) {
+  __shared__ dev::GaussTable gt;
+  __shared__ RowStage st;
+  __shared__ double tot[ST_ROWS];
   const int wb = blockIdx.y;
   const int w = wb / B, b = wb - w * B;
   if (mstatus[w] != 0) return;
-  __shared__ dev::Exp2Table e2;
-  e2.load();
-  __syncthreads();
   const BSet2Dev& bs = bsets[b];
-  const int lane = threadIdx.x & 31;
-  const int r = 1 + blockIdx.x * RY_ROWS + (threadIdx.x >> 5);  // main rows 1..n-1
-  if (r >= n) return;
-  const int sgn1 = bs.rowsgn[r];
-  const size_t ri = static_cast<size_t>(wb) * bs.nrows + r;
-  const double* __restrict__ row = rw + ri * bs.Ts * 3;
-  const int2 nt = rcnt[ri];
-  const unsigned hsm = (bs.hassign[0] ? 1u : 0u) | (bs.hassign[1] ? 2u : 0u) |
-                       (bs.hassign[2] ? 4u : 0u) | (bs.hassign[3] ? 8u : 0u);
-  double tot = 0.0;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int r0 = 1 + blockIdx.x, step = gridDim.x;
+  gt.load();
+  const bool staged = st.load(bs, wb, r0, step, nrb, n, rw, rcnt);
+  const double* __restrict__ tab = gt.lane();
+  const dev::GaussC gc;
+  if (threadIdx.x < ST_ROWS) tot[threadIdx.x] = 0.0;
+  __syncthreads();
+  const unsigned hsm = sign_mask(bs);
   for (int c0 = 0; c0 < nedge; c0 += 32 * RY_CPL) {
-    double lf2[RY_CPL], if2[RY_CPL], acc[RY_CPL];
-    unsigned cpos = 0, cneg = 0;
+    double lf2[RY_CPL], wt[RY_CPL];
+    ColMask m;
 #pragma unroll
     for (int q = 0; q < RY_CPL; ++q) {
       const int jj = c0 + lane + 32 * q;
       lf2[q] = 0.0;
-      if2[q] = 0.0;
-      acc[q] = 0.0;
+      wt[q] = 0.0;
       if (jj < nedge) {
-        const int j = n + jj;
-        if2[q] = bs.colinv[j];
-        lf2[q] = bs.collog[j];
-        if (if2[q] != 0.0) {
-          if (bs.colsgn[j]) cneg |= 1u << q;
-          else cpos |= 1u << q;
+        const double ci = bs.colinv[n + jj];
+        lf2[q] = bs.collog[n + jj];
+        wt[q] = (jj == 0 || jj == nedge - 1) ? 0.5 * ci : ci;
+        if (ci != 0.0) {
+          if (bs.colsgn[n + jj]) m.neg |= 1u << q;
+          else m.pos |= 1u << q;
         }
       }
     }
-    if (sgn1 >= 0) {
+    const bool plain = staged && hsm == 1u && __all_sync(0xffffffffu, m.neg == 0u);
+    for (int rr = wp; rr < nrb; rr += NT / 32) {
+      const int sgn1 = st.sgn[rr];
+      if (sgn1 < 0) continue;
+      double acc[RY_CPL];
 #pragma unroll
-      for (int fs = 0; fs < 2; ++fs) {
-        const unsigned cols = fs ? cneg : cpos;
-        if (!cols || !((hsm >> (sgn1 + fs)) & 1u)) continue;
-        const double* __restrict__ T = fs ? row + 3 * nt.x : row;
-        const int cnt = fs ? nt.y : nt.x;
-        for (int k = 0; k < cnt; ++k) {
-          const double a0 = __ldg(T + 3 * k), a1 = __ldg(T + 3 * k + 1), a2 = __ldg(T + 3 * k + 2);
-#pragma unroll
-          for (int q = 0; q < RY_CPL; ++q) {
-            if (!((cols >> q) & 1u)) continue;
-            const double t = lf2[q] - a1;
-            acc[q] += a0 * dev::exp2_tab(t * t * a2, e2.t);
-          }
-        }
+      for (int q = 0; q < RY_CPL; ++q) acc[q] = 0.0;
+      if (plain) {
+        const int o = st.off[rr];
+        row_sum_pos<RY_CPL>(st.term + 3 * o, st.off[rr + 1] - o, lf2, tab, gc, acc);
+      } else {
+        const double* L = staged ? st.term + 3 * st.off[rr]
+                                 : rw + (static_cast<size_t>(wb) * bs.nrows + r0 + rr * step) *
+                                            (3 * bs.Ts);
+        row_sum<RY_CPL>(L, st.cnt[rr], sgn1, hsm, m, lf2, tab, gc, acc);
       }
-    }
+      double s = 0.0;
 #pragma unroll
-    for (int q = 0; q < RY_CPL; ++q) {
-      const int jj = c0 + lane + 32 * q;
-      if (jj >= nedge) continue;
-      const double R = acc[q] * if2[q];
-      tot += (jj == 0 || jj == nedge - 1) ? 0.5 * R : R;
+      for (int q = 0; q < RY_CPL; ++q) s = fma(acc[q], wt[q], s);
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) tot[rr] += s;
     }
   }
-  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-  if (lane == 0) redge[static_cast<size_t>(wb) * (2 * n + 1) + n + r] = tot * bs.iRynorm;
+  __syncthreads();
+  if (threadIdx.x < nrb) {
+    const int r = r0 + threadIdx.x * step;
+    if (r < n) redge[static_cast<size_t>(wb) * (2 * n + 1) + n + r] = tot[threadIdx.x] * bs.iRynorm;
+  }
 }
 
 // Edge cells into the grid (times dflux1*dflux2), the remaining moment
 // contributions and the shift decisions (PDFactoryDouble.cc:560-585,
 // 1198-1213).
 __global__ void __launch_bounds__(NT)
-k_rfinish2(const BSet2Dev* __restrict__ bsets, int B, int n, int nc2,
+k_rfinish2(const BSet2Dev* __restrict__ bsets, int B, int n, int pitch,
            int edge, int nedge, int ngr, int nparts,
            const int* __restrict__ mstatus, const double* __restrict__ redge,
            const double* __restrict__ epart, const double* __restrict__ rpart,
@@ -561,10 +659,10 @@ k_rfinish2(const BSet2Dev* __restrict__ bsets, int B, int n, int nc2,
   const BSet2Dev& bs = bsets[b];
   const double fluxfac = bs.dflux1 * bs.dflux2;
   const double* E = redge + static_cast<size_t>(wb) * (2 * n + 1);
-  double* R = rbuf + static_cast<size_t>(wb) * n * nc2;
+  double* R = rbuf + static_cast<size_t>(wb) * n * pitch;
   const int ncol = n + nedge;
   const double* ep = epart + static_cast<size_t>(wb) * ngr * ncol;
-  double m1 = 0.0, v1 = 0.0, m2 = 0.0, v2 = 0.0;
+  double m1 = 0.0, v1 = 0.0, m2 = 0.0, v2 = 0.0, m0 = 0.0;
   const int j = blockIdx.x * NT + threadIdx.x;  // row-0 column / column-0 row
   if (j >= 1 && j < n) {
     // row 0 (row factor 1/2)
@@ -575,6 +673,7 @@ k_rfinish2(const BSet2Dev* __restrict__ bsets, int B, int n, int nc2,
       val = c * bs.iRxnorm * fluxfac;
     }
     R[j] = val;
+    m0 += val;
     const double cf1r0 = bs.rowflux[0];
     const double cR = 0.5 * val;
     const double wc = (j == n - 1) ? 0.5 : 1.0;
@@ -583,35 +682,53 @@ k_rfinish2(const BSet2Dev* __restrict__ bsets, int B, int n, int nc2,
     m1 += p1; v1 += cf1r0 * p1; m2 += p2; v2 += cf2 * p2;
     // column 0 (column factor 1/2), row j
     const double cv = edge ? E[n + j] * fluxfac : 0.0;
-    R[static_cast<size_t>(j) * nc2] = cv;
+    R[static_cast<size_t>(j) * pitch] = cv;
+    m0 += cv;
     const double cR2 = (j == n - 1) ? 0.5 * cv : cv;
     const double cf1 = bs.rowflux[j], cf20 = bs.rflux2[0];
     const double q1 = 0.5 * cf1 * cR2, q2 = 0.5 * cf20 * cR2;
     m1 += q1; v1 += cf1 * q1; m2 += q2; v2 += cf20 * q2;
   }
-  const double* pp = rpart + static_cast<size_t>(wb) * nparts * 4;
+  const double* pp = rpart + static_cast<size_t>(wb) * nparts * 5;
   for (int k = j; k < nparts; k += gridDim.x * NT) {
-    m1 += pp[4 * k]; v1 += pp[4 * k + 1]; m2 += pp[4 * k + 2]; v2 += pp[4 * k + 3];
+    m1 += pp[5 * k]; v1 += pp[5 * k + 1]; m2 += pp[5 * k + 2]; v2 += pp[5 * k + 3];
+    m0 += pp[5 * k + 4];
   }
   m1 = dev::block_sum<NT>(m1, shr);
   v1 = dev::block_sum<NT>(v1, shr);
   m2 = dev::block_sum<NT>(m2, shr);
   v2 = dev::block_sum<NT>(v2, shr);
+  m0 = dev::block_sum<NT>(m0, shr);
   if (threadIdx.x == 0) {
-    double* o = fpart + (static_cast<size_t>(wb) * gridDim.x + blockIdx.x) * 4;
-    o[0] = m1; o[1] = v1; o[2] = m2; o[3] = v2;
+    double* o = fpart + (static_cast<size_t>(wb) * gridDim.x + blockIdx.x) * 5;
+    o[0] = m1; o[1] = v1; o[2] = m2; o[3] = v2; o[4] = m0;
   }
+}
+
+// Last column of the half spectrum with a bin inside the noise line (n / 2
+// without noise in band 2): every bin of a later column lies past
+// dev::kNoiseZero.
+__device__ __forceinline__ int noise_cut2(double sigma1, double sigma2, double dflux2, int n) {
+  const int h = n / 2;
+  if (!(sigma1 > 0 || sigma2 > 0)) return h;
+  const double iflux2 = dev::kTwoPi / (static_cast<double>(n) * dflux2);
+  const double x = 12.0 / (fabs(sigma2) * iflux2);  // sqrt(2 * 72)
+  return (x >= static_cast<double>(h)) ? h : static_cast<int>(x) + 1;
 }
 
 // r[0,0] (the double edge integral, PDFactoryDouble.cc:426-467), its cell
 // and moment term, the moment sums and the shift decisions
 // (PDFactoryDouble.cc:560-585, 1198-1213); one block per proposal and beam
-// set.
+// set.  For the row and column transforms also R~00, the sum of R, and the
+// noise cut-offs of each dataset and of the beam set (the widest of its
+// datasets).
 __global__ void __launch_bounds__(NT)
-k_rfinal2(const BSet2Dev* __restrict__ bsets, int B, int n, int nc2, int edge,
+k_rfinal2(const BSet2Dev* __restrict__ bsets, int B, int n, int pitch, int edge,
           int nedge, int ngr, int nfp, const int* __restrict__ mstatus,
           const double* __restrict__ epart, const double* __restrict__ fpart,
-          double* __restrict__ rbuf, double* __restrict__ mom) {
+          double* __restrict__ rbuf, double* __restrict__ mom,
+          const DSet2Dev* __restrict__ dsets, int D, const double* __restrict__ sigmult,
+          double* __restrict__ r0buf, int* __restrict__ kcset, int* __restrict__ kcds) {
   __shared__ double shr[32];
   const int wb = blockIdx.x;
   const int w = wb / B, b = wb - w * B;
@@ -629,18 +746,20 @@ k_rfinal2(const BSet2Dev* __restrict__ bsets, int B, int n, int nc2, int edge,
     }
     r00 = dev::block_sum<NT>(r00, shr) * bs.iR00norm;
   }
-  double m1 = 0.0, v1 = 0.0, m2 = 0.0, v2 = 0.0;
-  const double* fp = fpart + static_cast<size_t>(wb) * nfp * 4;
+  double m1 = 0.0, v1 = 0.0, m2 = 0.0, v2 = 0.0, m0 = 0.0;
+  const double* fp = fpart + static_cast<size_t>(wb) * nfp * 5;
   for (int k = threadIdx.x; k < nfp; k += NT) {
-    m1 += fp[4 * k]; v1 += fp[4 * k + 1]; m2 += fp[4 * k + 2]; v2 += fp[4 * k + 3];
+    m1 += fp[5 * k]; v1 += fp[5 * k + 1]; m2 += fp[5 * k + 2]; v2 += fp[5 * k + 3];
+    m0 += fp[5 * k + 4];
   }
   m1 = dev::block_sum<NT>(m1, shr);
   v1 = dev::block_sum<NT>(v1, shr);
   m2 = dev::block_sum<NT>(m2, shr);
   v2 = dev::block_sum<NT>(v2, shr);
+  m0 = dev::block_sum<NT>(m0, shr);
   if (threadIdx.x == 0) {
     const double val = edge ? r00 * fluxfac : 0.0;
-    rbuf[static_cast<size_t>(wb) * n * nc2] = val;
+    rbuf[static_cast<size_t>(wb) * n * pitch] = val;
     // cell (0, 0): row factor 1/2, column weight 1/2
     const double cf1 = bs.rowflux[0], cf2 = bs.rflux2[0];
     const double p1 = 0.5 * cf1 * 0.5 * val, p2 = 0.5 * cf2 * 0.5 * val;
@@ -652,6 +771,16 @@ k_rfinal2(const BSet2Dev* __restrict__ bsets, int B, int n, int nc2, int edge,
     o[0] = m1; o[1] = m2; o[2] = v1; o[3] = v2;
     o[4] = d1 ? -m1 : 0.0; o[5] = d2 ? -m2 : 0.0;
     o[6] = d1 ? 1.0 : 0.0; o[7] = d2 ? 1.0 : 0.0;
+    r0buf[wb] = m0 + val;
+    int kmax = 0;
+    for (int dd = 0; dd < bs.nds; ++dd) {
+      const int d = bs.ds_begin + dd;
+      const int kc = noise_cut2(sigmult[2 * w] * dsets[d].sb1, sigmult[2 * w + 1] * dsets[d].sb2,
+                                bs.dflux2, n);
+      kcds[static_cast<size_t>(w) * D + d] = kc;
+      kmax = max(kmax, kc);
+    }
+    kcset[wb] = kmax;
   }
 }
 
@@ -1289,13 +1418,9 @@ __global__ void k_reduce2(const BSet2Dev* __restrict__ bsets,
 }
 
 // ------------------------------------------------------------------
-// Transforms of FFT mode 1 (n a power of two in [512, 4096]): the R grid,
-// its row transforms, the columns with the spectrum between their two
-// transforms, and the inverse row transforms with the marginal sums of the
-// P(D), in three kernels with one intermediate array.
+// Transforms of FFT mode 1 (n a power of two in [512, 4096]):
 //
-//   k_rowfwd2   R of a few rows (straight into registers, never stored),
-//               their forward row DFTs, columns 0 .. kc of the result
+//   k_rowfwd2   forward row DFTs of the R grid, columns 0 .. kc of the result
 //   k_colspec2  per column: forward DFT, spectrum, inverse DFT, in place
 //   k_rowinv2   inverse row DFTs of columns 0 .. kc, the P(D) rows and the
 //               marginal sums
@@ -1304,9 +1429,8 @@ __global__ void k_reduce2(const BSet2Dev* __restrict__ bsets,
 // k2 > kc lies past dev::kNoiseZero, so those columns are neither computed,
 // stored nor read (kc = 427 of 1024 at n = 2048, 2.8 mJy).  The intermediate
 // array is kept by columns, [k2][row], so that the column kernel, which
-// reads and writes it whole, streams; the row kernels take several rows at
-// a time and touch it in contiguous pieces of 2 G rows (64 bytes at n =
-// 2048).
+// reads and writes it whole, streams; the row kernels touch it in pieces of
+// a pair of rows, 32 bytes, with one vector access each.
 //
 // One DFT, n = 16 M, M = 16 M3, runs on M threads with 16 values each: with
 // input j = n1 M + u, u = m M3 + s and output k = k1 + 16 k2 + 256 k3,
@@ -1329,8 +1453,8 @@ struct Fft2 {
 };
 
 template <int S>
-__device__ __forceinline__ void tw16(double2* v, const double2* __restrict__ T) {
-  double2 w1 = __ldg(T), w2 = __ldg(T + 1), w4 = __ldg(T + 2), w8 = __ldg(T + 3);
+__device__ __forceinline__ void tw16(double2* v, const double2* __restrict__ T, int M) {
+  double2 w1 = __ldg(T), w2 = __ldg(T + M), w4 = __ldg(T + 2 * M), w8 = __ldg(T + 3 * M);
   if (S > 0) {
     w1.y = -w1.y;
     w2.y = -w2.y;
@@ -1363,7 +1487,7 @@ __device__ __forceinline__ void fft2_head(double2* v, double2* b, int u,
                                           const double2* __restrict__ TW) {
   using F = Fft2<N>;
   fft::dft<16, S>(v);
-  tw16<S>(v, TW + 4 * u);
+  tw16<S>(v, TW + u, F::M);
 #pragma unroll
   for (int k1 = 0; k1 < 16; ++k1) b[k1 * F::PITCH + u] = v[k1];
   __syncthreads();
@@ -1371,7 +1495,7 @@ __device__ __forceinline__ void fft2_head(double2* v, double2* b, int u,
 #pragma unroll
   for (int m = 0; m < 16; ++m) v[m] = b[k1 * F::PITCH + m * F::M3 + s];
   fft::dft<16, S>(v);
-  tw16<S>(v, TW + 64 * s);
+  tw16<S>(v, TW + 16 * s, F::M);
   __syncthreads();
 #pragma unroll
   for (int k2 = 0; k2 < 16; ++k2) b[(k1 + 16 * k2) * (F::M3 + 1) + s] = v[k2];
@@ -1387,7 +1511,7 @@ __device__ __forceinline__ void fft2_tail_inv(double2* v, double2* b, int u,
   const int k1 = u / F::M3, s = u % F::M3;
 #pragma unroll
   for (int k2 = 0; k2 < 16; ++k2) v[k2] = b[(k1 + 16 * k2) * (F::M3 + 1) + s];
-  tw16<1>(v, TW + 64 * s);
+  tw16<1>(v, TW + 16 * s, F::M);
   fft::dft<16, 1>(v);
   __syncthreads();
 #pragma unroll
@@ -1395,7 +1519,7 @@ __device__ __forceinline__ void fft2_tail_inv(double2* v, double2* b, int u,
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] = b[j * F::PITCH + u];
-  tw16<1>(v, TW + 4 * u);
+  tw16<1>(v, TW + u, F::M);
   fft::dft<16, 1>(v);
 }
 
@@ -1413,21 +1537,27 @@ __device__ __forceinline__ void ld32(const double2* p, double2& a, double2& b) {
                : "memory");
 }
 
-// Threads, DFTs (pairs of rows) and rows per block of the row kernels.
-template <int N>
-struct RowCfg {
-  static constexpr int M = N / 16;
-  static constexpr int T = N <= 512 ? 128 : 256;
-  static constexpr int G = T / M;
-  static constexpr int ROWS = 2 * G;
+// Threads, DFTs (pairs of rows) and rows per block of the row kernels: the
+// forward one, all arithmetic, in small blocks; the inverse one, which reads
+// the columns in pieces of its rows, with more rows (n = 2048, 64 proposals:
+// 1.24 ms with two pairs, 1.48 ms with one).
+template <int N, int THREADS>
+struct RowShape {
+  static constexpr int M = N / 16, T = THREADS;
+  static constexpr int G = T / M, ROWS = 2 * G;
 };
-inline int rowcfg_rows(int n) { return n <= 1024 ? 8 : (n == 2048 ? 4 : 2); }
-inline size_t rowfwd_smem(int n) {
-  return static_cast<size_t>(rowcfg_rows(n) / 2) * 256 * (n / 256 + 1) * sizeof(double2);
-}
+template <int N>
+using FwdCfg = RowShape<N, (N <= 2048 ? 128 : 256)>;
+template <int N>
+using InvCfg = RowShape<N, (N <= 512 ? 128 : 256)>;
 constexpr int RI_ROWS = 32;  // P(D) rows per block of k_rowinv2 (>= 2 G)
-inline size_t rowinv_smem(int n) {
-  return rowfwd_smem(n) + static_cast<size_t>(rowcfg_rows(n) / 2) * n * sizeof(double);
+template <int N>
+constexpr size_t rowfwd_smem() {
+  return static_cast<size_t>(FwdCfg<N>::G) * Fft2<N>::SL * sizeof(double2);
+}
+template <int N>
+constexpr size_t rowinv_smem() {
+  return static_cast<size_t>(InvCfg<N>::G) * (Fft2<N>::SL * sizeof(double2) + N * sizeof(double));
 }
 // columns per block of k_colspec2
 template <int N>
@@ -1442,262 +1572,56 @@ inline size_t colspec_smem(int n, bool several) {
          (several ? 2 : 1);
 }
 
-// Last column of the half spectrum with a bin inside the noise line (n / 2
-// without noise in band 2).
-__device__ __forceinline__ int noise_cut2(double sigma1, double sigma2, double dflux2, int n) {
-  const int h = n / 2;
-  if (!(sigma1 > 0 || sigma2 > 0)) return h;
-  const double iflux2 = dev::kTwoPi / (static_cast<double>(n) * dflux2);
-  const double x = 12.0 / (fabs(sigma2) * iflux2);  // sqrt(2 * 72): past kNoiseZero
-  return (x >= static_cast<double>(h)) ? h : static_cast<int>(x) + 1;
-}
-
-// The edge cells of row 0 (band-1 edge integral, the double integral at
-// [0, 0]; times dflux1*dflux2) before the row transforms, and the noise
-// cut-offs of each dataset and of each beam set (the widest of its
-// datasets).
-__global__ void __launch_bounds__(NT)
-k_redge0_2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dsets, int B, int D,
-           int n, int edge, int nedge, int ngr, const int* __restrict__ mstatus,
-           const double* __restrict__ sigmult, const double* __restrict__ epart,
-           double* __restrict__ row0, int* __restrict__ kcset, int* __restrict__ kcds) {
-  __shared__ double shr[32];
-  const int wb = blockIdx.y;
-  const int w = wb / B, b = wb - w * B;
-  if (mstatus[w] != 0) return;
-  const BSet2Dev& bs = bsets[b];
-  const double fluxfac = bs.dflux1 * bs.dflux2;
-  const int ncol = n + nedge;
-  const double* ep = epart + static_cast<size_t>(wb) * ngr * ncol;
-  const int j = blockIdx.x * NT + threadIdx.x;
-  if (j >= 1 && j < n) {
-    double c = 0.0;
-    if (edge)
-      for (int g = 0; g < ngr; ++g) c += ep[static_cast<size_t>(g) * ncol + j];
-    row0[static_cast<size_t>(wb) * n + j] = edge ? c * bs.iRxnorm * fluxfac : 0.0;
-  }
-  if (blockIdx.x != 0) return;
-  double r00 = 0.0;
-  if (edge) {
-    for (int jj = threadIdx.x; jj < nedge; jj += NT) {
-      double c = 0.0;
-      for (int g = 0; g < ngr; ++g) c += ep[static_cast<size_t>(g) * ncol + n + jj];
-      r00 += (jj == 0 || jj == nedge - 1) ? 0.5 * c : c;
-    }
-    r00 = dev::block_sum<NT>(r00, shr) * bs.iR00norm;
-  }
-  if (threadIdx.x == 0) {
-    row0[static_cast<size_t>(wb) * n] = edge ? r00 * fluxfac : 0.0;
-    const double sm1 = sigmult[2 * w], sm2 = sigmult[2 * w + 1];
-    int kmax = 0;
-    for (int dd = 0; dd < bs.nds; ++dd) {
-      const int d = bs.ds_begin + dd;
-      const int kc = noise_cut2(sm1 * dsets[d].sb1, sm2 * dsets[d].sb2, bs.dflux2, n);
-      kcds[static_cast<size_t>(w) * D + d] = kc;
-      kmax = max(kmax, kc);
-    }
-    kcset[wb] = kmax;
-  }
-}
-
-// R and its forward row transforms.  A block takes groups of ROWS = 2 G rows,
-// each pair of rows on M threads; a thread evaluates R at its 16 columns u,
-// u + M, ... of both rows (the colour terms as in k_rgrid2, read once per
-// thread for its 16 columns) straight into the 16 inputs of its first DFT,
-// the two rows as real and imaginary part.  Of the result Z the two rows'
-// spectra X0 = (Z_k + conj Z_{n-k}) / 2, X1 = (Z_k - conj Z_{n-k}) / 2i go out
-// for k <= kc.  Block partials of the trapezoid moments of getRStats
-// (PDFactoryDouble.cc:593-722) and of the DC bin: rpart[wb][block][5].
+// Forward row transforms of the R grid (pitch n), two rows as the real and
+// imaginary part of one DFT.  Of the result Z the rows' spectra X0 = (Z_k +
+// conj Z_{n-k}) / 2, X1 = (Z_k - conj Z_{n-k}) / 2i go out for k <= kc.
 template <int N>
-__global__ void __launch_bounds__(RowCfg<N>::T, 512 / RowCfg<N>::T)
-k_rowfwd2(const BSet2Dev* __restrict__ bsets, int B, int D, int edge, int gpb,
-          const int* __restrict__ mstatus, const double* __restrict__ rw,
-          const int2* __restrict__ rcnt, const double* __restrict__ row0,
-          const double* __restrict__ redge, const int* __restrict__ kcset,
-          double2* __restrict__ ybuf, double* __restrict__ rpart,
-          const double2* __restrict__ TW) {
+__global__ void __launch_bounds__(FwdCfg<N>::T, 512 / FwdCfg<N>::T)
+k_rowfwd2(const BSet2Dev* __restrict__ bsets, int B, int D, const int* __restrict__ mstatus,
+          const double* __restrict__ rgrid, const int* __restrict__ kcset,
+          double2* __restrict__ ybuf, const double2* __restrict__ TW) {
   using F = Fft2<N>;
-  using R = RowCfg<N>;
+  using R = FwdCfg<N>;
   constexpr int M = F::M, M3 = F::M3, G = R::G, T = R::T;
   constexpr int nc = N / 2 + 1;
   extern __shared__ double2 fsm[];  // [G][SL]
-  __shared__ double shr[32];
-  __shared__ dev::Exp2Table e2;
   const int wb = blockIdx.y;
   const int w = wb / B, bsi = wb - w * B;
   if (mstatus[w] != 0) return;
-  e2.load();
-  __syncthreads();
-  const BSet2Dev& bs = bsets[bsi];
   const int t = threadIdx.x, g = t / M, u = t % M;
   double2* b = fsm + g * F::SL;
-  const int nrows = bs.nrows, ts3 = 3 * bs.Ts;
-  const double fluxfac = bs.dflux1 * bs.dflux2;
-  const double* __restrict__ colinv = bs.colinv + u;
-  const double* __restrict__ collog = bs.collog + u;
-  const double* __restrict__ cflux2 = bs.rflux2 + u;
   const int kc = kcset[wb];
-  double2* Y = ybuf + (static_cast<size_t>(w) * D + bs.ds_begin) * N * nc;
-  unsigned cpos = 0, cneg = 0, czero = 0;
+  const int rbase = blockIdx.x * R::ROWS;
+  const double* R0 = rgrid + (static_cast<size_t>(wb) * N + rbase + 2 * g) * N + u;
+  double2 v[16];
 #pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    if (colinv[q * M] == 0.0) czero |= 1u << q;
-    else if (bs.colsgn[q * M + u]) cneg |= 1u << q;
-    else cpos |= 1u << q;
-  }
-  const unsigned hsm = (bs.hassign[0] ? 1u : 0u) | (bs.hassign[1] ? 2u : 0u) |
-                       (bs.hassign[2] ? 4u : 0u) | (bs.hassign[3] ? 8u : 0u);
-  double m1 = 0.0, v1 = 0.0, m2 = 0.0, v2 = 0.0, r0 = 0.0;
-  for (int gi = 0; gi < gpb; ++gi) {
-    const int rbase = (blockIdx.x * gpb + gi) * R::ROWS;
-    if (rbase >= N) break;
-    double2 v[16];
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      const int r = rbase + 2 * g + h;
-      double acc[16];
+  for (int q = 0; q < 16; ++q) v[q] = make_double2(R0[q * M], R0[N + q * M]);
+  fft2_head<N, -1>(v, b, u, TW);
 #pragma unroll
-      for (int q = 0; q < 16; ++q) acc[q] = 0.0;
-      if (r == 0) {
-        const double* e0 = row0 + static_cast<size_t>(wb) * N + u;
+  for (int pp = 0; pp < F::PP; ++pp) {
+    double2* s = b + (pp * M + u) * (M3 + 1);
+    double2 z[M3];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) acc[q] = e0[q * M];
-      } else {
-        const int sgn1 = bs.rowsgn[r];
-        if (sgn1 >= 0) {
-          const size_t ri = static_cast<size_t>(wb) * nrows + r;
-          const int2 nt = rcnt[ri];
-          const double* __restrict__ L = rw + ri * ts3;
-          double lf2[16];  // read again per row: not held through the DFT
+    for (int i = 0; i < M3; ++i) z[i] = s[i];
+    fft::dft<M3, -1>(z);
 #pragma unroll
-          for (int q = 0; q < 16; ++q) lf2[q] = collog[q * M];
-#pragma unroll 1
-          for (int fs = 0; fs < 2; ++fs) {
-            const unsigned cols = fs ? cneg : cpos;
-            if (!cols || !((hsm >> (sgn1 + fs)) & 1u)) continue;
-            const double* __restrict__ Tm = fs ? L + 3 * nt.x : L;
-            const int cnt = fs ? nt.y : nt.x;
-            if ((cols | czero) == 0xffffu) {  // every column of this sign
-              for (int k = 0; k < cnt; ++k) {
-                const double c0 = __ldg(Tm + 3 * k), c1 = __ldg(Tm + 3 * k + 1),
-                             c2 = __ldg(Tm + 3 * k + 2);
-#pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                  const double d = lf2[q] - c1;
-                  acc[q] += c0 * dev::exp2_tab(d * d * c2, e2.t);
-                }
-              }
-            } else {
-              for (int k = 0; k < cnt; ++k) {
-                const double c0 = __ldg(Tm + 3 * k), c1 = __ldg(Tm + 3 * k + 1),
-                             c2 = __ldg(Tm + 3 * k + 2);
-#pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                  if (!((cols >> q) & 1u)) continue;
-                  const double d = lf2[q] - c1;
-                  acc[q] += c0 * dev::exp2_tab(d * d * c2, e2.t);
-                }
-              }
-            }
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 16; ++q) acc[q] = acc[q] * colinv[q * M] * fluxfac;
-        if (u == 0) acc[0] = edge ? redge[static_cast<size_t>(wb) * (2 * N + 1) + N + r] * fluxfac : 0.0;
-      }
-      // moment sums of the row; the first and last column weigh a half
-      double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        double a = acc[q];
-        if ((q == 0 && u == 0) || (q == 15 && u == M - 1)) a *= 0.5;
-        const double cf = cflux2[q * M];
-        const double ca = cf * a;
-        s0 += a;
-        s1 += ca;
-        s2 += cf * ca;
-      }
-      const double wr = (r == 0 || r == N - 1) ? 0.5 : 1.0, cf1 = bs.rowflux[r];
-      s0 *= wr;
-      m1 += cf1 * s0;
-      v1 += cf1 * cf1 * s0;
-      m2 += wr * s1;
-      v2 += wr * s2;
-      // the first row waits in the thread's own slots of the exchange
-      double* keep = reinterpret_cast<double*>(b) + u;
-      if (h == 0) {
-#pragma unroll
-        for (int q = 0; q < 16; ++q) keep[q * M] = acc[q];
-      } else {
-#pragma unroll
-        for (int q = 0; q < 16; ++q) v[q] = make_double2(keep[q * M], acc[q]);
-      }
+    for (int i = 0; i < M3; ++i) {  // bins past the cut-off are not read
+      const int k = pp * M + u + 256 * i;
+      if (min(k, N - k) <= kc) s[i] = z[i];
     }
-    __syncthreads();
-    fft2_head<N, -1>(v, b, u, TW);
-#pragma unroll
-    for (int pp = 0; pp < F::PP; ++pp) {
-      double2* s = b + (pp * M + u) * (M3 + 1);
-      double2 z[M3];
-#pragma unroll
-      for (int i = 0; i < M3; ++i) z[i] = s[i];
-      fft::dft<M3, -1>(z);
-#pragma unroll
-      for (int i = 0; i < M3; ++i) s[i] = z[i];
-    }
-    __syncthreads();
-    for (int k = t; k <= kc; k += T) {
-      const int kn = (N - k) & (N - 1);
-      const int pk = (k & 255) * (M3 + 1) + (k >> 8), pn = (kn & 255) * (M3 + 1) + (kn >> 8);
-      double2* o = Y + static_cast<size_t>(k) * N + rbase;
-#pragma unroll
-      for (int gg = 0; gg < G; ++gg) {
-        const double2 a = fsm[gg * F::SL + pk], c = fsm[gg * F::SL + pn];
-        const double2 x0 = make_double2(0.5 * (a.x + c.x), 0.5 * (a.y - c.y));
-        const double2 x1 = make_double2(0.5 * (a.y + c.y), 0.5 * (c.x - a.x));
-        st32(o + 2 * gg, x0, x1);
-        if (k == 0) r0 += x0.x + x1.x;
-      }
-    }
-    __syncthreads();
   }
-  m1 = dev::block_sum<T>(m1, shr);
-  v1 = dev::block_sum<T>(v1, shr);
-  m2 = dev::block_sum<T>(m2, shr);
-  v2 = dev::block_sum<T>(v2, shr);
-  if (t == 0) {
-    double* o = rpart + (static_cast<size_t>(wb) * gridDim.x + blockIdx.x) * 5;
-    o[0] = m1; o[1] = v1; o[2] = m2; o[3] = v2; o[4] = r0;
-  }
-}
-
-// Moments, shift decisions (PDFactoryDouble.cc:560-585, 1198-1213) and the
-// DC bin R~00 from the row kernel's partials; one block per proposal and
-// beam set.
-__global__ void __launch_bounds__(NT)
-k_rmom2(const BSet2Dev* __restrict__ bsets, int B, int nparts, const int* __restrict__ mstatus,
-        const double* __restrict__ rpart, double* __restrict__ mom, double* __restrict__ r0buf) {
-  __shared__ double shr[32];
-  const int wb = blockIdx.x;
-  const int w = wb / B;
-  if (mstatus[w] != 0) return;
-  const BSet2Dev& bs = bsets[wb - w * B];
-  const double* p = rpart + static_cast<size_t>(wb) * nparts * 5;
-  double a[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int k = threadIdx.x; k < nparts; k += NT)
+  __syncthreads();
+  double2* Y = ybuf + (static_cast<size_t>(w) * D + bsets[bsi].ds_begin) * N * nc + rbase;
+  for (int k = t; k <= kc; k += T) {
+    const int kn = (N - k) & (N - 1);
+    const int pk = (k & 255) * (M3 + 1) + (k >> 8), pn = (kn & 255) * (M3 + 1) + (kn >> 8);
 #pragma unroll
-    for (int i = 0; i < 5; ++i) a[i] += p[5 * k + i];
-#pragma unroll
-  for (int i = 0; i < 5; ++i) a[i] = dev::block_sum<NT>(a[i], shr);
-  if (threadIdx.x == 0) {
-    const double s1 = sqrt(a[1]), s2 = sqrt(a[3]);
-    const bool d1 = (s1 > bs.dflux1) && (fabs(a[0]) > bs.dflux1);
-    const bool d2 = (s2 > bs.dflux2) && (fabs(a[2]) > bs.dflux2);
-    double* o = mom + static_cast<size_t>(wb) * 8;
-    o[0] = a[0]; o[1] = a[2]; o[2] = a[1]; o[3] = a[3];
-    o[4] = d1 ? -a[0] : 0.0; o[5] = d2 ? -a[2] : 0.0;
-    o[6] = d1 ? 1.0 : 0.0; o[7] = d2 ? 1.0 : 0.0;
-    r0buf[wb] = a[4];
+    for (int gg = 0; gg < G; ++gg) {
+      const double2 a = fsm[gg * F::SL + pk], c = fsm[gg * F::SL + pn];
+      st32(Y + static_cast<size_t>(k) * N + 2 * gg,
+           make_double2(0.5 * (a.x + c.x), 0.5 * (a.y - c.y)),
+           make_double2(0.5 * (a.y + c.y), 0.5 * (c.x - a.x)));
+    }
   }
 }
 
@@ -1855,13 +1779,13 @@ k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dset
 // sums of its rows in shared memory (each column of a pair's rows belongs to
 // one thread).  P(D) rows go out at pitch `pitch`.
 template <int N>
-__global__ void __launch_bounds__(RowCfg<N>::T, 512 / RowCfg<N>::T)
+__global__ void __launch_bounds__(InvCfg<N>::T, 512 / InvCfg<N>::T)
 k_rowinv2(int D, const int* __restrict__ mstatus, const int* __restrict__ kcds,
           const double2* __restrict__ ybuf, int pitch, double* __restrict__ pbuf,
           double* __restrict__ rowpart, double* __restrict__ colpart,
           const double2* __restrict__ TW) {
   using F = Fft2<N>;
-  using R = RowCfg<N>;
+  using R = InvCfg<N>;
   constexpr int M = F::M, M3 = F::M3, G = R::G, T = R::T;
   constexpr int nc = N / 2 + 1, H = N / 2;
   constexpr int WP = M / 32;  // warps per pair
@@ -2371,6 +2295,7 @@ void Engine2::build_static() {
     nq_ = static_cast<int>(kq.u.size());
   }
 
+  ck(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device_), "SM count");
   const unsigned n = n_;
   B_ = static_cast<unsigned>(sets_.size());
   h_bsets_.assign(B_, BSet2Dev{});
@@ -2523,7 +2448,7 @@ void Engine2::free_work() {
                   ws_.rpart, ws_.redge, ws_.epart, ws_.fpart, ws_.mom, ws_.pbuf, ws_.rowpart,
                   ws_.colpart, ws_.pinfo, ws_.gpart, ws_.pdout,
                   ws_.theta_in, ws_.logl, ws_.status, ws_.bonus, ws_.bcnt,
-                  ws_.bstatus, ws_.bsig, ws_.r0, ws_.row0, ws_.kcset, ws_.kcds};
+                  ws_.bstatus, ws_.bsig, ws_.r0, ws_.kcset, ws_.kcds};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (ws_.h_theta) cudaFreeHost(ws_.h_theta);
@@ -2560,16 +2485,15 @@ void Engine2::reserve(unsigned P) {
   ws_.rcnt = dal<int2>(static_cast<size_t>(P) * B_ * nrows);
   ws_.rrows = rbuf_rows();
   ws_.rbuf = dal<double>(static_cast<size_t>(P) * ws_.rrows * n * nc2);
-  ws_.row0 = dal<double>(static_cast<size_t>(P) * B_ * n);
   ws_.kcset = dal<int>(static_cast<size_t>(P) * B_);
   ws_.kcds = dal<int>(static_cast<size_t>(P) * D_);
-  ws_.rpart = dal<double>(static_cast<size_t>(P) * B_ * gx_ * gy_ * 4);
+  ws_.rpart = dal<double>(static_cast<size_t>(P) * B_ * gx_ * gy_ * 5);
   ws_.redge = dal<double>(static_cast<size_t>(P) * B_ * (2 * n + 1));
   const size_t ngr = edge_ ? (nedge_ + ER_MIN - 1) / ER_MIN : 0;
   ws_.epart = dal<double>(static_cast<size_t>(P) * B_ * (ngr ? ngr * (n + nedge_) : 1));
   ws_.mom = dal<double>(static_cast<size_t>(P) * B_ * 8);
   ws_.r0 = dal<double>(static_cast<size_t>(P) * B_);
-  ws_.fpart = dal<double>(static_cast<size_t>(P) * B_ * ((n + NT - 1) / NT) * 4);
+  ws_.fpart = dal<double>(static_cast<size_t>(P) * B_ * ((n + NT - 1) / NT) * 5);
   ws_.pbuf = dal<double>(static_cast<size_t>(P) * D_ * n * nc2);
   ws_.rowpart = dal<double>(static_cast<size_t>(P) * D_ * n * nct_);
   ws_.colpart = dal<double>(static_cast<size_t>(P) * D_ * nrt_ * n);
@@ -2589,14 +2513,15 @@ void Engine2::setup_colspec() {
   colspec_ = fft_mode_ == 1 && (n == 512 || n == 1024 || n == 2048 || n == 4096);
   if (!colspec_) return;
   if (!d_ctw_) {
-    // W_n^{u 2^i}, u < n / 16, i < 4 (the second stage's W_{n/16}^s is row 16 s)
+    // W_n^{u 2^i} at [i][u], u < n / 16, i < 4 (the second stage's W_{n/16}^s
+    // at u = 16 s)
     std::vector<double2> tw(n / 4);
     const long double tau = 6.283185307179586476925286766559005768L;
     for (unsigned u = 0; u < n / 16; ++u)
       for (unsigned i = 0; i < 4; ++i) {
         const unsigned e = (u << i) % n;
         const long double a = -tau * static_cast<long double>(e) / static_cast<long double>(n);
-        tw[4 * u + i] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
+        tw[i * (n / 16) + u] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
       }
     d_ctw_ = dal<double2>(tw.size());
     static_allocs_.push_back(d_ctw_);
@@ -2605,8 +2530,8 @@ void Engine2::setup_colspec() {
 #define POFD_ATTR2(NN)                                                                       \
   {                                                                                          \
     const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;                            \
-    ck(cudaFuncSetAttribute(k_rowfwd2<NN>, dyn, static_cast<int>(rowfwd_smem(NN))), "attr"); \
-    ck(cudaFuncSetAttribute(k_rowinv2<NN>, dyn, static_cast<int>(rowinv_smem(NN))), "attr"); \
+    ck(cudaFuncSetAttribute(k_rowfwd2<NN>, dyn, static_cast<int>(rowfwd_smem<NN>())), "attr"); \
+    ck(cudaFuncSetAttribute(k_rowinv2<NN>, dyn, static_cast<int>(rowinv_smem<NN>())), "attr"); \
     ck(cudaFuncSetAttribute(k_colspec2<NN>, dyn, static_cast<int>(colspec_smem(NN, true))),  \
        "attr");                                                                              \
     const auto pref = cudaFuncAttributePreferredSharedMemoryCarveout;                        \
@@ -2770,60 +2695,66 @@ void Engine2::launch_all(unsigned nprop, const float* theta, unsigned npar,
   {
     const unsigned nrows = static_cast<unsigned>(n + ne);
     const unsigned gxr = (nrows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK;
-    k_rows2<<<dim3(gxr, P * B), NT, 0, st>>>(d_bsets_, model_, B, 1.0 / std::log(2.),
-                                             ws_.mstatus, ws_.cnt, ws_.rw, ws_.rcnt);
+    k_rows2<<<dim3(gxr, P * B), NT, 0, st>>>(d_bsets_, model_, B, ws_.mstatus, ws_.cnt, ws_.rw, ws_.rcnt);
   }
   mark(2);
+  const int pitch = static_cast<int>(ppitch());  // of a P(D) row
+  // the R grid: in the P(D)'s place for the row and column kernels, which
+  // keep their columns in rbuf, else in rbuf at the transform's pitch
+  const bool own = colspec_ && !r_only;
+  double* rgrid = own ? ws_.pbuf : ws_.rbuf;
+  const int rpitch = own ? n : nc2;
+  // rows per block: four times the tuning's, but fewer where the batch is
+  // too small to fill the GPU several times over
+  const unsigned gxg = static_cast<unsigned>((n + RG_COLS - 1) / RG_COLS);
+  int rb = std::min(4 * tune_.rgrid_rows, ST_ROWS);
+  while (rb > 4 && static_cast<long>(P) * B * gxg * ((n - 1) / rb) < 12 * sm_count_) rb /= 2;
+  const unsigned gy = static_cast<unsigned>((n - 1 + rb - 1) / rb);
+  k_rgrid2<<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, rpitch, rb, ws_.mstatus, ws_.rw,
+                                                ws_.rcnt, rgrid, ws_.rpart);
+  mark(3);
   const int er = tune_.edge_rows;
   const int ngr = (ne + er - 1) / er;
-  auto edges = [&] {
-    if (!edge_) return;
+  if (edge_) {
     const unsigned gxe = static_cast<unsigned>((n + ne + RG_COLS - 1) / RG_COLS);
-    switch (er) {
-      case 4:
-        k_redge2<4><<<dim3(gxe, ngr, P * B), NT, 0, st>>>(d_bsets_, B, n, ne, ws_.mstatus, ws_.rw,
-                                                          ws_.rcnt, ws_.epart);
-        break;
-      case 16:
-        k_redge2<16><<<dim3(gxe, ngr, P * B), NT, 0, st>>>(d_bsets_, B, n, ne, ws_.mstatus, ws_.rw,
-                                                           ws_.rcnt, ws_.epart);
-        break;
-      default:
-        k_redge2<8><<<dim3(gxe, ngr, P * B), NT, 0, st>>>(d_bsets_, B, n, ne, ws_.mstatus, ws_.rw,
-                                                          ws_.rcnt, ws_.epart);
-    }
-    k_ry2<<<dim3((n - 1 + RY_ROWS - 1) / RY_ROWS, P * B), NT, 0, st>>>(
-        d_bsets_, B, n, ne, ws_.mstatus, ws_.rw, ws_.rcnt, ws_.redge);
-  };
-  const int pitch = static_cast<int>(ppitch());  // of a P(D) row
-  int nct = static_cast<int>(nct_), s = 2;       // marginal column tiles; stage
-  if (colspec_ && !r_only) {
-    edges();
-    k_redge0_2<<<dim3((n + NT - 1) / NT, P * B), NT, 0, st>>>(
-        d_bsets_, d_dsets_, B, D, n, edge_ ? 1 : 0, ne, ngr, ws_.mstatus, ws_.sigmult, ws_.epart,
-        ws_.row0, ws_.kcset, ws_.kcds);
-    mark(3);
-    // groups of rows per block: the tuning's rows per block, at least one
-    const int rows = rowcfg_rows(n), gpb = std::max(1, tune_.rgrid_rows / rows);
-    const int nblk = (n / rows + gpb - 1) / gpb;
+    k_redge2<<<dim3(gxe, ngr, P * B), NT, 0, st>>>(d_bsets_, B, n, ne, er, ws_.mstatus, ws_.rw,
+                                                   ws_.rcnt, ws_.epart);
+    int ry = ST_ROWS;
+    while (ry > 8 && static_cast<long>(P) * B * ((n - 1) / ry) < 6 * sm_count_) ry /= 2;
+    k_ry2<<<dim3((n - 1 + ry - 1) / ry, P * B), NT, 0, st>>>(
+        d_bsets_, B, n, ne, ry, ws_.mstatus, ws_.rw, ws_.rcnt, ws_.redge);
+  }
+  mark(4);
+  const int nfp = (n + NT - 1) / NT;
+  k_rfinish2<<<dim3(nfp, P * B), NT, 0, st>>>(d_bsets_, B, n, rpitch, edge_ ? 1 : 0, ne, ngr,
+                                              static_cast<int>(gxg * gy), ws_.mstatus,
+                                              ws_.redge, ws_.epart, ws_.rpart, rgrid, ws_.fpart);
+  k_rfinal2<<<P * B, NT, 0, st>>>(d_bsets_, B, n, rpitch, edge_ ? 1 : 0, ne, ngr, nfp,
+                                  ws_.mstatus, ws_.epart, ws_.fpart, rgrid, ws_.mom, d_dsets_, D,
+                                  ws_.sigmult, ws_.r0, ws_.kcset, ws_.kcds);
+  mark(5);
+  if (r_only) {
+    ck(cudaGetLastError(), "kernel launch");
+    return;
+  }
+  int nct = static_cast<int>(nct_), s = 9;  // marginal column tiles; stage
+  if (own) {
     double2* Y = reinterpret_cast<double2*>(ws_.rbuf);
     bool several = false;
     for (const auto& bs : h_bsets_) several = several || bs.nds > 1;
-#define POFD_ROWS2(NN)                                                                          \
-  {                                                                                             \
-    k_rowfwd2<NN><<<dim3(nblk, P * B), RowCfg<NN>::T, rowfwd_smem(NN), st>>>(                   \
-        d_bsets_, B, D, edge_ ? 1 : 0, gpb, ws_.mstatus, ws_.rw, ws_.rcnt, ws_.row0, ws_.redge, \
-        ws_.kcset, Y, ws_.rpart, d_ctw_);                                                       \
-    mark(4);                                                                                    \
-    k_rmom2<<<P * B, NT, 0, st>>>(d_bsets_, B, nblk, ws_.mstatus, ws_.rpart, ws_.mom, ws_.r0);  \
-    mark(5);                                                                                    \
-    k_colspec2<NN><<<dim3((nc + ColCfg<NN>::C - 1) / ColCfg<NN>::C, P * B), ColCfg<NN>::T,      \
-                     colspec_smem(NN, several), st>>>(d_bsets_, d_dsets_, B, D, ws_.mstatus,    \
-                                                      ws_.sigmult, ws_.mom, ws_.r0, ws_.kcset,  \
-                                                      ws_.kcds, Y, d_ctw_);                     \
-    mark(6);                                                                                    \
-    k_rowinv2<NN><<<dim3(n / RI_ROWS, P * D), RowCfg<NN>::T, rowinv_smem(NN), st>>>(            \
-        D, ws_.mstatus, ws_.kcds, Y, pitch, ws_.pbuf, ws_.rowpart, ws_.colpart, d_ctw_);        \
+#define POFD_ROWS2(NN)                                                                        \
+  {                                                                                           \
+    using R = FwdCfg<NN>;                                                                     \
+    using C = ColCfg<NN>;                                                                     \
+    k_rowfwd2<NN><<<dim3(NN / R::ROWS, P * B), R::T, rowfwd_smem<NN>(), st>>>(                \
+        d_bsets_, B, D, ws_.mstatus, rgrid, ws_.kcset, Y, d_ctw_);                            \
+    mark(6);                                                                                  \
+    k_colspec2<NN><<<dim3((nc + C::C - 1) / C::C, P * B), C::T, colspec_smem(NN, several),    \
+                     st>>>(d_bsets_, d_dsets_, B, D, ws_.mstatus, ws_.sigmult, ws_.mom,       \
+                           ws_.r0, ws_.kcset, ws_.kcds, Y, d_ctw_);                           \
+    mark(7);                                                                                  \
+    k_rowinv2<NN><<<dim3(NN / RI_ROWS, P * D), InvCfg<NN>::T, rowinv_smem<NN>(), st>>>(       \
+        D, ws_.mstatus, ws_.kcds, Y, pitch, ws_.pbuf, ws_.rowpart, ws_.colpart, d_ctw_);      \
   }
     switch (n) {
       case 512: POFD_ROWS2(512) break;
@@ -2834,39 +2765,8 @@ void Engine2::launch_all(unsigned nprop, const float* theta, unsigned npar,
     }
 #undef POFD_ROWS2
     nct = 1;
-    s = 7;
+    s = 8;
   } else {
-    const int rb = tune_.rgrid_rows;
-    const unsigned gy = static_cast<unsigned>((n - 1 + rb - 1) / rb);
-    const unsigned gxg = static_cast<unsigned>((n + RG_COLS - 1) / RG_COLS);
-    switch (rb) {
-      case 2:
-        k_rgrid2<2><<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, ws_.mstatus, ws_.rw,
-                                                         ws_.rcnt, ws_.rbuf, ws_.rpart);
-        break;
-      case 8:
-        k_rgrid2<8><<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, ws_.mstatus, ws_.rw,
-                                                         ws_.rcnt, ws_.rbuf, ws_.rpart);
-        break;
-      default:
-        k_rgrid2<4><<<dim3(gxg, gy, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, ws_.mstatus, ws_.rw,
-                                                         ws_.rcnt, ws_.rbuf, ws_.rpart);
-    }
-    mark(3);
-    edges();
-    mark(4);
-    const int nfp = (n + NT - 1) / NT;
-    k_rfinish2<<<dim3(nfp, P * B), NT, 0, st>>>(d_bsets_, B, n, nc2, edge_ ? 1 : 0, ne, ngr,
-                                                static_cast<int>(gxg * gy), ws_.mstatus,
-                                                ws_.redge, ws_.epart, ws_.rpart, ws_.rbuf,
-                                                ws_.fpart);
-    k_rfinal2<<<P * B, NT, 0, st>>>(d_bsets_, B, n, nc2, edge_ ? 1 : 0, ne, ngr, nfp,
-                                    ws_.mstatus, ws_.epart, ws_.fpart, ws_.rbuf, ws_.mom);
-    mark(5);
-    if (r_only) {
-      ck(cudaGetLastError(), "kernel launch");
-      return;
-    }
     fk(cufftSetStream(pl.fwd, st), "cufftSetStream");
     fk(cufftExecD2Z(pl.fwd, ws_.rbuf, reinterpret_cast<cufftDoubleComplex*>(ws_.rbuf)),
        "cufftExecD2Z 2D");
@@ -2881,7 +2781,6 @@ void Engine2::launch_all(unsigned nprop, const float* theta, unsigned npar,
     mark(8);
     k_pscan2<<<dim3(nct_, nrt_, P * D), NT, 0, st>>>(D, n, nc2, ws_.mstatus, ws_.pbuf,
                                                       ws_.rowpart, ws_.colpart);
-    s = 9;
   }
   mark(s);
   k_psplit2<<<P * D, SNT, 3 * static_cast<size_t>(n) * sizeof(double), st>>>(
@@ -3177,8 +3076,8 @@ const char* Engine2::stage_name(int i) {
 
 const char* Engine2::stage_name_now(int i) const {
   static const char* names[] = {
-      "k_model2", "k_rows2", "k_redge2+k_ry2+k_redge0_2", "k_rowfwd2", "k_rmom2",
-      "k_colspec2", "k_rowinv2", "k_psplit2", "k_pgather2", "k_reduce2"};
+      "k_model2", "k_rows2", "k_rgrid2", "k_redge2+k_ry2", "k_rfinish2+k_rfinal2",
+      "k_rowfwd2", "k_colspec2", "k_rowinv2", "k_psplit2", "k_pgather2", "k_reduce2"};
   if (!colspec_) return stage_name(i);
   return (i >= 0 && i < num_stages()) ? names[i] : "";
 }

@@ -99,7 +99,7 @@ struct PDInfo2 {
 // changes what is computed; the FFT mode changes the transform's rounding).
 struct Tune2 {
   int fft_mode = 1;     // see set_fft_mode
-  int rgrid_rows = 8;   // R-grid rows per block of k_rgrid2 (2, 4, 8)
+  int rgrid_rows = 8;   // R-grid rows per block of k_rgrid2 / 4 (2, 4, 8)
   int edge_rows = 16;   // band-1 edge rows per group of k_redge2 (4, 8, 16)
 };
 
@@ -144,11 +144,11 @@ class Engine2 {
   void profile_stages(unsigned nprop, const float* theta, unsigned npar,
                       int reps, double* stage_ms);
   static const char* stage_name(int i);
-  int num_stages() const { return colspec_ ? 10 : kNumStages; }
+  int num_stages() const { return colspec_ ? 11 : kNumStages; }
   // the stage names of the FFT mode in use
   const char* stage_name_now(int i) const;
   int kernels_per_eval() const {
-    return (edge_ ? 12 : 10) + (prior_.needs_bonus() ? 1 : 0) +
+    return (edge_ ? 12 : 10) + (colspec_ ? 1 : 0) + (prior_.needs_bonus() ? 1 : 0) +
            (refsum_ ? 1 : 0);
   }
   // Reference-order normalisation and means (k_pseq2 after the split
@@ -249,6 +249,7 @@ class Engine2 {
   std::vector<DSet2Dev> h_dsets_;
   unsigned B_ = 0, D_ = 0;
   int Tmax_ = 1;
+  int sm_count_ = 148;
   unsigned gx_ = 0, gy_ = 0;      // R grid blocks (columns, row groups)
   unsigned nrt_ = 0, nct_ = 0;    // P(D) row / column tiles
   unsigned gchunks_ = 1;          // gather chunks per dataset
@@ -282,17 +283,16 @@ class Engine2 {
                                 // (FFT mode 0), or the columns [P][D][nc][n]
                                 // of the transforms (mode 1)
     unsigned rrows = 0;         // rbuf_rows() it was made for
-    double* row0 = nullptr;     // [P][B][n] edge cells of row 0 (mode 1)
     int* kcset = nullptr;       // [P][B] noise cut-off columns (mode 1)
     int* kcds = nullptr;        // [P][D]
-    double* rpart = nullptr;    // [P][B][gy][gx][4]
+    double* rpart = nullptr;    // [P][B][gy][gx][5]
     double* redge = nullptr;    // [P][B][2n+1]: Ry at [n, 2n)
     double* epart = nullptr;    // [P][B][edge row groups][n + nedge]
     double* mom = nullptr;      // [P][B][8]
     double* r0 = nullptr;       // [P][B] R~00 (FFT mode 1)
-    double* fpart = nullptr;    // [P][B][n/256][4] edge-cell moment partials
+    double* fpart = nullptr;    // [P][B][n/256][5] edge-cell moment partials
     double* pbuf = nullptr;     // [P][D][n][2nc] spectrum and P(D) (mode 0);
-                                // P(D) at pitch n (mode 1)
+                                // R grid, then P(D), at pitch n (mode 1)
     double* rowpart = nullptr;  // [P][D][n][nct]
     double* colpart = nullptr;  // [P][D][nrt][n]
     PDInfo2* pinfo = nullptr;   // [P][D]
