@@ -40,6 +40,7 @@ constexpr int CHUNK = NT * 16;    // P(D) elements per reduction block
 constexpr int kSplineThreads = 1024;  // threads per node-spline block
 constexpr int KMAX = Engine1::KMAX;
 constexpr int MAXTERMS = 4096;    // beam terms held in shared memory
+constexpr double kThird = 1.0 / 3.0;
 
 void cuda_check(cudaError_t e, const char* what) {
   if (e != cudaSuccess) {
@@ -118,61 +119,98 @@ __device__ int model_solve(const Model1Dev& m, const float* __restrict__ th,
   return POFD_OK;
 }
 
-// Knot spline of every proposal: one block per proposal, thread 0 solving
-// in shared memory.  Publishes the model status and the sigma multiplier.
-__global__ void k_model1(Model1Dev m, const float* __restrict__ theta,
-                         int npar, double logfac, double* __restrict__ cnt,
-                         int* __restrict__ mstatus,
-                         double* __restrict__ sigmult) {
-  __shared__ double wk[8 * KMAX];
-  __shared__ double cs[4 * KMAX];
-  const int w = blockIdx.x;
-  const float* th = theta + static_cast<size_t>(w) * npar;
-  if (threadIdx.x == 0) {
-    const int st = model_solve(m, th, logfac, cs, wk);
-    mstatus[w] = st;
-    sigmult[w] = static_cast<double>(th[m.K]);
+// The same by one warp against the host-factored system (the matrix depends
+// only on the knot positions): the right-hand side and the coefficients by
+// lane, the two substitutions, K - 2 dependent steps each, by every lane
+// alike.  y and c: shared, KMAX each.  Returns the status.
+__device__ int model_solve_warp(const Model1Dev& m, const float* __restrict__ th, double logfac,
+                                double* __restrict__ y, double* __restrict__ c,
+                                double* __restrict__ out) {
+  const int K = m.K, N = K - 2, lane = threadIdx.x & 31;
+  bool bad = false;
+  for (int k = lane; k < K; k += 32) {
+    y[k] = logfac * static_cast<double>(th[k]);
+    bad = bad || isnan(y[k]);
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 4 * (m.K - 1); i += blockDim.x)
-    cnt[static_cast<size_t>(w) * 4 * KMAX + i] = cs[i];
+  if (__any_sync(0xffffffffu, bad)) return POFD_E_INVALID_MODEL;
+  __syncwarp();
+  for (int i = lane; i < N; i += 32)
+    c[1 + i] = 3.0 * ((y[i + 2] - y[i + 1]) * m.ih[i + 1] - (y[i + 1] - y[i]) * m.ih[i]);
+  __syncwarp();
+  if (lane == 0) {
+    for (int i = 1; i < N; ++i) c[1 + i] = c[1 + i] - m.gamma[i - 1] * c[i];
+    c[0] = 0.0;
+    c[K - 1] = 0.0;
+    c[N] = c[N] * m.ialpha[N - 1];
+    for (int i = N - 2; i >= 0; --i) c[1 + i] = c[1 + i] * m.ialpha[i] - m.gamma[i] * c[2 + i];
+  }
+  __syncwarp();
+  for (int i = lane; i < K - 1; i += 32) {
+    const double dx = m.logknots[i + 1] - m.logknots[i];
+    const double dy = y[i + 1] - y[i];
+    out[4 * i + 0] = y[i];
+    out[4 * i + 1] = dy * m.ih[i] - dx * (c[i + 1] + 2.0 * c[i]) / 3.0;
+    out[4 * i + 2] = c[i];
+    out[4 * i + 3] = (c[i + 1] - c[i]) * m.ih[i] / 3.0;
+  }
+  return POFD_OK;
 }
 
 // R at the interpolation nodes, one node per thread, terms summed in the
 // beam's order (numberCountsKnotsSpline.cc:495-526).  log2(x * ieta) is
 // formed as log2|x| + log2(ieta) from host-computed logs; the range test uses
-// the product itself, as the reference does.
+// the product itself, as the reference does.  Every block solves the
+// proposal's knot spline for itself in its first warp while the others bring
+// in the beam (a launch of its own cost 3 us and thread-serial divisions);
+// the proposal's first block publishes it with the status and the sigma
+// multiplier.  The terms go four at a time, so that the reads of their knot
+// intervals, one dependent read per term before, overlap.
 __global__ void k_rnodes1(const BSet1Dev* __restrict__ bsets, Model1Dev m,
                           int B, int NI, int maxterms,
-                          const double* __restrict__ cnt,
-                          const int* __restrict__ mstatus,
+                          const float* __restrict__ theta, int npar, double logfac,
+                          double* __restrict__ cnt, int* __restrict__ mstatus,
+                          double* __restrict__ sigmult,
                           double* __restrict__ nodes) {
   extern __shared__ double sm[];
+  __shared__ double my[KMAX], mc[KMAX];
+  __shared__ int s_st;
   const int row = blockIdx.y;  // (w*B + b)*2 + side
   const int side = row & 1;
   const int wb = row >> 1;
   const int w = wb / B, b = wb - w * B;
   const BSet1Dev& bs = bsets[b];
   const Side1Dev& sd = bs.side[side];
-  if (!sd.nodes || mstatus[w] != 0) return;
+  const bool publish = blockIdx.x == 0 && b == 0 && side == 0;
+  if (!sd.nodes && !publish) return;
   const int K = m.K;
   double* s_lk = sm;
   double* s_cs = s_lk + KMAX;
   double* s_w = s_cs + 4 * KMAX;
   double* s_le = s_w + maxterms;
-  double* s_ie = s_le + maxterms;
-  const double* cs = cnt + static_cast<size_t>(w) * 4 * KMAX;
+  const float* th = theta + static_cast<size_t>(w) * npar;
+  if (threadIdx.x < 32) {
+    const int st = model_solve_warp(m, th, logfac, my, mc, s_cs);
+    if (threadIdx.x == 0) s_st = st;
+  }
   for (int i = threadIdx.x; i < K; i += blockDim.x) s_lk[i] = m.logknots[i];
-  for (int i = threadIdx.x; i < 4 * (K - 1); i += blockDim.x) s_cs[i] = cs[i];
-  const int nt = sd.nterms;
+  const int nt = sd.nodes ? sd.nterms : 0;
   for (int i = threadIdx.x; i < nt; i += blockDim.x) {
-    s_w[i] = sd.w[i];
+    s_w[i] = sd.w[i] * sd.ieta[i];
     s_le[i] = sd.lie[i];
-    s_ie[i] = sd.ieta[i];
   }
   __shared__ dev::Exp2Table e2;
   e2.load();
   __syncthreads();
+  if (publish) {
+    if (threadIdx.x == 0) {
+      mstatus[w] = s_st;
+      sigmult[w] = static_cast<double>(th[K]);
+    }
+    if (s_st == 0)
+      for (int i = threadIdx.x; i < 4 * (K - 1); i += blockDim.x)
+        cnt[static_cast<size_t>(w) * 4 * KMAX + i] = s_cs[i];
+  }
+  if (s_st != 0 || !sd.nodes) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= NI) return;
   const double f = sd.x[i];
@@ -186,14 +224,25 @@ __global__ void k_rnodes1(const BSet1Dev* __restrict__ bsets, Model1Dev m,
     // terms outside the node's first-to-last in-range span are not visited
     const unsigned char* __restrict__ kt = sd.kidx + i;
     const int2 jr = sd.jrange[i];
-    for (int j = jr.x; j < jr.y; ++j) {
-      const int k = kt[static_cast<size_t>(j) * NI];
-      if (k == 255) continue;
-      const double delx = (lf + s_le[j]) - s_lk[k];
-      const double* q = s_cs + 4 * k;
-      const double cts =
-          dev::exp2_tab(q[0] + delx * (q[1] + delx * (q[2] + delx * q[3])), e2.t);
-      if (cts > 0) workval += s_w[j] * cts * s_ie[j];
+    constexpr int U = 4;
+    for (int j0 = jr.x; j0 < jr.y; j0 += U) {
+      int kk[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        kk[u] = (j0 + u < jr.y) ? kt[static_cast<size_t>(j0 + u) * NI] : 255;
+      double v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool in = kk[u] != 255;
+        const int k = in ? kk[u] : 0, j = in ? j0 + u : jr.x;
+        const double delx = (lf + s_le[j]) - s_lk[k];
+        const double* q = s_cs + 4 * k;
+        const double cts =
+            dev::exp2_tab(q[0] + delx * (q[1] + delx * (q[2] + delx * q[3])), e2.t);
+        v[u] = (in && cts > 0) ? s_w[j] * cts : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) workval += v[u];
     }
   }
   nodes[static_cast<size_t>(row) * NI + i] = bs.prefac * workval;
@@ -229,7 +278,7 @@ k_rspline1(const BSet1Dev* __restrict__ bsets, int B, int NI,
   const int s0 = threadIdx.x * E;
   const int s1 = min(s0 + E, N);
   const double* ih = sd.ih;
-  const double* al = sd.alpha;
+  const double* ial = sd.ialpha;
   const double* ga = sd.gamma;
   // forward: z_i = g_i - gamma_{i-1} z_{i-1}, z_0 = g_0; stored in c[1+i]
   double A = 1.0, Bv = 0.0;
@@ -247,7 +296,7 @@ k_rspline1(const BSet1Dev* __restrict__ bsets, int B, int NI,
     for (int i = s0; i < s1; ++i) {
       const double gi = c[1 + i];
       z = (i == 0) ? gi : gi - ga[i - 1] * z;
-      c[1 + i] = z / al[i];  // cc_i
+      c[1 + i] = z * ial[i];  // cc_i
     }
   }
   __syncthreads();
@@ -279,8 +328,8 @@ k_rspline1(const BSet1Dev* __restrict__ bsets, int B, int NI,
   for (int i = threadIdx.x; i < NI - 1; i += RT) {
     const double dx = x[i + 1] - x[i];
     const double dy = y[i + 1] - y[i];
-    out[2 * i] = make_double2(y[i], (dy / dx) - dx * (c[i + 1] + 2.0 * c[i]) / 3.0);
-    out[2 * i + 1] = make_double2(c[i], (c[i + 1] - c[i]) / (3.0 * dx));
+    out[2 * i] = make_double2(y[i], dy * ih[i] - dx * (c[i + 1] + 2.0 * c[i]) * kThird);
+    out[2 * i + 1] = make_double2(c[i], (c[i + 1] - c[i]) * ih[i] * kThird);
   }
 }
 
@@ -1890,6 +1939,15 @@ void Engine1::build_static() {
   model_.minknot = knots_.front();
   model_.maxknot = knots_.back();
   {
+    SplineSystem ks;
+    ks.factor(lk);
+    std::vector<double> ia(ks.alpha);
+    for (double& v : ia) v = 1.0 / v;
+    model_.ih = up(ks.ih);
+    model_.ialpha = up(ia);
+    model_.gamma = up(ks.gamma);
+  }
+  {
     // 64 panels of 20 points per knot interval
     KnotQuadrature kq;
     kq.build(lk.data(), static_cast<int>(K), 64, 20);
@@ -2019,7 +2077,11 @@ void Engine1::build_static() {
       sd.ieta = up(tie);
       sd.x = up(sys.x);
       sd.ih = up(sys.ih);
-      sd.alpha = up(sys.alpha);
+      {
+        std::vector<double> ia(sys.alpha);
+        for (double& v : ia) v = 1.0 / v;
+        sd.ialpha = up(ia);
+      }
       sd.gamma = up(sys.gamma);
       // grid ranges (PDFactory.cc:563-606)
       if (side == 0 && maxflux > 0) {
@@ -2353,15 +2415,15 @@ void Engine1::autotune(unsigned nprop, const float* theta, unsigned npar, int re
 
 const char* Engine1::stage_name(int i) const {
   static const char* lib[kNumStages] = {
-      "k_model1+k_rnodes1", "k_rspline1", "k_rfill1", "k_moments1",
+      "k_rnodes1", "k_rspline1", "k_rfill1", "k_moments1",
       "cufft_d2z", "k_spectrum1", "cufft_z2d", "k_pscan1", "k_pfinish1",
       "k_reduce1"};
   static const char* own[kNumStages] = {
-      "k_model1+k_rnodes1", "k_rspline1", "k_rfill1", "k_moments1",
+      "k_rnodes1", "k_rspline1", "k_rfill1", "k_moments1",
       "k_fftA1+k_fftB1", "k_spectrum1f", "k_fftA1+k_fftB1_inv", "k_pscan1", "k_pfinish1",
       "k_reduce1"};
   static const char* fused[kNumStages] = {
-      "k_model1+k_rnodes1", "k_rspline1", "k_fftAR1", "k_moments1",
+      "k_rnodes1", "k_rspline1", "k_fftAR1", "k_moments1",
       "k_fftB1", "k_spectrum1f", "k_fftA1+k_fftB1_inv", "k_pscan1", "k_pfinish1",
       "k_reduce1"};
   if (i < 0 || i >= kNumStages) return "";
@@ -2520,7 +2582,7 @@ void Engine1::reserve(unsigned P) {
   ws_.logl = dalloc<double>(P + (P + 1) / 2);
   ws_.status = reinterpret_cast<int*>(ws_.logl + P);
   cuda_check(cudaFuncSetAttribute(k_rnodes1, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>((KMAX + 4 * KMAX + 3 * MAXTERMS) * sizeof(double))),
+                                  static_cast<int>((KMAX + 4 * KMAX + 2 * MAXTERMS) * sizeof(double))),
              "smem attribute");
   cuda_check(cudaFuncSetAttribute(k_rspline1<kSplineThreads>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2566,19 +2628,18 @@ void Engine1::launch_all(unsigned nprop, const float* theta, unsigned npar,
   Plans& pl = plans_.at(nprop);
 
   mark(0);
-  k_model1<<<P, 32, 0, st>>>(model_, theta, static_cast<int>(npar), std::log2(10.0),
-                             ws_.cnt, ws_.mstatus, ws_.sigmult);
+  {
+    const size_t smem = (KMAX + 4 * KMAX + 2 * static_cast<size_t>(maxterms_)) * sizeof(double);
+    const int th = tune_.rnodes_threads;
+    dim3 grid((NI + th - 1) / th, P * B * 2);
+    k_rnodes1<<<grid, th, smem, st>>>(d_bsets_, model_, B, NI, maxterms_, theta,
+                                      static_cast<int>(npar), std::log2(10.0), ws_.cnt,
+                                      ws_.mstatus, ws_.sigmult, ws_.nodes);
+  }
   if (prior_.needs_bonus())
     k_bonus1<<<P, kBonusThreads, 0, st>>>(model_, const_cast<float*>(theta), static_cast<int>(npar),
                                           std::log2(10.0), ws_.cnt, ws_.mstatus, d_qu_, d_qs_,
                                           d_qw_, qper_, ws_.bonus, -1);
-  {
-    const size_t smem = (KMAX + 4 * KMAX + 3 * static_cast<size_t>(maxterms_)) * sizeof(double);
-    const int th = tune_.rnodes_threads;
-    dim3 grid((NI + th - 1) / th, P * B * 2);
-    k_rnodes1<<<grid, th, smem, st>>>(d_bsets_, model_, B, NI, maxterms_,
-                                      ws_.cnt, ws_.mstatus, ws_.nodes);
-  }
   mark(1);
   {
     const size_t smem = (2 * static_cast<size_t>(NI) + 64) * sizeof(double);
@@ -2868,11 +2929,10 @@ void Engine1::rgrid_host(int bs, const float* theta, unsigned npar, double* out)
   const int NI = static_cast<int>(ninterp_), n = static_cast<int>(n_);
   const int nc2 = 2 * (n / 2 + 1);
   const int B = static_cast<int>(B_);
-  k_model1<<<1, 32, 0, stream_>>>(model_, ws_.theta_in, static_cast<int>(npar),
-                                  std::log2(10.0), ws_.cnt, ws_.mstatus, ws_.sigmult);
   k_rnodes1<<<dim3((NI + 127) / 128, B * 2), 128,
-              (KMAX + 4 * KMAX + 3 * static_cast<size_t>(maxterms_)) * sizeof(double), stream_>>>(
-      d_bsets_, model_, B, NI, maxterms_, ws_.cnt, ws_.mstatus, ws_.nodes);
+              (KMAX + 4 * KMAX + 2 * static_cast<size_t>(maxterms_)) * sizeof(double), stream_>>>(
+      d_bsets_, model_, B, NI, maxterms_, ws_.theta_in, static_cast<int>(npar), std::log2(10.0),
+      ws_.cnt, ws_.mstatus, ws_.sigmult, ws_.nodes);
   k_rspline1<kSplineThreads><<<B * 2, kSplineThreads, (2 * static_cast<size_t>(NI) + 64) * sizeof(double), stream_>>>(
       d_bsets_, B, NI, ws_.mstatus, ws_.nodes, ws_.spl);
   launch_rfill(tune_.rfill_per, tune_.rfill_mode >= 2, dim3(ntile_, B), stream_, d_bsets_, B, n,

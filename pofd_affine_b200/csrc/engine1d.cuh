@@ -31,7 +31,7 @@ struct Side1Dev {
   const double* ieta;
   const double* x;      // ninterp node fluxes
   const double* ih;     // 1/(x[i+1]-x[i])
-  const double* alpha;  // LDL^T diagonal (ninterp-2)
+  const double* ialpha; // 1 / LDL^T diagonal (ninterp-2)
   const double* gamma;  // LDL^T sub-diagonal ratio (ninterp-2)
   const double* lxa;    // log2|x| of the nodes
   const double* lie;    // log2 of the inverse beam terms
@@ -78,6 +78,9 @@ struct DSet1Dev {
 struct Model1Dev {
   int K;
   const double* logknots;  // log2 knot positions
+  const double* ih;        // their spline system: 1 / spacing (K - 1)
+  const double* ialpha;    // and its factors, as Side1Dev's (K - 2)
+  const double* gamma;
   double minknot, maxknot;
 };
 
@@ -187,7 +190,7 @@ class Engine1 {
                    double* x_out, double* r_out);
   void rgrid_host(int bs, const float* theta, unsigned npar, double* out);
   int kernels_per_eval() const {
-    return (own_fft_ ? (fused_fill() ? 12 : 13) : 9) + (prior_.needs_bonus() ? 1 : 0);
+    return (own_fft_ ? (fused_fill() ? 11 : 12) : 8) + (prior_.needs_bonus() ? 1 : 0);
   }
   // the R grid fill runs inside the forward FFT pass A (own FFT, plain passes)
   bool fused_fill() const {
