@@ -521,7 +521,7 @@ int pofd_like1_profile(pofd_like1* L, unsigned nprop, const float* theta,
     need(reps > 0, "reps must be > 0");
     cudaSetDevice(L->ctx->device);
     L->eng->profile_stages(nprop, theta, npar, reps, stage_ms);
-    *nstages = pofd::Engine1::kNumStages;
+    *nstages = L->eng->num_stages();
     return POFD_OK;
   });
 }
@@ -533,6 +533,7 @@ const char* pofd_like1_stage_name(const pofd_like1* L, int i) {
 int pofd_like1_set_fft(pofd_like1* L, int mode) {
   return guard([&] {
     need(L != nullptr, "null argument");
+    need(mode == 0 || mode == 1, "fft mode must be 0 (own) or 1 (cuFFT)");
     L->eng->set_fft_mode(mode);
     return POFD_OK;
   });

@@ -19,7 +19,36 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Programmatic dependent launch: the kernel may start while its predecessor
+// on the stream (or in the captured graph) still runs, and waits for its
+// results with dev::pdl_wait() before touching them.
+template <class... KArgs, class... Args>
+inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                       cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 namespace dev {
+
+// Waits until every kernel this one was launched to overlap has finished and
+// its writes are visible (returns at once where there is none).  Pointers to
+// such writes must not be const __restrict__: the compiler takes loads
+// through those as invariant and may move them ahead of the wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel on the stream start its prologue.
+__device__ __forceinline__ void pdl_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 constexpr double kTwoPi = 6.283185307179586476925286766559005768394;
 constexpr double kSmallLogVal = -30.0;

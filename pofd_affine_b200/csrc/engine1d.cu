@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "fft1d.cuh"
+#include "fft2.cuh"
 
 namespace pofd {
 
@@ -164,13 +165,19 @@ __device__ int model_solve_warp(const Model1Dev& m, const float* __restrict__ th
 // in the beam (a launch of its own cost 3 us and thread-serial divisions);
 // the proposal's first block publishes it with the status and the sigma
 // multiplier.  The terms go four at a time, so that the reads of their knot
-// intervals, one dependent read per term before, overlap.
+// intervals, one dependent read per term before, overlap.  LN lanes share a
+// node, each every LN-th group of its terms: a node has up to half the
+// beam's terms, and with few rows their chain is what the kernel waits for
+// (LN = 4); with many rows it is throughput (LN = 1).  nodes: log2 R,
+// which the node spline goes through (PDFactory.cc:466-474); rout (may be
+// null): R itself.
+template <int LN>
 __global__ void k_rnodes1(const BSet1Dev* __restrict__ bsets, Model1Dev m,
                           int B, int NI, int maxterms,
                           const float* __restrict__ theta, int npar, double logfac,
                           double* __restrict__ cnt, int* __restrict__ mstatus,
                           double* __restrict__ sigmult,
-                          double* __restrict__ nodes) {
+                          double* __restrict__ nodes, double* __restrict__ rout) {
   extern __shared__ double sm[];
   __shared__ double my[KMAX], mc[KMAX];
   __shared__ int s_st;
@@ -181,6 +188,7 @@ __global__ void k_rnodes1(const BSet1Dev* __restrict__ bsets, Model1Dev m,
   const BSet1Dev& bs = bsets[b];
   const Side1Dev& sd = bs.side[side];
   const bool publish = blockIdx.x == 0 && b == 0 && side == 0;
+  dev::pdl_launch();
   if (!sd.nodes && !publish) return;
   const int K = m.K;
   double* s_lk = sm;
@@ -211,41 +219,48 @@ __global__ void k_rnodes1(const BSet1Dev* __restrict__ bsets, Model1Dev m,
         cnt[static_cast<size_t>(w) * 4 * KMAX + i] = s_cs[i];
   }
   if (s_st != 0 || !sd.nodes) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= NI) return;
-  const double f = sd.x[i];
-  const double lf = sd.lxa[i];
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = id / LN, ln = id % LN;
   double workval = 0.0;
-  const bool posb = (f > 0 && bs.haspos && f <= bs.rr_hi);
-  const bool negb = !posb && (bs.hasneg && f < 0 && f >= bs.rr_lo);
-  if (posb || negb) {
-    // the knot interval and the range test of every term at this node come
-    // from the host-built table (the reference searches them per call);
-    // terms outside the node's first-to-last in-range span are not visited
-    const unsigned char* __restrict__ kt = sd.kidx + i;
-    const int2 jr = sd.jrange[i];
-    constexpr int U = 4;
-    for (int j0 = jr.x; j0 < jr.y; j0 += U) {
-      int kk[U];
+  if (i < NI) {
+    const double f = sd.x[i];
+    const double lf = sd.lxa[i];
+    const bool posb = (f > 0 && bs.haspos && f <= bs.rr_hi);
+    const bool negb = !posb && (bs.hasneg && f < 0 && f >= bs.rr_lo);
+    if (posb || negb) {
+      // the knot interval and the range test of every term at this node come
+      // from the host-built table (the reference searches them per call);
+      // terms outside the node's first-to-last in-range span are not visited
+      const unsigned char* __restrict__ kt = sd.kidx + i;
+      const int2 jr = sd.jrange[i];
+      constexpr int U = 4;
+      for (int j0 = jr.x + ln * U; j0 < jr.y; j0 += U * LN) {
+        int kk[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        kk[u] = (j0 + u < jr.y) ? kt[static_cast<size_t>(j0 + u) * NI] : 255;
-      double v[U];
+        for (int u = 0; u < U; ++u)
+          kk[u] = (j0 + u < jr.y) ? kt[static_cast<size_t>(j0 + u) * NI] : 255;
+        double v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const bool in = kk[u] != 255;
-        const int k = in ? kk[u] : 0, j = in ? j0 + u : jr.x;
-        const double delx = (lf + s_le[j]) - s_lk[k];
-        const double* q = s_cs + 4 * k;
-        const double cts =
-            dev::exp2_tab(q[0] + delx * (q[1] + delx * (q[2] + delx * q[3])), e2.t);
-        v[u] = (in && cts > 0) ? s_w[j] * cts : 0.0;
+        for (int u = 0; u < U; ++u) {
+          const bool in = kk[u] != 255;
+          const int k = in ? kk[u] : 0, j = in ? j0 + u : jr.x;
+          const double delx = (lf + s_le[j]) - s_lk[k];
+          const double* q = s_cs + 4 * k;
+          const double cts =
+              dev::exp2_tab(q[0] + delx * (q[1] + delx * (q[2] + delx * q[3])), e2.t);
+          v[u] = (in && cts > 0) ? s_w[j] * cts : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) workval += v[u];
       }
-#pragma unroll
-      for (int u = 0; u < U; ++u) workval += v[u];
     }
   }
-  nodes[static_cast<size_t>(row) * NI + i] = bs.prefac * workval;
+#pragma unroll
+  for (int o = 1; o < LN; o <<= 1) workval += __shfl_xor_sync(0xffffffffu, workval, o);
+  if (i >= NI || ln != 0) return;
+  const double R = bs.prefac * workval;
+  nodes[static_cast<size_t>(row) * NI + i] = (R > 0) ? log2(R) : dev::kSmallLogVal;
+  if (rout) rout[static_cast<size_t>(row) * NI + i] = R;
 }
 
 // Natural cubic spline through (x_i, log2 R_i) over the NI nodes: RHS of
@@ -268,10 +283,7 @@ k_rspline1(const BSet1Dev* __restrict__ bsets, int B, int NI,
   double* c = y + NI;         // NI (full second-derivative/2 array)
   double* scr = c + NI;       // 64
   const double* R = nodes + static_cast<size_t>(row) * NI;
-  for (int i = threadIdx.x; i < NI; i += RT) {
-    const double v = R[i];
-    y[i] = (v > 0) ? log2(v) : dev::kSmallLogVal;
-  }
+  for (int i = threadIdx.x; i < NI; i += RT) y[i] = R[i];
   __syncthreads();
   const int N = NI - 2;
   const int E = (N + RT - 1) / RT;
@@ -338,84 +350,74 @@ k_rspline1(const BSet1Dev* __restrict__ bsets, int B, int NI,
 // second flux moments (PDFactory.cc:634-665).  The node interval of every
 // grid point is parameter-independent and comes from a host-built table
 // (gidx, -1 outside the covered ranges).
-struct GridFill1 {
+struct Fill1 {
   double dflux, minflux_R, off0, off1;
-  int wrap, NI;
-  const double* __restrict__ x0;
-  const double* __restrict__ x1;
-  const double* __restrict__ S0;   // this row's node spline [2][NI][4]
+  int wrap;
   const double* __restrict__ e2;   // exp2 table in shared memory
+  // the node spline on one interval: left node, (y, b), (c, d)
+  struct Coef {
+    double x;
+    double2 yb, cd;
+  };
 
-  __device__ __forceinline__ GridFill1(const BSet1Dev& bs, const double* spl_row, int ni,
-                                       const double* tab)
+  __device__ __forceinline__ Fill1(const BSet1Dev& bs, const double* tab)
       : dflux(bs.dflux), minflux_R(bs.minflux_R), off0(bs.side[0].grid_off),
-        off1(bs.side[1].grid_off), wrap(bs.wrapRidx), NI(ni), x0(bs.side[0].x),
-        x1(bs.side[1].x), S0(spl_row), e2(tab) {}
+        off1(bs.side[1].grid_off), wrap(bs.wrapRidx), e2(tab) {}
 
-  // R at grid index i (di = i as a double) with node interval q (< 0: not
-  // covered), and its moment terms added to mn, var: weight 0 at i = 0 (its
-  // flux is 0), 1/2 at the positive edge, 1 elsewhere
-  __device__ __forceinline__ double point(int i, double di, int q, double& mn,
-                                          double& var) const {
-    const bool neg = i > wrap;
-    const double pd = __dmul_rn(di, dflux);
-    double r = 0.0;
-    if (q >= 0) {
-      const double cflux = __dadd_rn(pd, neg ? off1 : off0);
-      const double2* S = reinterpret_cast<const double2*>(S0 + (neg ? 4 * NI : 0)) + 2 * q;
-      const double2 yb = S[0], cd = S[1];
-      const double delx = cflux - (neg ? x1 : x0)[q];
-      const double v = yb.x + delx * (yb.y + delx * (cd.x + delx * cd.y));
-      r = dev::exp2_tab(v, e2) * dflux;
-    }
-    const double cf = neg ? static_cast<double>(i - wrap - 1) * dflux + minflux_R : pd;
+  // R at a covered grid index i
+  __device__ __forceinline__ double value(const Coef& c, int i) const {
+    const double cflux = __dadd_rn(__dmul_rn(static_cast<double>(i), dflux), i > wrap ? off1 : off0);
+    const double delx = cflux - c.x;
+    return dev::exp2_tab(c.yb.x + delx * (c.yb.y + delx * (c.cd.x + delx * c.cd.y)), e2) * dflux;
+  }
+  // the moment terms of R = r at grid index i added to mn, var: weight 0 at
+  // i = 0 (its flux is 0), 1/2 at the positive edge, 1 elsewhere
+  __device__ __forceinline__ void moments(int i, double r, double& mn, double& var) const {
+    const double cf = (i > wrap) ? static_cast<double>(i - wrap - 1) * dflux + minflux_R
+                                 : __dmul_rn(static_cast<double>(i), dflux);
     double prod = cf * r;
     if (i == wrap) prod *= 0.5;
     mn += prod;
     var += cf * prod;
-    return r;
   }
 
-  // R at the len (<= 16) consecutive grid indices of one run (i0, q) --
-  // points of one covered node interval q on one side of the wrap -- into
-  // the shared tile at out[pad(o + k)], with their moment terms.  The cubic
-  // exponent v(t) of point i0 + t has constant third differences, so 2^v
-  // follows from three running products: R(t+1) = R(t) E1(t), E1(t+1) =
-  // E1(t) E2(t), E2(t+1) = E2(t) E3, with E1(0) = 2^(v(1) - v(0)), E2(0) =
-  // 2^(second difference), E3 = 2^(third difference), the differences taken
-  // analytically from the cubic: four exp2 per run instead of one per
-  // point, and no per-point cubic or table lookup.  The products add at
-  // most ~16^3/6 roundings (< 1e-13 relative) to each value.  A run whose
+  // R at the len (<= 16) consecutive grid indices from i0 -- points of one
+  // covered node interval on one side of the wrap -- into the shared tile at
+  // out[pad(o + k)], with their moment terms.  The cubic exponent v(t) of
+  // point i0 + t has constant third differences, so 2^v follows from three
+  // running products: R(t+1) = R(t) E1(t), E1(t+1) = E1(t) E2(t), E2(t+1) =
+  // E2(t) E3, with E1(0) = 2^(v(1) - v(0)), E2(0) = 2^(second difference),
+  // E3 = 2^(third difference), the differences taken analytically from the
+  // cubic: four exp2 per run instead of one per point, and no per-point
+  // cubic or table lookup.  The products add at most ~16^3/6 roundings
+  // (< 1e-13 relative) to each value.  The grid index is carried as a
+  // double, since a conversion costs four times an addition.  A run whose
   // exponents leave the safe range goes point by point.
-  __device__ __forceinline__ void run_products(int i0, int len, int q, double* out, int o,
-                                               double& mn, double& var) const {
+  __device__ __forceinline__ void run(const Coef& c, int i0, int len, double* out, int o,
+                                      double& mn, double& var) const {
     const bool neg = i0 > wrap;
-    const double2* S = reinterpret_cast<const double2*>(S0 + (neg ? 4 * NI : 0)) + 2 * q;
-    const double2 yb = S[0], cd = S[1];
     const double h = dflux;
-    const double d0 = __dadd_rn(__dmul_rn(static_cast<double>(i0), dflux), neg ? off1 : off0) -
-                      (neg ? x1 : x0)[q];
-    const double v0 = yb.x + d0 * (yb.y + d0 * (cd.x + d0 * cd.y));
-    const double D1 = h * (yb.y + cd.x * (2.0 * d0 + h) + cd.y * (3.0 * d0 * (d0 + h) + h * h));
-    const double D2 = h * h * (2.0 * cd.x + 6.0 * cd.y * (d0 + h));
-    const double D3 = 6.0 * cd.y * h * h * h;
+    const double d0 = __dadd_rn(__dmul_rn(static_cast<double>(i0), dflux), neg ? off1 : off0) - c.x;
+    const double v0 = c.yb.x + d0 * (c.yb.y + d0 * (c.cd.x + d0 * c.cd.y));
+    const double D1 = h * (c.yb.y + c.cd.x * (2.0 * d0 + h) + c.cd.y * (3.0 * d0 * (d0 + h) + h * h));
+    const double D2 = h * h * (2.0 * c.cd.x + 6.0 * c.cd.y * (d0 + h));
+    const double D3 = 6.0 * c.cd.y * h * h * h;
     if (fabs(v0) < 500.0 && fabs(D1) < 16.0 && fabs(D2) < 4.0 && fabs(D3) < 2.0) {
       double R = dev::exp2_tab(v0, e2) * dflux;
       double E1 = dev::exp2_tab(D1, e2), E2 = dev::exp2_tab(D2, e2);
       const double E3 = dev::exp2_tab(D3, e2);
       const double cb = neg ? minflux_R : 0.0;
-      const int ib = neg ? wrap + 1 : 0;
+      double di = static_cast<double>(neg ? i0 - wrap - 1 : i0);
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
         if (k >= len) break;
-        const int i = i0 + k;
         out[pad(o + k)] = R;
-        const double cf = neg ? static_cast<double>(i - ib) * dflux + cb
-                              : __dmul_rn(static_cast<double>(i), dflux);
+        const double cf = fma(di, dflux, cb);
         double prod = cf * R;
-        if (i == wrap) prod *= 0.5;
+        if (i0 + k == wrap) prod *= 0.5;
         mn += prod;
         var += cf * prod;
+        di += 1.0;
         R *= E1;
         E1 *= E2;
         E2 *= E3;
@@ -423,13 +425,60 @@ struct GridFill1 {
       return;
     }
     for (int k = 0; k < len; ++k) {
-      const int i = i0 + k;
-      out[pad(o + k)] = point(i, static_cast<double>(i), q, mn, var);
+      const double r = value(c, i0 + k);
+      out[pad(o + k)] = r;
+      moments(i0 + k, r, mn, var);
     }
   }
   // shared tile index of span offset j: one pad word per 16 values, so that
   // threads starting runs ~16 values apart do not share a bank
   __device__ __forceinline__ static int pad(int j) { return j + (j >> 4); }
+};
+
+// The fill from the node-spline records in global memory.
+struct GridFill1 : Fill1 {
+  int NI;
+  const double* __restrict__ x0;
+  const double* __restrict__ x1;
+  const double* __restrict__ S0;   // this row's node spline [2][NI][4]
+
+  __device__ __forceinline__ GridFill1(const BSet1Dev& bs, const double* spl_row, int ni,
+                                       const double* tab)
+      : Fill1(bs, tab), NI(ni), x0(bs.side[0].x), x1(bs.side[1].x), S0(spl_row) {}
+
+  __device__ __forceinline__ Coef coef(int q, bool neg) const {
+    const double2* S = reinterpret_cast<const double2*>(S0 + (neg ? 4 * NI : 0)) + 2 * q;
+    return Coef{(neg ? x1 : x0)[q], S[0], S[1]};
+  }
+  // R at grid index i with node interval q (< 0: not covered), and its
+  // moment terms
+  __device__ __forceinline__ double point(int i, int q, double& mn, double& var) const {
+    const double r = (q >= 0) ? value(coef(q, i > wrap), i) : 0.0;
+    moments(i, r, mn, var);
+    return r;
+  }
+};
+
+// The fill from a side's node values and second derivatives in shared
+// memory (padded by row1_pad), as the single-block kernel holds them.
+__host__ __device__ constexpr int row1_pad(int i) { return i + (i >> 3); }
+struct RowFill1 : Fill1 {
+  const double* __restrict__ x;
+  const double* __restrict__ ih;
+  const double* y;
+  const double* c;
+
+  __device__ __forceinline__ RowFill1(const BSet1Dev& bs, const Side1Dev& sd, const double* yc,
+                                      int ni, const double* tab)
+      : Fill1(bs, tab), x(sd.x), ih(sd.ih), y(yc), c(yc + row1_pad(ni) + 1) {}
+
+  __device__ __forceinline__ Coef coef(int q) const { return coef(q, x[q], x[q + 1] - x[q], ih[q]); }
+  __device__ __forceinline__ Coef coef(int q, double x0, double dx, double i) const {
+    const double y0 = y[row1_pad(q)], c0 = c[row1_pad(q)], c1 = c[row1_pad(q + 1)];
+    return Coef{x0,
+                make_double2(y0, (y[row1_pad(q + 1)] - y0) * i - dx * (c1 + 2.0 * c0) * kThird),
+                make_double2(c0, (c1 - c0) * i * kThird)};
+  }
 };
 
 // The R grid materialised (cuFFT path, and the own path when the fill is
@@ -463,7 +512,7 @@ k_rfill1(const BSet1Dev* __restrict__ bsets, int B, int n, int NI,
   for (int k = 0; k < PER; ++k) {
     const int i = base + k * NT;
     if (q[k] == -2) break;
-    R[i] = rg.point(i, static_cast<double>(i), q[k], mn, var);
+    R[i] = rg.point(i, q[k], mn, var);
   }
   mn = dev::block_sum<NT>(mn, shr);
   var = dev::block_sum<NT>(var, shr);
@@ -479,7 +528,7 @@ k_rfill1(const BSet1Dev* __restrict__ bsets, int B, int n, int NI,
 // consecutive points that share one node interval and one side of the wrap
 // (bs.runs: x = first index, y = (q + 1) << 8 | len << 2 | kind; kind 0:
 // uncovered, R = 0; 1: shorter than four points, evaluated point by point;
-// 2: running products, GridFill1::run_products).  Block k takes runs
+// 2: running products, Fill1::run).  Block k takes runs
 // [k NT, k NT + NT) of its row -- one per thread, so no thread's run crosses
 // an interval and warps do not diverge on interval changes -- stages their
 // contiguous span of the grid (at most 16 NT values) in shared memory and
@@ -512,11 +561,11 @@ k_rfill1_run(const BSet1Dev* __restrict__ bsets, int B, int NI, int nc2, int nti
       const int len = (d.y >> 2) & 31, kind = d.y & 3, q = (d.y >> 8) - 1;
       const int o = d.x - span0;
       if (kind == 2) {
-        rg.run_products(d.x, len, q, tile, o, mn, var);
+        rg.run(rg.coef(q, d.x > rg.wrap), d.x, len, tile, o, mn, var);
       } else if (kind == 1) {
         for (int k = 0; k < len; ++k) {
           const int i = d.x + k;
-          tile[GridFill1::pad(o + k)] = rg.point(i, static_cast<double>(i), q, mn, var);
+          tile[GridFill1::pad(o + k)] = rg.point(i, q, mn, var);
         }
       } else {
         for (int k = 0; k < len; ++k) tile[GridFill1::pad(o + k)] = 0.0;
@@ -826,11 +875,11 @@ k_fftAR(const BSet1Dev* __restrict__ bsets, int B, int NI, int rowsz,
         const int len = (d.y >> 2) & 31, kind = d.y & 3, q = (d.y >> 8) - 1;
         const int o = (d.x >> 9) * (2 * CB) + (d.x & 511) - 2 * b0;
         if (kind == 2) {
-          rg.run_products(d.x, len, q, stage, o, mn, var);
+          rg.run(rg.coef(q, d.x > rg.wrap), d.x, len, stage, o, mn, var);
         } else if (kind == 1) {
           for (int e = 0; e < len; ++e) {
             const int i = d.x + e;
-            stage[GridFill1::pad(o + e)] = rg.point(i, static_cast<double>(i), q, mn, var);
+            stage[GridFill1::pad(o + e)] = rg.point(i, q, mn, var);
           }
         } else {
           for (int e = 0; e < len; ++e) stage[GridFill1::pad(o + e)] = 0.0;
@@ -852,9 +901,8 @@ k_fftAR(const BSet1Dev* __restrict__ bsets, int B, int NI, int rowsz,
       for (int n1 = 0; n1 < L1; ++n1) {
         const int i = 2 * ((L2 * n1 + n2) * M2 + b0 + b);
         const int2 q = __ldg(reinterpret_cast<const int2*>(gidx + i));
-        const double di = static_cast<double>(i);
-        const double r0 = rg.point(i, di, q.x, mn, var);
-        const double r1 = rg.point(i + 1, di + 1.0, q.y, mn, var);
+        const double r0 = rg.point(i, q.x, mn, var);
+        const double r1 = rg.point(i + 1, q.y, mn, var);
         if (i == iw) Rrow[i] = r0;
         if (i + 1 == iw) Rrow[i + 1] = r1;
         v[n1] = make_double2(r0, r1);
@@ -1203,48 +1251,35 @@ __device__ __forceinline__ double logp_at(const double* __restrict__ p, int n,
   return (v > 0.0) ? log2(v) : dev::kSmallLogVal;
 }
 
+// What the split search needs of a row's clipped values.
+struct RowMin1 {
+  double peak, minval;  // largest value; smallest inside the search window
+  int minidx;
+};
+
 // Split point, unwrap, normalisation, mean and the log-likelihood of one
 // (proposal, dataset): PDFactory.cc:691-1009, PD.cc:146-274, 557-677,
-// calcLike.cc:419-425.
-__global__ void __launch_bounds__(NT)
-k_pfinish1(const BSet1Dev* __restrict__ bsets,
-           const DSet1Dev* __restrict__ dsets, int B, int D, int n, int nc2,
-           int nchunk, double log2toe, const int* __restrict__ mstatus,
-           const double* __restrict__ sigmult, const double* __restrict__ mom,
-           const double* __restrict__ pbuf, const double* __restrict__ ppart,
-           const int* __restrict__ pmidx, PDInfo1* __restrict__ pinfo) {
-  __shared__ double shd[32];
+// calcLike.cc:419-425.  p: the wrapped P(D) row in global or shared memory;
+// sums(split, S, W, T) gives the sum and the index-weighted sum of the row
+// and the sum below the split, to every thread.  rs: thread 0's is used.
+template <int NTH, class Sums>
+__device__ __forceinline__ void finish_row(const BSet1Dev& bs, const DSet1Dev& ds,
+                                           const SplitParams& sp, const double* p, int n,
+                                           const RowMin1& rs, double log2toe, double* shd,
+                                           PDInfo1& info, Sums sums) {
   __shared__ int shi[32];
   __shared__ int s_state;   // 0 need search, 1 done, <0 error
   __shared__ int s_split;
   __shared__ double s_jitter;
-  const int wd = blockIdx.x;
-  const int w = wd / D, d = wd - w * D;
-  PDInfo1& info = pinfo[wd];
-  if (mstatus[w] != 0) {
-    if (threadIdx.x == 0) info.status = mstatus[w];
-    return;
-  }
-  const DSet1Dev& ds = dsets[d];
-  const BSet1Dev& bs = bsets[ds.bs];
-  const double var = mom[(static_cast<size_t>(w) * B + ds.bs) * 4 + 1];
-  const SplitParams sp = split_params(bs, var, sigmult[w] * ds.sigma_base);
-  const double* p = pbuf + static_cast<size_t>(wd) * nc2;
   const double dflux = bs.dflux;
-  const double* pp = ppart + static_cast<size_t>(wd) * nchunk * 4;
-  const int* pm = pmidx + static_cast<size_t>(wd) * nchunk;
-
   if (threadIdx.x == 0) {
     int st = 0;
     int split = -1;
     double jitter = 0.0;
-    const double fluxrange = n * dflux;
-    double peak = -1.0e308, minval = 1.0e308;
-    int minidx = 0x7fffffff;
-    for (int c = 0; c < nchunk; ++c) {
-      if (pp[4 * c] > peak) peak = pp[4 * c];
-      dev::argmin_merge(minval, minidx, pp[4 * c + 3], pm[c]);
-    }
+    const double fluxrange = n * bs.dflux;
+    const double peak = rs.peak;
+    double minval = rs.minval;
+    int minidx = rs.minidx;
     const long long botidx = sp.botidx, topidx = sp.topidx;
     if (sp.sgpos <= 0 || sp.sgneg <= 0) st = POFD_E_SPLIT_RANGE;
     else if (fluxrange < (sp.n1sigpos + sp.n1signeg)) st = POFD_E_SPLIT_RANGE;
@@ -1313,20 +1348,20 @@ k_pfinish1(const BSet1Dev* __restrict__ bsets,
     // first hit of the element-by-element search
     const double jitter = s_jitter;
     int found = -1;
-    for (long long top = sp.topidx - 1; top >= sp.botidx; top -= NT * kSearchPer) {
+    for (long long top = sp.topidx - 1; top >= sp.botidx; top -= NTH * kSearchPer) {
       double pv[kSearchPer];
 #pragma unroll
       for (int k = 0; k < kSearchPer; ++k) {
-        const long long i = top - threadIdx.x - static_cast<long long>(NT) * k;
+        const long long i = top - threadIdx.x - static_cast<long long>(NTH) * k;
         pv[k] = (i >= sp.botidx) ? p[i] : 1.0e308;
       }
       int hit = -1;
 #pragma unroll
       for (int k = kSearchPer - 1; k >= 0; --k) {
-        const long long i = top - threadIdx.x - static_cast<long long>(NT) * k;
+        const long long i = top - threadIdx.x - static_cast<long long>(NTH) * k;
         if (i >= sp.botidx && clip0(pv[k]) < jitter) hit = static_cast<int>(i);
       }
-      const int m = dev::block_max_int<NT>(hit, shi);
+      const int m = dev::block_max_int<NTH>(hit, shi);
       if (m >= 0) { found = m; break; }
     }
     if (found >= 0) { state = 1; if (threadIdx.x == 0) s_split = found + 1; }
@@ -1341,18 +1376,8 @@ k_pfinish1(const BSet1Dev* __restrict__ bsets,
     return;
   }
   const int split = s_split;
-  // Sum below the split: whole chunks from the partials, the rest read.
-  const int cfull = split / CHUNK;
-  double part = 0.0;
-  for (int i = cfull * CHUNK + threadIdx.x; i < split; i += NT) part += clip0(p[i]);
-  part = dev::block_sum<NT>(part, shd);
-  double S = 0.0, W = 0.0, T = 0.0;
-  for (int c = 0; c < nchunk; ++c) {
-    S += pp[4 * c + 1];
-    W += static_cast<double>(c) * CHUNK * pp[4 * c + 1] + pp[4 * c + 2];
-    if (c < cfull) T += pp[4 * c + 1];
-  }
-  T += part;
+  double S, W, T;  // sum, index-weighted sum, sum below the split
+  sums(split, S, W, T);
   const double q0 = clip0(p[split]);
   const double qlast = clip0(p[split == 0 ? n - 1 : split - 1]);
   const double tot = (S - 0.5 * q0 - 0.5 * qlast) * dflux;
@@ -1368,40 +1393,37 @@ k_pfinish1(const BSet1Dev* __restrict__ bsets,
   const double maxflux = minflux + static_cast<double>(n - 1) * dflux;
   const double maxfluxval = maxflux - dflux;
   const double idflux = 1.0 / dflux;
+  // several bins or pixels at a time: their reads, and the logarithms, overlap
   double ll = 0.0;
-  if (ds.binned) {
-    for (int e = threadIdx.x; e < ds.nnz; e += NT) {
-      const double cnt = ds.nzcnt[e];
-      const double cflux = ds.bincent0 + static_cast<double>(ds.nzidx[e]) * ds.bindelta;
-      double v;
-      if (cflux < minflux) v = cnt * logp_at(p, n, split, itot, 0);
-      else if (cflux > maxfluxval) v = cnt * logp_at(p, n, split, itot, n - 1);
-      else {
-        const double delt = (cflux - minflux) * idflux;
-        const int idx = static_cast<int>(delt);
-        const double t = delt - static_cast<double>(idx);
-        v = ((1.0 - t) * logp_at(p, n, split, itot, idx) +
-             t * logp_at(p, n, split, itot, idx + 1)) * cnt;
-      }
-      ll += v;
+  constexpr int U = NTH > 256 ? 2 : 4;
+  for (int e0 = threadIdx.x; e0 < ds.nnz; e0 += U * NTH) {
+    double cnt[U], cflux[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = min(e0 + u * NTH, ds.nnz - 1);
+      cnt[u] = ds.binned ? ds.nzcnt[e] : 1.0;
+      cflux[u] = ds.binned ? ds.bincent0 + static_cast<double>(ds.nzidx[e]) * ds.bindelta
+                           : ds.flux[e];
     }
-  } else {
-    for (int e = threadIdx.x; e < ds.nnz; e += NT) {
-      const double cflux = ds.flux[e];
-      double v;
-      if (cflux <= minflux) v = logp_at(p, n, split, itot, 0);
-      else if (cflux >= maxfluxval) v = logp_at(p, n, split, itot, n - 1);
-      else {
-        const double delt = (cflux - minflux) * idflux;
-        const int idx = static_cast<int>(delt);
-        const double t = delt - static_cast<double>(idx);
-        v = (1.0 - t) * logp_at(p, n, split, itot, idx) +
-            t * logp_at(p, n, split, itot, idx + 1);
-      }
-      ll += v;
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      // outside the grid its end values (the unbinned form includes the edge
+      // values themselves)
+      const bool lo = ds.binned ? cflux[u] < minflux : cflux[u] <= minflux;
+      const bool hi = ds.binned ? cflux[u] > maxfluxval : cflux[u] >= maxfluxval;
+      const double delt = (cflux[u] - minflux) * idflux;
+      const int idx = lo ? 0 : (hi ? n - 1 : static_cast<int>(delt));
+      const double t = delt - static_cast<double>(idx);
+      const double a = logp_at(p, n, split, itot, idx);
+      const double b = logp_at(p, n, split, itot, (lo || hi) ? idx : idx + 1);
+      v[u] = (lo || hi) ? a : (1.0 - t) * a + t * b;
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (e0 + u * NTH < ds.nnz) ll += ds.binned ? v[u] * cnt[u] : v[u];
   }
-  ll = dev::block_sum<NT>(ll, shd);
+  ll = dev::block_sum<NTH>(ll, shd);
   if (threadIdx.x == 0) {
     info.status = 0;
     info.split = split;
@@ -1413,23 +1435,60 @@ k_pfinish1(const BSet1Dev* __restrict__ bsets,
   }
 }
 
+// finish_row on a row in global memory, from the chunk reductions of
+// k_pscan1; one block per (proposal, dataset).
+__global__ void __launch_bounds__(NT)
+k_pfinish1(const BSet1Dev* __restrict__ bsets,
+           const DSet1Dev* __restrict__ dsets, int B, int D, int n, int nc2,
+           int nchunk, double log2toe, const int* __restrict__ mstatus,
+           const double* __restrict__ sigmult, const double* __restrict__ mom,
+           const double* __restrict__ pbuf, const double* __restrict__ ppart,
+           const int* __restrict__ pmidx, PDInfo1* __restrict__ pinfo) {
+  __shared__ double shd[32];
+  const int wd = blockIdx.x;
+  const int w = wd / D, d = wd - w * D;
+  PDInfo1& info = pinfo[wd];
+  if (mstatus[w] != 0) {
+    if (threadIdx.x == 0) info.status = mstatus[w];
+    return;
+  }
+  const DSet1Dev& ds = dsets[d];
+  const BSet1Dev& bs = bsets[ds.bs];
+  const double var = mom[(static_cast<size_t>(w) * B + ds.bs) * 4 + 1];
+  const SplitParams sp = split_params(bs, var, sigmult[w] * ds.sigma_base);
+  const double* p = pbuf + static_cast<size_t>(wd) * nc2;
+  const double* pp = ppart + static_cast<size_t>(wd) * nchunk * 4;
+  const int* pm = pmidx + static_cast<size_t>(wd) * nchunk;
+  RowMin1 rs{-1.0e308, 1.0e308, 0x7fffffff};
+  if (threadIdx.x == 0)
+    for (int c = 0; c < nchunk; ++c) {
+      if (pp[4 * c] > rs.peak) rs.peak = pp[4 * c];
+      dev::argmin_merge(rs.minval, rs.minidx, pp[4 * c + 3], pm[c]);
+    }
+  finish_row<NT>(bs, ds, sp, p, n, rs, log2toe, shd, info,
+                 [&](int split, double& S, double& W, double& T) {
+                   // whole chunks below the split from the partials, the rest read
+                   const int cfull = split / CHUNK;
+                   double part = 0.0;
+                   for (int i = cfull * CHUNK + threadIdx.x; i < split; i += NT) part += clip0(p[i]);
+                   part = dev::block_sum<NT>(part, shd);
+                   S = W = T = 0.0;
+                   for (int c = 0; c < nchunk; ++c) {
+                     S += pp[4 * c + 1];
+                     W += static_cast<double>(c) * CHUNK * pp[4 * c + 1] + pp[4 * c + 2];
+                     if (c < cfull) T += pp[4 * c + 1];
+                   }
+                   T += part;
+                 });
+}
+
 // Per-proposal sum over beam sets and datasets in the reference's order;
 // a negative sigma multiplier gives bad_like for the beam set
 // (calcLike.cc:404, 916-920).
-__global__ void k_reduce1(const BSet1Dev* __restrict__ bsets, int B, int D,
-                          int nprop, const int* __restrict__ mstatus,
-                          const double* __restrict__ sigmult,
-                          const PDInfo1* __restrict__ pinfo, Prior1 pr,
-                          const double* __restrict__ bonus,
-                          double* __restrict__ logl, int* __restrict__ status) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= nprop) return;
-  if (mstatus[w] != 0) {
-    logl[w] = __longlong_as_double(0x7ff8000000000000LL);
-    status[w] = mstatus[w];
-    return;
-  }
-  const double sm = sigmult[w];
+__device__ __forceinline__ void reduce_one(const BSet1Dev* __restrict__ bsets, int B, int D,
+                                           int w, double sm, const PDInfo1* pinfo,
+                                           const Prior1& pr, const double* __restrict__ bonus,
+                                           double* __restrict__ logl, int* __restrict__ status) {
   double LogLike = 0.0;
   int st = 0;
   for (int b = 0; b < B; ++b) {
@@ -1460,6 +1519,416 @@ __global__ void k_reduce1(const BSet1Dev* __restrict__ bsets, int B, int D,
   if (pr.alpha > 0.0) LogLike += pr.alpha * bonus[4 * static_cast<size_t>(w) + 2];
   status[w] = st;
   logl[w] = (st == 0) ? LogLike : __longlong_as_double(0x7ff8000000000000LL);
+}
+
+__global__ void k_reduce1(const BSet1Dev* __restrict__ bsets, int B, int D,
+                          int nprop, const int* __restrict__ mstatus,
+                          const double* __restrict__ sigmult,
+                          const PDInfo1* __restrict__ pinfo, Prior1 pr,
+                          const double* __restrict__ bonus,
+                          double* __restrict__ logl, int* __restrict__ status) {
+  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= nprop) return;
+  if (mstatus[w] != 0) {
+    logl[w] = __longlong_as_double(0x7ff8000000000000LL);
+    status[w] = mstatus[w];
+    return;
+  }
+  reduce_one(bsets, B, D, w, sigmult[w], pinfo, pr, bonus, logl, status);
+}
+
+// ------------------------------------------------------------------
+// Small grids (n = 2m, m a power of two in [512, 4096], up to ROW1_MAXNI
+// nodes): one block takes a (proposal, beam set) row from the R nodes to the
+// log-likelihood of its datasets -- node spline, R grid, forward transform,
+// spectrum, inverse transform, split search, normalisation and gather --
+// without leaving shared memory.  As separate kernels (with cuFFT) these are
+// nine launches of 2-6 us each for rows of 32-64 KB.  Bound by latency: a
+// dozen barriers and the transforms' exchanges on one SM.  Launched to
+// overlap the nodes kernel's end: what that kernel (or the bonus kernel)
+// writes comes through pointers without __restrict__, since the compiler may
+// move a load it takes for invariant ahead of the wait.
+constexpr int RU = 3;  // runs per thread whose static data is read ahead
+constexpr int ROW1_MAXN = 8192;
+constexpr int ROW1_MAXNI = 4096;
+constexpr int ROW1_MAXDS = 64;  // datasets per beam set
+
+struct Row1Mem {  // sizes in doubles of the block's shared memory regions
+  int a, b, d;
+  int several;    // P(D) in d, where b keeps the spectrum for the next dataset
+};
+inline Row1Mem row1_mem(int n, int ni, bool several) {
+  const int m = n / 2, pn = row1_pad(ni) + 1;
+  Row1Mem r;
+  r.a = 2 * 256 * (m / 256 + 1);              // transform slots; R grid padded
+  r.b = std::max(2 * pn, 2 * (m + 1));        // spline y, c; then the spectrum; P(D)
+  r.d = std::max(2 * pn, several ? n : 0);    // spline factors; P(D)
+  r.several = several ? 1 : 0;
+  return r;
+}
+inline size_t row1_smem(const Row1Mem& r) {
+  return static_cast<size_t>(r.a + r.b + r.d) * sizeof(double);
+}
+
+template <int M2, int T>
+__global__ void __launch_bounds__(T, 512 / T)
+k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, int B, int D,
+       int NI, Row1Mem mem, double log2toe, const int* mstatus,
+       const double* sigmult, const double* nodes,
+       const double2* __restrict__ Wn, const double2* __restrict__ TW, double* __restrict__ mom,
+       double* __restrict__ pbuf, PDInfo1* __restrict__ pinfo, Prior1 pr,
+       const double* bonus, double* __restrict__ logl, int* __restrict__ status) {
+  using F = fft::Fft2<M2>;
+  constexpr int M = F::M, M3 = F::M3, n = 2 * M2, m = M2;
+  constexpr int nc2 = 2 * (n / 2 + 1);
+  extern __shared__ double rs[];
+  double* A = rs;
+  double* Bm = A + mem.a;
+  double* Dm = Bm + mem.b;
+  double2* z = reinterpret_cast<double2*>(A);
+  __shared__ double scr[64];
+  __shared__ double red[4][T / 32];
+  __shared__ int redi[T / 32], s_kc[ROW1_MAXDS];
+  __shared__ dev::Exp2Table e2;
+  const int wb = blockIdx.x;
+  const int w = wb / B, b = wb - w * B;
+  const int t = threadIdx.x;
+  const BSet1Dev& bs = bsets[b];
+  // what does not depend on the nodes kernel, before waiting for it: the
+  // exp2 table, and of the thread's first runs the descriptors and nodes
+  e2.load();
+  int2 rd[RU];
+  double rx[RU], rdx[RU], rih[RU];
+#pragma unroll
+  for (int k = 0; k < RU; ++k) {
+    const int r = t + k * T;
+    rd[k] = (r < bs.nruns) ? __ldg(&bs.runs[r]) : make_int2(0, 0);
+  }
+#pragma unroll
+  for (int k = 0; k < RU; ++k) {
+    const int q = (rd[k].y >> 8) - 1;
+    rx[k] = rdx[k] = rih[k] = 0.0;
+    if (q >= 0) {
+      const Side1Dev& sd = bs.side[rd[k].x > bs.wrapRidx ? 1 : 0];
+      rx[k] = sd.x[q];
+      rdx[k] = sd.x[q + 1];
+      rih[k] = sd.ih[q];
+    }
+  }
+  dev::pdl_wait();
+  const int st0 = mstatus[w];
+  if (st0 != 0) {
+    for (int dd = t; dd < bs.nds; dd += T) pinfo[static_cast<size_t>(w) * D + bs.ds_begin + dd].status = st0;
+    if (B == 1 && t == 0) {
+      logl[w] = __longlong_as_double(0x7ff8000000000000LL);
+      status[w] = st0;
+    }
+    return;
+  }
+  const double dflux = bs.dflux;
+  const int wrap = bs.wrapRidx;
+  const double sm = sigmult[w];
+  if (t < bs.nds) s_kc[t] = noise_cut(sm * dsets[bs.ds_begin + t].sigma_base, dflux, n);
+  double mn = 0.0, var = 0.0;
+  for (int side = 0; side < 2; ++side) {
+    const Side1Dev& sd = bs.side[side];
+    if (sd.nodes) {
+      // ---- natural spline through (x, log2 R): k_rspline1's steps
+      double* y = Bm;
+      double* c = Bm + row1_pad(NI) + 1;
+      double* gam = Dm;
+      double* ial = Dm + row1_pad(NI) + 1;
+      const double* R = nodes + (static_cast<size_t>(wb) * 2 + side) * NI;
+      const int N = NI - 2;
+#pragma unroll 4
+      for (int i = t; i < NI; i += T) {
+        const int k = min(i, N - 1);
+        const double v = R[i], ga = sd.gamma[k], ia = sd.ialpha[k];
+        y[row1_pad(i)] = v;
+        gam[row1_pad(k)] = ga;
+        ial[row1_pad(k)] = ia;
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int i = t; i < N; i += T) {
+        const double h0 = sd.ih[i], h1 = sd.ih[i + 1];
+        const double y1 = y[row1_pad(i + 1)];
+        c[row1_pad(i + 1)] = 3.0 * ((y[row1_pad(i + 2)] - y1) * h1 - (y1 - y[row1_pad(i)]) * h0);
+      }
+      __syncthreads();
+      const int E = (N + T - 1) / T;
+      const int s0 = t * E, s1 = min(s0 + E, N);
+      double Am = 1.0, Bv = 0.0;
+      for (int i = s0; i < s1; ++i) {
+        const double a = (i == 0) ? 0.0 : -gam[row1_pad(i - 1)];
+        Bv = a * Bv + c[row1_pad(i + 1)];
+        Am = a * Am;
+      }
+      {
+        double zz = dev::block_affine_scan_w<T>(Am, Bv, scr);
+        for (int i = s0; i < s1; ++i) {
+          const double g = c[row1_pad(i + 1)];
+          zz = (i == 0) ? g : g - gam[row1_pad(i - 1)] * zz;
+          c[row1_pad(i + 1)] = zz * ial[row1_pad(i)];
+        }
+      }
+      __syncthreads();
+      Am = 1.0;
+      Bv = 0.0;
+      for (int i = s1 - 1; i >= s0; --i) {
+        const double a = (i == N - 1) ? 0.0 : -gam[row1_pad(i)];
+        Bv = a * Bv + c[row1_pad(i + 1)];
+        Am = a * Am;
+      }
+      {
+        double cn = dev::block_affine_rscan_w<T>(Am, Bv, scr);
+        for (int i = s1 - 1; i >= s0; --i) {
+          const double cc = c[row1_pad(i + 1)];
+          cn = (i == N - 1) ? cc : cc - gam[row1_pad(i)] * cn;
+          c[row1_pad(i + 1)] = cn;
+        }
+      }
+      if (t == 0) {
+        c[0] = 0.0;
+        c[row1_pad(NI - 1)] = 0.0;
+      }
+      __syncthreads();
+    }
+    // ---- the side's part of the R grid by running products over the static
+    // runs, padded, with the moment partials; uncovered points with side 0
+    const RowFill1 rf(bs, sd, Bm, NI, e2.t);
+    auto fill = [&](int2 d, auto coef) {
+      const int len = (d.y >> 2) & 31, kind = d.y & 3;
+      if (kind == 0) {
+        if (side == 0)
+          for (int k = 0; k < len; ++k) A[Fill1::pad(d.x + k)] = 0.0;
+        return;
+      }
+      if ((d.x > wrap) != (side == 1)) return;
+      const Fill1::Coef cf = coef();
+      if (kind == 2) {
+        rf.run(cf, d.x, len, A, d.x, mn, var);
+      } else {
+        for (int k = 0; k < len; ++k) {
+          const double r = rf.value(cf, d.x + k);
+          A[Fill1::pad(d.x + k)] = r;
+          rf.moments(d.x + k, r, mn, var);
+        }
+      }
+    };
+#pragma unroll
+    for (int k = 0; k < RU; ++k)
+      fill(rd[k], [&] { return rf.coef((rd[k].y >> 8) - 1, rx[k], rdx[k] - rx[k], rih[k]); });
+    for (int r = t + RU * T; r < bs.nruns; r += T) {
+      const int2 d = __ldg(&bs.runs[r]);
+      fill(d, [&] { return rf.coef((d.y >> 8) - 1); });
+    }
+    __syncthreads();
+  }
+  // ---- moments and the shift (k_moments1)
+  for (int o = 16; o > 0; o >>= 1) {
+    mn += __shfl_xor_sync(0xffffffffu, mn, o);
+    var += __shfl_xor_sync(0xffffffffu, var, o);
+  }
+  if ((t & 31) == 0) {
+    red[0][t >> 5] = mn;
+    red[1][t >> 5] = var;
+  }
+  __syncthreads();
+  mn = red[0][0];
+  var = red[1][0];
+#pragma unroll
+  for (int k = 1; k < T / 32; ++k) {
+    mn += red[0][k];
+    var += red[1][k];
+  }
+  if (wrap < n - 1) {
+    const double cf = bs.minflux_R;
+    const double prod = 0.5 * cf * A[Fill1::pad(wrap - 1)];
+    mn -= prod;
+    var -= cf * prod;
+  }
+  const bool doshift = (sqrt(var) > dflux) && (fabs(mn) > dflux);
+  if (t == 0) {
+    double* o = mom + static_cast<size_t>(wb) * 4;
+    o[0] = mn;
+    o[1] = var;
+    o[2] = doshift ? -mn : 0.0;
+    o[3] = doshift ? 1.0 : 0.0;
+  }
+  int kcmax = 0;
+  for (int dd = 0; dd < bs.nds; ++dd) kcmax = max(kcmax, s_kc[dd]);
+  const int qmax = min(m / 2, kcmax);
+  // ---- forward transform of z_j = R_2j + i R_2j+1
+  const bool act = t < M;
+  double2 v[16];
+  if (act) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const int i = 2 * (k * M + t);
+      v[k] = make_double2(A[Fill1::pad(i)], A[Fill1::pad(i + 1)]);
+    }
+    fft::fft2_sync<M2>(1);
+    fft::fft2_head<M2, -1>(v, z, t, TW, 1);
+#pragma unroll
+    for (int pp = 0; pp < F::PP; ++pp) {
+      double2* s = z + (pp * M + t) * (M3 + 1);
+      double2 u[M3];
+#pragma unroll
+      for (int i = 0; i < M3; ++i) u[i] = s[i];
+      fft::dft<M3, -1>(u);
+#pragma unroll
+      for (int i = 0; i < M3; ++i) s[i] = u[i];
+    }
+  }
+  __syncthreads();
+  // ---- spectrum on pairs (q, m - q), before the noise
+  const double iflux = dev::kTwoPi / (static_cast<double>(n) * dflux);
+  const double shiftw = doshift ? -mn * iflux : 0.0;
+  double2* S = reinterpret_cast<double2*>(Bm);
+  auto slot = [](int k) { return (k & 255) * (M3 + 1) + (k >> 8); };
+  {
+    const double2 z0 = z[0];
+    const double r0 = z0.x + z0.y;  // X_0
+    for (int q = t; q <= qmax; q += T) {
+      const int kb = m - q;
+      double2 Xa, Xb;
+      if (q == 0) {
+        Xa = make_double2(r0, 0.0);
+        Xb = make_double2(z0.x - z0.y, 0.0);  // X_m
+      } else {
+        const double2 a = z[slot(q)], c = z[slot(kb)];
+        const double2 Ea = make_double2(0.5 * (a.x + c.x), 0.5 * (a.y - c.y));
+        const double2 Oa = make_double2(0.5 * (a.y + c.y), -0.5 * (a.x - c.x));
+        const double2 Eb = make_double2(Ea.x, -Ea.y);
+        const double2 Ob = make_double2(0.5 * (c.y + a.y), -0.5 * (c.x - a.x));
+        Xa = fft::cadd(Ea, fft::cmul(__ldg(Wn + q), Oa));
+        Xb = fft::cadd(Eb, fft::cmul(__ldg(Wn + kb), Ob));
+      }
+      S[q] = spec_p(Xa, r0, q, m, doshift, shiftw);
+      // the pair's other bin lies past every cut-off unless nothing is cut
+      S[kb] = (kb <= kcmax) ? spec_p(Xb, r0, kb, m, doshift, shiftw) : make_double2(0.0, 0.0);
+    }
+  }
+  __syncthreads();
+  double* P = mem.several ? Dm : Bm;
+  for (int dd = 0; dd < bs.nds; ++dd) {
+    const int d = bs.ds_begin + dd;
+    const double sigma = sm * dsets[d].sigma_base;
+    const int kc = s_kc[dd];
+    const double sigfac = -0.5 * sigma * sigma;
+    // ---- noise and the merge of the inverse real transform (k_spectrum1f)
+    for (int q = t; q <= min(m / 2, kc); q += T) {
+      const int kb = m - q;
+      double2 Pa = S[q], Pb = S[kb];
+      if (sigma > 0) {
+        if (q > 0) {
+          const double wv = iflux * q;
+          const double ef = exp(sigfac * wv * wv);
+          Pa = make_double2(ef * Pa.x, ef * Pa.y);
+        }
+        const double wv = iflux * kb;
+        const double ef = exp(sigfac * wv * wv);
+        Pb = make_double2(ef * Pb.x, ef * Pb.y);
+      }
+      {
+        const double2 e = make_double2(Pa.x + Pb.x, Pa.y - Pb.y);
+        const double2 o = fft::cmul(make_double2(Pa.x - Pb.x, Pa.y + Pb.y), fft::conj(__ldg(Wn + q)));
+        z[q] = make_double2(e.x - o.y, e.y + o.x);
+      }
+      if (q != 0 && kb != q) {
+        const double2 e = make_double2(Pb.x + Pa.x, Pb.y - Pa.y);
+        const double2 o = fft::cmul(make_double2(Pb.x - Pa.x, Pb.y + Pa.y), fft::conj(__ldg(Wn + kb)));
+        z[kb] = make_double2(e.x - o.y, e.y + o.x);
+      }
+    }
+    __syncthreads();
+    // ---- inverse transform: the wrapped P(D) row
+    double2* p2 = reinterpret_cast<double2*>(P);
+    if (act) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const int i = k * M + t;
+        v[k] = (min(i, m - i) <= kc) ? z[i] : make_double2(0.0, 0.0);
+      }
+      fft::fft2_sync<M2>(1);
+      fft::fft2_head<M2, 1>(v, z, t, TW, 1);
+#pragma unroll
+      for (int pp = 0; pp < F::PP; ++pp) {
+        const int p = pp * M + t;
+        double2 u[M3];
+#pragma unroll
+        for (int i = 0; i < M3; ++i) u[i] = z[p * (M3 + 1) + i];
+        fft::dft<M3, 1>(u);
+#pragma unroll
+        for (int i = 0; i < M3; ++i) {
+          p2[p + 256 * i] = u[i];
+        }
+      }
+    }
+    __syncthreads();
+    // ---- chunk reductions over the whole row (k_pscan1)
+    const SplitParams sp = split_params(bs, var, sigma);
+    double2* prow = reinterpret_cast<double2*>(pbuf + (static_cast<size_t>(w) * D + d) * nc2);
+    double mx = -1.0e308, sum = 0.0, wsum = 0.0, mnv = 1.0e308;
+    int mni = 0x7fffffff;
+#pragma unroll 4
+    for (int j = t; j < m; j += T) {
+      const double2 x = p2[j];
+      prow[j] = x;
+      const double xa = clip0(x.x), xb = clip0(x.y);
+      const int i = 2 * j;
+      if (xa > mx) mx = xa;
+      if (xb > mx) mx = xb;
+      sum += xa + xb;
+      wsum += static_cast<double>(i) * xa + static_cast<double>(i + 1) * xb;
+      if (i >= sp.botidx && i <= sp.topidx) dev::argmin_merge(mnv, mni, xa, i);
+      if (i + 1 >= sp.botidx && i + 1 <= sp.topidx) dev::argmin_merge(mnv, mni, xb, i + 1);
+    }
+    // the five reductions in one round; every thread folds the warps' results
+    for (int o = 16; o > 0; o >>= 1) {
+      mx = dev::dmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+      const double v2 = __shfl_xor_sync(0xffffffffu, mnv, o);
+      const int i2 = __shfl_xor_sync(0xffffffffu, mni, o);
+      dev::argmin_merge(mnv, mni, v2, i2);
+    }
+    if ((t & 31) == 0) {
+      const int k = t >> 5;
+      red[0][k] = mx;
+      red[1][k] = sum;
+      red[2][k] = wsum;
+      red[3][k] = mnv;
+      redi[k] = mni;
+    }
+    __syncthreads();
+    mx = red[0][0];
+    sum = red[1][0];
+    wsum = red[2][0];
+    mnv = red[3][0];
+    mni = redi[0];
+#pragma unroll
+    for (int k = 1; k < T / 32; ++k) {
+      mx = dev::dmax(mx, red[0][k]);
+      sum += red[1][k];
+      wsum += red[2][k];
+      dev::argmin_merge(mnv, mni, red[3][k], redi[k]);
+    }
+    const RowMin1 rsum{mx, mnv, mni};
+    PDInfo1& info = pinfo[static_cast<size_t>(w) * D + d];
+    finish_row<T>(bs, dsets[d], sp, P, n, rsum, log2toe, scr, info,
+                  [&](int split, double& Sx, double& Wx, double& Tx) {
+                    double part = 0.0;
+                    for (int i = t; i < split; i += T) part += clip0(P[i]);
+                    Tx = dev::block_sum<T>(part, scr);
+                    Sx = sum;
+                    Wx = wsum;
+                  });
+    __syncthreads();
+  }
+  if (B == 1 && t == 0)
+    reduce_one(bsets, B, D, w, sm, pinfo, pr, bonus, logl, status);
 }
 
 // Bonus integrals and the slope penalty of each proposal's knot model, one
@@ -1857,8 +2326,8 @@ void Engine1::set_virtual_sigma(int bs, double sigma) {
   const int d = h_bsets_[bs].ds_begin + h_bsets_[bs].nds - 1;
   h_dsets_[d].sigma_base = sigma;
   h_bsets_[bs].maxsb = sigma;
-  cuda_check(cudaMemcpy(d_dsets_ + d, &h_dsets_[d], sizeof(DSet1Dev), cudaMemcpyHostToDevice), "upload");
-  cuda_check(cudaMemcpy(d_bsets_ + bs, &h_bsets_[bs], sizeof(BSet1Dev), cudaMemcpyHostToDevice), "upload");
+  cuda_check(cudaMemcpyAsync(d_dsets_ + d, &h_dsets_[d], sizeof(DSet1Dev), cudaMemcpyHostToDevice, stream_), "upload");
+  cuda_check(cudaMemcpyAsync(d_bsets_ + bs, &h_bsets_[bs], sizeof(BSet1Dev), cudaMemcpyHostToDevice, stream_), "upload");
 }
 
 void Engine1::set_rrange_explicit(int bs, double minR, double maxR) {
@@ -1921,14 +2390,14 @@ void Engine1::build_static() {
     double* p = dalloc<double>(v.size() ? v.size() : 1);
     static_allocs_.push_back(p);
     if (!v.empty())
-      cuda_check(cudaMemcpy(p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice), "upload");
+      cuda_check(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, stream_), "upload");
     return p;
   };
   auto upi = [&](const std::vector<int>& v) -> const int* {
     int* p = dalloc<int>(v.size() ? v.size() : 1);
     static_allocs_.push_back(p);
     if (!v.empty())
-      cuda_check(cudaMemcpy(p, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice), "upload");
+      cuda_check(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, stream_), "upload");
     return p;
   };
   const unsigned K = static_cast<unsigned>(knots_.size());
@@ -2049,7 +2518,7 @@ void Engine1::build_static() {
         unsigned char* d = nullptr;
         cuda_check(cudaMalloc(&d, kt.size() + 16), "cudaMalloc");
         static_allocs_.push_back(d);
-        cuda_check(cudaMemcpy(d, kt.data(), kt.size(), cudaMemcpyHostToDevice), "upload");
+        cuda_check(cudaMemcpyAsync(d, kt.data(), kt.size(), cudaMemcpyHostToDevice, stream_), "upload");
         sd.kidx = d;
         // per node, the first and one past the last term inside the knot
         // range: the only terms the node's sum visits
@@ -2066,7 +2535,7 @@ void Engine1::build_static() {
         int2* dj = nullptr;
         cuda_check(cudaMalloc(&dj, jr.size() * sizeof(int2) + 16), "cudaMalloc");
         static_allocs_.push_back(dj);
-        cuda_check(cudaMemcpy(dj, jr.data(), jr.size() * sizeof(int2), cudaMemcpyHostToDevice),
+        cuda_check(cudaMemcpyAsync(dj, jr.data(), jr.size() * sizeof(int2), cudaMemcpyHostToDevice, stream_),
                    "upload");
         sd.jrange = dj;
       }
@@ -2229,45 +2698,50 @@ void Engine1::build_static() {
   D_ = static_cast<unsigned>(h_dsets_.size());
   d_bsets_ = dalloc<BSet1Dev>(B_);
   static_allocs_.push_back(d_bsets_);
-  cuda_check(cudaMemcpy(d_bsets_, h_bsets_.data(), B_ * sizeof(BSet1Dev), cudaMemcpyHostToDevice), "upload");
+  cuda_check(cudaMemcpyAsync(d_bsets_, h_bsets_.data(), B_ * sizeof(BSet1Dev), cudaMemcpyHostToDevice, stream_), "upload");
   d_dsets_ = dalloc<DSet1Dev>(D_);
   static_allocs_.push_back(d_dsets_);
-  cuda_check(cudaMemcpy(d_dsets_, h_dsets_.data(), D_ * sizeof(DSet1Dev), cudaMemcpyHostToDevice), "upload");
+  cuda_check(cudaMemcpyAsync(d_dsets_, h_dsets_.data(), D_ * sizeof(DSet1Dev), cudaMemcpyHostToDevice, stream_), "upload");
   ntile_ = fill_tiles();
   nchunk_ = (n_ + CHUNK - 1) / CHUNK;
   // own FFT: n = 2m, m = m1 * 256 with m1 a power of two in [8, 256].  By
   // default (no FFT mode set) from n = 8192: at n = 4096 batched cuFFT is
   // ~5 % faster on the B200, above it the own FFT is faster (1.6x at
   // n = 65536 and 131072); on request (set_fft_mode(0)) from n = 4096.
-  own_fft_ = (fft_mode_ == 0 || (fft_mode_ < 0 && n_ >= 8192)) && n_ >= 4096 && n_ <= 131072 &&
+  own_fft_ = (fft_mode_ == 0 || (fft_mode_ < 0 && n_ >= kOwnFftMin)) && n_ >= 4096 && n_ <= 131072 &&
              (n_ & (n_ - 1)) == 0;
   tune_.own_fft = own_fft_ ? 1 : 0;
-  if (own_fft_) {
+  {
     const size_t m = n_ / 2;
-    std::vector<double2> wh(m / 128), wl(128), wn(m + 1);
     const long double tau = 6.283185307179586476925286766559005768L;
-    for (size_t j = 0; j < m / 128; ++j) {
-      const long double a = -tau * static_cast<long double>(128 * j) / static_cast<long double>(m);
-      wh[j] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
+    auto table = [&](size_t len, size_t step, size_t period) -> const double2* {
+      std::vector<double2> v(len);
+      for (size_t j = 0; j < len; ++j) {
+        const long double a = -tau * static_cast<long double>(step * j) / static_cast<long double>(period);
+        v[j] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
+      }
+      double2* d = dalloc<double2>(len);
+      static_allocs_.push_back(d);
+      cuda_check(cudaMemcpyAsync(d, v.data(), len * sizeof(double2), cudaMemcpyHostToDevice, stream_), "upload");
+      return d;
+    };
+    const bool small = n_ >= 1024 && n_ <= 8192 && (n_ & (n_ - 1)) == 0;
+    d_wh_ = d_wl_ = d_wn_ = d_tw_ = nullptr;
+    if (own_fft_) {
+      d_wh_ = table(m / 128, 128, m);
+      d_wl_ = table(128, 1, m);
     }
-    for (size_t i = 0; i < 128; ++i) {
-      const long double a = -tau * static_cast<long double>(i) / static_cast<long double>(m);
-      wl[i] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
+    if (own_fft_ || small) d_wn_ = table(m + 1, 1, n_);
+    if (small) {
+      const std::vector<double2> tw = fft::fft2_twiddles(static_cast<unsigned>(m));
+      double2* d = dalloc<double2>(tw.size());
+      static_allocs_.push_back(d);
+      cuda_check(cudaMemcpyAsync(d, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, stream_), "upload");
+      d_tw_ = d;
     }
-    for (size_t k = 0; k <= m; ++k) {
-      const long double a = -tau * static_cast<long double>(k) / static_cast<long double>(n_);
-      wn[k] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
-    }
-    d_wh_ = dalloc<double2>(m / 128);
-    static_allocs_.push_back(d_wh_);
-    d_wl_ = dalloc<double2>(128);
-    static_allocs_.push_back(d_wl_);
-    d_wn_ = dalloc<double2>(m + 1);
-    static_allocs_.push_back(d_wn_);
-    cuda_check(cudaMemcpy(d_wh_, wh.data(), wh.size() * sizeof(double2), cudaMemcpyHostToDevice), "upload");
-    cuda_check(cudaMemcpy(d_wl_, wl.data(), wl.size() * sizeof(double2), cudaMemcpyHostToDevice), "upload");
-    cuda_check(cudaMemcpy(d_wn_, wn.data(), (m + 1) * sizeof(double2), cudaMemcpyHostToDevice), "upload");
   }
+  // the uploads went through this engine's stream; launches may go to others
+  cuda_check(cudaStreamSynchronize(stream_), "uploads");
   static_ok_ = true;
   // shapes changed: old plans/graphs/work space no longer match
   drop_graphs();
@@ -2299,12 +2773,12 @@ void Engine1::profile_stages(unsigned nprop, const float* theta, unsigned npar,
   eval_host(nprop, theta, npar, lls.data(), sts.data());  // staging + warm
   cudaEvent_t ev[kNumStages + 1];
   for (auto& e : ev) cuda_check(cudaEventCreate(&e), "event create");
-  for (int k = 0; k < kNumStages; ++k) stage_ms[k] = 0.0;
+  for (int k = 0; k < num_stages(); ++k) stage_ms[k] = 0.0;
   (void)ll;
   for (int r = 0; r < reps; ++r) {
     launch_all(nprop, ws_.theta_in, npar, ws_.logl, ws_.status, stream_, ev);
     cuda_check(cudaStreamSynchronize(stream_), "synchronize");
-    for (int k = 0; k < kNumStages; ++k) {
+    for (int k = 0; k < num_stages(); ++k) {
       float ms = 0.f;
       cuda_check(cudaEventElapsedTime(&ms, ev[k], ev[k + 1]), "elapsed");
       stage_ms[k] += ms / reps;
@@ -2344,7 +2818,12 @@ void Engine1::set_tuning(const Tune1& t) {
   const bool fft_changed = (t.own_fft != 0) != (tune_.own_fft != 0);
   tune_ = t;
   tune_.own_fft = t.own_fft ? 1 : 0;
-  if (fft_changed) set_fft_mode(tune_.own_fft ? 0 : 1);  // rebuilds tables, plans, work space
+  if (fft_changed) {  // rebuilds tables, plans, work space
+    // off again where it is not the automatic choice either: automatic, not
+    // cuFFT, so that the single-block kernel stays in use
+    const bool automatic = !tune_.own_fft && n_ < kOwnFftMin;
+    set_fft_mode(tune_.own_fft ? 0 : automatic ? -1 : 1);
+  }
   if (static_ok_) ntile_ = fill_tiles();
   drop_graphs();
 }
@@ -2426,7 +2905,9 @@ const char* Engine1::stage_name(int i) const {
       "k_rnodes1", "k_rspline1", "k_fftAR1", "k_moments1",
       "k_fftB1", "k_spectrum1f", "k_fftA1+k_fftB1_inv", "k_pscan1", "k_pfinish1",
       "k_reduce1"};
-  if (i < 0 || i >= kNumStages) return "";
+  if (i < 0 || i >= num_stages()) return "";
+  static const char* row[] = {"k_rnodes1", "k_row1", "k_reduce1"};
+  if (row1()) return row[i];
   if (!own_fft_) return lib[i];
   return fused_fill() ? fused[i] : own[i];
 }
@@ -2515,8 +2996,8 @@ void Engine1::fill_bonus(unsigned nprop, float* theta_dev, unsigned npar, cudaSt
   cuda_check(cudaGetLastError(), "k_bonus1");
 }
 
+// -1: automatic (the state of a new engine; the C entry takes 0 and 1 only)
 void Engine1::set_fft_mode(int mode) {
-  if (mode != 0 && mode != 1) throw Error(POFD_E_ARG, "fft mode must be 0 (own) or 1 (cuFFT)");
   tune_.own_fft = (mode == 0) ? 1 : 0;
   if (mode == fft_mode_) return;
   fft_mode_ = mode;
@@ -2581,21 +3062,25 @@ void Engine1::reserve(unsigned P) {
   // logL [P] then status [P] in one allocation: one download per call
   ws_.logl = dalloc<double>(P + (P + 1) / 2);
   ws_.status = reinterpret_cast<int*>(ws_.logl + P);
-  cuda_check(cudaFuncSetAttribute(k_rnodes1, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>((KMAX + 4 * KMAX + 2 * MAXTERMS) * sizeof(double))),
-             "smem attribute");
+  for (auto k : {k_rnodes1<1>, k_rnodes1<4>})
+    cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>((KMAX + 4 * KMAX + 2 * MAXTERMS) * sizeof(double))),
+               "smem attribute");
   cuda_check(cudaFuncSetAttribute(k_rspline1<kSplineThreads>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>((2 * 8192 + 64) * sizeof(double))),
              "smem attribute");
-  cuda_check(cudaMemset(ws_.nodes, 0, static_cast<size_t>(P) * B_ * 2 * NI * sizeof(double)), "memset");
+  cuda_check(cudaMemsetAsync(ws_.nodes, 0, static_cast<size_t>(P) * B_ * 2 * NI * sizeof(double),
+                             stream_), "memset");
+  cuda_check(cudaStreamSynchronize(stream_), "memset");
 }
 
 void Engine1::ensure_plans(unsigned nprop) {
   auto it = plans_.find(nprop);
-  if (it != plans_.end() && (it->second.fwd || own_fft_)) return;
+  if (it != plans_.end() && (it->second.fwd || own_fft_ || row1())) return;
   Plans pl;
-  if (own_fft_) {  // the own FFT needs no cuFFT plans; the entry holds graphs
+  if (it != plans_.end()) pl = it->second;
+  if (own_fft_ || row1()) {  // the own FFT needs no cuFFT plans; the entry holds graphs
     plans_[nprop] = pl;
     return;
   }
@@ -2611,6 +3096,35 @@ void Engine1::ensure_plans(unsigned nprop) {
   plans_[nprop] = pl;
 }
 
+
+// The single-block kernel where the transform may be the library's own, the
+// fill is by running products and the row fits a block: at any batch.  One
+// likelihood call (2048 nodes, host to host), this kernel's sequence and the
+// one of eight to nine kernels: n = 4096, 1 row 46.0 and 63.8 us, 148 rows
+// 59.5 and 85.3, 600 rows (a third wave hardly begun) 162 and 188, 2048 rows
+// 424 and 508; n = 1024, 1 row 43.7 and 57.0, 2048 rows 371 and 399; n = 8192
+// (one row to an SM), 1 row 49.7 and 71.2, 148 rows 63 and 98, 600 rows (a
+// fifth wave hardly begun) 207 and 226, 1000 rows 312 and 345.
+bool Engine1::row1() const {
+  for (const auto& s : sets_)
+    if (s.data.size() > static_cast<size_t>(ROW1_MAXDS)) return false;
+  return fft_mode_ != 1 && tune_.rfill_mode == 3 && n_ >= 1024 && n_ <= 8192 &&
+         (n_ & (n_ - 1)) == 0 && ninterp_ <= static_cast<unsigned>(ROW1_MAXNI);
+}
+
+namespace {
+template <int M2, int T, class... Args>
+void launch_row1_t(int rows, size_t smem, cudaStream_t st, Args... args) {
+  cuda_check(cudaFuncSetAttribute(k_row1<M2, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(smem)), "attr");
+  launch_pdl(k_row1<M2, T>, dim3(rows), dim3(T), smem, st, args...);
+}
+template <int M2, class... Args>
+void launch_row1(bool wide, int rows, size_t smem, cudaStream_t st, Args... args) {
+  if (wide || M2 == ROW1_MAXN / 2) launch_row1_t<M2, 512>(rows, smem, st, args...);
+  else if constexpr (M2 < ROW1_MAXN / 2) launch_row1_t<M2, 256>(rows, smem, st, args...);
+}
+}  // namespace
 
 void Engine1::launch_all(unsigned nprop, const float* theta, unsigned npar,
                          double* logl, int* status, cudaStream_t st,
@@ -2631,16 +3145,54 @@ void Engine1::launch_all(unsigned nprop, const float* theta, unsigned npar,
   {
     const size_t smem = (KMAX + 4 * KMAX + 2 * static_cast<size_t>(maxterms_)) * sizeof(double);
     const int th = tune_.rnodes_threads;
-    dim3 grid((NI + th - 1) / th, P * B * 2);
-    k_rnodes1<<<grid, th, smem, st>>>(d_bsets_, model_, B, NI, maxterms_, theta,
-                                      static_cast<int>(npar), std::log2(10.0), ws_.cnt,
-                                      ws_.mstatus, ws_.sigmult, ws_.nodes);
+    // four lanes a node up to 16384 nodes a side.  One likelihood of n = 4096
+    // with 2048 nodes and binned beams, four lanes or one: 1 row 45.0 and
+    // 46.0 us, 8 rows 46.8 and 48.7, 12 rows 50.4 and 48.1, 40 rows 57.6 and
+    // 51.6; 500 nodes: 1 row 42.1 and 43.5, 30 rows 45.0 and 46.9, 60 rows
+    // 47.0 and 46.7; 2048 nodes, unbinned beams: 50.5 and 56.1 at 1 row, 57.3
+    // and 60.0 at 16, 62.2 and 60.9 at 24.
+    const bool few = static_cast<long>(P) * B * NI <= 16384;
+    dim3 grid((NI * (few ? 4 : 1) + th - 1) / th, P * B * 2);
+    (few ? k_rnodes1<4> : k_rnodes1<1>)<<<grid, th, smem, st>>>(
+        d_bsets_, model_, B, NI, maxterms_, theta, static_cast<int>(npar), std::log2(10.0),
+        ws_.cnt, ws_.mstatus, ws_.sigmult, ws_.nodes, nullptr);
   }
   if (prior_.needs_bonus())
     k_bonus1<<<P, kBonusThreads, 0, st>>>(model_, const_cast<float*>(theta), static_cast<int>(npar),
                                           std::log2(10.0), ws_.cnt, ws_.mstatus, d_qu_, d_qs_,
                                           d_qw_, qper_, ws_.bonus, -1);
   mark(1);
+  if (row1()) {
+    bool several = false;
+    for (const auto& bs : h_bsets_) several = several || bs.nds > 1;
+    const Row1Mem mem = row1_mem(n, NI, several);
+    const size_t smem = row1_smem(mem);
+    // 512 threads a row while every row has an SM to itself, and at n = 8192,
+    // whose rows never share one; else 256, two rows to an SM.  One likelihood
+    // with 512 and 256 threads a row: n = 4096, 1 row 45.2 and 49.2 us, 148
+    // rows 60.4 and 66.4, 150 rows 81.7 and 66.1, 296 rows 95 and 78, 592 rows
+    // 166 and 133; n = 1024, 148 rows 61.9 and 65.7, 592 rows 150 and 123; n =
+    // 8192, 1 row 49.3 and 53.4, 150 rows 90 and 100, 592 rows 180 and 207.
+    const bool wide = P * B <= sm_count_;
+#define POFD_ROW1(M2)                                                                          \
+  launch_row1<M2>(wide, P * B, smem, st, d_bsets_, d_dsets_, B, D, NI, mem, std::log(2.0),           \
+                  ws_.mstatus, ws_.sigmult, ws_.nodes, d_wn_, d_tw_, ws_.mom, ws_.pbuf,        \
+                  ws_.pinfo, prior_, ws_.bonus, logl, status)
+    switch (n) {
+      case 1024: POFD_ROW1(512); break;
+      case 2048: POFD_ROW1(1024); break;
+      case 4096: POFD_ROW1(2048); break;
+      default: POFD_ROW1(4096); break;
+    }
+#undef POFD_ROW1
+    mark(2);
+    if (B > 1)
+      k_reduce1<<<(P + 127) / 128, 128, 0, st>>>(d_bsets_, B, D, P, ws_.mstatus, ws_.sigmult,
+                                                ws_.pinfo, prior_, ws_.bonus, logl, status);
+    mark(3);
+    cuda_check(cudaGetLastError(), "kernel launch");
+    return;
+  }
   {
     const size_t smem = (2 * static_cast<size_t>(NI) + 64) * sizeof(double);
     k_rspline1<kSplineThreads><<<P * B * 2, kSplineThreads, smem, st>>>(d_bsets_, B, NI, ws_.mstatus,
@@ -2795,8 +3347,8 @@ cudaGraphExec_t Engine1::graph_for(unsigned nprop, const float* theta,
   return ge;
 }
 
-// The upload of theta, the launch sequence and the download of logL and
-// status, captured together for each batch size after its first (eager) use.
+// The upload of theta and the launch sequence, whose last kernel writes logL
+// and status to the host, captured together for each batch size after its first (eager) use.
 cudaGraphExec_t Engine1::host_graph_for(unsigned nprop, unsigned npar) {
   Plans& pl = plans_.at(nprop);
   if (pl.no_graph || !pl.warmed) return nullptr;
@@ -2813,10 +3365,9 @@ cudaGraphExec_t Engine1::host_graph_for(unsigned nprop, unsigned npar) {
       cuda_check(cudaMemcpyAsync(ws_.theta_in, ws_.h_theta,
                                  static_cast<size_t>(nprop) * npar * sizeof(float),
                                  cudaMemcpyHostToDevice, stream_), "H2D theta");
-      launch_all(nprop, ws_.theta_in, npar, ws_.logl, ws_.status, stream_, nullptr);
-      cuda_check(cudaMemcpyAsync(ws_.h_logl, ws_.logl,
-                                 ws_.P * sizeof(double) + nprop * sizeof(int),
-                                 cudaMemcpyDeviceToHost, stream_), "D2H results");
+      // the last kernel writes its 12 bytes a row into the pinned host buffer:
+      // a copy of its own costs 3 us
+      launch_all(nprop, ws_.theta_in, npar, ws_.h_logl, ws_.h_status, stream_, nullptr);
     } catch (...) {
       threw = true;
     }
@@ -2912,9 +3463,19 @@ void Engine1::rnodes_host(int bs, int side, const float* theta, unsigned npar,
   const Side1Dev& sd = h_bsets_[bs].side[side & 1];
   if (!sd.nodes) throw Error(POFD_E_ARG, "beam has no such side");
   const size_t NI = ninterp_;
-  cuda_check(cudaMemcpy(x_out, sd.x, NI * sizeof(double), cudaMemcpyDeviceToHost), "D2H x");
-  cuda_check(cudaMemcpy(r_out, ws_.nodes + (static_cast<size_t>(bs) * 2 + (side & 1)) * NI,
-                        NI * sizeof(double), cudaMemcpyDeviceToHost), "D2H R");
+  double* R = dalloc<double>(static_cast<size_t>(B_) * 2 * NI);
+  k_rnodes1<1><<<dim3(static_cast<unsigned>((NI + 127) / 128), B_ * 2), 128,
+              (KMAX + 4 * KMAX + 2 * static_cast<size_t>(maxterms_)) * sizeof(double), stream_>>>(
+      d_bsets_, model_, static_cast<int>(B_), static_cast<int>(NI), maxterms_, ws_.theta_in,
+      static_cast<int>(npar), std::log2(10.0), ws_.cnt, ws_.mstatus, ws_.sigmult, ws_.nodes, R);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+  if (e == cudaSuccess) e = cudaMemcpy(x_out, sd.x, NI * sizeof(double), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(r_out, R + (static_cast<size_t>(bs) * 2 + (side & 1)) * NI, NI * sizeof(double),
+                   cudaMemcpyDeviceToHost);
+  cudaFree(R);
+  cuda_check(e, "R nodes");
 }
 
 void Engine1::rgrid_host(int bs, const float* theta, unsigned npar, double* out) {
@@ -2925,14 +3486,14 @@ void Engine1::rgrid_host(int bs, const float* theta, unsigned npar, double* out)
     int st;
     eval_host(1, theta, npar, &ll, &st);  // allocates staging
   }
-  cuda_check(cudaMemcpy(ws_.theta_in, theta, npar * sizeof(float), cudaMemcpyHostToDevice), "H2D");
+  cuda_check(cudaMemcpyAsync(ws_.theta_in, theta, npar * sizeof(float), cudaMemcpyHostToDevice, stream_), "H2D");
   const int NI = static_cast<int>(ninterp_), n = static_cast<int>(n_);
   const int nc2 = 2 * (n / 2 + 1);
   const int B = static_cast<int>(B_);
-  k_rnodes1<<<dim3((NI + 127) / 128, B * 2), 128,
+  k_rnodes1<1><<<dim3((NI + 127) / 128, B * 2), 128,
               (KMAX + 4 * KMAX + 2 * static_cast<size_t>(maxterms_)) * sizeof(double), stream_>>>(
       d_bsets_, model_, B, NI, maxterms_, ws_.theta_in, static_cast<int>(npar), std::log2(10.0),
-      ws_.cnt, ws_.mstatus, ws_.sigmult, ws_.nodes);
+      ws_.cnt, ws_.mstatus, ws_.sigmult, ws_.nodes, nullptr);
   k_rspline1<kSplineThreads><<<B * 2, kSplineThreads, (2 * static_cast<size_t>(NI) + 64) * sizeof(double), stream_>>>(
       d_bsets_, B, NI, ws_.mstatus, ws_.nodes, ws_.spl);
   launch_rfill(tune_.rfill_per, tune_.rfill_mode >= 2, dim3(ntile_, B), stream_, d_bsets_, B, n,

@@ -190,6 +190,7 @@ class Engine1 {
                    double* x_out, double* r_out);
   void rgrid_host(int bs, const float* theta, unsigned npar, double* out);
   int kernels_per_eval() const {
+    if (row1()) return 1 + 1 + (B_ > 1 ? 1 : 0) + (prior_.needs_bonus() ? 1 : 0);
     return (own_fft_ ? (fused_fill() ? 11 : 12) : 8) + (prior_.needs_bonus() ? 1 : 0);
   }
   // the R grid fill runs inside the forward FFT pass A (own FFT, plain passes)
@@ -221,6 +222,8 @@ class Engine1 {
   // the same written into theta_dev[i][nknots + 1], [nknots + 2] (device)
   void fill_bonus(unsigned nprop, float* theta_dev, unsigned npar, cudaStream_t st);
   static constexpr int kNumStages = 10;
+  static constexpr size_t kOwnFftMin = 8192;  // automatic four-step FFT from here
+  int num_stages() const { return row1() ? 3 : kNumStages; }
   void profile_stages(unsigned nprop, const float* theta, unsigned npar,
                       int reps, double* stage_ms);
   const char* stage_name(int i) const;
@@ -286,8 +289,8 @@ class Engine1 {
     std::vector<std::pair<GraphKey, cudaGraphExec_t>> graphs;
     bool warmed = false;
     bool no_graph = false;
-    // eval_host's graph: theta upload, the launch sequence and the result
-    // download in one launch (for host_npar parameters per row)
+    // eval_host's graph: theta upload and the launch sequence in one launch
+    // (for host_npar parameters per row)
     cudaGraphExec_t host_graph = nullptr;
     unsigned host_npar = 0;
   };
@@ -300,9 +303,11 @@ class Engine1 {
   int fft_mode_ = -1;  // -1 automatic (own FFT from n = 8192), 0 own, 1 cuFFT
   bool own_fft_ = false;
   int sm_count_ = 148;
-  double2* d_wh_ = nullptr;  // e^{-2 pi i 128 j / m}, j < m / 128
-  double2* d_wl_ = nullptr;  // e^{-2 pi i i / m}, i < 128
-  double2* d_wn_ = nullptr;  // e^{-2 pi i k / n}, k <= m
+  const double2* d_wh_ = nullptr;  // e^{-2 pi i 128 j / m}, j < m / 128
+  const double2* d_wl_ = nullptr;  // e^{-2 pi i i / m}, i < 128
+  const double2* d_wn_ = nullptr;  // e^{-2 pi i k / n}, k <= m
+  const double2* d_tw_ = nullptr;  // fft::fft2_twiddles(m) (the single-block kernel)
+  bool row1() const;
   double time_sequence(unsigned nprop, const float* theta, unsigned npar, int reps);
   Tune1 tune_;
   // priors and the knot quadrature of the bonus integrals

@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "fft1d.cuh"
+#include "fft2.cuh"
 
 namespace pofd {
 
@@ -1431,97 +1432,7 @@ __global__ void k_reduce2(const BSet2Dev* __restrict__ bsets,
 // array is kept by columns, [k2][row], so that the column kernel, which
 // reads and writes it whole, streams; the row kernels touch it in pieces of
 // a pair of rows, 32 bytes, with one vector access each.
-//
-// One DFT, n = 16 M, M = 16 M3, runs on M threads with 16 values each: with
-// input j = n1 M + u, u = m M3 + s and output k = k1 + 16 k2 + 256 k3,
-//   stage 1: 16-point register DFTs over n1, times W_n^{u k1};
-//   stage 2: 16-point register DFTs over m, times W_M^{s k2};
-//   stage 3: M3-point register DFTs over s;
-// thread u holds (k1, s) = (u / M3, u % M3) in stage 2 and the outputs of
-// p = k1 + 16 k2 = u, u + M, ... in stage 3.  The two exchanges go through
-// shared memory, pitched so that neither side has bank conflicts.  A column
-// goes back through the same stages transposed.  Twiddle powers come from
-// four table entries per thread and stage (W^x, W^2x, W^4x, W^8x, made in
-// long double), the other eleven by one product each: a table of all of
-// them would cost as much shared memory traffic again as the exchanges.
-template <int N>
-struct Fft2 {
-  static constexpr int M = N / 16, M3 = N / 256;
-  static constexpr int PITCH = M + M3;        // of the first exchange, [k1][u]
-  static constexpr int SL = 256 * (M3 + 1);   // slots per DFT: [p][s], one pad
-  static constexpr int PP = 16 / M3;          // stage-3 DFTs per thread
-};
-
-template <int S>
-__device__ __forceinline__ void tw16(double2* v, const double2* __restrict__ T, int M) {
-  double2 w1 = __ldg(T), w2 = __ldg(T + M), w4 = __ldg(T + 2 * M), w8 = __ldg(T + 3 * M);
-  if (S > 0) {
-    w1.y = -w1.y;
-    w2.y = -w2.y;
-    w4.y = -w4.y;
-    w8.y = -w8.y;
-  }
-  const double2 w3 = fft::cmul(w1, w2);
-  v[1] = fft::cmul(v[1], w1);
-  v[2] = fft::cmul(v[2], w2);
-  v[3] = fft::cmul(v[3], w3);
-  v[4] = fft::cmul(v[4], w4);
-  v[8] = fft::cmul(v[8], w8);
-  v[9] = fft::cmul(v[9], fft::cmul(w1, w8));
-  v[10] = fft::cmul(v[10], fft::cmul(w2, w8));
-  v[11] = fft::cmul(v[11], fft::cmul(w3, w8));
-  const double2 w5 = fft::cmul(w1, w4), w6 = fft::cmul(w2, w4), w7 = fft::cmul(w3, w4);
-  v[5] = fft::cmul(v[5], w5);
-  v[6] = fft::cmul(v[6], w6);
-  v[7] = fft::cmul(v[7], w7);
-  v[12] = fft::cmul(v[12], fft::cmul(w4, w8));
-  v[13] = fft::cmul(v[13], fft::cmul(w5, w8));
-  v[14] = fft::cmul(v[14], fft::cmul(w6, w8));
-  v[15] = fft::cmul(v[15], fft::cmul(w7, w8));
-}
-
-// Stages 1 and 2: v[n1] = input n1 M + u of the thread; leaves the stage-3
-// inputs in the slots b[p (M3 + 1) + s].
-template <int N, int S>
-__device__ __forceinline__ void fft2_head(double2* v, double2* b, int u,
-                                          const double2* __restrict__ TW) {
-  using F = Fft2<N>;
-  fft::dft<16, S>(v);
-  tw16<S>(v, TW + u, F::M);
-#pragma unroll
-  for (int k1 = 0; k1 < 16; ++k1) b[k1 * F::PITCH + u] = v[k1];
-  __syncthreads();
-  const int k1 = u / F::M3, s = u % F::M3;
-#pragma unroll
-  for (int m = 0; m < 16; ++m) v[m] = b[k1 * F::PITCH + m * F::M3 + s];
-  fft::dft<16, S>(v);
-  tw16<S>(v, TW + 16 * s, F::M);
-  __syncthreads();
-#pragma unroll
-  for (int k2 = 0; k2 < 16; ++k2) b[(k1 + 16 * k2) * (F::M3 + 1) + s] = v[k2];
-  __syncthreads();
-}
-
-// The transposed stages 2 and 1 of the inverse, from the slots to v[n1] =
-// output n1 M + u.
-template <int N>
-__device__ __forceinline__ void fft2_tail_inv(double2* v, double2* b, int u,
-                                              const double2* __restrict__ TW) {
-  using F = Fft2<N>;
-  const int k1 = u / F::M3, s = u % F::M3;
-#pragma unroll
-  for (int k2 = 0; k2 < 16; ++k2) v[k2] = b[(k1 + 16 * k2) * (F::M3 + 1) + s];
-  tw16<1>(v, TW + 16 * s, F::M);
-  fft::dft<16, 1>(v);
-  __syncthreads();
-#pragma unroll
-  for (int m = 0; m < 16; ++m) b[k1 * F::PITCH + m * F::M3 + s] = v[m];
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = b[j * F::PITCH + u];
-  tw16<1>(v, TW + u, F::M);
-  fft::dft<16, 1>(v);
-}
+// The DFTs are those of fft2.cuh.
 
 // 32 bytes in one store (both values' cells adjoin and are 32-byte aligned)
 __device__ __forceinline__ void st32(double2* p, double2 a, double2 b) {
@@ -1553,11 +1464,11 @@ using InvCfg = RowShape<N, (N <= 512 ? 128 : 256)>;
 constexpr int RI_ROWS = 32;  // P(D) rows per block of k_rowinv2 (>= 2 G)
 template <int N>
 constexpr size_t rowfwd_smem() {
-  return static_cast<size_t>(FwdCfg<N>::G) * Fft2<N>::SL * sizeof(double2);
+  return static_cast<size_t>(FwdCfg<N>::G) * fft::Fft2<N>::SL * sizeof(double2);
 }
 template <int N>
 constexpr size_t rowinv_smem() {
-  return static_cast<size_t>(InvCfg<N>::G) * (Fft2<N>::SL * sizeof(double2) + N * sizeof(double));
+  return static_cast<size_t>(InvCfg<N>::G) * (fft::Fft2<N>::SL * sizeof(double2) + N * sizeof(double));
 }
 // columns per block of k_colspec2
 template <int N>
@@ -1580,7 +1491,7 @@ __global__ void __launch_bounds__(FwdCfg<N>::T, 512 / FwdCfg<N>::T)
 k_rowfwd2(const BSet2Dev* __restrict__ bsets, int B, int D, const int* __restrict__ mstatus,
           const double* __restrict__ rgrid, const int* __restrict__ kcset,
           double2* __restrict__ ybuf, const double2* __restrict__ TW) {
-  using F = Fft2<N>;
+  using F = fft::Fft2<N>;
   using R = FwdCfg<N>;
   constexpr int M = F::M, M3 = F::M3, G = R::G, T = R::T;
   constexpr int nc = N / 2 + 1;
@@ -1596,7 +1507,7 @@ k_rowfwd2(const BSet2Dev* __restrict__ bsets, int B, int D, const int* __restric
   double2 v[16];
 #pragma unroll
   for (int q = 0; q < 16; ++q) v[q] = make_double2(R0[q * M], R0[N + q * M]);
-  fft2_head<N, -1>(v, b, u, TW);
+  fft::fft2_head<N, -1>(v, b, u, TW, 1 + g);
 #pragma unroll
   for (int pp = 0; pp < F::PP; ++pp) {
     double2* s = b + (pp * M + u) * (M3 + 1);
@@ -1672,7 +1583,7 @@ k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dset
            const double* __restrict__ mom, const double* __restrict__ r0buf,
            const int* __restrict__ kcset, const int* __restrict__ kcds,
            double2* __restrict__ ybuf, const double2* __restrict__ TW) {
-  using F = Fft2<N>;
+  using F = fft::Fft2<N>;
   constexpr int M = F::M, M3 = F::M3, C = ColCfg<N>::C;
   constexpr int nc = N / 2 + 1;
   extern __shared__ double2 csm[];  // [C][SL], with several datasets twice
@@ -1702,12 +1613,13 @@ k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dset
   // spectrum through shared memory
   const bool staged = several || c0 == 0 || (c0 <= N / 2 && N / 2 < c0 + C);
   const bool self = i2 == 0 || i2 == N / 2;
+  const int bar = 1 + t / M;
   double2 v[16];
   double2* Yc = ybuf + (static_cast<size_t>(w) * D + bs.ds_begin) * N * nc +
                 static_cast<size_t>(i2) * N + u;
 #pragma unroll
   for (int n1 = 0; n1 < 16; ++n1) v[n1] = live ? Yc[n1 * M] : make_double2(0.0, 0.0);
-  fft2_head<N, -1>(v, b, u, TW);
+  fft::fft2_head<N, -1>(v, b, u, TW, bar);
   if (staged) {
 #pragma unroll 1
     for (int pp = 0; pp < F::PP; ++pp) {
@@ -1719,7 +1631,7 @@ k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dset
 #pragma unroll
       for (int i = 0; i < M3; ++i) zs[p * (M3 + 1) + i] = z[i];
     }
-    __syncthreads();
+    fft::fft2_sync<N>(bar);
   }
   for (int dd = 0; dd < bs.nds; ++dd) {
     const int d = bs.ds_begin + dd;
@@ -1742,7 +1654,7 @@ k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dset
         oc[j * M] = self ? sp.bin_self<N>(X, zs[(j1 & 255) * (M3 + 1) + (j1 >> 8)], i1, i2)
                          : sp.bin<N>(X, i1, i2);
       }
-      __syncthreads();
+      fft::fft2_sync<N>(bar);
     }
 #pragma unroll
     for (int pp = 0; pp < F::PP; ++pp) {
@@ -1763,13 +1675,13 @@ k_colspec2(const BSet2Dev* __restrict__ bsets, const DSet2Dev* __restrict__ dset
 #pragma unroll
       for (int i = 0; i < M3; ++i) b[p * (M3 + 1) + i] = z[i];
     }
-    __syncthreads();
-    fft2_tail_inv<N>(v, b, u, TW);
+    fft::fft2_sync<N>(bar);
+    fft::fft2_tail_inv<N>(v, b, u, TW, bar);
     if (i2 <= kd) {
 #pragma unroll
       for (int n1 = 0; n1 < 16; ++n1) oc[n1 * M] = v[n1];
     }
-    __syncthreads();
+    fft::fft2_sync<N>(bar);
   }
 }
 
@@ -1784,7 +1696,7 @@ k_rowinv2(int D, const int* __restrict__ mstatus, const int* __restrict__ kcds,
           const double2* __restrict__ ybuf, int pitch, double* __restrict__ pbuf,
           double* __restrict__ rowpart, double* __restrict__ colpart,
           const double2* __restrict__ TW) {
-  using F = Fft2<N>;
+  using F = fft::Fft2<N>;
   using R = InvCfg<N>;
   constexpr int M = F::M, M3 = F::M3, G = R::G, T = R::T;
   constexpr int nc = N / 2 + 1, H = N / 2;
@@ -1829,8 +1741,8 @@ k_rowinv2(int D, const int* __restrict__ mstatus, const int* __restrict__ kcds,
       const int i = n1 * M + u;
       v[n1] = (min(i, N - i) <= kc) ? b[i] : make_double2(0.0, 0.0);
     }
-    __syncthreads();
-    fft2_head<N, 1>(v, b, u, TW);
+    fft::fft2_sync<N>(1 + g);
+    fft::fft2_head<N, 1>(v, b, u, TW, 1 + g);
     double s0 = 0.0, s1 = 0.0;
     double* p0 = pbuf + (static_cast<size_t>(wd) * N + rbase + 2 * g) * pitch;
     double* p1 = p0 + pitch;
@@ -2197,8 +2109,8 @@ void Engine2::set_virtual_sigma(int bs, double sigma1, double sigma2) {
   h_dsets_[d].sb2 = sigma2;
   h_bsets_[bs].maxsb1 = sigma1;
   h_bsets_[bs].maxsb2 = sigma2;
-  ck(cudaMemcpy(d_dsets_ + d, &h_dsets_[d], sizeof(DSet2Dev), cudaMemcpyHostToDevice), "upload");
-  ck(cudaMemcpy(d_bsets_ + bs, &h_bsets_[bs], sizeof(BSet2Dev), cudaMemcpyHostToDevice), "upload");
+  ck(cudaMemcpyAsync(d_dsets_ + d, &h_dsets_[d], sizeof(DSet2Dev), cudaMemcpyHostToDevice, stream_), "upload");
+  ck(cudaMemcpyAsync(d_bsets_ + bs, &h_bsets_[bs], sizeof(BSet2Dev), cudaMemcpyHostToDevice, stream_), "upload");
 }
 
 void Engine2::set_rrange_explicit(int bs, double min1, double max1, double min2, double max2) {
@@ -2254,13 +2166,13 @@ void Engine2::build_static() {
   auto up = [&](const std::vector<double>& v) -> const double* {
     double* q = dal<double>(v.size() ? v.size() : 1);
     static_allocs_.push_back(q);
-    if (!v.empty()) ck(cudaMemcpy(q, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice), "upload");
+    if (!v.empty()) ck(cudaMemcpyAsync(q, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, stream_), "upload");
     return q;
   };
   auto upi = [&](const std::vector<int>& v) -> const int* {
     int* q = dal<int>(v.size() ? v.size() : 1);
     static_allocs_.push_back(q);
-    if (!v.empty()) ck(cudaMemcpy(q, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice), "upload");
+    if (!v.empty()) ck(cudaMemcpyAsync(q, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, stream_), "upload");
     return q;
   };
   std::vector<double> lk(knots_.size());
@@ -2289,7 +2201,7 @@ void Engine2::build_static() {
     ck(cudaMalloc(&qk, (kq.kidx.size() + 1) * sizeof(int)), "cudaMalloc");
     static_allocs_.push_back(qk);
     if (!kq.kidx.empty())
-      ck(cudaMemcpy(qk, kq.kidx.data(), kq.kidx.size() * sizeof(int), cudaMemcpyHostToDevice),
+      ck(cudaMemcpyAsync(qk, kq.kidx.data(), kq.kidx.size() * sizeof(int), cudaMemcpyHostToDevice, stream_),
          "upload");
     d_qk_ = qk;
     nq_ = static_cast<int>(kq.u.size());
@@ -2426,10 +2338,10 @@ void Engine2::build_static() {
   for (auto& bd : h_bsets_) bd.Ts = Tmax_;  // common row stride of rw
   d_bsets_ = dal<BSet2Dev>(B_);
   static_allocs_.push_back(d_bsets_);
-  ck(cudaMemcpy(d_bsets_, h_bsets_.data(), B_ * sizeof(BSet2Dev), cudaMemcpyHostToDevice), "upload");
+  ck(cudaMemcpyAsync(d_bsets_, h_bsets_.data(), B_ * sizeof(BSet2Dev), cudaMemcpyHostToDevice, stream_), "upload");
   d_dsets_ = dal<DSet2Dev>(D_);
   static_allocs_.push_back(d_dsets_);
-  ck(cudaMemcpy(d_dsets_, h_dsets_.data(), D_ * sizeof(DSet2Dev), cudaMemcpyHostToDevice), "upload");
+  ck(cudaMemcpyAsync(d_dsets_, h_dsets_.data(), D_ * sizeof(DSet2Dev), cudaMemcpyHostToDevice, stream_), "upload");
   gx_ = (n + NT - 1) / NT;
   gy_ = (n - 1 + RB_MIN - 1) / RB_MIN;  // the most row groups any tuning uses
   nrt_ = (n + RTILE - 1) / RTILE;
@@ -2438,6 +2350,8 @@ void Engine2::build_static() {
   static_ok_ = true;
   drop_plans();
   setup_colspec();
+  // the uploads went through this engine's stream; launches may go to others
+  ck(cudaStreamSynchronize(stream_), "uploads");
   const unsigned P = ws_.P;
   free_work();
   if (P) reserve(P);
@@ -2502,7 +2416,9 @@ void Engine2::reserve(unsigned P) {
   ws_.pdout = dal<double>(n * n);
   ws_.logl = dal<double>(P);
   ws_.status = dal<int>(P);
-  ck(cudaMemset(ws_.redge, 0, static_cast<size_t>(P) * B_ * (2 * n + 1) * sizeof(double)), "memset");
+  ck(cudaMemsetAsync(ws_.redge, 0, static_cast<size_t>(P) * B_ * (2 * n + 1) * sizeof(double),
+                     stream_), "memset");
+  ck(cudaStreamSynchronize(stream_), "memset");
   ck(cudaFuncSetAttribute(k_psplit2, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           static_cast<int>(3 * 8192 * sizeof(double))), "attr");
 }
@@ -2513,19 +2429,10 @@ void Engine2::setup_colspec() {
   colspec_ = fft_mode_ == 1 && (n == 512 || n == 1024 || n == 2048 || n == 4096);
   if (!colspec_) return;
   if (!d_ctw_) {
-    // W_n^{u 2^i} at [i][u], u < n / 16, i < 4 (the second stage's W_{n/16}^s
-    // at u = 16 s)
-    std::vector<double2> tw(n / 4);
-    const long double tau = 6.283185307179586476925286766559005768L;
-    for (unsigned u = 0; u < n / 16; ++u)
-      for (unsigned i = 0; i < 4; ++i) {
-        const unsigned e = (u << i) % n;
-        const long double a = -tau * static_cast<long double>(e) / static_cast<long double>(n);
-        tw[i * (n / 16) + u] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
-      }
+    const std::vector<double2> tw = fft::fft2_twiddles(n);
     d_ctw_ = dal<double2>(tw.size());
     static_allocs_.push_back(d_ctw_);
-    ck(cudaMemcpy(d_ctw_, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice), "upload");
+    ck(cudaMemcpyAsync(d_ctw_, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, stream_), "upload");
   }
 #define POFD_ATTR2(NN)                                                                       \
   {                                                                                          \
@@ -2561,8 +2468,12 @@ void Engine2::set_fft_mode(int mode) {
   fft_mode_ = mode;
   if (device_ >= 0) ck(cudaSetDevice(device_), "cudaSetDevice");
   drop_plans();
-  if (static_ok_) setup_colspec();
-  else colspec_ = false;
+  if (static_ok_) {
+    setup_colspec();
+    ck(cudaStreamSynchronize(stream_), "uploads");
+  } else {
+    colspec_ = false;
+  }
   if (ws_.rbuf && ws_.rrows < rbuf_rows()) {  // the modes keep different grids in rbuf
     const unsigned P = ws_.P;
     free_work();
@@ -3036,7 +2947,7 @@ void Engine2::rgrid_host(int bs, const float* theta, unsigned npar, double* out)
   double ll;
   int st;
   eval_host(1, theta, npar, &ll, &st);  // staging, plans
-  ck(cudaMemcpy(ws_.theta_in, theta, npar * sizeof(float), cudaMemcpyHostToDevice), "H2D");
+  ck(cudaMemcpyAsync(ws_.theta_in, theta, npar * sizeof(float), cudaMemcpyHostToDevice, stream_), "H2D");
   launch_all(1, ws_.theta_in, npar, ws_.logl, ws_.status, stream_, nullptr, true);
   const size_t n = n_, nc2 = 2 * (n / 2 + 1);
   ck(cudaMemcpy2DAsync(out, n * sizeof(double), ws_.rbuf + static_cast<size_t>(bs) * n * nc2,
