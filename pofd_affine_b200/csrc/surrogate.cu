@@ -8,6 +8,7 @@
 //   FP32 master weights and Adam moments.
 #include "surrogate.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <limits>
@@ -52,16 +53,27 @@ __device__ __forceinline__ float dsilu(float z) {
   const int m0 = blockIdx.x * umma::kRows, n0 = blockIdx.y * g.ntile;         \
   const uint32_t tb = umma::mainloop(g, &tmA, &tmB, m0, n0, smem, bs);        \
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;                 \
-  const int row = m0 + warp * 32 + lane;                                      \
-  const uint32_t tlane = static_cast<uint32_t>(warp * 32) << 16;
+  const int row = m0 + (warp & 3) * 32 + lane;                                \
+  const uint32_t tlane = static_cast<uint32_t>((warp & 3) * 32) << 16;        \
+  const int wg = warp >> 2; /* warps w, w + 4, ... share the rows' columns */
 
-__device__ __forceinline__ void st_bf16x16(bf16* dst, const float* v) {
-  __align__(16) bf16 h[16];
+__device__ __forceinline__ void st_bf16x4(bf16* dst, const float* v) {
+  __align__(8) bf16 h[4];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) h[j] = __float2bfloat16_rn(v[j]);
-  reinterpret_cast<uint4*>(dst)[0] = reinterpret_cast<const uint4*>(h)[0];
-  reinterpret_cast<uint4*>(dst)[1] = reinterpret_cast<const uint4*>(h)[1];
+  for (int j = 0; j < 4; ++j) h[j] = __float2bfloat16_rn(v[j]);
+  *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(h);
 }
+
+// The kernels of a training iteration overlap their launches (each waits for
+// the one before it inside, umma::mainloop or pdl_wait).  What an earlier
+// kernel of the sequence writes therefore comes through pointers without
+// __restrict__: the compiler may move loads that it takes for invariant
+// ahead of the wait.
+//
+// The epilogues are chains of dependent special functions and divisions over
+// few elements: with four columns a thread (512 threads a block; 16 columns a
+// tile) instead of sixteen they are a quarter as long.
+constexpr int NTE = 512;
 
 // Plain product C = A B^T in FP32 (a checkable entry point of the tensor-core
 // main loop).
@@ -81,78 +93,74 @@ __global__ void __launch_bounds__(NT) k_gemm_f32(const __grid_constant__ CUtenso
   umma::release(bs, g.ntile);
 }
 
-// Hidden layer forward: z = A W^T + b, h = silu(z); writes h (bf16,
-// [M][ldh]) and, when given, z (fp32 [M][N]) and h^T (bf16 [N][ldt]).  The
-// last hidden layer also writes this column tile's part of the network
-// output, ypart[tile][row] = h . w4 (+ b4 in tile 0).
-__global__ void __launch_bounds__(NT) k_fwd(const __grid_constant__ CUtensorMap tmA,
-                                            const __grid_constant__ CUtensorMap tmB,
-                                            umma::GemmShape g, const float* __restrict__ bias,
-                                            bf16* __restrict__ h, int ldh,
-                                            float* __restrict__ z, bf16* __restrict__ ht,
-                                            int ldt, const float* __restrict__ w4,
-                                            const float* __restrict__ b4,
-                                            float* __restrict__ ypart) {
+// Hidden layer forward: z = A W^T + b, h = silu(z); writes what is given of
+// h (bf16, [M][ldh]), z (fp32 [M][N]) and h^T (bf16 [N][ldt]).  The last
+// hidden layer also writes this column tile's part of the network output,
+// ypart[tile][row] = h . w4 (+ b4 in tile 0), summed in column order.
+__global__ void __launch_bounds__(NTE) k_fwd(const __grid_constant__ CUtensorMap tmA,
+                                             const __grid_constant__ CUtensorMap tmB,
+                                             umma::GemmShape g, const float* bias, bf16* h,
+                                             int ldh, float* z, bf16* ht, int ldt,
+                                             const float* w4, const float* b4, float* ypart) {
   UMMA_PROLOGUE
   if (tb != 0xFFFFFFFFu) {
     float yacc = 0.0f;
-    for (int c0 = 0; c0 < g.ntile; c0 += 16) {
-      float v[16], hv[16];
-      umma::tmem_ld16(tb + tlane + c0, v);
+    float* hs = reinterpret_cast<float*>(smem);  // the operands are done with
+    for (int c0 = wg * 4; c0 < g.ntile; c0 += 16) {
+      float v[4], hv[4];
+      umma::tmem_ld4(tb + tlane + c0, v);
       const int cb = n0 + c0;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
+      for (int j = 0; j < 4; ++j) {
         v[j] += bias[cb + j];
         hv[j] = silu(v[j]);
       }
       if (row < g.M) {
-        st_bf16x16(h + static_cast<size_t>(row) * ldh + cb, hv);
-        if (z) {
-          float4* zp = reinterpret_cast<float4*>(z + static_cast<size_t>(row) * g.N + cb);
+        if (h) st_bf16x4(h + static_cast<size_t>(row) * ldh + cb, hv);
+        if (z)
+          *reinterpret_cast<float4*>(z + static_cast<size_t>(row) * g.N + cb) =
+              make_float4(v[0], v[1], v[2], v[3]);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) zp[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
+        for (int j = 0; j < 4; ++j) {
           const bf16 hb = __float2bfloat16_rn(hv[j]);
           if (ht) ht[static_cast<size_t>(cb + j) * ldt + row] = hb;
-          if (w4) yacc += __bfloat162float(hb) * w4[cb + j];
+          if (w4) hs[(c0 + j) * umma::kRows + (row - m0)] = __bfloat162float(hb);
         }
       }
     }
-    if (w4 && row < g.M)
-      ypart[static_cast<size_t>(blockIdx.y) * g.M + row] = yacc + (blockIdx.y == 0 ? b4[0] : 0.0f);
+    if (w4) {
+      __syncthreads();
+      if (wg == 0 && row < g.M) {
+        for (int c = 0; c < g.ntile; ++c) yacc += hs[c * umma::kRows + (row - m0)] * w4[n0 + c];
+        ypart[static_cast<size_t>(blockIdx.y) * g.M + row] = yacc + (blockIdx.y == 0 ? b4[0] : 0.0f);
+      }
+    }
   }
   umma::release(bs, g.ntile);
 }
 
 // Backward through a hidden layer: dh = dZ_next W_next (this GEMM, with B =
-// W_next^T), dz = dh * silu'(z); writes dz (bf16 [M][N]) and dz^T (bf16
-// [N][ldt]).
-__global__ void __launch_bounds__(NT) k_bwd_dx(const __grid_constant__ CUtensorMap tmA,
-                                               const __grid_constant__ CUtensorMap tmB,
-                                               umma::GemmShape g, const float* __restrict__ z,
-                                               bf16* __restrict__ dz, bf16* __restrict__ dzt,
-                                               int ldt) {
+// W_next^T), dz = dh * silu'(z); writes dz (bf16 [M][N], when given) and dz^T
+// (bf16 [N][ldt]).
+__global__ void __launch_bounds__(NTE) k_bwd_dx(const __grid_constant__ CUtensorMap tmA,
+                                                const __grid_constant__ CUtensorMap tmB,
+                                                umma::GemmShape g, const float* z, bf16* dz,
+                                                bf16* dzt, int ldt) {
   UMMA_PROLOGUE
   if (tb != 0xFFFFFFFFu) {
-    for (int c0 = 0; c0 < g.ntile; c0 += 16) {
-      float v[16];
-      umma::tmem_ld16(tb + tlane + c0, v);
+    for (int c0 = wg * 4; c0 < g.ntile; c0 += 16) {
+      float v[4];
+      umma::tmem_ld4(tb + tlane + c0, v);
       const int cb = n0 + c0;
       if (row < g.M) {
-        const float4* zp = reinterpret_cast<const float4*>(z + static_cast<size_t>(row) * g.N + cb);
+        const float4 zz = *reinterpret_cast<const float4*>(z + static_cast<size_t>(row) * g.N + cb);
+        v[0] *= dsilu(zz.x);
+        v[1] *= dsilu(zz.y);
+        v[2] *= dsilu(zz.z);
+        v[3] *= dsilu(zz.w);
+        if (dz) st_bf16x4(dz + static_cast<size_t>(row) * g.N + cb, v);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 zz = zp[q];
-          v[4 * q] *= dsilu(zz.x);
-          v[4 * q + 1] *= dsilu(zz.y);
-          v[4 * q + 2] *= dsilu(zz.z);
-          v[4 * q + 3] *= dsilu(zz.w);
-        }
-        st_bf16x16(dz + static_cast<size_t>(row) * g.N + cb, v);
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
+        for (int j = 0; j < 4; ++j)
           dzt[static_cast<size_t>(cb + j) * ldt + row] = __float2bfloat16_rn(v[j]);
       }
     }
@@ -164,195 +172,229 @@ struct AdamArgs {
   float lr, b1, b2, eps, bc1, bc2;  // bc = 1 - beta^t
 };
 
-// Weight gradient G = dZ^T X (this GEMM: A = dZ^T [Nout x M], B = X^T
-// [Nin x M]) followed by the Adam step of W [Nout][Nin]; writes the bf16
-// copies W (row-major) and W^T.  grad_out, when given, receives G instead
-// of the update (gradient checks).
-__global__ void __launch_bounds__(NT) k_wgrad_adam(const __grid_constant__ CUtensorMap tmA,
-                                                   const __grid_constant__ CUtensorMap tmB,
-                                                   umma::GemmShape g, AdamArgs ad,
-                                                   float* __restrict__ W, float* __restrict__ m,
-                                                   float* __restrict__ v, bf16* __restrict__ Wb,
-                                                   int ldwb, bf16* __restrict__ Wt, int ldwt,
-                                                   float* __restrict__ grad_out) {
-  UMMA_PROLOGUE
-  if (tb != 0xFFFFFFFFu) {
-    for (int c0 = 0; c0 < g.ntile; c0 += 16) {
-      float gv[16];
-      umma::tmem_ld16(tb + tlane + c0, gv);
-      const int cb = n0 + c0;
-      if (row >= g.M) continue;
-      const size_t i0 = static_cast<size_t>(row) * g.N + cb;
-      if (grad_out) {
-        float4* gp = reinterpret_cast<float4*>(grad_out + i0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) gp[q] = make_float4(gv[4 * q], gv[4 * q + 1], gv[4 * q + 2], gv[4 * q + 3]);
-        continue;
-      }
-      float w[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const size_t i = i0 + j;
-        const float mm = ad.b1 * m[i] + (1.0f - ad.b1) * gv[j];
-        const float vv = ad.b2 * v[i] + (1.0f - ad.b2) * gv[j] * gv[j];
-        m[i] = mm;
-        v[i] = vv;
-        w[j] = W[i] - ad.lr * (mm / ad.bc1) / (sqrtf(vv / ad.bc2) + ad.eps);
-        W[i] = w[j];
-      }
-      st_bf16x16(Wb + static_cast<size_t>(row) * ldwb + cb, w);
-      if (Wt)
-        for (int j = 0; j < 16; ++j)
-          Wt[static_cast<size_t>(cb + j) * ldwt + row] = __float2bfloat16_rn(w[j]);
-    }
-  }
-  umma::release(bs, g.ntile);
-}
-
-// ------------------------------------------------------ elementwise kernels
-// Whitened, zero-padded bf16 inputs x [Mp][16] and x^T [16][Mp] from theta
-// rows (free parameters only): x = W (theta_free - mu), W [16][16] row-major
-// (lower triangular); rows >= M are zero.
-__global__ void k_pack_inputs(int M, int Mp, const float* __restrict__ theta, int npar,
-                              const int* __restrict__ idx, int nin,
-                              const float* __restrict__ mu, const float* __restrict__ wm,
-                              const int* __restrict__ rows, bf16* __restrict__ x,
-                              bf16* __restrict__ xt) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= Mp) return;
-  const int src = (r < M) ? (rows ? rows[r] : r) : -1;
-  float d[Surrogate::kInPad];
-#pragma unroll
-  for (int j = 0; j < Surrogate::kInPad; ++j)
-    d[j] = (src >= 0 && j < nin) ? theta[static_cast<size_t>(src) * npar + idx[j]] - mu[j] : 0.0f;
-#pragma unroll
-  for (int k = 0; k < Surrogate::kInPad; ++k) {
-    float v = 0.0f;
-#pragma unroll
-    for (int j = 0; j < Surrogate::kInPad; ++j) v = fmaf(wm[k * Surrogate::kInPad + j], d[j], v);
-    const bf16 b = __float2bfloat16_rn(v);
-    x[static_cast<size_t>(r) * Surrogate::kInPad + k] = b;
-    if (xt) xt[static_cast<size_t>(k) * Mp + r] = b;
-  }
-}
-
-// Network output y = sum of the column-tile parts, the loss and
-// dy = 2 (y - t) / M.
-__global__ void k_out_loss(int M, int Mp, int ntiles, const float* __restrict__ ypart,
-                           const float* __restrict__ t, float* __restrict__ y,
-                           float* __restrict__ dy_out, float* __restrict__ loss) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= Mp) return;
-  float yy = 0.0f;
-  for (int k = 0; k < ntiles; ++k) yy += ypart[static_cast<size_t>(k) * Mp + r];
-  y[r] = yy;
-  const float d = (r < M) ? (yy - t[r]) : 0.0f;
-  dy_out[r] = 2.0f * d / static_cast<float>(M);
-  if (r < M) atomicAdd(loss, d * d / static_cast<float>(M));
-}
-
-// dz3 = dy w4 * silu'(z3), one thread per (16-column chunk, row).
-__global__ void k_out_dz(int Mp, int H, const float* __restrict__ dy,
-                         const float* __restrict__ w4, const float* __restrict__ z3,
-                         bf16* __restrict__ dz3, bf16* __restrict__ dz3t) {
-  const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= static_cast<long long>(Mp) * (H / 16)) return;
-  const int r = static_cast<int>(e % Mp), c0 = static_cast<int>(e / Mp) * 16;
-  const float d = dy[r];
-  const float4* zp = reinterpret_cast<const float4*>(z3 + static_cast<size_t>(r) * H + c0);
-  float v[16];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const float4 zz = zp[q];
-    v[4 * q] = d * w4[c0 + 4 * q] * dsilu(zz.x);
-    v[4 * q + 1] = d * w4[c0 + 4 * q + 1] * dsilu(zz.y);
-    v[4 * q + 2] = d * w4[c0 + 4 * q + 2] * dsilu(zz.z);
-    v[4 * q + 3] = d * w4[c0 + 4 * q + 3] * dsilu(zz.w);
-  }
-  st_bf16x16(dz3 + static_cast<size_t>(r) * H + c0, v);
-#pragma unroll
-  for (int j = 0; j < 16; ++j) dz3t[static_cast<size_t>(c0 + j) * Mp + r] = __float2bfloat16_rn(v[j]);
+// One Adam step of one weight.  The roundings are spelled out: which product
+// of a sum goes into the fused operation is the compiler's choice otherwise,
+// and the weights and the biases keep the one that each has had.
+template <bool kBias>
+__device__ __forceinline__ void adam_step(const AdamArgs& ad, float g, float* p, float* m,
+                                          float* v) {
+  const float g1 = 1.0f - ad.b1, g2 = (1.0f - ad.b2) * g;
+  *m = kBias ? __fmaf_rn(g1, g, __fmul_rn(ad.b1, *m)) : __fmaf_rn(ad.b1, *m, __fmul_rn(g1, g));
+  *v = kBias ? __fmaf_rn(g2, g, __fmul_rn(ad.b2, *v)) : __fmaf_rn(ad.b2, *v, __fmul_rn(g2, g));
+  *p = __fsub_rn(*p, ad.lr * (*m / ad.bc1) / (sqrtf(*v / ad.bc2) + ad.eps));
 }
 
 // Gradients of w4 (sum_r dy h3[r]), b4 (sum dy) and the hidden biases
-// (column sums of dz), then their Adam steps; one block per vector entry.
+// (column sums of dz) and their Adam steps.
 struct BiasArgs {
   int Mp, H;
   const float* dy;
-  const bf16* h3;
-  const bf16* dz[3];
+  const bf16* h3t;      // [H][Mp]
+  const bf16* dzt[3];   // [H][Mp]
   float* p[5];   // b1, b2, b3, w4, b4
   float* m[5];
   float* v[5];
   float* grad_out[5];
 };
 
-__global__ void k_bias_adam(BiasArgs a, AdamArgs ad) {
-  __shared__ float sh[32];
-  const int H = a.H;
-  const int e = blockIdx.x;  // 0..3H: b1, b2, b3, w4 entries; 4H: b4
-  int which, c;
-  if (e < 3 * H) { which = e / H; c = e - which * H; }
-  else if (e < 4 * H) { which = 3; c = e - 3 * H; }
-  else { which = 4; c = 0; }
-  float s = 0.0f;
-  for (int r = threadIdx.x; r < a.Mp; r += blockDim.x) {
-    if (which < 3) s += __bfloat162float(a.dz[which][static_cast<size_t>(r) * H + c]);
-    else if (which == 3) s += a.dy[r] * __bfloat162float(a.h3[static_cast<size_t>(r) * H + c]);
-    else s += a.dy[r];
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float g = 0.0f;
-    for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) g += sh[w];
-    if (a.grad_out[which]) {
-      a.grad_out[which][c] = g;
-      return;
+// One warp per entry e: 0 .. 3H - 1 the hidden biases, 3H .. 4H - 1 w4, 4H
+// b4.  256 partial sums over rows 256 apart, each 32 of them (a lane's w-th)
+// added across the lanes, the eight in order.
+__device__ __forceinline__ void bias_adam(const BiasArgs& a, const AdamArgs& ad, int e) {
+  const int H = a.H, lane = threadIdx.x & 31;
+  if (e > 4 * H) return;
+  const int which = e / H, c = e - which * H;
+  const bf16* col = which < 3 ? a.dzt[which] + static_cast<size_t>(c) * a.Mp
+                   : which == 3 ? a.h3t + static_cast<size_t>(c) * a.Mp : nullptr;
+  float s[8];
+#pragma unroll
+  for (int w = 0; w < 8; ++w) s[w] = 0.0f;
+  for (int r0 = lane; r0 < a.Mp; r0 += 256) {
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const int r = r0 + 32 * w;
+      if (r < a.Mp) {
+        if (which < 3) s[w] += __bfloat162float(col[r]);
+        else if (which == 3) s[w] = __fadd_rn(s[w], __fmul_rn(a.dy[r], __bfloat162float(col[r])));
+        else s[w] += a.dy[r];
+      }
     }
-    float* p = a.p[which];
-    float* m = a.m[which];
-    float* v = a.v[which];
-    const float mm = ad.b1 * m[c] + (1.0f - ad.b1) * g;
-    const float vv = ad.b2 * v[c] + (1.0f - ad.b2) * g * g;
-    m[c] = mm;
-    v[c] = vv;
-    p[c] -= ad.lr * (mm / ad.bc1) / (sqrtf(vv / ad.bc2) + ad.eps);
+  }
+#pragma unroll
+  for (int w = 0; w < 8; ++w)
+    for (int o = 16; o > 0; o >>= 1) s[w] += __shfl_xor_sync(0xffffffffu, s[w], o);
+  if (lane == 0) {
+    float g = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) g += s[w];
+    if (a.grad_out[which]) a.grad_out[which][c] = g;
+    else adam_step<true>(ad, g, &a.p[which][c], &a.m[which][c], &a.v[which][c]);
   }
 }
 
-// Minibatch rows: Philox-free LCG hash of (iteration, slot) over the pairs
-// held (uniform with replacement).
-__global__ void k_pick_rows(int Mb, unsigned n, unsigned long long it,
-                            unsigned long long seed, int* __restrict__ rows) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= Mb) return;
-  unsigned long long x = seed ^ (it * 0x9E3779B97F4A7C15ull) ^ (static_cast<unsigned long long>(r) *
-                                                                 0xBF58476D1CE4E5B9ull);
+// One weight matrix of k_update: G = dZ^T X (A = dZ^T [Nout x M], B = X^T
+// [Nin x M]), the Adam step of W [Nout][Nin] and its bf16 copies W
+// (row-major) and W^T (may be null).  grad_out, when given, receives G
+// instead of the update (gradient checks).
+struct UpdateArgs {
+  CUtensorMap a, b;
+  umma::GemmShape g;
+  int blocks, rowtiles;
+  float *W, *m, *v, *grad_out;
+  bf16 *Wb, *Wt;
+};
+struct UpdateAll {
+  UpdateArgs w[3];
+};
+
+// All updates of an iteration in one launch: the tiles of the three weight
+// gradients, then the bias entries, 16 to a block.  They are independent once
+// the backward pass is through, and a few dozen tiles each: as launches of
+// their own, with 16 elements of Adam a thread, the three took 78 us and the
+// biases (one block per entry, columns of dz 2 H bytes apart) 6.5 us of the
+// iteration's 150 (512 rows, H = 256).
+__global__ void __launch_bounds__(NTE) k_update(const __grid_constant__ UpdateAll u, BiasArgs ba,
+                                                AdamArgs ad) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ umma::Barriers bs;
+  int blk = static_cast<int>(blockIdx.x), l = 0;
+  while (l < 3 && blk >= u.w[l].blocks) blk -= u.w[l++].blocks;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (l == 3) {
+    dev::pdl_launch();
+    dev::pdl_wait();
+    bias_adam(ba, ad, blk * (NTE / 32) + warp);
+    return;
+  }
+  const UpdateArgs& q = u.w[l];
+  const umma::GemmShape g = q.g;
+  const int m0 = (blk % q.rowtiles) * umma::kRows, n0 = (blk / q.rowtiles) * g.ntile;
+  const uint32_t tb = umma::mainloop(g, &q.a, &q.b, m0, n0, smem, bs);
+  const int row = m0 + (warp & 3) * 32 + lane;
+  const uint32_t tlane = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  if (tb != 0xFFFFFFFFu) {
+    for (int c0 = (warp >> 2) * 4; c0 < g.ntile; c0 += 16) {
+      float gv[4];
+      umma::tmem_ld4(tb + tlane + c0, gv);
+      const int cb = n0 + c0;
+      if (row < g.M) {
+        const size_t i0 = static_cast<size_t>(row) * g.N + cb;
+        if (q.grad_out) {
+          *reinterpret_cast<float4*>(q.grad_out + i0) = make_float4(gv[0], gv[1], gv[2], gv[3]);
+        } else {
+          const float4 m4 = *reinterpret_cast<const float4*>(q.m + i0);
+          const float4 v4 = *reinterpret_cast<const float4*>(q.v + i0);
+          const float4 w4 = *reinterpret_cast<const float4*>(q.W + i0);
+          float m[4] = {m4.x, m4.y, m4.z, m4.w}, v[4] = {v4.x, v4.y, v4.z, v4.w};
+          float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) adam_step<false>(ad, gv[j], &w[j], &m[j], &v[j]);
+          *reinterpret_cast<float4*>(q.m + i0) = make_float4(m[0], m[1], m[2], m[3]);
+          *reinterpret_cast<float4*>(q.v + i0) = make_float4(v[0], v[1], v[2], v[3]);
+          *reinterpret_cast<float4*>(q.W + i0) = make_float4(w[0], w[1], w[2], w[3]);
+          st_bf16x4(q.Wb + i0, w);
+          if (q.Wt)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              q.Wt[static_cast<size_t>(cb + j) * g.M + row] = __float2bfloat16_rn(w[j]);
+        }
+      }
+    }
+  }
+  umma::release(bs, g.ntile);
+}
+
+// ------------------------------------------------------ elementwise kernels
+__device__ __forceinline__ int pick_row(const Pick& p, int r) {
+  if (p.n == 0) return r;
+  unsigned long long x = p.seed ^ (p.it * 0x9E3779B97F4A7C15ull) ^
+                         (static_cast<unsigned long long>(r) * 0xBF58476D1CE4E5B9ull);
   // splitmix64 finaliser (Steele, Lea & Flood 2014)
   x ^= x >> 30;
   x *= 0xBF58476D1CE4E5B9ull;
   x ^= x >> 27;
   x *= 0x94D049BB133111EBull;
   x ^= x >> 31;
-  rows[r] = static_cast<int>((x >> 32) * static_cast<unsigned long long>(n) >> 32);
+  return static_cast<int>((x >> 32) * static_cast<unsigned long long>(p.n) >> 32);
 }
 
-// Targets (logL - ymax, floored at -clip) / ys.
-__global__ void k_gather_targets(int M, const int* __restrict__ rows,
-                                 const double* __restrict__ logl, double ymax, double clip,
-                                 double iys, float* __restrict__ t) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= M) return;
-  const double d = logl[rows ? rows[r] : r] - ymax;
-  t[r] = static_cast<float>((d < -clip ? -clip : d) * iys);
+
+// Whitened, zero-padded bf16 inputs x [Mp][16] and x^T [16][Mp] (may be
+// null) from theta rows (free parameters only): x = W (theta_free - mu), W
+// [16][16] row-major (lower triangular); rows >= M are zero.  And the rows'
+// targets, and the loss to zero.  A thread per (row, input): with a thread
+// per row its 256 loads of W and products were 12 us for 512 rows.
+__global__ void __launch_bounds__(256) k_pack_inputs(int M, int Mp, const float* theta, int npar,
+                                                     const int* idx, int nin, const float* mu,
+                                                     const float* wm, Pick pick, Targets tg,
+                                                     bf16* x, bf16* xt) {
+  static_assert(Surrogate::kInPad == 16, "half a warp to a row");
+  dev::pdl_launch();
+  dev::pdl_wait();
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = e >> 4, k = e & 15;  // Mp * 16 is a multiple of the block size
+  const int src = (r < M) ? pick_row(pick, r) : -1;
+  const float dk =
+      (src >= 0 && k < nin) ? theta[static_cast<size_t>(src) * npar + idx[k]] - mu[k] : 0.0f;
+  float w[16];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 f = reinterpret_cast<const float4*>(wm)[k * 4 + q];
+    w[4 * q] = f.x;
+    w[4 * q + 1] = f.y;
+    w[4 * q + 2] = f.z;
+    w[4 * q + 3] = f.w;
+  }
+  float v = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v = fmaf(w[j], __shfl_sync(0xffffffffu, dk, j, 16), v);
+  const bf16 b = __float2bfloat16_rn(v);
+  x[e] = b;
+  if (xt) xt[static_cast<size_t>(k) * Mp + r] = b;
+  if (tg.t && k == 0) {
+    if (r == 0) *tg.loss = 0.0f;
+    if (r < M) {
+      const double d = tg.logl[src] - tg.ymax;
+      tg.t[r] = static_cast<float>((d < -tg.clip ? -tg.clip : d) * tg.iys);
+    }
+  }
+}
+
+// Network output y = sum of the column-tile parts, the loss, dy = 2 (y - t)
+// / M and dz3 = dy w4 * silu'(z3); one thread per (4-column chunk, row), the
+// first chunk's writes the row's values.
+__global__ void __launch_bounds__(256) k_out_dz(int M, int Mp, int H, int ntiles,
+                                                const float* ypart, const float* t, float* y,
+                                                float* dy_out, float* loss, const float* w4,
+                                                const float* z3, bf16* dz3, bf16* dz3t) {
+  dev::pdl_launch();
+  dev::pdl_wait();
+  const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e >= static_cast<long long>(Mp) * (H / 4)) return;
+  const int r = static_cast<int>(e % Mp), c0 = static_cast<int>(e / Mp) * 4;
+  const float4 zz = *reinterpret_cast<const float4*>(z3 + static_cast<size_t>(r) * H + c0);
+  float yy = 0.0f;
+  for (int k = 0; k < ntiles; ++k) yy += ypart[static_cast<size_t>(k) * Mp + r];
+  const float d = (r < M) ? (yy - t[r]) : 0.0f;
+  const float dy = 2.0f * d / static_cast<float>(M);
+  if (c0 == 0) {
+    y[r] = yy;
+    dy_out[r] = dy;
+    float q = d * d / static_cast<float>(M);  // 0 past M; a warp is 32 rows
+    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(loss, q);
+  }
+  const float v[4] = {dy * w4[c0] * dsilu(zz.x), dy * w4[c0 + 1] * dsilu(zz.y),
+                      dy * w4[c0 + 2] * dsilu(zz.z), dy * w4[c0 + 3] * dsilu(zz.w)};
+  st_bf16x4(dz3 + static_cast<size_t>(r) * H + c0, v);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) dz3t[static_cast<size_t>(c0 + j) * Mp + r] = __float2bfloat16_rn(v[j]);
 }
 
 // Network output to log-likelihood units: logL = ymax + ys * y.
-__global__ void k_unscale(int M, int Mp, int ntiles, const float* __restrict__ ypart,
-                          double ymax, double ys, double* __restrict__ out,
-                          int* __restrict__ status) {
+__global__ void k_unscale(int M, int Mp, int ntiles, const float* ypart, double ymax, double ys,
+                          double* out, int* status) {
+  dev::pdl_wait();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= M) return;
   float yy = 0.0f;
@@ -423,23 +465,22 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-// A row-major bf16 matrix [rows][K] (leading dimension ld elements) viewed
-// as [K/8][rows][8] so that a {8, box_rows, 8} box lands in the canonical
-// no-swizzle K-major layout; rows and K beyond the matrix read as zero.
+// A row-major bf16 matrix [rows][K] (leading dimension ld elements) in boxes
+// of box_rows x 64, 128 bytes of K a row, swizzled as the MMA descriptors of
+// umma::mainloop assume; rows and K beyond the matrix read as zero.
 CUtensorMap kmajor_map(const bf16* base, int rows, int K, int ld, int box_rows) {
   if (reinterpret_cast<uintptr_t>(base) % 16 || ld % 8 || K % 16)
     throw Error(POFD_E_ARG, "tensor map: base 16-byte aligned, ld multiple of 8, K multiple of 16");
   CUtensorMap m;
-  const cuuint64_t dims[3] = {8, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(K / 8)};
-  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, 16};
-  // the box is always {8, box_rows, 8}: rows and K groups past the matrix
-  // are zero-filled, so every stage holds exactly stage_bytes() and keeps the
-  // layout the MMA descriptors assume
-  const cuuint32_t box[3] = {8, static_cast<cuuint32_t>(box_rows), 8};
-  const cuuint32_t es[3] = {1, 1, 1};
-  const CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(base),
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
+  // the box is always whole: rows and K past the matrix are zero-filled, so
+  // every stage holds exactly stage_bytes()
+  const cuuint32_t box[2] = {umma::kKChunk, static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t es[2] = {1, 1};
+  const CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(base),
                                  dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw Error(POFD_E_CUDA, "cuTensorMapEncodeTiled failed");
   return m;
@@ -492,7 +533,7 @@ void set_gemm_attributes() {
   ck(cudaFuncSetAttribute(k_gemm_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr");
   ck(cudaFuncSetAttribute(k_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr");
   ck(cudaFuncSetAttribute(k_bwd_dx, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr");
-  ck(cudaFuncSetAttribute(k_wgrad_adam, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr");
+  ck(cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr");
   done = true;
 }
 
@@ -549,7 +590,7 @@ Surrogate::~Surrogate() {
   void* q[] = {idx_, mu_, wm_, w1b_, w2b_, w3b_, w2t_, w3t_, ptheta_, plogl_, counters_, err_,
                ws_.x, ws_.xt, ws_.h[0], ws_.h[1], ws_.h[2], ws_.ht[0], ws_.ht[1], ws_.ht[2],
                ws_.z[0], ws_.z[1], ws_.z[2], ws_.dz[0], ws_.dz[1], ws_.dz[2], ws_.dzt[0],
-               ws_.dzt[1], ws_.dzt[2], ws_.y, ws_.ypart, ws_.t, ws_.dy, ws_.rows, ws_.loss};
+               ws_.dzt[1], ws_.dzt[2], ws_.y, ws_.ypart, ws_.t, ws_.dy, ws_.loss};
   for (void* p : q)
     if (p) cudaFree(p);
 }
@@ -623,7 +664,7 @@ void Surrogate::ensure_work(int Mp) {
   if (Mp <= ws_.Mp) return;
   void* q[] = {ws_.x, ws_.xt, ws_.h[0], ws_.h[1], ws_.h[2], ws_.ht[0], ws_.ht[1], ws_.ht[2],
                ws_.z[0], ws_.z[1], ws_.z[2], ws_.dz[0], ws_.dz[1], ws_.dz[2], ws_.dzt[0],
-               ws_.dzt[1], ws_.dzt[2], ws_.y, ws_.ypart, ws_.t, ws_.dy, ws_.rows, ws_.loss};
+               ws_.dzt[1], ws_.dzt[2], ws_.y, ws_.ypart, ws_.t, ws_.dy, ws_.loss};
   for (void* p : q)
     if (p) cudaFree(p);
   ws_ = Work{};
@@ -642,19 +683,19 @@ void Surrogate::ensure_work(int Mp) {
   ws_.ypart = dal<float>(M * (umma::kMaxN / 16));
   ws_.t = dal<float>(M);
   ws_.dy = dal<float>(M);
-  ws_.rows = dal<int>(M);
   ws_.loss = dal<float>(1);
 }
 
-// Forward of M rows of theta (optionally gathered through rows) into
-// ws_.y; keeps z, h and h^T when train.
-void Surrogate::forward(int M, const float* theta, int npar, const int* rows, bool train,
+// Forward of M rows of theta (row r, or the picked one) into ws_.ypart; when
+// targets are given (training) keeps z and h^T and writes them too.
+void Surrogate::forward(int M, const float* theta, int npar, const Pick& pick, const Targets& tg,
                         cudaStream_t st) {
   const int Mp = (M + umma::kRows - 1) / umma::kRows * umma::kRows;
   ensure_work(Mp);
   const int H = static_cast<int>(H_);
-  k_pack_inputs<<<(Mp + 127) / 128, 128, 0, st>>>(M, Mp, theta, npar, idx_, static_cast<int>(nin_),
-                                                  mu_, wm_, rows, ws_.x, train ? ws_.xt : nullptr);
+  const bool train = tg.t != nullptr;
+  launch_pdl(k_pack_inputs, dim3(Mp * kInPad / 256), dim3(256), 0, st, M, Mp, theta, npar, idx_,
+             static_cast<int>(nin_), mu_, wm_, pick, tg, ws_.x, train ? ws_.xt : nullptr);
   const bf16* Ws[3] = {w1b_, w2b_, w3b_};
   const bf16* in = ws_.x;
   int ldin = kInPad;
@@ -662,9 +703,10 @@ void Surrogate::forward(int M, const float* theta, int npar, const int* rows, bo
     const int K = (l == 0) ? kInPad : H;
     const Gemm q = plan_gemm(Mp, H, K, in, ldin, Ws[l], K, err_);
     const bool last = (l == 2);
-    k_fwd<<<q.grid, NT, q.smem, st>>>(q.a, q.b, q.g, p_[2 * l + 1], ws_.h[l], H,
-                                      train ? ws_.z[l] : nullptr, train ? ws_.ht[l] : nullptr, Mp,
-                                      last ? p_[6] : nullptr, last ? p_[7] : nullptr, ws_.ypart);
+    launch_pdl(k_fwd, q.grid, dim3(NTE), q.smem, st, q.a, q.b, q.g, p_[2 * l + 1],
+               last ? nullptr : ws_.h[l], H, train ? ws_.z[l] : nullptr,
+               train ? ws_.ht[l] : nullptr, Mp, last ? p_[6] : nullptr, last ? p_[7] : nullptr,
+               ws_.ypart);
     in = ws_.h[l];
     ldin = H;
   }
@@ -677,11 +719,11 @@ void Surrogate::predict(unsigned n, const float* theta, unsigned npar, double* o
   if (npar < npar_) throw Error(POFD_E_ARG, "Not enough elements in params");
   ck(cudaSetDevice(device_), "cudaSetDevice");
   if (!st) st = stream_;
-  forward(static_cast<int>(n), theta, static_cast<int>(npar), nullptr, false, st);
+  forward(static_cast<int>(n), theta, static_cast<int>(npar), Pick{}, Targets{}, st);
   const int Mp = (static_cast<int>(n) + umma::kRows - 1) / umma::kRows * umma::kRows;
   const int ntiles = static_cast<int>(H_) / ntile_for(Mp, static_cast<int>(H_));
-  k_unscale<<<(n + 127) / 128, 128, 0, st>>>(static_cast<int>(n), Mp, ntiles, ws_.ypart, ymax_, ys_,
-                                             out, status);
+  launch_pdl(k_unscale, dim3((n + 127) / 128), dim3(128), 0, st, static_cast<int>(n), Mp, ntiles,
+             ws_.ypart, ymax_, ys_, out, status);
   ck(cudaGetLastError(), "k_unscale");
 }
 
@@ -818,52 +860,50 @@ void Surrogate::refresh_scaling() {
   scaled_ = true;
 }
 
-// One training iteration on Mb rows (rows of the pair buffer, or the first
-// Mb pairs when rows is null).  grads (8 tensors), when given, receive the
-// loss gradients and the weights are not updated.
-float Surrogate::iteration(int Mb, const int* rows, float lr, float** grads, cudaStream_t st) {
+// One training iteration on Mb rows (picked from the pair buffer, or its
+// first Mb).  grads (8 tensors), when given, receive the loss gradients and
+// the weights are not updated.  Eight launches: inputs and targets, three
+// layers forward, output, two layers backward, all updates.
+void Surrogate::iteration(int Mb, const Pick& pick, float lr, float** grads, cudaStream_t st) {
   const int Mp = (Mb + umma::kRows - 1) / umma::kRows * umma::kRows;
   const int H = static_cast<int>(H_);
-  forward(Mb, ptheta_, static_cast<int>(npar_), rows, true, st);
-  k_gather_targets<<<(Mb + 127) / 128, 128, 0, st>>>(Mb, rows, plogl_, ymax_, clip_, 1.0 / ys_,
-                                                     ws_.t);
-  ck(cudaMemsetAsync(ws_.loss, 0, sizeof(float), st), "memset");
+  forward(Mb, ptheta_, static_cast<int>(npar_), pick,
+          Targets{plogl_, ymax_, clip_, 1.0 / ys_, ws_.t, ws_.loss}, st);
   const int ntiles = H / ntile_for(Mp, H);
-  k_out_loss<<<(Mp + 127) / 128, 128, 0, st>>>(Mb, Mp, ntiles, ws_.ypart, ws_.t, ws_.y, ws_.dy,
-                                               ws_.loss);
-  {
-    const long long ne = static_cast<long long>(Mp) * (H / 16);
-    k_out_dz<<<static_cast<unsigned>((ne + 127) / 128), 128, 0, st>>>(Mp, H, ws_.dy, p_[6],
-                                                                     ws_.z[2], ws_.dz[2],
-                                                                     ws_.dzt[2]);
-  }
+  const long long ne = static_cast<long long>(Mp) * (H / 4);
+  launch_pdl(k_out_dz, dim3(static_cast<unsigned>((ne + 255) / 256)), dim3(256), 0, st, Mb, Mp, H,
+             ntiles, ws_.ypart, ws_.t, ws_.y, ws_.dy, ws_.loss, p_[6], ws_.z[2], ws_.dz[2],
+             ws_.dzt[2]);
   ++step_;
   AdamArgs ad{lr, 0.9f, 0.999f, 1e-8f, 1.0f - std::pow(0.9f, static_cast<float>(step_)),
               1.0f - std::pow(0.999f, static_cast<float>(step_))};
-  const bf16* Wt[3] = {nullptr, w2t_, w3t_};
   bf16* Wb[3] = {w1b_, w2b_, w3b_};
-  bf16* Wtw[3] = {nullptr, w2t_, w3t_};
-  for (int l = 2; l >= 0; --l) {
-    if (l > 0) {
-      // dh_{l-1} = dz_l W_l: A = dz_l [Mp x H], B = W_l^T [H x H]
-      const Gemm q = plan_gemm(Mp, H, H, ws_.dz[l], H, Wt[l], H, err_);
-      k_bwd_dx<<<q.grid, NT, q.smem, st>>>(q.a, q.b, q.g, ws_.z[l - 1], ws_.dz[l - 1],
-                                           ws_.dzt[l - 1], Mp);
-    }
+  bf16* Wt[3] = {nullptr, w2t_, w3t_};
+  for (int l = 2; l > 0; --l) {
+    // dh_{l-1} = dz_l W_l: A = dz_l [Mp x H], B = W_l^T [H x H]
+    const Gemm q = plan_gemm(Mp, H, H, ws_.dz[l], H, Wt[l], H, err_);
+    launch_pdl(k_bwd_dx, q.grid, dim3(NTE), q.smem, st, q.a, q.b, q.g, ws_.z[l - 1],
+               l > 1 ? ws_.dz[l - 1] : nullptr, ws_.dzt[l - 1], Mp);
+  }
+  UpdateAll u;
+  size_t smem = 0;
+  int blocks = 0;
+  for (int l = 0; l < 3; ++l) {
     // G_l = dz_l^T X_l: A = dz_l^T [H x Mp], B = X_l^T [Nin x Mp]
     const int nin = (l == 0) ? kInPad : H;
-    const bf16* XT = (l == 0) ? ws_.xt : ws_.ht[l - 1];
-    const Gemm q = plan_gemm(H, nin, Mp, ws_.dzt[l], Mp, XT, Mp, err_);
-    k_wgrad_adam<<<q.grid, NT, q.smem, st>>>(q.a, q.b, q.g, ad, p_[2 * l], m_[2 * l], v_[2 * l],
-                                             Wb[l], nin, Wtw[l], H,
-                                             grads ? grads[2 * l] : nullptr);
+    const Gemm q = plan_gemm(H, nin, Mp, ws_.dzt[l], Mp, (l == 0) ? ws_.xt : ws_.ht[l - 1], Mp, err_);
+    u.w[l] = UpdateArgs{q.a, q.b, q.g, static_cast<int>(q.grid.x * q.grid.y),
+                        static_cast<int>(q.grid.x), p_[2 * l], m_[2 * l], v_[2 * l],
+                        grads ? grads[2 * l] : nullptr, Wb[l], Wt[l]};
+    blocks += u.w[l].blocks;
+    smem = std::max(smem, q.smem);
   }
   BiasArgs ba{};
   ba.Mp = Mp;
   ba.H = H;
   ba.dy = ws_.dy;
-  ba.h3 = ws_.h[2];
-  for (int l = 0; l < 3; ++l) ba.dz[l] = ws_.dz[l];
+  ba.h3t = ws_.ht[2];
+  for (int l = 0; l < 3; ++l) ba.dzt[l] = ws_.dzt[l];
   const int map[5] = {1, 3, 5, 6, 7};
   for (int q = 0; q < 5; ++q) {
     ba.p[q] = p_[map[q]];
@@ -871,9 +911,9 @@ float Surrogate::iteration(int Mb, const int* rows, float lr, float** grads, cud
     ba.v[q] = v_[map[q]];
     ba.grad_out[q] = grads ? grads[map[q]] : nullptr;
   }
-  k_bias_adam<<<4 * H + 1, 256, 0, st>>>(ba, ad);
+  blocks += (4 * H + 1 + NTE / 32 - 1) / (NTE / 32);
+  launch_pdl(k_update, dim3(blocks), dim3(NTE), smem, st, u, ba, ad);
   ck(cudaGetLastError(), "surrogate training");
-  return 0.0f;
 }
 
 void Surrogate::train(unsigned iters, unsigned batch, float lr, float* last_loss) {
@@ -885,9 +925,7 @@ void Surrogate::train(unsigned iters, unsigned batch, float lr, float* last_loss
   ensure_work((Mb + umma::kRows - 1) / umma::kRows * umma::kRows);
   ck(cudaMemset(err_, 0, sizeof(int)), "memset");
   for (unsigned it = 0; it < iters; ++it) {
-    k_pick_rows<<<(Mb + 127) / 128, 128, 0, stream_>>>(Mb, n, static_cast<unsigned long long>(step_) + 1,
-                                                     seed_, ws_.rows);
-    iteration(Mb, ws_.rows, lr, nullptr, stream_);
+    iteration(Mb, Pick{n, static_cast<unsigned long long>(step_) + 1, seed_}, lr, nullptr, stream_);
   }
   ck(cudaStreamSynchronize(stream_), "synchronize");
   check_err();
@@ -901,7 +939,7 @@ void Surrogate::gradients(unsigned n, float** grads_dev, float* loss) {
   ensure_work((static_cast<int>(n) + umma::kRows - 1) / umma::kRows * umma::kRows);
   ck(cudaMemset(err_, 0, sizeof(int)), "memset");
   const unsigned s0 = step_;
-  iteration(static_cast<int>(n), nullptr, 0.0f, grads_dev, stream_);
+  iteration(static_cast<int>(n), Pick{}, 0.0f, grads_dev, stream_);
   step_ = s0;
   ck(cudaStreamSynchronize(stream_), "synchronize");
   check_err();

@@ -12,6 +12,21 @@
 
 namespace pofd {
 
+// Minibatch rows of iteration it: a hash of (iteration, slot) over the n
+// pairs held (uniform with replacement); n = 0: row r itself.
+struct Pick {
+  unsigned n = 0;
+  unsigned long long it = 0, seed = 0;
+};
+
+// Targets (logL - ymax, floored at -clip) / ys; t null: no targets.
+struct Targets {
+  const double* logl = nullptr;
+  double ymax = 0.0, clip = 0.0, iys = 0.0;
+  float* t = nullptr;
+  float* loss = nullptr;
+};
+
 class Surrogate {
  public:
   static constexpr int kInPad = 16;      // inputs padded to one MMA K step
@@ -49,9 +64,9 @@ class Surrogate {
   void init_weights();
   void refresh_bf16(const std::vector<std::vector<float>>& host);
   void ensure_work(int Mp);
-  void forward(int M, const float* theta, int npar, const int* rows, bool train,
+  void forward(int M, const float* theta, int npar, const Pick& pick, const Targets& tg,
                cudaStream_t st);
-  float iteration(int Mb, const int* rows, float lr, float** grads, cudaStream_t st);
+  void iteration(int Mb, const Pick& pick, float lr, float** grads, cudaStream_t st);
   void check_err();
 
   int device_;
@@ -84,7 +99,6 @@ class Surrogate {
     __nv_bfloat16* dz[3] = {};
     __nv_bfloat16* dzt[3] = {};
     float *y = nullptr, *ypart = nullptr, *t = nullptr, *dy = nullptr, *loss = nullptr;
-    int* rows = nullptr;
   } ws_;
 };
 
