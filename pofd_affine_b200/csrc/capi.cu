@@ -1263,11 +1263,7 @@ int pofd_surrogate_get_params(pofd_surrogate* s, int t, float* out, size_t* size
     need(s != nullptr, "null argument");
     need(t >= 0 && t < pofd::Surrogate::kNumTensors, "tensor index out of range");
     if (size) *size = s->s->tensor_size(t);
-    if (out) {
-      std::vector<std::vector<float>> h;
-      s->s->get_params_host(h);
-      std::memcpy(out, h[t].data(), h[t].size() * sizeof(float));
-    }
+    if (out) s->s->get_param_host(t, out);
     return POFD_OK;
   });
 }
@@ -1275,12 +1271,8 @@ int pofd_surrogate_get_params(pofd_surrogate* s, int t, float* out, size_t* size
 int pofd_surrogate_set_params(pofd_surrogate* s, const float* const* tensors) {
   return guard([&] {
     need(s && tensors, "null argument");
-    std::vector<std::vector<float>> h(pofd::Surrogate::kNumTensors);
-    for (int t = 0; t < pofd::Surrogate::kNumTensors; ++t) {
-      need(tensors[t] != nullptr, "null tensor");
-      h[t].assign(tensors[t], tensors[t] + s->s->tensor_size(t));
-    }
-    s->s->set_params_host(h);
+    for (int t = 0; t < pofd::Surrogate::kNumTensors; ++t) need(tensors[t] != nullptr, "null tensor");
+    s->s->set_params_host(tensors);
     return POFD_OK;
   });
 }

@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(NT) k_gemm_f32(const __grid_constant__ CUtenso
                                                  umma::GemmShape g, float* __restrict__ C,
                                                  int ldc) {
   UMMA_PROLOGUE
+  static_cast<void>(wg);
   if (tb != 0xFFFFFFFFu) {
     for (int c0 = 0; c0 < g.ntile; c0 += 16) {
       float v[16];
@@ -446,6 +447,144 @@ __global__ void k_append_pairs(int n, const float* __restrict__ theta, int npar,
   }
 }
 
+// --------------------------------------------- weights and scaling on device
+// bf16 copies of the weights, W and W^T.
+__global__ void k_pack_weights(int H, const float* __restrict__ W1, const float* __restrict__ W2,
+                               const float* __restrict__ W3, bf16* __restrict__ w1b,
+                               bf16* __restrict__ w2b, bf16* __restrict__ w2t,
+                               bf16* __restrict__ w3b, bf16* __restrict__ w3t) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < H * Surrogate::kInPad) w1b[i] = __float2bfloat16_rn(W1[i]);
+  if (i >= H * H) return;
+  const int r = i / H, k = i - r * H;
+  const bf16 b = __float2bfloat16_rn(W2[i]), c = __float2bfloat16_rn(W3[i]);
+  w2b[i] = b;
+  w2t[k * H + r] = b;
+  w3b[i] = c;
+  w3t[k * H + r] = c;
+}
+
+// Sums for the scaling of inputs and target over the n pairs held, in FP64:
+// three passes, since each needs the one before (the largest logL; the means
+// over the pairs near it; the covariance about them).  Block b takes rows [b
+// R, (b + 1) R); every entry is one thread's, which walks the block's rows;
+// the blocks' parts are added by whoever needs them next, in block order.  On
+// the host, with the pairs copied there, this was 0.5 ms for 8000 pairs of 14
+// inputs and grew with the pairs held; now 0.12 ms with the transfers.
+constexpr int kScT = 160;           // threads: covariance entries and more
+constexpr int kScCov = Surrogate::kInPad * (Surrogate::kInPad + 1) / 2;
+constexpr int kScPart = 160;        // doubles a block writes per pass
+// pass 1: sums over the pairs near the maximum and over all, count, target
+constexpr int kScAll = 16, kScCount = 32, kScTarget = 33;
+static_assert(kScCov < kScT && kScCov < kScPart, "one thread per entry");
+
+struct ScaleArgs {
+  int n, R, G, npar, nin;
+  double clip;
+  const float* theta;
+  const double* logl;
+  const int* idx;
+  double* part[3];  // [G][kScPart] of each pass
+  double* out;      // [kScPart] pass 1 sums, [kScPart] pass 2 sums, max
+};
+
+__device__ __forceinline__ double scale_max(const ScaleArgs& a, double* sh) {
+  const double none = -__longlong_as_double(0x7ff0000000000000ll);
+  double mx = none;
+  for (int b = threadIdx.x; b < a.G; b += kScT) mx = fmax(mx, a.part[0][static_cast<size_t>(b) * kScPart]);
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = sh[0];
+  for (int w = 1; w < kScT / 32; ++w) mx = fmax(mx, sh[w]);
+  __syncthreads();
+  return mx;
+}
+
+__device__ __forceinline__ double scale_total(const ScaleArgs& a, int pass, int e) {
+  double s = 0.0;
+#pragma unroll 8
+  for (int b = 0; b < a.G; ++b) s += a.part[pass][static_cast<size_t>(b) * kScPart + e];
+  return s;
+}
+
+template <int PASS>
+__global__ void __launch_bounds__(kScT) k_scale(ScaleArgs a) {
+  __shared__ double sh[kScT], mean[Surrogate::kInPad];
+  const int e = threadIdx.x, b = blockIdx.x, K = a.nin;
+  const int r0 = min(b * a.R, a.n), r1 = min(r0 + a.R, a.n);
+  if (PASS == 0) {
+    double mx = -__longlong_as_double(0x7ff0000000000000ll);
+    for (int r = r0 + e; r < r1; r += kScT) mx = fmax(mx, a.logl[r]);
+    sh[e] = mx;
+    __syncthreads();
+    if (e == 0) {
+      for (int w = 1; w < kScT; ++w) mx = fmax(mx, sh[w]);
+      a.part[0][static_cast<size_t>(b) * kScPart] = mx;
+    }
+    return;
+  }
+  const double mx = scale_max(a, sh);
+  if (PASS == 1) {
+    double s = 0.0;
+    const bool col = e < K || (e >= kScAll && e < kScAll + K);
+    if (col) {
+      const int p = a.idx[e & 15];
+#pragma unroll 8
+      for (int r = r0; r < r1; ++r) {
+        const double v = a.theta[static_cast<size_t>(r) * a.npar + p];
+        s += (e >= kScAll || a.logl[r] - mx > -a.clip) ? v : 0.0;
+      }
+    } else if (e == kScCount) {
+      for (int r = r0; r < r1; ++r) s += (a.logl[r] - mx > -a.clip) ? 1.0 : 0.0;
+    } else if (e == kScTarget) {
+#pragma unroll 8
+      for (int r = r0; r < r1; ++r) {
+        const double d = a.logl[r] - mx;
+        s += d < -a.clip ? -a.clip : d;
+      }
+    }
+    a.part[1][static_cast<size_t>(b) * kScPart + e] = s;
+    return;
+  }
+  // means over the pairs within the clip of the maximum if they are enough
+  sh[e] = e <= kScTarget ? scale_total(a, 1, e) : 0.0;
+  __syncthreads();
+  const bool all = sh[kScCount] < (2 * K > 64 ? 2 * K : 64);
+  const double nu = all ? a.n : sh[kScCount];
+  if (e < K) mean[e] = sh[(all ? kScAll : 0) + e] / nu;
+  const double m = sh[kScTarget] / a.n;
+  if (b == 0) {
+    a.out[e] = sh[e];
+    if (e == 0) a.out[2 * kScPart] = mx;
+  }
+  __syncthreads();
+  double s = 0.0;
+  if (e < K * (K + 1) / 2) {
+    int i = 0;
+    while ((i + 1) * (i + 2) / 2 <= e) ++i;
+    const int j = e - i * (i + 1) / 2, pi = a.idx[i], pj = a.idx[j];
+#pragma unroll 8
+    for (int r = r0; r < r1; ++r) {
+      const float* t = a.theta + static_cast<size_t>(r) * a.npar;
+      const double q = (t[pi] - mean[i]) * (t[pj] - mean[j]);
+      s += (all || a.logl[r] - mx > -a.clip) ? q : 0.0;
+    }
+  } else if (e == kScT - 1) {
+#pragma unroll 8
+    for (int r = r0; r < r1; ++r) {
+      const double d = a.logl[r] - mx;
+      const double q = (d < -a.clip ? -a.clip : d) - m;
+      s += q * q;
+    }
+  }
+  a.part[2][static_cast<size_t>(b) * kScPart + e] = s;
+}
+
+__global__ void __launch_bounds__(kScT) k_scale_out(ScaleArgs a) {
+  a.out[kScPart + threadIdx.x] = scale_total(a, 2, threadIdx.x);
+}
+
 // ----------------------------------------------------------- tensor maps
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                               const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -554,8 +693,8 @@ Surrogate::Surrogate(int device, cudaStream_t stream, unsigned npar, const int* 
   ck(cudaSetDevice(device_), "cudaSetDevice");
   idx_ = dal<int>(kInPad);
   ck(cudaMemcpy(idx_, free_idx, nin * sizeof(int), cudaMemcpyHostToDevice), "upload");
-  mu_ = dal<float>(kInPad);
-  wm_ = dal<float>(kInPad * kInPad);
+  wm_ = dal<float>(kInPad * kInPad + kInPad);
+  mu_ = wm_ + kInPad * kInPad;
   std::vector<float> eye(kInPad * kInPad, 0.0f);
   for (int k = 0; k < kInPad; ++k) eye[k * kInPad + k] = 1.0f;
   ck(cudaMemcpy(wm_, eye.data(), eye.size() * sizeof(float), cudaMemcpyHostToDevice), "upload");
@@ -563,9 +702,16 @@ Surrogate::Surrogate(int device, cudaStream_t stream, unsigned npar, const int* 
   const size_t sz[kNumTensors] = {H * kInPad, H, H * H, H, H * H, H, H, 1};
   for (int t = 0; t < kNumTensors; ++t) {
     size_[t] = sz[t];
-    p_[t] = dal<float>(sz[t]);
-    m_[t] = dal<float>(sz[t]);
-    v_[t] = dal<float>(sz[t]);
+    slab_ += (sz[t] + 63) / 64 * 64;
+  }
+  p_[0] = dal<float>(slab_);  // all tensors in one allocation, 256-byte aligned
+  m_[0] = dal<float>(slab_);
+  v_[0] = dal<float>(slab_);
+  for (int t = 1; t < kNumTensors; ++t) {
+    const size_t step = (sz[t - 1] + 63) / 64 * 64;
+    p_[t] = p_[t - 1] + step;
+    m_[t] = m_[t - 1] + step;
+    v_[t] = v_[t - 1] + step;
   }
   w1b_ = dal<bf16>(H * kInPad);
   w2b_ = dal<bf16>(H * H);
@@ -576,18 +722,20 @@ Surrogate::Surrogate(int device, cudaStream_t stream, unsigned npar, const int* 
   plogl_ = dal<double>(cap_);
   counters_ = dal<unsigned>(4);
   err_ = dal<int>(1);
+  int sms = 0;
+  ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "attr");
+  scale_blocks_ = sms > 0 ? sms : 1;
+  scale_ = dal<double>(static_cast<size_t>(3 * scale_blocks_ + 3) * kScPart);
+  static_assert(3 * kScPart * sizeof(double) >= (kInPad + 1) * kInPad * sizeof(float), "staging");
+  ck(cudaMallocHost(reinterpret_cast<void**>(&h_stage_), 3 * kScPart * sizeof(double)), "cudaMallocHost");
   set_gemm_attributes();
   init_weights();
 }
 
 Surrogate::~Surrogate() {
   cudaSetDevice(device_);
-  for (int t = 0; t < kNumTensors; ++t) {
-    cudaFree(p_[t]);
-    cudaFree(m_[t]);
-    cudaFree(v_[t]);
-  }
-  void* q[] = {idx_, mu_, wm_, w1b_, w2b_, w3b_, w2t_, w3t_, ptheta_, plogl_, counters_, err_,
+  if (h_stage_) cudaFreeHost(h_stage_);
+  void* q[] = {p_[0], m_[0], v_[0], scale_, idx_, wm_, w1b_, w2b_, w3b_, w2t_, w3t_, ptheta_, plogl_, counters_, err_,
                ws_.x, ws_.xt, ws_.h[0], ws_.h[1], ws_.h[2], ws_.ht[0], ws_.ht[1], ws_.ht[2],
                ws_.z[0], ws_.z[1], ws_.z[2], ws_.dz[0], ws_.dz[1], ws_.dz[2], ws_.dzt[0],
                ws_.dzt[1], ws_.dzt[2], ws_.y, ws_.ypart, ws_.t, ws_.dy, ws_.loss};
@@ -618,46 +766,29 @@ void Surrogate::init_weights() {
       host[t][i] = static_cast<float>((2.0 * next() - 1.0) * a);
     }
   }
-  set_params_host(host);
+  const float* ptr[kNumTensors];
+  for (int t = 0; t < kNumTensors; ++t) ptr[t] = host[t].data();
+  set_params_host(ptr);
 }
 
-void Surrogate::set_params_host(const std::vector<std::vector<float>>& host) {
+void Surrogate::set_params_host(const float* const* host) {
   ck(cudaSetDevice(device_), "cudaSetDevice");
-  for (int t = 0; t < kNumTensors; ++t) {
-    ck(cudaMemcpy(p_[t], host[t].data(), size_[t] * sizeof(float), cudaMemcpyHostToDevice), "upload");
-    ck(cudaMemset(m_[t], 0, size_[t] * sizeof(float)), "memset");
-    ck(cudaMemset(v_[t], 0, size_[t] * sizeof(float)), "memset");
-  }
+  for (int t = 0; t < kNumTensors; ++t)
+    ck(cudaMemcpyAsync(p_[t], host[t], size_[t] * sizeof(float), cudaMemcpyHostToDevice, stream_), "upload");
+  ck(cudaMemsetAsync(m_[0], 0, slab_ * sizeof(float), stream_), "memset");
+  ck(cudaMemsetAsync(v_[0], 0, slab_ * sizeof(float), stream_), "memset");
   step_ = 0;
-  refresh_bf16(host);
+  const int H = static_cast<int>(H_);
+  k_pack_weights<<<(H * H + 255) / 256, 256, 0, stream_>>>(H, p_[0], p_[2], p_[4], w1b_, w2b_, w2t_,
+                                                         w3b_, w3t_);
+  ck(cudaGetLastError(), "k_pack_weights");
+  ck(cudaStreamSynchronize(stream_), "synchronize");  // other streams may use the weights
 }
 
-void Surrogate::refresh_bf16(const std::vector<std::vector<float>>& host) {
-  const size_t H = H_;
-  std::vector<bf16> a(H * kInPad), b(H * H), bt(H * H), c(H * H), ct(H * H);
-  for (size_t i = 0; i < H * kInPad; ++i) a[i] = __float2bfloat16_rn(host[0][i]);
-  for (size_t r = 0; r < H; ++r)
-    for (size_t k = 0; k < H; ++k) {
-      b[r * H + k] = __float2bfloat16_rn(host[2][r * H + k]);
-      bt[k * H + r] = b[r * H + k];
-      c[r * H + k] = __float2bfloat16_rn(host[4][r * H + k]);
-      ct[k * H + r] = c[r * H + k];
-    }
-  ck(cudaMemcpy(w1b_, a.data(), a.size() * sizeof(bf16), cudaMemcpyHostToDevice), "upload");
-  ck(cudaMemcpy(w2b_, b.data(), b.size() * sizeof(bf16), cudaMemcpyHostToDevice), "upload");
-  ck(cudaMemcpy(w2t_, bt.data(), bt.size() * sizeof(bf16), cudaMemcpyHostToDevice), "upload");
-  ck(cudaMemcpy(w3b_, c.data(), c.size() * sizeof(bf16), cudaMemcpyHostToDevice), "upload");
-  ck(cudaMemcpy(w3t_, ct.data(), ct.size() * sizeof(bf16), cudaMemcpyHostToDevice), "upload");
-}
-
-void Surrogate::get_params_host(std::vector<std::vector<float>>& host) const {
+void Surrogate::get_param_host(int t, float* out) const {
   ck(cudaSetDevice(device_), "cudaSetDevice");
+  ck(cudaMemcpyAsync(out, p_[t], size_[t] * sizeof(float), cudaMemcpyDeviceToHost, stream_), "D2H");
   ck(cudaStreamSynchronize(stream_), "synchronize");
-  host.resize(kNumTensors);
-  for (int t = 0; t < kNumTensors; ++t) {
-    host[t].resize(size_[t]);
-    ck(cudaMemcpy(host[t].data(), p_[t], size_[t] * sizeof(float), cudaMemcpyDeviceToHost), "D2H");
-  }
 }
 
 void Surrogate::ensure_work(int Mp) {
@@ -757,50 +888,45 @@ void Surrogate::pairs_host(unsigned n, float* theta, double* logl) const {
 
 // Standardisation of the inputs (mean, 1/sd of the free parameters) and of
 // the target (running max, sd of logL) from the pairs held.
-void Surrogate::refresh_scaling() {
+unsigned Surrogate::refresh_scaling() {
   const unsigned n = npairs();
   if (n < 2) throw Error(POFD_E_ARG, "need at least two training pairs");
-  std::vector<float> th(static_cast<size_t>(n) * npar_);
-  std::vector<double> ll(n);
-  ck(cudaMemcpy(th.data(), ptheta_, th.size() * sizeof(float), cudaMemcpyDeviceToHost), "D2H");
-  ck(cudaMemcpy(ll.data(), plogl_, n * sizeof(double), cudaMemcpyDeviceToHost), "D2H");
-  std::vector<int> idx(kInPad, 0);
-  ck(cudaMemcpy(idx.data(), idx_, kInPad * sizeof(int), cudaMemcpyDeviceToHost), "D2H");
   // inputs standardised over the pairs whose target is not clipped (the
   // region the sampler explores once burnt in), when there are enough of
   // them; far-off burn-in points then sit at large |x| instead of setting
   // the scale
-  double lmax = -std::numeric_limits<double>::infinity();
-  for (double v : ll) lmax = std::max(lmax, v);
-  const double clip0 = 25.0 + 2.5 * nin_;
-  std::vector<unsigned> use;
-  for (unsigned i = 0; i < n; ++i)
-    if (ll[i] - lmax > -clip0) use.push_back(i);
-  if (use.size() < std::max<size_t>(2 * nin_, 64)) {
-    use.resize(n);
-    for (unsigned i = 0; i < n; ++i) use[i] = i;
-  }
+  const double clip = 25.0 + 2.5 * nin_;
+  const unsigned K = nin_;
+  ScaleArgs a{};
+  a.n = static_cast<int>(n);
+  a.R = static_cast<int>((n + scale_blocks_ - 1) / scale_blocks_);
+  a.G = (a.n + a.R - 1) / a.R;
+  a.npar = static_cast<int>(npar_);
+  a.nin = static_cast<int>(K);
+  a.clip = clip;
+  a.theta = ptheta_;
+  a.logl = plogl_;
+  a.idx = idx_;
+  for (int k = 0; k < 3; ++k) a.part[k] = scale_ + static_cast<size_t>(k) * scale_blocks_ * kScPart;
+  a.out = scale_ + static_cast<size_t>(3) * scale_blocks_ * kScPart;
+  k_scale<0><<<a.G, kScT, 0, stream_>>>(a);
+  k_scale<1><<<a.G, kScT, 0, stream_>>>(a);
+  k_scale<2><<<a.G, kScT, 0, stream_>>>(a);
+  k_scale_out<<<1, kScT, 0, stream_>>>(a);
+  ck(cudaGetLastError(), "k_scale");
+  ck(cudaMemcpyAsync(h_stage_, a.out, 3 * kScPart * sizeof(double), cudaMemcpyDeviceToHost, stream_), "D2H");
+  ck(cudaStreamSynchronize(stream_), "synchronize");
   // Whitening: mean and covariance of the inputs over those pairs, W = L^-1
   // with L L^T the covariance (Cholesky), so that the network sees
   // decorrelated unit-variance inputs (the knot values of a P(D) posterior
   // are strongly correlated).  A covariance that is not positive definite
   // falls back to the diagonal (1/sd) scaling.
-  const double nu = static_cast<double>(use.size());
-  const unsigned K = nin_;
+  const bool all = h_stage_[kScCount] < std::max<size_t>(2 * K, 64);
+  const double nu = all ? n : h_stage_[kScCount];
   std::vector<double> mean_in(K, 0.0), cov(K * K, 0.0);
-  for (unsigned k = 0; k < K; ++k) {
-    double s = 0;
-    for (unsigned i : use) s += th[static_cast<size_t>(i) * npar_ + idx[k]];
-    mean_in[k] = s / nu;
-  }
-  for (unsigned i : use) {
-    double d[kInPad];
-    for (unsigned k = 0; k < K; ++k) d[k] = th[static_cast<size_t>(i) * npar_ + idx[k]] - mean_in[k];
-    for (unsigned a = 0; a < K; ++a)
-      for (unsigned b = 0; b <= a; ++b) cov[a * K + b] += d[a] * d[b];
-  }
-  for (unsigned a = 0; a < K; ++a)
-    for (unsigned b = 0; b <= a; ++b) cov[a * K + b] /= nu;
+  for (unsigned k = 0; k < K; ++k) mean_in[k] = h_stage_[(all ? kScAll : 0) + k] / nu;
+  for (unsigned i = 0, e = 0; i < K; ++i)
+    for (unsigned j = 0; j <= i; ++j, ++e) cov[i * K + j] = h_stage_[kScPart + e] / nu;
   std::vector<double> L(K * K, 0.0), Winv(K * K, 0.0);
   bool chol = true;
   for (unsigned a = 0; a < K && chol; ++a) {
@@ -832,32 +958,27 @@ void Surrogate::refresh_scaling() {
       Winv[k * K + k] = sd > 0 ? 1.0 / sd : 1.0;
     }
   }
-  std::vector<float> mu(kInPad, 0.0f), wm(kInPad * kInPad, 0.0f);
+  // target: logL - max, floored at -clip so that far-off burn-in points do
+  // not set the scale; the floor grows with the number of inputs (a
+  // chi-square of nin degrees of freedom sits near -nin/2)
+  const double mx = h_stage_[2 * kScPart], s2 = h_stage_[kScPart + kScT - 1];
+  float* wm = reinterpret_cast<float*>(h_stage_);  // the sums are done with
+  float* mu = wm + kInPad * kInPad;
+  std::fill(wm, mu + kInPad, 0.0f);
   for (unsigned a = 0; a < K; ++a) {
     mu[a] = static_cast<float>(mean_in[a]);
     for (unsigned b = 0; b < K; ++b) wm[a * kInPad + b] = static_cast<float>(Winv[a * K + b]);
   }
   whitened_ = chol;
-  // target: logL - max, floored at -clip so that far-off burn-in points do
-  // not set the scale; the floor grows with the number of inputs (a
-  // chi-square of nin degrees of freedom sits near -nin/2)
-  double mx = -std::numeric_limits<double>::infinity();
-  for (double v : ll) mx = std::max(mx, v);
-  const double clip = 25.0 + 2.5 * nin_;
-  double s = 0, s2 = 0;
-  for (double v : ll) s += std::max(v - mx, -clip);
-  const double m = s / n;
-  for (double v : ll) {
-    const double d = std::max(v - mx, -clip) - m;
-    s2 += d * d;
-  }
   const double sd = std::sqrt(s2 / n);
   ymax_ = mx;
   clip_ = clip;
   ys_ = (sd > 0) ? sd : 1.0;
-  ck(cudaMemcpy(mu_, mu.data(), kInPad * sizeof(float), cudaMemcpyHostToDevice), "upload");
-  ck(cudaMemcpy(wm_, wm.data(), wm.size() * sizeof(float), cudaMemcpyHostToDevice), "upload");
+  ck(cudaMemcpyAsync(wm_, wm, (kInPad + 1) * kInPad * sizeof(float), cudaMemcpyHostToDevice, stream_),
+     "upload");
+  ck(cudaStreamSynchronize(stream_), "synchronize");  // other streams may use them
   scaled_ = true;
+  return n;
 }
 
 // One training iteration on Mb rows (picked from the pair buffer, or its
@@ -919,8 +1040,7 @@ void Surrogate::iteration(int Mb, const Pick& pick, float lr, float** grads, cud
 void Surrogate::train(unsigned iters, unsigned batch, float lr, float* last_loss) {
   if (batch == 0 || batch > 65536) throw Error(POFD_E_ARG, "batch must be in [1, 65536]");
   ck(cudaSetDevice(device_), "cudaSetDevice");
-  refresh_scaling();
-  const unsigned n = npairs();
+  const unsigned n = refresh_scaling();
   const int Mb = static_cast<int>(batch);
   ensure_work((Mb + umma::kRows - 1) / umma::kRows * umma::kRows);
   ck(cudaMemset(err_, 0, sizeof(int)), "memset");

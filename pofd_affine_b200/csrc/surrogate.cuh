@@ -50,19 +50,18 @@ class Surrogate {
   // Loss gradients over the first n pairs (no update): grads_dev[8] device
   // buffers of the tensor sizes.
   void gradients(unsigned n, float** grads_dev, float* loss);
-  void get_params_host(std::vector<std::vector<float>>& host) const;
-  void set_params_host(const std::vector<std::vector<float>>& host);
+  void get_param_host(int t, float* out) const;
+  void set_params_host(const float* const* host);  // kNumTensors arrays
   size_t tensor_size(int t) const { return size_[t]; }
   // mu[16], W[16][16], ymax, ys, clip, whitened (276 values)
   void scaling(double* out) const;
-  void refresh_scaling();
+  unsigned refresh_scaling();  // returns the pairs held
   unsigned hidden() const { return H_; }
   unsigned nin() const { return nin_; }
   unsigned npar() const { return npar_; }
 
  private:
   void init_weights();
-  void refresh_bf16(const std::vector<std::vector<float>>& host);
   void ensure_work(int Mp);
   void forward(int M, const float* theta, int npar, const Pick& pick, const Targets& tg,
                cudaStream_t st);
@@ -78,12 +77,16 @@ class Surrogate {
   double ymax_ = 0.0, ys_ = 1.0, clip_ = 1e300;
   int* idx_ = nullptr;
   float* mu_ = nullptr;
-  float* wm_ = nullptr;    // input whitening W [16][16]
+  float* wm_ = nullptr;    // input whitening W [16][16], then mu_
+  double* scale_ = nullptr;    // parts and sums of the scaling passes
+  int scale_blocks_ = 0;
+  double* h_stage_ = nullptr;  // pinned: the sums, then W and mu
   bool whitened_ = false;
   float* p_[kNumTensors] = {};
   float* m_[kNumTensors] = {};
   float* v_[kNumTensors] = {};
   size_t size_[kNumTensors] = {};
+  size_t slab_ = 0;  // floats of all tensors
   __nv_bfloat16 *w1b_ = nullptr, *w2b_ = nullptr, *w3b_ = nullptr;
   __nv_bfloat16 *w2t_ = nullptr, *w3t_ = nullptr;
   float* ptheta_ = nullptr;

@@ -81,3 +81,39 @@ def test_first_step_is_adams(gpu_ctx, k, H, n, batch):
         big = np.abs(g) > 0.2 * np.abs(g).max()
         step = (p1.astype(np.float64) - p0).ravel()[big]
         assert np.max(np.abs(step + lr * np.sign(g[big]))) < 1e-2 * lr, name
+
+
+@pytest.mark.parametrize("k,n,far,same", [(1, 2, 0, False), (16, 65, 0, False), (3, 160, 120, False),
+                                          (5, 149, 0, True), (14, 8001, 3000, False),
+                                          (7, 70000, 0, False)])
+def test_scaling_matches_float64(gpu_ctx, k, n, far, same):
+    """Mean, whitening and target scaling against numpy in 64 bits: few and
+    many pairs (blocks of one row and of several hundred), most of them far
+    below the maximum (too few near it: all are used), two equal inputs (no
+    Cholesky factor: diagonal scaling).  The mean and W are stored in FP32
+    (6e-8); the sums differ by their order only, and W by that times the
+    covariance's condition (< 1e3 here)."""
+    from pofd_affine_b200.surrogate import Surrogate
+    th, ll = _pairs(n, k, 11)
+    th[:, :k] += 5.0
+    if same:
+        th[:, 1] = th[:, 0]
+    ll[:far] -= 500.0
+    S = Surrogate(gpu_ctx, k + 1, list(range(k)), hidden=16, capacity=max(n, 128), seed=1)
+    S.addPairs(th, ll)
+    S.gradients(2)
+    sc = S.scaling()
+    clip = 25.0 + 2.5 * k
+    d = np.maximum(ll - ll.max(), -clip)
+    assert sc["ymax"] == ll.max() and sc["clip"] == clip
+    assert abs(sc["ys"] - d.std()) <= 1e-12 * d.std()
+    use = ll - ll.max() > -clip
+    if use.sum() < max(2 * k, 64):
+        use[:] = True
+    x = th[use, :k].astype(np.float64)
+    assert np.max(np.abs(sc["mu"][:k] - x.mean(0)) / np.abs(x.mean(0))) < 1e-7
+    cov = np.cov(x.T, bias=True).reshape(k, k)
+    W = np.zeros((16, 16))
+    W[:k, :k] = np.diag(1 / np.sqrt(np.diag(cov))) if same else np.linalg.inv(np.linalg.cholesky(cov))
+    assert sc["whitened"] == (not same)
+    assert np.max(np.abs(sc["W"] - W)) < 1e-7 * np.abs(W).max()
