@@ -600,6 +600,34 @@ void launch_rfill(int per, bool seg, dim3 grid, cudaStream_t st, const BSet1Dev*
   }
 }
 
+struct SplitParams {
+  double sgpos, sgneg, n1sigpos, n1signeg;
+  long long botidx, topidx;
+};
+
+__device__ __forceinline__ long long to_index(double v) {
+  // (int) conversion of the reference, saturated so that huge values stay
+  // out of range instead of wrapping.
+  if (!(v < 9.0e15)) return 0x7fffffffffffLL;
+  if (!(v > -9.0e15)) return -0x7fffffffffffLL;
+  return static_cast<long long>(v);
+}
+
+__device__ __forceinline__ SplitParams split_params(const BSet1Dev& bs,
+                                                    double var, double sigma) {
+  SplitParams sp;
+  sp.sgpos = sqrt(var + sigma * sigma);
+  sp.sgneg = (9 * sigma * sigma > var) ? sigma : sp.sgpos;
+  sp.n1sigpos = 2.5 * sp.sgpos;
+  sp.n1signeg = 2.5 * sp.sgneg;
+  sp.botidx = to_index(sp.n1sigpos / bs.dflux);
+  if (sp.n1sigpos > fabs(bs.minflux_R))
+    sp.topidx = bs.wrapRidx;
+  else
+    sp.topidx = to_index(-(sp.n1signeg + bs.minflux_R) / bs.dflux + bs.wrapRidx + 1);
+  return sp;
+}
+
 // Moments, sigma estimate and the shift decision (PDFactory.cc:660-679,
 // 1067-1076), one thread per (proposal, beam set).
 // Noise cut-off of the half-length spectrum (own-FFT path): with noise sigma
@@ -621,6 +649,15 @@ __device__ __forceinline__ bool row_cut(int a, int m, int kc) {
   return min(256 * a, m - 256 * a - 255) > kc;
 }
 
+// Whether the inverse takes a row's spectrum in one pass: at most 8 rows of
+// 256 bins not cut (row_cut), at both ends together.  256 rows of n = 65536:
+// 69 us at 2 rows, 73 at 4, 83 at 8, 101 with pass A; 128 of n = 131072 71,
+// 75, 85 and 108; 512 of n = 16384 40, 42, 48 and 57: two more rows cost 4 us,
+// so that little is left past 8, and each would hold 8 KB of shared memory.
+__device__ __forceinline__ bool few_rows(int m1, int kc) {
+  return kc < 1024 && (kc >> 8) + 1 + ((kc + 255) >> 8) <= min(8, m1 / 2);
+}
+
 __global__ void k_moments1(const BSet1Dev* __restrict__ bsets,
                            const DSet1Dev* __restrict__ dsets, int B, int D, int n,
                            int nc2, int ntile, int nrow,
@@ -629,12 +666,17 @@ __global__ void k_moments1(const BSet1Dev* __restrict__ bsets,
                            const double* __restrict__ rbuf,
                            const double* __restrict__ rpart,
                            double* __restrict__ mom, int* __restrict__ kcut_set,
-                           int* __restrict__ kcut_ds) {
+                           int* __restrict__ kcut_ds, int4* __restrict__ rinfo) {
   const int wb = blockIdx.x * blockDim.x + threadIdx.x;
   if (wb >= nrow) return;
   const int w = wb / B, b = wb - w * B;
-  if (mstatus[w] != 0) return;
   const BSet1Dev& bs = bsets[b];
+  if (mstatus[w] != 0) {
+    if (rinfo)
+      for (int dd = 0; dd < bs.nds; ++dd)
+        rinfo[static_cast<size_t>(w) * D + bs.ds_begin + dd] = make_int4(mstatus[w], 0, 0, 0);
+    return;
+  }
   if (kcut_set) {
     // bins the spectrum kernel reads: the widest cut-off of the set's
     // datasets; per dataset for the inverse transform's input
@@ -660,6 +702,15 @@ __global__ void k_moments1(const BSet1Dev* __restrict__ bsets,
     mn -= prod;
     var -= cf * prod;
   }
+  if (rinfo)  // what k_inv1 needs of each dataset's row
+    for (int dd = 0; dd < bs.nds; ++dd) {
+      const int d = bs.ds_begin + dd;
+      const SplitParams sp = split_params(bs, var, sigmult[w] * dsets[d].sigma_base);
+      rinfo[static_cast<size_t>(w) * D + d] =
+          make_int4(0, kcut_ds[static_cast<size_t>(w) * D + d],
+                    static_cast<int>(max(-1ll, min(sp.botidx, 0x7fffffffll))),
+                    static_cast<int>(max(-1ll, min(sp.topidx, 0x7ffffffell))));
+    }
   const double sg = sqrt(var);
   const bool doshift = (sg > bs.dflux) && (fabs(mn) > bs.dflux);
   double* o = mom + static_cast<size_t>(wb) * 4;
@@ -761,6 +812,7 @@ k_fftA(int rowsz, int nrows_per_w, const int* __restrict__ mstatus,
   double2* Ts = Hs + NH + 128;  // inter-stage twiddles W_m^{(m / M1) n2 k1}
   const int row = blockIdx.y;
   if (mstatus[row / nrows_per_w] != 0) return;
+  if (kcut && few_rows(M1, kcut[row])) return;  // k_inv1 does without this pass
   const int b0 = blockIdx.x * CB;
   const int t = threadIdx.x;
   const double2* src = in + static_cast<size_t>(row) * rowsz;
@@ -950,9 +1002,8 @@ k_fftAR(const BSet1Dev* __restrict__ bsets, int B, int NI, int rowsz,
   }
 }
 
-// Pass B: 256-point DFTs along rows c0..c0+15 of Y (16 x 16 split), stored
+// Forward pass B: 256-point DFTs along rows c0..c0+15 of Y (16 x 16 split), stored
 // in natural order Z[c + m1 d].
-template <int S>
 __global__ void __launch_bounds__(256, 2)
 k_fftB(int m1, int rowsz, int nrows_per_w, const int* __restrict__ mstatus,
        const double2* __restrict__ in, double2* __restrict__ out,
@@ -961,8 +1012,7 @@ k_fftB(int m1, int rowsz, int nrows_per_w, const int* __restrict__ mstatus,
   extern __shared__ double2 fs[];  // [(k1 * 16 + n2) * 17 + r], then T
   double2* Ts = fs + 16 * 16 * 17;  // inter-stage twiddles W_256^{n2 k1} (symmetric)
   // blocks take the rows last-written-first: the tail of pass A's output is
-  // still in L2 when this pass starts (and the P(D) scan after the inverse,
-  // in natural order, then starts on this pass's last-written rows)
+  // still in L2 when this pass starts
   const int row = gridDim.y - 1 - blockIdx.y;
   if (mstatus[row / nrows_per_w] != 0) return;
   const int rb = min(FRB, m1);
@@ -978,11 +1028,11 @@ k_fftB(int m1, int rowsz, int nrows_per_w, const int* __restrict__ mstatus,
 #pragma unroll
     for (int n1 = 0; n1 < 16; ++n1) v[n1] = src[(c0 + r) * 256 + 16 * n1 + n2];
   }
-  Ts[t] = fft::tw2<S>(WH, WL, (m / 256) * (t >> 4) * (t & 15));
+  Ts[t] = fft::tw2<-1>(WH, WL, (m / 256) * (t >> 4) * (t & 15));
   __syncthreads();
   if (t < 16 * rb) {
     const int n2 = t & 15, r = t >> 4;
-    fft::dft<16, S>(v);
+    fft::dft<16, -1>(v);
 #pragma unroll
     for (int k1 = 0; k1 < 16; ++k1) {
       if (n2 * k1) v[k1] = fft::cmul(v[k1], Ts[k1 * 16 + n2]);
@@ -995,7 +1045,7 @@ k_fftB(int m1, int rowsz, int nrows_per_w, const int* __restrict__ mstatus,
     double2 u[16];
 #pragma unroll
     for (int n2 = 0; n2 < 16; ++n2) u[n2] = fs[(k1 * 16 + n2) * 17 + r];
-    fft::dft<16, S>(u);
+    fft::dft<16, -1>(u);
 #pragma unroll
     for (int k2 = 0; k2 < 16; ++k2) {
       // bins beyond the noise cut-off are never read (forward transform)
@@ -1039,7 +1089,7 @@ k_spectrum1f(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ ds
              int D, int n, int rowsz, const int* __restrict__ mstatus,
              const double* __restrict__ sigmult, const double* __restrict__ mom,
              const double2* __restrict__ zbuf, double2* __restrict__ pbuf,
-             const double2* __restrict__ Wn, const int* __restrict__ kcut_set,
+             double2* __restrict__ tbuf, const double2* __restrict__ Wn, const int* __restrict__ kcut_set,
              const int* __restrict__ kcut_ds) {
   const int wb = blockIdx.y;
   const int w = wb / B, b = wb - w * B;
@@ -1095,10 +1145,10 @@ k_spectrum1f(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ ds
         const double ef = exp(sigfac * wv * wv);
         Pb = make_double2(ef * pb.x, ef * pb.y);
       }
-      double2* out = pbuf + static_cast<size_t>(w * D + d) * rowsz;
       // rows the inverse transform does not read (every bin beyond the noise
-      // cut-off, hence zero) are not written
+      // cut-off, hence zero) are not written; k_inv1 takes few rows from tbuf
       const int kc = kcut_ds[static_cast<size_t>(w) * D + d];
+      double2* out = (few_rows(m >> 8, kc) ? tbuf : pbuf) + static_cast<size_t>(w * D + d) * rowsz;
       // Z'_k = (P_k + conj P_{m-k}) + i (P_k - conj P_{m-k}) e^{+2 pi i k / n}
       if (!row_cut(ka >> 8, m, kc)) {
         const double2 e = make_double2(Pa.x + Pb.x, Pa.y - Pb.y);
@@ -1114,37 +1164,214 @@ k_spectrum1f(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ ds
   }
 }
 
-struct SplitParams {
-  double sgpos, sgneg, n1sigpos, n1signeg;
-  long long botidx, topidx;
-};
-
 constexpr int kSearchPer = 8;  // values per thread per window of the split search
 
-__device__ __forceinline__ long long to_index(double v) {
-  // (int) conversion of the reference, saturated so that huge values stay
-  // out of range instead of wrapping.
-  if (!(v < 9.0e15)) return 0x7fffffffffffLL;
-  if (!(v > -9.0e15)) return -0x7fffffffffffLL;
-  return static_cast<long long>(v);
-}
-
-__device__ __forceinline__ SplitParams split_params(const BSet1Dev& bs,
-                                                    double var, double sigma) {
-  SplitParams sp;
-  sp.sgpos = sqrt(var + sigma * sigma);
-  sp.sgneg = (9 * sigma * sigma > var) ? sigma : sp.sgpos;
-  sp.n1sigpos = 2.5 * sp.sgpos;
-  sp.n1signeg = 2.5 * sp.sgneg;
-  sp.botidx = to_index(sp.n1sigpos / bs.dflux);
-  if (sp.n1sigpos > fabs(bs.minflux_R))
-    sp.topidx = bs.wrapRidx;
-  else
-    sp.topidx = to_index(-(sp.n1signeg + bs.minflux_R) / bs.dflux + bs.wrapRidx + 1);
-  return sp;
-}
-
 __device__ __forceinline__ double clip0(double v) { return (v < 0) ? 0.0 : v; }
+
+// What k_inv1 leaves per block of a P(D) row: the sums over the row's 16
+// chunks of 32 m1 values, the peak, the index-weighted sum, the smallest value
+// inside the split search window (its index in pmidx).
+constexpr int INV_PART = 20, INV_CHUNKS = 16;
+inline int inv_blocks(size_t n) { return static_cast<int>(n / 512 < FRB ? 1 : n / 512 / FRB); }
+
+// Inverse pass B straight into the P(D) row, with the row's reductions
+// (PDFactory.cc:779-815, PD.cc:123-140, 245-274) from registers: 256-point
+// DFTs along rows c0 .. c0 + 15 of Y, stored in natural order z[c + m1 d].
+// Where few rows of 256 bins are not cut by the noise (few_rows), their
+// contribution Y[c][b] = W_m^{cb} sum_a X[a][b] W_m1^{ac} is formed here from
+// the spectrum itself and pass A leaves the row out; else Y is pass A's.
+// With the rows read from memory, written back and read again by pass A and
+// the scan apart, the three took 181 us for 384 rows of n = 65536 (126 for
+// the transform, 55 for the scan) and 143 for 132 of n = 131072; this takes
+// 116 and 78.  Bound by latency at 16 warps an SM (128 registers: 16 values
+// and as many products): FP64 pipe 33 %, shared memory 33 %, DRAM 20 %; the
+// writes alone are 31 us.
+__global__ void __launch_bounds__(256, 2)
+k_inv1(int m1, int rowsz, const int4* __restrict__ rinfo, const double2* __restrict__ in,
+       double2* __restrict__ out, const double2* __restrict__ WH, const double2* __restrict__ WL,
+       double* __restrict__ ppart, int* __restrict__ pmidx) {
+  extern __shared__ double2 fs[];  // [(k1 * 16 + n2) * 17 + r], then T
+  __shared__ double shs[8][INV_CHUNKS], shd[24];
+  __shared__ int shi[8];
+  double2* Ts = fs + 16 * 16 * 17;  // inter-stage twiddles W_256^{n2 k1} (symmetric)
+  // blocks take the rows last-written-first: the tail of pass A's output is
+  // still in L2 when this pass starts
+  const int row = gridDim.y - 1 - blockIdx.y;
+  const int4 info = rinfo[row];  // status, noise cut-off, split search window
+  if (info.x != 0) return;
+  const int rb = min(FRB, m1);
+  const int blk = gridDim.x - 1 - blockIdx.x, c0 = blk * rb;
+  const int m = m1 * 256;
+  const int t = threadIdx.x;
+  const double2* src = in + static_cast<size_t>(row) * rowsz;
+  double2* dst = out + static_cast<size_t>(row) * rowsz;
+  const int kc = info.y;
+  const bool few = few_rows(m1, kc);
+  const int n2 = few ? t / rb : t & 15, r = few ? t % rb : t >> 4;
+  Ts[t] = fft::tw2<1>(WH, WL, (m / 256) * (t >> 4) * (t & 15));
+  double2 v[16];
+  if (!few) {
+    if (t < 16 * rb) {
+#pragma unroll
+      for (int n1 = 0; n1 < 16; ++n1) v[n1] = src[(c0 + r) * 256 + 16 * n1 + n2];
+    }
+  } else {
+    // all loads go out before the first wait: the rows, then the twiddles
+    const int lo = kc >> 8;  // <= 3
+    const bool odd = ((kc + 255) >> 8) > lo;
+    const int c = c0 + r;
+    double2 A[3], Bh[3], x0 = src[t], xo = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int h = 1; h <= 3; ++h)
+      if (h <= lo) {
+        A[h - 1] = src[256 * h + t];
+        Bh[h - 1] = src[256 * (m1 - h) + t];
+      }
+    if (odd) xo = src[256 * (m1 - lo - 1) + t];
+    const double2 e1 = fft::tw2<1>(WH, WL, (256 * c) & (m - 1));
+    // W_m^{c (16 n1 + n2)} from W^{c n2} and W^{16 c 2^i}
+    const double2 w1 = fft::tw2<1>(WH, WL, (16 * c) & (m - 1));
+    const double2 w2 = fft::tw2<1>(WH, WL, (32 * c) & (m - 1));
+    const double2 w4 = fft::tw2<1>(WH, WL, (64 * c) & (m - 1));
+    const double2 w8 = fft::tw2<1>(WH, WL, (128 * c) & (m - 1));
+    const double2 g0 = fft::tw2<1>(WH, WL, (c * n2) & (m - 1));
+    // rows h and m1 - h enter as A e^{ix} + B e^{-ix}: A + B and i (A - B),
+    // the same for every c, are made once per block
+    fs[t] = x0;
+#pragma unroll
+    for (int h = 1; h <= 3; ++h)
+      if (h <= lo) {
+        fs[(2 * h - 1) * 256 + t] = fft::cadd(A[h - 1], Bh[h - 1]);
+        fs[2 * h * 256 + t] = make_double2(Bh[h - 1].y - A[h - 1].y, A[h - 1].x - Bh[h - 1].x);
+      }
+    if (odd) fs[(2 * lo + 1) * 256 + t] = xo;
+    __syncthreads();
+    if (t < 16 * rb) {
+      const double2* x = fs + n2;  // a warp reads two neighbouring values
+#pragma unroll
+      for (int n1 = 0; n1 < 16; ++n1) v[n1] = x[16 * n1];
+      double2 e = e1;
+      for (int h = 1; h <= lo; ++h) {
+        const double2 *S = x + (2 * h - 1) * 256, *Q = S + 256;
+#pragma unroll
+        for (int n1 = 0; n1 < 16; ++n1) {
+          const double2 sa = S[16 * n1], qa = Q[16 * n1];
+          v[n1].x = fma(sa.x, e.x, fma(qa.x, e.y, v[n1].x));
+          v[n1].y = fma(sa.y, e.x, fma(qa.y, e.y, v[n1].y));
+        }
+        e = fft::cmul(e, e1);
+      }
+      if (odd) {
+        const double2* S = x + (2 * lo + 1) * 256;
+#pragma unroll
+        for (int n1 = 0; n1 < 16; ++n1) {
+          const double2 q = S[16 * n1];
+          v[n1].x = fma(q.x, e.x, fma(q.y, e.y, v[n1].x));
+          v[n1].y = fma(q.y, e.x, fma(-q.x, e.y, v[n1].y));
+        }
+      }
+      double2 g = g0, g1 = fft::cmul(g0, w1);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[i] = fft::cmul(v[i], g);
+        v[8 + i] = fft::cmul(v[8 + i], fft::cmul(g, w8));
+        const double2 g4 = fft::cmul(g, w4);
+        v[4 + i] = fft::cmul(v[4 + i], g4);
+        v[12 + i] = fft::cmul(v[12 + i], fft::cmul(g4, w8));
+        g = (i == 0) ? g1 : (i == 1) ? fft::cmul(g0, w2) : fft::cmul(g1, w2);
+      }
+    }
+  }
+  __syncthreads();
+  if (t < 16 * rb) {
+    fft::dft<16, 1>(v);
+#pragma unroll
+    for (int k1 = 0; k1 < 16; ++k1) {
+      if (n2 * k1) v[k1] = fft::cmul(v[k1], Ts[k1 * 16 + n2]);
+      fs[(k1 * 16 + n2) * 17 + r] = v[k1];
+    }
+  }
+  __syncthreads();
+  // Values are clipped at 0, so that their bit patterns order like the values:
+  // clipping, peak and minimum go by integers and leave the FP64 pipe alone.
+  // (NaN: no peak, which the split search reports.)
+  double s[INV_CHUNKS], wsum = 0.0;
+  long long mxb = 0, mnb = 0x7fe1ccf385ebc8a0ll;  // 1e308
+  int mni = 0x7fffffff;
+#pragma unroll
+  for (int k2 = 0; k2 < 16; ++k2) s[k2] = 0.0;
+  if (t < 16 * rb) {
+    const int rr = t % rb, k1 = t / rb;
+    double2 u[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) u[q] = fs[(k1 * 16 + q) * 17 + rr];
+    fft::dft<16, 1>(u);
+    const int bot = info.z, top = info.w;
+    double fi = static_cast<double>(2 * (c0 + rr + m1 * k1));
+#pragma unroll
+    for (int k2 = 0; k2 < 16; ++k2) {
+      const int j = (c0 + rr) + m1 * (k1 + 16 * k2), i = 2 * j;
+      dst[j] = u[k2];
+      long long ba = __double_as_longlong(u[k2].x), bb = __double_as_longlong(u[k2].y);
+      ba = ba < 0 ? 0 : ba;
+      bb = bb < 0 ? 0 : bb;
+      mxb = max(mxb, max(ba, bb));
+      if (i >= bot && i <= top && ba < mnb) { mnb = ba; mni = i; }
+      if (i + 1 >= bot && i + 1 <= top && bb < mnb) { mnb = bb; mni = i + 1; }
+      const double xb = __longlong_as_double(bb);
+      s[k2] = __longlong_as_double(ba) + xb;
+      wsum = fma(fi, s[k2], wsum + xb);
+      fi += static_cast<double>(32 * m1);
+    }
+  }
+  double mx = __longlong_as_double(mxb), mnv = __longlong_as_double(mnb);
+  // across the warp: the chunk sums by halving (lane l ends with chunk l / 2),
+  // the others by butterflies
+  const int wp = t >> 5, l = t & 31;
+#pragma unroll
+  for (int h = 8; h > 0; h >>= 1) {
+    const bool up = (l & (2 * h)) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double give = up ? s[i] : s[i + h], keep = up ? s[i + h] : s[i];
+      s[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+    }
+  }
+  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+  for (int o = 16; o > 0; o >>= 1) {
+    mx = dev::dmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+    const double v2 = __shfl_xor_sync(0xffffffffu, mnv, o);
+    const int i2 = __shfl_xor_sync(0xffffffffu, mni, o);
+    dev::argmin_merge(mnv, mni, v2, i2);
+  }
+  if ((l & 1) == 0) shs[wp][l >> 1] = s[0];
+  if (l == 0) {
+    shd[wp] = mx;
+    shd[8 + wp] = wsum;
+    shd[16 + wp] = mnv;
+    shi[wp] = mni;
+  }
+  __syncthreads();
+  double* o = ppart + (static_cast<size_t>(row) * gridDim.x + blk) * INV_PART;
+  if (t < INV_CHUNKS) {
+    double a = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) a += shs[q][t];
+    o[t] = a;
+  } else if (t == 32) {
+    for (int q = 0; q < 8; ++q) {
+      mx = dev::dmax(mx, shd[q]);
+      dev::argmin_merge(mnv, mni, shd[16 + q], shi[q]);
+    }
+    wsum = 0.0;
+    for (int q = 0; q < 8; ++q) wsum += shd[8 + q];
+    o[16] = mx;
+    o[17] = wsum;
+    o[18] = mnv;
+    pmidx[static_cast<size_t>(row) * gridDim.x + blk] = mni;
+  }
+}
 
 // Chunk reductions over the P(D) after the inverse transform: peak, sum,
 // index-weighted sum and the minimum inside the split search window
@@ -1435,16 +1662,18 @@ __device__ __forceinline__ void finish_row(const BSet1Dev& bs, const DSet1Dev& d
   }
 }
 
-// finish_row on a row in global memory, from the chunk reductions of
-// k_pscan1; one block per (proposal, dataset).
+// finish_row on a row in global memory, from its npart partial reductions:
+// chunks of k_pscan1, or blocks of k_inv1 (OWN); one block per (proposal,
+// dataset).
+template <bool OWN>
 __global__ void __launch_bounds__(NT)
 k_pfinish1(const BSet1Dev* __restrict__ bsets,
            const DSet1Dev* __restrict__ dsets, int B, int D, int n, int nc2,
-           int nchunk, double log2toe, const int* __restrict__ mstatus,
+           int npart, double log2toe, const int* __restrict__ mstatus,
            const double* __restrict__ sigmult, const double* __restrict__ mom,
            const double* __restrict__ pbuf, const double* __restrict__ ppart,
            const int* __restrict__ pmidx, PDInfo1* __restrict__ pinfo) {
-  __shared__ double shd[32];
+  __shared__ double shd[32], shc[INV_CHUNKS + 1];
   const int wd = blockIdx.x;
   const int w = wd / D, d = wd - w * D;
   PDInfo1& info = pinfo[wd];
@@ -1457,26 +1686,46 @@ k_pfinish1(const BSet1Dev* __restrict__ bsets,
   const double var = mom[(static_cast<size_t>(w) * B + ds.bs) * 4 + 1];
   const SplitParams sp = split_params(bs, var, sigmult[w] * ds.sigma_base);
   const double* p = pbuf + static_cast<size_t>(wd) * nc2;
-  const double* pp = ppart + static_cast<size_t>(wd) * nchunk * 4;
-  const int* pm = pmidx + static_cast<size_t>(wd) * nchunk;
+  constexpr int PW = OWN ? INV_PART : 4;
+  const double* pp = ppart + static_cast<size_t>(wd) * npart * PW;
+  const int* pm = pmidx + static_cast<size_t>(wd) * npart;
   RowMin1 rs{-1.0e308, 1.0e308, 0x7fffffff};
   if (threadIdx.x == 0)
-    for (int c = 0; c < nchunk; ++c) {
-      if (pp[4 * c] > rs.peak) rs.peak = pp[4 * c];
-      dev::argmin_merge(rs.minval, rs.minidx, pp[4 * c + 3], pm[c]);
+    for (int c = 0; c < npart; ++c) {
+      const double* q = pp + PW * c + (OWN ? INV_CHUNKS : 0);  // peak, (sum,) wsum, min
+      if (q[0] > rs.peak) rs.peak = q[0];
+      dev::argmin_merge(rs.minval, rs.minidx, q[OWN ? 2 : 3], pm[c]);
     }
+  if (OWN) {  // the blocks' chunk sums and index-weighted sums
+    const int e = static_cast<int>(threadIdx.x) - 32;
+    if (e >= 0 && e <= INV_CHUNKS) {
+      double a = 0.0;
+      for (int c = 0; c < npart; ++c) a += pp[PW * c + (e < INV_CHUNKS ? e : INV_CHUNKS + 1)];
+      shc[e] = a;
+    }
+    __syncthreads();
+  }
   finish_row<NT>(bs, ds, sp, p, n, rs, log2toe, shd, info,
                  [&](int split, double& S, double& W, double& T) {
                    // whole chunks below the split from the partials, the rest read
-                   const int cfull = split / CHUNK;
+                   const int chunk = OWN ? n / INV_CHUNKS : CHUNK;
+                   const int cfull = split / chunk;
                    double part = 0.0;
-                   for (int i = cfull * CHUNK + threadIdx.x; i < split; i += NT) part += clip0(p[i]);
+                   for (int i = cfull * chunk + threadIdx.x; i < split; i += NT) part += clip0(p[i]);
                    part = dev::block_sum<NT>(part, shd);
                    S = W = T = 0.0;
-                   for (int c = 0; c < nchunk; ++c) {
-                     S += pp[4 * c + 1];
-                     W += static_cast<double>(c) * CHUNK * pp[4 * c + 1] + pp[4 * c + 2];
-                     if (c < cfull) T += pp[4 * c + 1];
+                   if (OWN) {
+                     for (int c = 0; c < INV_CHUNKS; ++c) {
+                       S += shc[c];
+                       if (c < cfull) T += shc[c];
+                     }
+                     W = shc[INV_CHUNKS];
+                   } else {
+                     for (int c = 0; c < npart; ++c) {
+                       S += pp[4 * c + 1];
+                       W += static_cast<double>(c) * CHUNK * pp[4 * c + 1] + pp[4 * c + 2];
+                       if (c < cfull) T += pp[4 * c + 1];
+                     }
                    }
                    T += part;
                  });
@@ -2146,11 +2395,9 @@ void fftA_attr() {
   cuda_check(cudaFuncSetAttribute(k_fftA<16, 16, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm), "attr");
 }
 
-constexpr size_t kFftBSmemMax = (16 * 16 * 17 + 256) * sizeof(double2);
-
 // pass B: the exchange and the inter-stage table (its twiddles are W_256
 // powers only)
-inline size_t fftB_smem(int) { return kFftBSmemMax; }
+constexpr size_t kFftBSmem = (16 * 16 * 17 + 256) * sizeof(double2);
 }  // namespace
 
 
@@ -2897,13 +3144,13 @@ const char* Engine1::stage_name(int i) const {
       "k_rnodes1", "k_rspline1", "k_rfill1", "k_moments1",
       "cufft_d2z", "k_spectrum1", "cufft_z2d", "k_pscan1", "k_pfinish1",
       "k_reduce1"};
-  static const char* own[kNumStages] = {
+  static const char* own[] = {
       "k_rnodes1", "k_rspline1", "k_rfill1", "k_moments1",
-      "k_fftA1+k_fftB1", "k_spectrum1f", "k_fftA1+k_fftB1_inv", "k_pscan1", "k_pfinish1",
+      "k_fftA1+k_fftB1", "k_spectrum1f", "k_fftA1+k_inv1", "k_pfinish1",
       "k_reduce1"};
-  static const char* fused[kNumStages] = {
+  static const char* fused[] = {
       "k_rnodes1", "k_rspline1", "k_fftAR1", "k_moments1",
-      "k_fftB1", "k_spectrum1f", "k_fftA1+k_fftB1_inv", "k_pscan1", "k_pfinish1",
+      "k_fftB1", "k_spectrum1f", "k_fftA1+k_inv1", "k_pfinish1",
       "k_reduce1"};
   if (i < 0 || i >= num_stages()) return "";
   static const char* row[] = {"k_rnodes1", "k_row1", "k_reduce1"};
@@ -3008,7 +3255,7 @@ void Engine1::free_work() {
   void* ptrs[] = {ws_.cnt, ws_.mstatus, ws_.sigmult, ws_.nodes, ws_.spl,
                   ws_.rbuf, ws_.rpart, ws_.mom, ws_.pbuf, ws_.ppart,
                   ws_.pmidx, ws_.pinfo, ws_.pdout, ws_.theta_in, ws_.logl,
-                  ws_.tmp, ws_.bonus, ws_.kcut_set, ws_.kcut_ds};
+                  ws_.tmp, ws_.bonus, ws_.kcut_set, ws_.kcut_ds, ws_.rinfo};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (ws_.h_theta) cudaFreeHost(ws_.h_theta);
@@ -3046,17 +3293,19 @@ void Engine1::reserve(unsigned P) {
     fftA_attr<-1>();
     fftA_attr<1>();
     fftAR_attr();
-    cuda_check(cudaFuncSetAttribute(k_fftB<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(kFftBSmemMax)), "attr");
-    cuda_check(cudaFuncSetAttribute(k_fftB<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(kFftBSmemMax)), "attr");
+    cuda_check(cudaFuncSetAttribute(k_fftB, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(kFftBSmem)), "attr");
+    cuda_check(cudaFuncSetAttribute(k_inv1, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(kFftBSmem)), "attr");
   }
   ws_.mom = dalloc<double>(static_cast<size_t>(P) * B_ * 4);
   ws_.kcut_set = dalloc<int>(static_cast<size_t>(P) * B_);
   ws_.kcut_ds = dalloc<int>(static_cast<size_t>(P) * D_);
+  ws_.rinfo = dalloc<int4>(static_cast<size_t>(P) * D_);
   ws_.pbuf = dalloc<double>(static_cast<size_t>(P) * D_ * nc2);
-  ws_.ppart = dalloc<double>(static_cast<size_t>(P) * D_ * nchunk_ * 4);
-  ws_.pmidx = dalloc<int>(static_cast<size_t>(P) * D_ * nchunk_);
+  const size_t npart = own_fft_ ? inv_blocks(n_) : nchunk_;
+  ws_.ppart = dalloc<double>(static_cast<size_t>(P) * D_ * npart * (own_fft_ ? INV_PART : 4));
+  ws_.pmidx = dalloc<int>(static_cast<size_t>(P) * D_ * npart);
   ws_.pinfo = dalloc<PDInfo1>(static_cast<size_t>(P) * D_);
   ws_.pdout = dalloc<double>(n_);
   // logL [P] then status [P] in one allocation: one download per call
@@ -3220,25 +3469,25 @@ void Engine1::launch_all(unsigned nprop, const float* theta, unsigned npar,
     k_moments1<<<(P * B + 127) / 128, 128, 0, st>>>(d_bsets_, d_dsets_, B, D, n, nc2,
                                                     ntile, P * B,
                                                     ws_.mstatus, ws_.sigmult, ws_.rbuf, ws_.rpart,
-                                                    ws_.mom, ws_.kcut_set, ws_.kcut_ds);
+                                                    ws_.mom, ws_.kcut_set, ws_.kcut_ds, ws_.rinfo);
     mark(4);
     const int rb_rows = m1 < FRB ? m1 : FRB;
     if (!fused)
       launch_fftA<-1>(m1, P * B, st, rowsz, B, ws_.mstatus, rb, tmp, d_wh_, d_wl_, nullptr);
-    k_fftB<-1><<<dim3(m1 / rb_rows, P * B), 256, fftB_smem(m1), st>>>(
+    k_fftB<<<dim3(m1 / rb_rows, P * B), 256, kFftBSmem, st>>>(
         m1, rowsz, B, ws_.mstatus, tmp, rb, d_wh_, d_wl_, ws_.kcut_set);
     mark(5);
     {
       // a few blocks per row loop over the pairs up to the row's cut-off
       dim3 grid(std::min((m / 2 + 1 + NT - 1) / NT, tune_.spec_blocks), P * B);
       k_spectrum1f<<<grid, NT, 0, st>>>(d_bsets_, d_dsets_, B, D, n, rowsz, ws_.mstatus,
-                                        ws_.sigmult, ws_.mom, rb, pb, d_wn_, ws_.kcut_set,
+                                        ws_.sigmult, ws_.mom, rb, pb, tmp, d_wn_, ws_.kcut_set,
                                         ws_.kcut_ds);
     }
     mark(6);
     launch_fftA<1>(m1, P * D, st, rowsz, D, ws_.mstatus, pb, tmp, d_wh_, d_wl_, ws_.kcut_ds);
-    k_fftB<1><<<dim3(m1 / rb_rows, P * D), 256, fftB_smem(m1), st>>>(
-        m1, rowsz, D, ws_.mstatus, tmp, pb, d_wh_, d_wl_, nullptr);
+    k_inv1<<<dim3(m1 / rb_rows, P * D), 256, kFftBSmem, st>>>(
+        m1, rowsz, ws_.rinfo, tmp, pb, d_wh_, d_wl_, ws_.ppart, ws_.pmidx);
   } else {
     {
       dim3 grid(ntile_, P * B);
@@ -3249,7 +3498,7 @@ void Engine1::launch_all(unsigned nprop, const float* theta, unsigned npar,
     k_moments1<<<(P * B + 127) / 128, 128, 0, st>>>(d_bsets_, d_dsets_, B, D, n, nc2,
                                                     static_cast<int>(ntile_), P * B,
                                                     ws_.mstatus, ws_.sigmult, ws_.rbuf,
-                                                    ws_.rpart, ws_.mom, nullptr, nullptr);
+                                                    ws_.rpart, ws_.mom, nullptr, nullptr, nullptr);
     mark(4);
     cufft_check(cufftSetStream(pl.fwd, st), "cufftSetStream");
     cufft_check(cufftExecD2Z(pl.fwd, ws_.rbuf, reinterpret_cast<cufftDoubleComplex*>(ws_.rbuf)),
@@ -3266,23 +3515,26 @@ void Engine1::launch_all(unsigned nprop, const float* theta, unsigned npar,
                 "cufftExecZ2D");
   }
   mark(7);
-  {
-    dim3 grid(nchunk_, P * D);
-    k_pscan1<<<grid, NT, 0, st>>>(d_bsets_, d_dsets_, B, D, n, nc2,
-                                  static_cast<int>(nchunk_), ws_.mstatus,
-                                  ws_.sigmult, ws_.mom, ws_.pbuf, ws_.ppart,
-                                  ws_.pmidx);
+  if (!own_fft_) {
+    k_pscan1<<<dim3(nchunk_, P * D), NT, 0, st>>>(d_bsets_, d_dsets_, B, D, n, nc2,
+                                                  static_cast<int>(nchunk_), ws_.mstatus,
+                                                  ws_.sigmult, ws_.mom, ws_.pbuf, ws_.ppart,
+                                                  ws_.pmidx);
+    mark(8);
   }
-  mark(8);
-  k_pfinish1<<<P * D, NT, 0, st>>>(d_bsets_, d_dsets_, B, D, n, nc2,
-                                   static_cast<int>(nchunk_), std::log(2.0),
-                                   ws_.mstatus, ws_.sigmult, ws_.mom, ws_.pbuf,
-                                   ws_.ppart, ws_.pmidx, ws_.pinfo);
-  mark(9);
+  const int npart = own_fft_ ? inv_blocks(n) : static_cast<int>(nchunk_);
+#define POFD_FINISH(OWN)                                                                      \
+  k_pfinish1<OWN><<<P * D, NT, 0, st>>>(d_bsets_, d_dsets_, B, D, n, nc2, npart, std::log(2.0), \
+                                        ws_.mstatus, ws_.sigmult, ws_.mom, ws_.pbuf, ws_.ppart, \
+                                        ws_.pmidx, ws_.pinfo)
+  if (own_fft_) POFD_FINISH(true);
+  else POFD_FINISH(false);
+#undef POFD_FINISH
+  mark(own_fft_ ? 8 : 9);
   k_reduce1<<<(P + 127) / 128, 128, 0, st>>>(d_bsets_, B, D, P, ws_.mstatus,
                                             ws_.sigmult, ws_.pinfo, prior_, ws_.bonus,
                                             logl, status);
-  mark(10);
+  mark(own_fft_ ? 9 : 10);
   cuda_check(cudaGetLastError(), "kernel launch");
 }
 

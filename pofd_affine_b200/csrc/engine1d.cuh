@@ -120,6 +120,7 @@ struct Workspace1 {
   double* mom = nullptr;     // [P][B][4] mean, var, shift, doshift
   int* kcut_set = nullptr;   // [P][B] noise cut-off of the forward spectrum
   int* kcut_ds = nullptr;    // [P][D] noise cut-off of each dataset's spectrum
+  int4* rinfo = nullptr;  // [P][D] status, noise cut-off, split search window
   double* pbuf = nullptr;    // [P][D][2*(n/2+1)] spectrum / P(D)
   double* tmp = nullptr;     // [P][max(B,D)][2*(n/2+1)] own-FFT pass-A rows
   double* ppart = nullptr;   // [P][D][nchunk][4] max, sum, wsum, minval
@@ -191,7 +192,7 @@ class Engine1 {
   void rgrid_host(int bs, const float* theta, unsigned npar, double* out);
   int kernels_per_eval() const {
     if (row1()) return 1 + 1 + (B_ > 1 ? 1 : 0) + (prior_.needs_bonus() ? 1 : 0);
-    return (own_fft_ ? (fused_fill() ? 11 : 12) : 8) + (prior_.needs_bonus() ? 1 : 0);
+    return (own_fft_ ? (fused_fill() ? 10 : 11) : 8) + (prior_.needs_bonus() ? 1 : 0);
   }
   // the R grid fill runs inside the forward FFT pass A (own FFT, plain passes)
   bool fused_fill() const {
@@ -223,7 +224,7 @@ class Engine1 {
   void fill_bonus(unsigned nprop, float* theta_dev, unsigned npar, cudaStream_t st);
   static constexpr int kNumStages = 10;
   static constexpr size_t kOwnFftMin = 8192;  // automatic four-step FFT from here
-  int num_stages() const { return row1() ? 3 : kNumStages; }
+  int num_stages() const { return row1() ? 3 : own_fft_ ? kNumStages - 1 : kNumStages; }
   void profile_stages(unsigned nprop, const float* theta, unsigned npar,
                       int reps, double* stage_ms);
   const char* stage_name(int i) const;
