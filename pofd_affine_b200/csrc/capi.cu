@@ -92,6 +92,7 @@ struct pofd_ensemble {
 struct pofd_pdfactory1 {
   pofd_ctx* ctx = nullptr;
   unsigned ninterp = 2048;
+  pofd::BlockPool pool;  // outlives the engine
   std::unique_ptr<pofd::Engine1> eng;
   std::vector<float> theta;  // knot values + noise slot
   bool inited = false;
@@ -299,7 +300,8 @@ int pofd_pdfactory1_initpd(pofd_pdfactory1* f, unsigned n, double minflux,
       if (std::isnan(static_cast<double>(knotvals[k])))
         throw pofd::Error(POFD_E_INVALID_MODEL, "Invalid model");
     cudaSetDevice(f->ctx->device);
-    f->eng.reset(new pofd::Engine1(f->ctx->device, f->ctx->stream));
+    f->eng.reset();  // its blocks go to the next one
+    f->eng.reset(new pofd::Engine1(f->ctx->device, f->ctx->stream, &f->pool));
     f->eng->configure(nknots, knotpos, n, f->ninterp, true, 1);
     const int bs = f->eng->add_beamset(beam->b, 0.0);
     f->eng->add_virtual_dataset(bs, 1.0);
@@ -324,6 +326,7 @@ int pofd_pdfactory1_getpd(pofd_pdfactory1* f, double sigma, int setlog,
     const int st = f->eng->pd_host(0, 0, f->theta.data(),
                                    static_cast<unsigned>(f->theta.size()),
                                    setlog != 0, pd_out, info);
+    f->pool.trim();  // every block that this engine uses is taken by now
     if (minflux_out) *minflux_out = info[10];
     if (dflux_out) *dflux_out = info[0];
     if (st != 0) throw pofd::Error(st, "P(D) unwrap failed (split point or mean)");

@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <sstream>
 
 #include "common.cuh"
@@ -2285,13 +2286,6 @@ __global__ void k_pdwrite1(const double* __restrict__ p, int n, int split,
   out[i] = setlog ? ((v > 0.0) ? log2(v) : dev::kSmallLogVal) : v;
 }
 
-template <class T>
-T* dalloc(size_t n) {
-  void* p = nullptr;
-  cuda_check(cudaMalloc(&p, n * sizeof(T) + 16), "cudaMalloc");
-  return static_cast<T*>(p);
-}
-
 }  // namespace
 
 // ===================================================================== host
@@ -2401,8 +2395,76 @@ constexpr size_t kFftBSmem = (16 * 16 * 17 + 256) * sizeof(double2);
 }  // namespace
 
 
-Engine1::Engine1(int device, cudaStream_t stream)
-    : device_(device), stream_(stream) {}
+void BlockPool::release(const Block& b) {
+  if (b.pinned) cudaFreeHost(b.p);
+  else cudaFree(b.p);
+}
+
+BlockPool::~BlockPool() {
+  for (const Block& b : free_) release(b);
+  for (const Block& b : used_) release(b);
+}
+
+void BlockPool::trim() {
+  for (const Block& b : free_) release(b);
+  free_.clear();
+}
+
+// The smallest free block of the kind that holds the bytes and is at most
+// twice as large, else a new one.
+void* BlockPool::get(size_t bytes, bool pinned) {
+  size_t best = free_.size();
+  for (size_t i = 0; i < free_.size(); ++i) {
+    const Block& b = free_[i];
+    if (b.pinned == pinned && b.bytes >= bytes && b.bytes <= 2 * bytes &&
+        (best == free_.size() || b.bytes < free_[best].bytes))
+      best = i;
+  }
+  used_.reserve(used_.size() + 1);
+  free_.reserve(free_.size() + used_.size() + 1);  // put() never throws
+  if (best < free_.size()) {
+    used_.push_back(free_[best]);
+    free_.erase(free_.begin() + static_cast<long>(best));
+  } else {
+    void* p = nullptr;
+    cudaError_t e = pinned ? cudaMallocHost(&p, bytes) : cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation && !free_.empty()) {
+      cudaGetLastError();
+      trim();
+      e = pinned ? cudaMallocHost(&p, bytes) : cudaMalloc(&p, bytes);
+    }
+    cuda_check(e, pinned ? "cudaMallocHost" : "cudaMalloc");
+    used_.push_back(Block{p, bytes, pinned});
+  }
+  return used_.back().p;
+}
+
+void BlockPool::put(void* p) {
+  for (size_t i = 0; i < used_.size(); ++i)
+    if (used_[i].p == p) {
+      free_.push_back(used_[i]);
+      used_.erase(used_.begin() + static_cast<long>(i));
+      return;
+    }
+}
+
+void* Engine1::take(size_t bytes, bool pinned) {
+  if (pool_) return pool_->get(bytes, pinned);
+  void* p = nullptr;
+  if (pinned) cuda_check(cudaMallocHost(&p, bytes), "cudaMallocHost");
+  else cuda_check(cudaMalloc(&p, bytes), "cudaMalloc");
+  return p;
+}
+
+void Engine1::give(void* p, bool pinned) {
+  if (!p) return;
+  if (pool_) pool_->put(p);
+  else if (pinned) cudaFreeHost(p);
+  else cudaFree(p);
+}
+
+Engine1::Engine1(int device, cudaStream_t stream, BlockPool* pool)
+    : device_(device), stream_(stream), pool_(pool) {}
 
 Engine1::~Engine1() {
   if (device_ < 0) return;  // host-only: nothing was allocated on a GPU
@@ -2412,6 +2474,7 @@ Engine1::~Engine1() {
     if (kv.second.fwd) { fftwork_.forget(kv.second.fwd); cufftDestroy(kv.second.fwd); }
     if (kv.second.inv) { fftwork_.forget(kv.second.inv); cufftDestroy(kv.second.inv); }
   }
+  if (pool_) cudaDeviceSynchronize();  // freeing waits by itself; putting back does not
   free_work();
   free_static();
 }
@@ -2613,7 +2676,7 @@ void Engine1::dataset_info(int bs, int ds, double* o, uint32_t* bins) const {
 }
 
 void Engine1::free_static() {
-  for (void* p : static_allocs_) cudaFree(p);
+  for (void* p : static_allocs_) give(p);
   static_allocs_.clear();
   d_bsets_ = nullptr;
   d_dsets_ = nullptr;
@@ -2633,19 +2696,34 @@ void Engine1::build_static() {
   free_static();
   if (sets_.empty()) throw Error(POFD_E_ARG, "no beam sets");
   runblk_ = 0;
-  auto up = [&](const std::vector<double>& v) -> const double* {
-    double* p = dalloc<double>(v.size() ? v.size() : 1);
-    static_allocs_.push_back(p);
-    if (!v.empty())
-      cuda_check(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, stream_), "upload");
-    return p;
+  // The tables are a few dozen arrays, most of some kilobytes: they share
+  // device chunks and go up in one copy per chunk (an allocation and a copy
+  // each had been a third of the 0.25 ms that uploads took).
+  struct Chunk {
+    char* dev;
+    std::vector<char> host;
+    size_t used, size;
   };
-  auto upi = [&](const std::vector<int>& v) -> const int* {
-    int* p = dalloc<int>(v.size() ? v.size() : 1);
-    static_allocs_.push_back(p);
-    if (!v.empty())
-      cuda_check(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, stream_), "upload");
-    return p;
+  std::vector<Chunk> chunks;
+  auto upload = [&](const void* src, size_t bytes) -> void* {
+    const size_t need = (bytes + 16 + 255) / 256 * 256;
+    if (chunks.empty() || chunks.back().used + need > chunks.back().size) {
+      const size_t size = std::max<size_t>(need, size_t(1) << 20);
+      chunks.push_back(Chunk{dalloc<char>(size), {}, 0, size});
+      static_allocs_.push_back(chunks.back().dev);
+    }
+    Chunk& c = chunks.back();
+    char* d = c.dev + c.used;
+    c.host.resize(c.used + need);
+    if (bytes) std::memcpy(c.host.data() + c.used, src, bytes);
+    c.used += need;
+    return d;
+  };
+  auto up = [&](const std::vector<double>& v) {
+    return static_cast<const double*>(upload(v.data(), v.size() * sizeof(double)));
+  };
+  auto upi = [&](const std::vector<int>& v) {
+    return static_cast<const int*>(upload(v.data(), v.size() * sizeof(int)));
   };
   const unsigned K = static_cast<unsigned>(knots_.size());
   std::vector<double> lk(K);
@@ -2746,45 +2824,29 @@ void Engine1::build_static() {
         // knot interval of every (term, node): parameter independent, as
         // the range test on |x| / eta and log2|x| + log2(1/eta) are
         const size_t nt = tie.size();
-        std::vector<double> lk(knots_.size());
-        for (size_t k = 0; k < knots_.size(); ++k) lk[k] = std::log2(knots_[k]);
         const int K = static_cast<int>(knots_.size());
+        const double k0 = knots_.front(), k1 = knots_.back();
+        std::vector<double> ax(NI);
+        for (unsigned i = 0; i < NI; ++i) ax[i] = std::fabs(sys.x[i]);
         std::vector<unsigned char> kt(nt * NI, 255);
-        for (size_t j = 0; j < nt; ++j)
-          for (unsigned i = 0; i < NI; ++i) {
-            const double currarg = std::fabs(sys.x[i]) * tie[j];
-            if (currarg < knots_.front() || currarg >= knots_.back()) continue;
-            const double u = lxa[i] + lie[j];
-            int ilo = 0, ihi = K - 1;
-            while (ihi > ilo + 1) {
-              const int mid = (ihi + ilo) >> 1;
-              if (lk[mid] > u) ihi = mid; else ilo = mid;
-            }
-            kt[j * NI + i] = static_cast<unsigned char>(ilo);
-          }
-        unsigned char* d = nullptr;
-        cuda_check(cudaMalloc(&d, kt.size() + 16), "cudaMalloc");
-        static_allocs_.push_back(d);
-        cuda_check(cudaMemcpyAsync(d, kt.data(), kt.size(), cudaMemcpyHostToDevice, stream_), "upload");
-        sd.kidx = d;
         // per node, the first and one past the last term inside the knot
         // range: the only terms the node's sum visits
         std::vector<int2> jr(NI, make_int2(0, 0));
-        for (unsigned i = 0; i < NI; ++i) {
-          int lo = -1, hi = -1;
-          for (size_t j = 0; j < nt; ++j)
-            if (kt[j * NI + i] != 255) {
-              if (lo < 0) lo = static_cast<int>(j);
-              hi = static_cast<int>(j) + 1;
-            }
-          if (lo >= 0) jr[i] = make_int2(lo, hi);
+        for (size_t j = 0; j < nt; ++j) {
+          int ilo = 0;  // moves a step at a time: neighbouring nodes are close
+          for (unsigned i = 0; i < NI; ++i) {
+            const double currarg = ax[i] * tie[j];
+            if (currarg < k0 || currarg >= k1) continue;
+            const double u = lxa[i] + lie[j];
+            while (ilo < K - 2 && !(lk[ilo + 1] > u)) ++ilo;
+            while (ilo > 0 && lk[ilo] > u) --ilo;
+            kt[j * NI + i] = static_cast<unsigned char>(ilo);
+            if (jr[i].y == 0) jr[i].x = static_cast<int>(j);
+            jr[i].y = static_cast<int>(j) + 1;
+          }
         }
-        int2* dj = nullptr;
-        cuda_check(cudaMalloc(&dj, jr.size() * sizeof(int2) + 16), "cudaMalloc");
-        static_allocs_.push_back(dj);
-        cuda_check(cudaMemcpyAsync(dj, jr.data(), jr.size() * sizeof(int2), cudaMemcpyHostToDevice, stream_),
-                   "upload");
-        sd.jrange = dj;
+        sd.kidx = static_cast<const unsigned char*>(upload(kt.data(), kt.size()));
+        sd.jrange = static_cast<const int2*>(upload(jr.data(), jr.size() * sizeof(int2)));
       }
       sd.nodes = 1;
       sd.nterms = static_cast<int>(tie.size());
@@ -2819,14 +2881,12 @@ void Engine1::build_static() {
         sd.grid_hi = static_cast<int>(hi);
         sd.grid_off = g.minflux_R - static_cast<double>(g.wrapRidx + 1) * g.dflux;
       }
-      // interval of every covered grid point (gsl-style bisection)
+      // interval of every covered grid point: the last node not above it,
+      // as gsl's bisection gives it (the fluxes ascend)
+      size_t lo = 0;
       for (int i = sd.grid_lo; i <= sd.grid_hi; ++i) {
         const double cflux = static_cast<double>(i) * g.dflux + sd.grid_off;
-        size_t lo = 0, hi = NI - 1;
-        while (hi > lo + 1) {
-          const size_t mid = (hi + lo) / 2;
-          if (x[mid] > cflux) hi = mid; else lo = mid;
-        }
+        while (lo + 2 < NI && !(x[lo + 1] > cflux)) ++lo;
         gidx[i] = static_cast<int>(lo);
       }
     }
@@ -2890,21 +2950,29 @@ void Engine1::build_static() {
           std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
             return cost(blk[a].second) > cost(blk[b].second);
           });
-          std::vector<std::vector<int>> per(256);
-          std::vector<long> load(256, 0);
+          // the least loaded thread, the lowest of equals, is a heap's top
+          std::vector<std::pair<long, int>> heap(256);
+          for (int t2 = 0; t2 < 256; ++t2) heap[t2] = {0, t2};
+          const std::greater<std::pair<long, int>> later;
+          std::vector<int> owner(blk.size()), cnt(257, 0), slot(blk.size());
           for (int k : order) {
-            int tmin = 0;
-            for (int t2 = 1; t2 < 256; ++t2)
-              if (load[t2] < load[tmin]) tmin = t2;
-            per[tmin].push_back(k);
-            load[tmin] += cost(blk[k].second);
+            std::pop_heap(heap.begin(), heap.end(), later);
+            auto& h = heap.back();
+            owner[k] = h.second;
+            slot[k] = cnt[h.second + 1]++;
+            h.first += cost(blk[k].second);
+            std::push_heap(heap.begin(), heap.end(), later);
           }
+          const int base = static_cast<int>(ar.size() / 2);
           for (int t2 = 0; t2 < 256; ++t2) {
-            off[static_cast<size_t>(bx) * 257 + t2] = static_cast<int>(ar.size() / 2);
-            for (int k : per[t2]) {
-              ar.push_back(blk[k].first);
-              ar.push_back(blk[k].second);
-            }
+            cnt[t2 + 1] += cnt[t2];
+            off[static_cast<size_t>(bx) * 257 + t2] = base + cnt[t2];
+          }
+          ar.resize(ar.size() + 2 * blk.size());
+          for (size_t k = 0; k < blk.size(); ++k) {
+            const size_t o = 2 * (base + static_cast<size_t>(cnt[owner[k]]) + slot[k]);
+            ar[o] = blk[k].first;
+            ar[o + 1] = blk[k].second;
           }
           off[static_cast<size_t>(bx) * 257 + 256] = static_cast<int>(ar.size() / 2);
         }
@@ -2943,12 +3011,8 @@ void Engine1::build_static() {
     }
   }
   D_ = static_cast<unsigned>(h_dsets_.size());
-  d_bsets_ = dalloc<BSet1Dev>(B_);
-  static_allocs_.push_back(d_bsets_);
-  cuda_check(cudaMemcpyAsync(d_bsets_, h_bsets_.data(), B_ * sizeof(BSet1Dev), cudaMemcpyHostToDevice, stream_), "upload");
-  d_dsets_ = dalloc<DSet1Dev>(D_);
-  static_allocs_.push_back(d_dsets_);
-  cuda_check(cudaMemcpyAsync(d_dsets_, h_dsets_.data(), D_ * sizeof(DSet1Dev), cudaMemcpyHostToDevice, stream_), "upload");
+  d_bsets_ = static_cast<BSet1Dev*>(upload(h_bsets_.data(), B_ * sizeof(BSet1Dev)));
+  d_dsets_ = static_cast<DSet1Dev*>(upload(h_dsets_.data(), D_ * sizeof(DSet1Dev)));
   ntile_ = fill_tiles();
   nchunk_ = (n_ + CHUNK - 1) / CHUNK;
   // own FFT: n = 2m, m = m1 * 256 with m1 a power of two in [8, 256].  By
@@ -2960,33 +3024,47 @@ void Engine1::build_static() {
   tune_.own_fft = own_fft_ ? 1 : 0;
   {
     const size_t m = n_ / 2;
-    const long double tau = 6.283185307179586476925286766559005768L;
-    auto table = [&](size_t len, size_t step, size_t period) -> const double2* {
-      std::vector<double2> v(len);
-      for (size_t j = 0; j < len; ++j) {
-        const long double a = -tau * static_cast<long double>(step * j) / static_cast<long double>(period);
-        v[j] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
-      }
-      double2* d = dalloc<double2>(len);
-      static_allocs_.push_back(d);
-      cuda_check(cudaMemcpyAsync(d, v.data(), len * sizeof(double2), cudaMemcpyHostToDevice, stream_), "upload");
-      return d;
-    };
     const bool small = n_ >= 1024 && n_ <= 8192 && (n_ & (n_ - 1)) == 0;
     d_wh_ = d_wl_ = d_wn_ = d_tw_ = nullptr;
-    if (own_fft_) {
-      d_wh_ = table(m / 128, 128, m);
-      d_wl_ = table(128, 1, m);
-    }
-    if (own_fft_ || small) d_wn_ = table(m + 1, 1, n_);
-    if (small) {
-      const std::vector<double2> tw = fft::fft2_twiddles(static_cast<unsigned>(m));
-      double2* d = dalloc<double2>(tw.size());
-      static_allocs_.push_back(d);
-      cuda_check(cudaMemcpyAsync(d, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, stream_), "upload");
-      d_tw_ = d;
+    if (own_fft_ || small) {  // n is a power of two >= 1024
+      // e^{-2 pi i e / n}, from the first octant in long double
+      const size_t q = n_ / 4, o = n_ / 8;
+      std::vector<double2> oct(o + 1);
+      const long double tau = 6.283185307179586476925286766559005768L;
+      for (size_t e = 0; e <= o; ++e) {
+        const long double a = tau * static_cast<long double>(e) / static_cast<long double>(n_);
+        oct[e] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
+      }
+      auto root = [&](size_t e) {
+        const size_t quad = e / q, r = e % q;
+        const double2 w = (r <= o) ? oct[r] : make_double2(oct[q - r].y, oct[q - r].x);
+        switch (quad) {
+          case 0: return make_double2(w.x, -w.y);
+          case 1: return make_double2(-w.y, -w.x);
+          case 2: return make_double2(-w.x, w.y);
+          default: return make_double2(w.y, w.x);
+        }
+      };
+      auto table = [&](size_t len, size_t step) {  // e^{-2 pi i step j / n}
+        std::vector<double2> v(len);
+        for (size_t j = 0; j < len; ++j) v[j] = root(step * j);
+        return static_cast<const double2*>(upload(v.data(), len * sizeof(double2)));
+      };
+      if (own_fft_) {
+        d_wh_ = table(m / 128, 256);
+        d_wl_ = table(128, 2);
+      }
+      d_wn_ = table(m + 1, 1);
+      if (small) {  // fft::fft2_twiddles(m)
+        std::vector<double2> v(m / 4);
+        for (size_t u = 0; u < m / 16; ++u)
+          for (size_t i = 0; i < 4; ++i) v[i * (m / 16) + u] = root(2 * ((u << i) % m));
+        d_tw_ = static_cast<const double2*>(upload(v.data(), v.size() * sizeof(double2)));
+      }
     }
   }
+  for (const Chunk& c : chunks)
+    cuda_check(cudaMemcpyAsync(c.dev, c.host.data(), c.used, cudaMemcpyHostToDevice, stream_), "upload");
   // the uploads went through this engine's stream; launches may go to others
   cuda_check(cudaStreamSynchronize(stream_), "uploads");
   static_ok_ = true;
@@ -3257,9 +3335,9 @@ void Engine1::free_work() {
                   ws_.pmidx, ws_.pinfo, ws_.pdout, ws_.theta_in, ws_.logl,
                   ws_.tmp, ws_.bonus, ws_.kcut_set, ws_.kcut_ds, ws_.rinfo};
   for (void* p : ptrs)
-    if (p) cudaFree(p);
-  if (ws_.h_theta) cudaFreeHost(ws_.h_theta);
-  if (ws_.h_logl) cudaFreeHost(ws_.h_logl);  // h_status lies in the same block
+    give(p);
+  give(ws_.h_theta, true);
+  give(ws_.h_logl, true);  // h_status lies in the same block
   ws_ = Workspace1{};
 }
 
@@ -3644,17 +3722,16 @@ void Engine1::eval_host(unsigned nprop, const float* theta, unsigned npar,
   if (!static_ok_ || ws_.P < nprop) reserve(std::max(nprop, ws_.P));
   cuda_check(cudaSetDevice(device_), "cudaSetDevice");
   if (!ws_.theta_in || ws_.h_npar < npar) {
-    if (ws_.theta_in) cudaFree(ws_.theta_in);
-    if (ws_.h_theta) cudaFreeHost(ws_.h_theta);
+    give(ws_.theta_in);
+    give(ws_.h_theta, true);
     ws_.theta_in = dalloc<float>(static_cast<size_t>(ws_.P) * npar);
-    cuda_check(cudaMallocHost(&ws_.h_theta, static_cast<size_t>(ws_.P) * npar * sizeof(float)), "cudaMallocHost");
+    ws_.h_theta = static_cast<float*>(take(static_cast<size_t>(ws_.P) * npar * sizeof(float), true));
     ws_.h_npar = npar;
     drop_graphs();
   }
   if (!ws_.h_logl) {
     // logL [P] then status [P], as on the device
-    cuda_check(cudaMallocHost(&ws_.h_logl, ws_.P * (sizeof(double) + sizeof(int))),
-               "cudaMallocHost");
+    ws_.h_logl = static_cast<double*>(take(ws_.P * (sizeof(double) + sizeof(int)), true));
     ws_.h_status = reinterpret_cast<int*>(ws_.h_logl + ws_.P);
   }
   std::memcpy(ws_.h_theta, theta, static_cast<size_t>(nprop) * npar * sizeof(float));
@@ -3726,7 +3803,7 @@ void Engine1::rnodes_host(int bs, int side, const float* theta, unsigned npar,
   if (e == cudaSuccess)
     e = cudaMemcpy(r_out, R + (static_cast<size_t>(bs) * 2 + (side & 1)) * NI, NI * sizeof(double),
                    cudaMemcpyDeviceToHost);
-  cudaFree(R);
+  give(R);
   cuda_check(e, "R nodes");
 }
 

@@ -154,10 +154,36 @@ struct Tune1 {
                             // runs inside the forward pass A (own FFT)
 };
 
+// Device and pinned blocks handed from one engine to the next of the same
+// owner (a P(D) factory sets up an engine per call, whose two dozen blocks
+// cost up to 10 ms to map and pin each time).  Bounded by trim(), which frees
+// what the current engine did not take; the rest goes with the pool.  One
+// thread at a time; a block is put back only when its work is done.
+class BlockPool {
+ public:
+  BlockPool() = default;
+  BlockPool(const BlockPool&) = delete;
+  BlockPool& operator=(const BlockPool&) = delete;
+  ~BlockPool();
+  void* get(size_t bytes, bool pinned);  // throws Error
+  void put(void* p);                     // null: nothing
+  void trim();
+
+ private:
+  struct Block {
+    void* p;
+    size_t bytes;
+    bool pinned;
+  };
+  static void release(const Block& b);
+  std::vector<Block> free_, used_;
+};
+
 class Engine1 {
  public:
   static constexpr int KMAX = 64;
-  Engine1(int device, cudaStream_t stream);
+  // pool (may be null): where the engine's memory comes from and goes back to
+  Engine1(int device, cudaStream_t stream, BlockPool* pool = nullptr);
   ~Engine1();
 
   // configuration (host set-up)
@@ -253,8 +279,14 @@ class Engine1 {
   void launch_all(unsigned nprop, const float* theta, unsigned npar,
                   double* logl, int* status, cudaStream_t st, cudaEvent_t* ev);
 
+  void* take(size_t bytes, bool pinned = false);
+  void give(void* p, bool pinned = false);
+  template <class T>
+  T* dalloc(size_t n) { return static_cast<T*>(take(n * sizeof(T) + 16)); }
+
   int device_;
   cudaStream_t stream_;
+  BlockPool* pool_;
   // configuration
   std::vector<double> knots_;
   unsigned n_ = 0, ninterp_ = 2048, nbins_ = 1000;

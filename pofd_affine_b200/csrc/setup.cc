@@ -655,16 +655,27 @@ void KnotQuadrature::build_breaks(const double* logknots, int K, std::vector<dou
   br.erase(std::unique(br.begin(), br.end()), br.end());
   const long double ln2 = 0.693147180559945309417232121458176568L;
   int k = 0;
+  const size_t total = (br.size() - 1) * static_cast<size_t>(nper);
+  u.reserve(total);
+  s.reserve(total);
+  w.reserve(total);
+  kidx.reserve(total);
+  std::vector<long double> off(q), eoff(q);
   for (size_t i = 0; i + 1 < br.size(); ++i) {
     while (k + 2 < K && br[i] >= logknots[k + 1]) ++k;
     const long double a = br[i], b = br[i + 1];
     const long double h = (b - a) / panels;
+    // 2^(lo + off) as 2^lo 2^off: the exponentials of an interval's panels
+    // and of a panel's points apart, 84 instead of 1280
+    for (int g = 0; g < q; ++g) {
+      off[g] = 0.5L * h * (gx[g] + 1.0L);
+      eoff[g] = std::exp2(off[g]);
+    }
     for (int p = 0; p < panels; ++p) {
-      const long double lo = a + p * h;
+      const long double lo = a + p * h, elo = std::exp2(lo);
       for (int g = 0; g < q; ++g) {
-        const long double uu = lo + 0.5L * h * (gx[g] + 1.0L);
-        u.push_back(static_cast<double>(uu));
-        s.push_back(static_cast<double>(std::exp2(uu)));
+        u.push_back(static_cast<double>(lo + off[g]));
+        s.push_back(static_cast<double>(elo * eoff[g]));
         w.push_back(static_cast<double>(ln2 * 0.5L * h * gw[g]));
         kidx.push_back(k);
       }
