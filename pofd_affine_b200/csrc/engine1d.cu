@@ -2734,7 +2734,7 @@ void Engine1::build_static() {
   model_.maxknot = knots_.back();
   {
     SplineSystem ks;
-    ks.factor(lk);
+    ks.factor(lk, false);
     std::vector<double> ia(ks.alpha);
     for (double& v : ia) v = 1.0 / v;
     model_.ih = up(ks.ih);

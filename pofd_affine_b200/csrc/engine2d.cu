@@ -71,98 +71,70 @@ __device__ __forceinline__ long long sat_index(double v) {
 __device__ __forceinline__ double clip0(double v) { return (v < 0) ? 0.0 : v; }
 
 // ------------------------------------------------------------- model
-// Natural cubic spline through (x, y), written per interval as (y,b,c,d);
-// out[4*(n-1)] holds y[n-1].
-__device__ void nat_spline(const double* x, const double* y, int n,
-                           double* out, double* wk) {
-  double* c = wk;
-  double* g = c + KMAX;
-  double* diag = g + KMAX;
-  double* off = diag + KMAX;
-  double* alp = off + KMAX;
-  double* gam = alp + KMAX;
-  for (int k = 0; k < n; ++k) c[k] = 0.0;
-  const int N = n - 2;
-  for (int i = 0; i < N; ++i) {
-    const double h_i = x[i + 1] - x[i], h_ip1 = x[i + 2] - x[i + 1];
-    const double g_i = (h_i != 0.0) ? 1.0 / h_i : 0.0;
-    const double g_ip1 = (h_ip1 != 0.0) ? 1.0 / h_ip1 : 0.0;
-    off[i] = h_ip1;
-    diag[i] = 2.0 * (h_ip1 + h_i);
-    g[i] = 3.0 * ((y[i + 2] - y[i + 1]) * g_ip1 - (y[i + 1] - y[i]) * g_i);
+// Natural cubic spline through (x, y) by one warp, against the system that the
+// host factored (it depends only on the knots), written per interval as
+// (y,b,c,d); out[4*(n-1)] holds y[n-1].  Right-hand side and coefficients by
+// lane, the two substitutions, n - 2 dependent steps each, by the first.
+// y (n values) and c: shared, KMAX each.
+__device__ void nat_spline_warp(const Curve2Dev& m, const double* y, double* c, double* out) {
+  const int n = m.n, N = n - 2, lane = threadIdx.x & 31;
+  for (int i = lane; i < N; i += 32)
+    c[1 + i] = 3.0 * ((y[i + 2] - y[i + 1]) * m.ih[i + 1] - (y[i + 1] - y[i]) * m.ih[i]);
+  __syncwarp();
+  if (lane == 0) {
+    for (int i = 1; i < N; ++i) c[1 + i] = c[1 + i] - m.gamma[i - 1] * c[i];
+    c[0] = 0.0;
+    c[n - 1] = 0.0;
+    if (N > 0) c[N] = c[N] * m.ialpha[N - 1];
+    for (int i = N - 2; i >= 0; --i) c[1 + i] = c[1 + i] * m.ialpha[i] - m.gamma[i] * c[2 + i];
   }
-  if (N == 1) {
-    c[1] = g[0] / diag[0];
-  } else if (N > 1) {
-    alp[0] = diag[0];
-    gam[0] = off[0] / alp[0];
-    for (int i = 1; i < N - 1; ++i) {
-      alp[i] = diag[i] - off[i - 1] * gam[i - 1];
-      gam[i] = off[i] / alp[i];
-    }
-    alp[N - 1] = diag[N - 1] - off[N - 2] * gam[N - 2];
-    for (int i = 1; i < N; ++i) g[i] = g[i] - gam[i - 1] * g[i - 1];
-    for (int i = 0; i < N; ++i) g[i] = g[i] / alp[i];
-    c[N] = g[N - 1];
-    for (int i = N - 2; i >= 0; --i) c[1 + i] = g[i] - gam[i] * c[2 + i];
-  }
-  for (int i = 0; i < n - 1; ++i) {
-    const double dx = x[i + 1] - x[i];
+  __syncwarp();
+  for (int i = lane; i < n - 1; i += 32) {
+    const double dx = m.x[i + 1] - m.x[i];
     const double dy = y[i + 1] - y[i];
     out[4 * i + 0] = y[i];
-    out[4 * i + 1] = (dy / dx) - dx * (c[i + 1] + 2.0 * c[i]) / 3.0;
+    out[4 * i + 1] = dy * m.ih[i] - dx * (c[i + 1] + 2.0 * c[i]) / 3.0;
     out[4 * i + 2] = c[i];
-    out[4 * i + 3] = (c[i + 1] - c[i]) / (3.0 * dx);
+    out[4 * i + 3] = (c[i + 1] - c[i]) * m.ih[i] / 3.0;
   }
-  out[4 * (n - 1)] = y[n - 1];
+  if (lane == 0) out[4 * (n - 1)] = y[n - 1];
 }
 
 // Knot counts (log2-log2 natural spline), sigma and offset curves of one
 // proposal (numberCountsDoubleLogNormal.cc:1010-1052): cnt layout
 // [0,4K) counts, [4K,8K) sigma, [8K,12K) offset; values of 1- or 2-knot
 // curves sit at stride 4.
-__global__ void k_model2(Model2Dev m, const float* __restrict__ theta,
-                         int npar, double logfac, double* __restrict__ cnt,
-                         int* __restrict__ mstatus,
-                         double* __restrict__ sigmult) {
-  __shared__ double wk[6 * KMAX];
-  __shared__ double y[KMAX];
-  __shared__ double o[12 * KMAX];
-  const int w = blockIdx.x;
+// A warp per curve; one thread solving all three from the start, divisions
+// and all, took 15 us.
+__global__ void __launch_bounds__(96)
+k_model2(Model2Dev m, const float* __restrict__ theta, int npar, double logfac,
+         double* __restrict__ cnt, int* __restrict__ mstatus, double* __restrict__ sigmult) {
+  __shared__ double y[3][KMAX], c[3][KMAX];
+  __shared__ int bad[3];
+  const int w = blockIdx.x, q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* th = theta + static_cast<size_t>(w) * npar;
-  if (threadIdx.x == 0) {
-    int st = 0;
-    const int K = m.K, ns = m.ns, no = m.no;
-    for (int k = 0; k < K; ++k) {
-      y[k] = logfac * static_cast<double>(th[k]);
-      if (isnan(y[k])) st = POFD_E_INVALID_MODEL;
-    }
-    if (st == 0) nat_spline(m.logknots, y, K, o, wk);
-    for (int k = 0; k < ns; ++k) {
-      const double v = static_cast<double>(th[K + k]);
-      if (isnan(v) || isinf(v)) st = POFD_E_INVALID_MODEL;
-      y[k] = v;
-    }
-    if (st == 0) {
-      if (ns > 2) nat_spline(m.sk, y, ns, o + 4 * KMAX, wk);
-      else for (int k = 0; k < ns; ++k) o[4 * KMAX + 4 * k] = y[k];
-    }
-    for (int k = 0; k < no; ++k) {
-      const double v = static_cast<double>(th[K + ns + k]);
-      if (isnan(v)) st = POFD_E_INVALID_MODEL;
-      y[k] = v;
-    }
-    if (st == 0) {
-      if (no > 2) nat_spline(m.ok, y, no, o + 8 * KMAX, wk);
-      else for (int k = 0; k < no; ++k) o[8 * KMAX + 4 * k] = y[k];
-    }
-    mstatus[w] = st;
-    sigmult[2 * w] = static_cast<double>(th[K + ns + no]);
-    sigmult[2 * w + 1] = static_cast<double>(th[K + ns + no + 1]);
+  const Curve2Dev& cv = m.curve[q];
+  const float* v = th + (q > 0 ? m.K : 0) + (q > 1 ? m.ns : 0);
+  bool b = false;
+  for (int k = lane; k < cv.n; k += 32) {
+    const double t = static_cast<double>(v[k]);
+    y[q][k] = q ? t : logfac * t;
+    b = b || isnan(t) || (q == 1 && isinf(t));
+  }
+  b = __any_sync(0xffffffffu, b);
+  __syncwarp();
+  if (lane == 0) bad[q] = b;
+  double* o = cnt + static_cast<size_t>(w) * 12 * KMAX + 4 * KMAX * q;
+  if (!b) {
+    if (q == 0 || cv.n > 2) nat_spline_warp(cv, y[q], c[q], o);
+    else if (lane < cv.n) o[4 * lane] = y[q][lane];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 12 * KMAX; i += blockDim.x)
-    cnt[static_cast<size_t>(w) * 12 * KMAX + i] = o[i];
+  if (threadIdx.x == 0) {
+    mstatus[w] = (bad[0] || bad[1] || bad[2]) ? POFD_E_INVALID_MODEL : 0;
+    sigmult[2 * w] = static_cast<double>(th[m.K + m.ns + m.no]);
+    sigmult[2 * w + 1] = static_cast<double>(th[m.K + m.ns + m.no + 1]);
+  }
 }
 
 __device__ __forceinline__ double spline_at(const double* x, const double* s,
@@ -1029,10 +1001,24 @@ __device__ int split_marginal(const double* data, int n, double dflux,
 
 // Marginals, split points, normalisation and means of one (proposal,
 // dataset) (PDFactoryDouble.cc:978-1118, PDDouble.cc:142-208, 355-447).
+// The column sums of a P(D) from its nrt partial rows, into the first of them,
+// in their order.  k_psplit2, one block per P(D), took 80 us for 128 partial
+// rows of n = 4096 (4 MB read by one SM), now 54 with this.
+__global__ void __launch_bounds__(NT)
+k_pcol2(int D, int n, int nrt, const int* __restrict__ mstatus, double* colpart) {
+  const int wd = blockIdx.y, i = blockIdx.x * NT + threadIdx.x;
+  if (mstatus[wd / D] != 0 || i >= n) return;
+  double* cp = colpart + static_cast<size_t>(wd) * nrt * n + i;
+  double c = 0.0;
+#pragma unroll 16
+  for (int k = 0; k < nrt; ++k) c += cp[static_cast<size_t>(k) * n];
+  cp[0] = c;
+}
+
 __global__ void __launch_bounds__(SNT)
 k_psplit2(const BSet2Dev* __restrict__ bsets,
           const DSet2Dev* __restrict__ dsets, int B, int D, int n, int nc2,
-          int nct, int nrt, const int* __restrict__ mstatus,
+          int nct, int nrt, int nrt_sum, const int* __restrict__ mstatus,
           const double* __restrict__ sigmult, const double* __restrict__ mom,
           const double* __restrict__ pbuf, const double* __restrict__ rowpart,
           const double* __restrict__ colpart, PDInfo2* __restrict__ pinfo) {
@@ -1068,7 +1054,7 @@ k_psplit2(const BSet2Dev* __restrict__ bsets,
     for (int k = 0; k < nct; ++k) s += rp[static_cast<size_t>(i) * nct + k];
     Srow[i] = s;
     double c = 0.0;
-    for (int k = 0; k < nrt; ++k) c += cp[static_cast<size_t>(k) * n + i];
+    for (int k = 0; k < nrt_sum; ++k) c += cp[static_cast<size_t>(k) * n + i];
     Scol[i] = c;
   }
   __syncthreads();
@@ -2180,9 +2166,22 @@ void Engine2::build_static() {
   model_.K = static_cast<int>(knots_.size());
   model_.ns = static_cast<int>(sigk_.size());
   model_.no = static_cast<int>(offk_.size());
-  model_.logknots = up(lk);
-  model_.sk = up(sigk_);
-  model_.ok = up(offk_);
+  const std::vector<double>* curves[3] = {&lk, &sigk_, &offk_};
+  for (int q = 0; q < 3; ++q) {
+    const std::vector<double>& x = *curves[q];
+    Curve2Dev& c = model_.curve[q];
+    c = Curve2Dev{static_cast<int>(x.size()), up(x), nullptr, nullptr, nullptr};
+    if (q > 0 && x.size() <= 2) continue;  // a constant or a line
+    SplineSystem ks;
+    ks.factor(x, false);
+    for (double& v : ks.alpha) v = 1.0 / v;
+    c.ih = up(ks.ih);
+    c.ialpha = up(ks.alpha);
+    c.gamma = up(ks.gamma);
+  }
+  model_.logknots = model_.curve[0].x;
+  model_.sk = model_.curve[1].x;
+  model_.ok = model_.curve[2].x;
   model_.minknot = knots_.front();
   model_.maxknot = knots_.back();
   model_.min_sigma = 0.0;
@@ -2596,7 +2595,7 @@ void Engine2::launch_all(unsigned nprop, const float* theta, unsigned npar,
   const int ne = edge_ ? static_cast<int>(nedge_) : 0;
   Plans& pl = plans_.at(nprop);
   mark(0);
-  k_model2<<<P, 32, 0, st>>>(model_, theta, static_cast<int>(npar), std::log2(10.0),
+  k_model2<<<P, 96, 0, st>>>(model_, theta, static_cast<int>(npar), std::log2(10.0),
                              ws_.cnt, ws_.mstatus, ws_.sigmult);
   if (prior_.needs_bonus())
     k_bonus2<<<P, kBonus2Threads, 0, st>>>(model_, const_cast<float*>(theta), static_cast<int>(npar),
@@ -2694,8 +2693,11 @@ void Engine2::launch_all(unsigned nprop, const float* theta, unsigned npar,
                                                       ws_.rowpart, ws_.colpart);
   }
   mark(s);
+  const int nrt = static_cast<int>(nrt_);
+  if (cols_first())
+    k_pcol2<<<dim3((n + NT - 1) / NT, P * D), NT, 0, st>>>(D, n, nrt, ws_.mstatus, ws_.colpart);
   k_psplit2<<<P * D, SNT, 3 * static_cast<size_t>(n) * sizeof(double), st>>>(
-      d_bsets_, d_dsets_, B, D, n, pitch, nct, static_cast<int>(nrt_),
+      d_bsets_, d_dsets_, B, D, n, pitch, nct, nrt, cols_first() ? 1 : nrt,
       ws_.mstatus, ws_.sigmult, ws_.mom, ws_.pbuf, ws_.rowpart, ws_.colpart, ws_.pinfo);
   if (refsum_)
     k_pseq2<<<P * D, NT, static_cast<size_t>(n) * sizeof(double), st>>>(
@@ -2851,7 +2853,7 @@ void Engine2::set_regularization(double alpha) {
 void Engine2::bonus_launch(unsigned nprop, float* theta_dev, unsigned npar, int fill_at,
                            cudaStream_t st) {
   const int P = static_cast<int>(nprop);
-  k_model2<<<P, 32, 0, st>>>(model_, theta_dev, static_cast<int>(npar), std::log2(10.0),
+  k_model2<<<P, 96, 0, st>>>(model_, theta_dev, static_cast<int>(npar), std::log2(10.0),
                              ws_.bcnt, ws_.bstatus, ws_.bsig);
   k_bonus2<<<P, kBonus2Threads, 0, st>>>(model_, theta_dev, static_cast<int>(npar),
                                          std::log2(10.0), ws_.bcnt, ws_.bstatus, d_qu_, d_qs_,

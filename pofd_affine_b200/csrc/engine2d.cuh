@@ -68,8 +68,13 @@ struct DSet2Dev {
   double bc1, bc2, bd1, bd2;
 };
 
+struct Curve2Dev {  // a model curve's knots and factored spline system
+  int n;
+  const double *x, *ih, *ialpha, *gamma;
+};
 struct Model2Dev {
   int K, ns, no;
+  Curve2Dev curve[3];  // counts (log2 knots), sigma, offset
   const double* logknots;
   const double* sk;
   const double* ok;
@@ -147,9 +152,13 @@ class Engine2 {
   int num_stages() const { return colspec_ ? 11 : kNumStages; }
   // the stage names of the FFT mode in use
   const char* stage_name_now(int i) const;
+  // The P(D)'s column sums are made by a kernel of their own where one block
+  // would read long: split search and sums with and without it 54 and 80 us
+  // at 128 partial rows (n = 4096), 36 and 38 at 64, 26 and 22 at 32.
+  bool cols_first() const { return nrt_ >= 64; }
   int kernels_per_eval() const {
-    return (edge_ ? 12 : 10) + (colspec_ ? 1 : 0) + (prior_.needs_bonus() ? 1 : 0) +
-           (refsum_ ? 1 : 0);
+    return (edge_ ? 12 : 10) + (colspec_ ? 1 : 0) + (cols_first() ? 1 : 0) +
+           (prior_.needs_bonus() ? 1 : 0) + (refsum_ ? 1 : 0);
   }
   // Reference-order normalisation and means (k_pseq2 after the split
   // search): the P(D) integral and the two means summed in one sequential

@@ -107,15 +107,15 @@ void Beam1::terms(bool negside, std::vector<double>& w,
 // off-diagonal h_i+1, factored as L D L^T (the factorisation the reference's
 // spline library performs each time it fits the spline, e.g.
 // PDFactory.cc:522 for the R nodes).
-void SplineSystem::factor(const std::vector<double>& xn) {
+void SplineSystem::factor(const std::vector<double>& xn, bool distinct) {
   x = xn;
   const size_t n = x.size();
   if (n < 3) throw Error(POFD_E_ARG, "spline needs at least 3 nodes");
   ih.resize(n - 1);
   for (size_t i = 0; i + 1 < n; ++i) {
     const double h = x[i + 1] - x[i];
-    if (!(h > 0)) throw Error(POFD_E_ARG, "spline nodes must increase");
-    ih[i] = 1.0 / h;
+    if (distinct && !(h > 0)) throw Error(POFD_E_ARG, "spline nodes must increase");
+    ih[i] = (h != 0.0) ? 1.0 / h : 0.0;
   }
   const size_t N = n - 2;
   std::vector<double> diag(N), off(N);

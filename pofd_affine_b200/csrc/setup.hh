@@ -65,7 +65,9 @@ struct Beam1 {
 // and two first-order recurrences.
 struct SplineSystem {
   std::vector<double> x, ih, alpha, gamma;  // ih: 1/h_i (n-1); alpha,gamma: n-2
-  void factor(const std::vector<double>& xn);
+  // distinct: equal neighbours are an error, else intervals without inverse
+  // (the logarithms of knots an ulp apart may be equal)
+  void factor(const std::vector<double>& xn, bool distinct = true);
 };
 
 // Data set: mean-subtracted pixels, binned.
