@@ -31,6 +31,7 @@
 #include "common.cuh"
 #include "fft1d.cuh"
 #include "fft2.cuh"
+#include "fftmix.cuh"
 
 namespace pofd {
 
@@ -1788,8 +1789,8 @@ __global__ void k_reduce1(const BSet1Dev* __restrict__ bsets, int B, int D,
 }
 
 // ------------------------------------------------------------------
-// Small grids (n = 2m, m a power of two in [512, 4096], up to ROW1_MAXNI
-// nodes): one block takes a (proposal, beam set) row from the R nodes to the
+// Small grids (n = 2m <= 8192, m a power of two from 512 or 2^a 3^b 5^c 7^d,
+// up to ROW1_MAXNI nodes): one block takes a (proposal, beam set) row from the R nodes to the
 // log-likelihood of its datasets -- node spline, R grid, forward transform,
 // spectrum, inverse transform, split search, normalisation and gather --
 // without leaving shared memory.  As separate kernels (with cuFFT) these are
@@ -1800,17 +1801,29 @@ __global__ void k_reduce1(const BSet1Dev* __restrict__ bsets, int B, int D,
 // move a load it takes for invariant ahead of the wait.
 constexpr int RU = 3;  // runs per thread whose static data is read ahead
 constexpr int ROW1_MAXN = 8192;
+constexpr unsigned ROW1_MIXMIN = 256;  // below, no measurements
 constexpr int ROW1_MAXNI = 4096;
 constexpr int ROW1_MAXDS = 64;  // datasets per beam set
 
 struct Row1Mem {  // sizes in doubles of the block's shared memory regions
   int a, b, d;
   int several;    // P(D) in d, where b keeps the spectrum for the next dataset
+  int split;      // a block per dataset, each doing the set's part again
+  int n, nf;      // grid size and, of a mixed transform, its stages' radices
+  unsigned char f[fft::MIX_STAGES];
 };
+inline bool row1_pow2(int n) { return n >= 1024 && (n & (n - 1)) == 0; }
 inline Row1Mem row1_mem(int n, int ni, bool several) {
   const int m = n / 2, pn = row1_pad(ni) + 1;
-  Row1Mem r;
+  Row1Mem r{};
+  r.n = n;
   r.a = 2 * 256 * (m / 256 + 1);              // transform slots; R grid padded
+  if (!row1_pow2(n)) {
+    int f[fft::MIX_STAGES];
+    r.nf = fft::mix_factor(m, f);
+    for (int k = 0; k < r.nf; ++k) r.f[k] = static_cast<unsigned char>(f[k]);
+    r.a = (n + n / 16 + 2) & ~1;
+  }
   r.b = std::max(2 * pn, 2 * (m + 1));        // spline y, c; then the spectrum; P(D)
   r.d = std::max(2 * pn, several ? n : 0);    // spline factors; P(D)
   r.several = several ? 1 : 0;
@@ -1820,6 +1833,8 @@ inline size_t row1_smem(const Row1Mem& r) {
   return static_cast<size_t>(r.a + r.b + r.d) * sizeof(double);
 }
 
+// M2: m where it is a power of two from 512 (fft2.cuh), 0 for other sizes
+// (fftmix.cuh).
 template <int M2, int T>
 __global__ void __launch_bounds__(T, 512 / T)
 k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, int B, int D,
@@ -1828,9 +1843,10 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
        const double2* __restrict__ Wn, const double2* __restrict__ TW, double* __restrict__ mom,
        double* __restrict__ pbuf, PDInfo1* __restrict__ pinfo, Prior1 pr,
        const double* bonus, double* __restrict__ logl, int* __restrict__ status) {
-  using F = fft::Fft2<M2>;
-  constexpr int M = F::M, M3 = F::M3, n = 2 * M2, m = M2;
-  constexpr int nc2 = 2 * (n / 2 + 1);
+  using F = fft::Fft2<M2 ? M2 : 512>;
+  constexpr int M = F::M, M3 = F::M3;
+  const int n = M2 ? 2 * M2 : mem.n, m = n / 2;
+  const int nc2 = 2 * (n / 2 + 1);
   extern __shared__ double rs[];
   double* A = rs;
   double* Bm = A + mem.a;
@@ -1840,13 +1856,19 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
   __shared__ double red[4][T / 32];
   __shared__ int redi[T / 32], s_kc[ROW1_MAXDS];
   __shared__ dev::Exp2Table e2;
-  const int wb = blockIdx.x;
-  const int w = wb / B, b = wb - w * B;
+  const int w = blockIdx.x / (mem.split ? D : B);
+  const int b = mem.split ? dsets[blockIdx.x - w * D].bs : blockIdx.x - w * B;
+  const int wb = w * B + b;
   const int t = threadIdx.x;
   const BSet1Dev& bs = bsets[b];
+  const int d0 = mem.split ? static_cast<int>(blockIdx.x) - w * D - bs.ds_begin : 0;
+  const int d1 = mem.split ? d0 + 1 : bs.nds;
   // what does not depend on the nodes kernel, before waiting for it: the
   // exp2 table, and of the thread's first runs the descriptors and nodes
   e2.load();
+  if constexpr (M2 == 0)  // the twiddles, a line a thread
+    for (int i = t; i < (m + 7) / 8; i += T)
+      asm volatile("prefetch.global.L1 [%0];" : : "l"(TW + 8 * i));
   int2 rd[RU];
   double rx[RU], rdx[RU], rih[RU];
 #pragma unroll
@@ -1868,8 +1890,8 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
   dev::pdl_wait();
   const int st0 = mstatus[w];
   if (st0 != 0) {
-    for (int dd = t; dd < bs.nds; dd += T) pinfo[static_cast<size_t>(w) * D + bs.ds_begin + dd].status = st0;
-    if (B == 1 && t == 0) {
+    for (int dd = d0 + t; dd < d1; dd += T) pinfo[static_cast<size_t>(w) * D + bs.ds_begin + dd].status = st0;
+    if (B == 1 && !mem.split && t == 0) {
       logl[w] = __longlong_as_double(0x7ff8000000000000LL);
       status[w] = st0;
     }
@@ -1999,7 +2021,7 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
     var -= cf * prod;
   }
   const bool doshift = (sqrt(var) > dflux) && (fabs(mn) > dflux);
-  if (t == 0) {
+  if (t == 0 && d0 == 0) {
     double* o = mom + static_cast<size_t>(wb) * 4;
     o[0] = mn;
     o[1] = var;
@@ -2007,11 +2029,14 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
     o[3] = doshift ? 1.0 : 0.0;
   }
   int kcmax = 0;
-  for (int dd = 0; dd < bs.nds; ++dd) kcmax = max(kcmax, s_kc[dd]);
+  for (int dd = d0; dd < d1; ++dd) kcmax = max(kcmax, s_kc[dd]);
   const int qmax = min(m / 2, kcmax);
   // ---- forward transform of z_j = R_2j + i R_2j+1
-  const bool act = t < M;
-  double2 v[16];
+  [[maybe_unused]] const bool act = t < M;
+  [[maybe_unused]] double2 v[16];
+  if constexpr (M2 == 0) {
+    fft::mix_fft<T>(m, mem.nf, mem.f, TW, z, fft::MixIo{A, m, false, z});
+  } else {
   if (act) {
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
@@ -2032,11 +2057,12 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
     }
   }
   __syncthreads();
+  }
   // ---- spectrum on pairs (q, m - q), before the noise
   const double iflux = dev::kTwoPi / (static_cast<double>(n) * dflux);
   const double shiftw = doshift ? -mn * iflux : 0.0;
   double2* S = reinterpret_cast<double2*>(Bm);
-  auto slot = [](int k) { return (k & 255) * (M3 + 1) + (k >> 8); };
+  auto slot = [](int k) { return M2 ? (k & 255) * (M3 + 1) + (k >> 8) : k; };
   {
     const double2 z0 = z[0];
     const double r0 = z0.x + z0.y;  // X_0
@@ -2062,7 +2088,7 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
   }
   __syncthreads();
   double* P = mem.several ? Dm : Bm;
-  for (int dd = 0; dd < bs.nds; ++dd) {
+  for (int dd = d0; dd < d1; ++dd) {
     const int d = bs.ds_begin + dd;
     const double sigma = sm * dsets[d].sigma_base;
     const int kc = s_kc[dd];
@@ -2095,6 +2121,9 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
     __syncthreads();
     // ---- inverse transform: the wrapped P(D) row
     double2* p2 = reinterpret_cast<double2*>(P);
+    if constexpr (M2 == 0) {  // by the forward one, parts exchanged
+      fft::mix_fft<T>(m, mem.nf, mem.f, TW, z, fft::MixIo{nullptr, kc, true, p2});
+    } else {
     if (act) {
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
@@ -2117,6 +2146,7 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
       }
     }
     __syncthreads();
+    }
     // ---- chunk reductions over the whole row (k_pscan1)
     const SplitParams sp = split_params(bs, var, sigma);
     double2* prow = reinterpret_cast<double2*>(pbuf + (static_cast<size_t>(w) * D + d) * nc2);
@@ -2177,7 +2207,7 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
                   });
     __syncthreads();
   }
-  if (B == 1 && t == 0)
+  if (B == 1 && !mem.split && t == 0)
     reduce_one(bsets, B, D, w, sm, pinfo, pr, bonus, logl, status);
 }
 
@@ -3024,19 +3054,24 @@ void Engine1::build_static() {
   tune_.own_fft = own_fft_ ? 1 : 0;
   {
     const size_t m = n_ / 2;
-    const bool small = n_ >= 1024 && n_ <= 8192 && (n_ & (n_ - 1)) == 0;
+    const bool small = n_ <= 8192 && row1_pow2(static_cast<int>(n_));
+    int f[fft::MIX_STAGES];
+    const bool mixed = !small && n_ >= ROW1_MIXMIN && n_ <= static_cast<unsigned>(ROW1_MAXN) &&
+                       n_ % 2 == 0 && fft::mix_factor(static_cast<int>(m), f) > 0;
     d_wh_ = d_wl_ = d_wn_ = d_tw_ = nullptr;
-    if (own_fft_ || small) {  // n is a power of two >= 1024
-      // e^{-2 pi i e / n}, from the first octant in long double
-      const size_t q = n_ / 4, o = n_ / 8;
+    if (own_fft_ || small || mixed) {
+      // e^{-2 pi i e / n}, from the first octant in long double; where 8 does
+      // not divide n (mixed sizes), of the multiples that it divides
+      const size_t mul = (n_ % 8 == 0) ? 1 : (n_ % 4 == 0) ? 2 : 4;
+      const size_t nn = n_ * mul, q = nn / 4, o = nn / 8;
       std::vector<double2> oct(o + 1);
       const long double tau = 6.283185307179586476925286766559005768L;
       for (size_t e = 0; e <= o; ++e) {
-        const long double a = tau * static_cast<long double>(e) / static_cast<long double>(n_);
+        const long double a = tau * static_cast<long double>(e) / static_cast<long double>(nn);
         oct[e] = make_double2(static_cast<double>(cosl(a)), static_cast<double>(sinl(a)));
       }
-      auto root = [&](size_t e) {
-        const size_t quad = e / q, r = e % q;
+      auto root = [&](size_t en) {  // en < n
+        const size_t e = en * mul, quad = e / q, r = e % q;
         const double2 w = (r <= o) ? oct[r] : make_double2(oct[q - r].y, oct[q - r].x);
         switch (quad) {
           case 0: return make_double2(w.x, -w.y);
@@ -3055,6 +3090,7 @@ void Engine1::build_static() {
         d_wl_ = table(128, 2);
       }
       d_wn_ = table(m + 1, 1);
+      if (mixed) d_tw_ = table(m, 2);
       if (small) {  // fft::fft2_twiddles(m)
         std::vector<double2> v(m / 4);
         for (size_t u = 0; u < m / 16; ++u)
@@ -3096,6 +3132,7 @@ void Engine1::profile_stages(unsigned nprop, const float* theta, unsigned npar,
   std::vector<double> lls(nprop);
   std::vector<int> sts(nprop);
   eval_host(nprop, theta, npar, lls.data(), sts.data());  // staging + warm
+  prof_rows_ = nprop;
   cudaEvent_t ev[kNumStages + 1];
   for (auto& e : ev) cuda_check(cudaEventCreate(&e), "event create");
   for (int k = 0; k < num_stages(); ++k) stage_ms[k] = 0.0;
@@ -3232,7 +3269,7 @@ const char* Engine1::stage_name(int i) const {
       "k_reduce1"};
   if (i < 0 || i >= num_stages()) return "";
   static const char* row[] = {"k_rnodes1", "k_row1", "k_reduce1"};
-  if (row1()) return row[i];
+  if (row1(prof_rows_)) return row[i];
   if (!own_fft_) return lib[i];
   return fused_fill() ? fused[i] : own[i];
 }
@@ -3404,10 +3441,10 @@ void Engine1::reserve(unsigned P) {
 
 void Engine1::ensure_plans(unsigned nprop) {
   auto it = plans_.find(nprop);
-  if (it != plans_.end() && (it->second.fwd || own_fft_ || row1())) return;
+  if (it != plans_.end() && (it->second.fwd || own_fft_ || row1(nprop))) return;
   Plans pl;
   if (it != plans_.end()) pl = it->second;
-  if (own_fft_ || row1()) {  // the own FFT needs no cuFFT plans; the entry holds graphs
+  if (own_fft_ || row1(nprop)) {  // the own FFT needs no cuFFT plans; the entry holds graphs
     plans_[nprop] = pl;
     return;
   }
@@ -3424,19 +3461,28 @@ void Engine1::ensure_plans(unsigned nprop) {
 }
 
 
-// The single-block kernel where the transform may be the library's own, the
-// fill is by running products and the row fits a block: at any batch.  One
+// The single-block kernel where the transform may be the library's own (a
+// power of two, or an even size with no prime above 7), the fill is by running
+// products and the row fits a block: at any batch.  One
 // likelihood call (2048 nodes, host to host), this kernel's sequence and the
 // one of eight to nine kernels: n = 4096, 1 row 46.0 and 63.8 us, 148 rows
 // 59.5 and 85.3, 600 rows (a third wave hardly begun) 162 and 188, 2048 rows
 // 424 and 508; n = 1024, 1 row 43.7 and 57.0, 2048 rows 371 and 399; n = 8192
 // (one row to an SM), 1 row 49.7 and 71.2, 148 rows 63 and 98, 600 rows (a
-// fifth wave hardly begun) 207 and 226, 1000 rows 312 and 345.
-bool Engine1::row1() const {
+// fifth wave hardly begun) 207 and 226, 1000 rows 312 and 345.  Mixed sizes
+// while each dataset's row has an SM to itself: n = 6000, 1 row 69 and 75 us,
+// 25 rows 74 and 84, 148 rows 82 and 109, 296 rows 143 and 153; n = 1000, 1 row
+// 47 and 55, 148 rows 61 and 72, but 296 rows 94 and 85; n = 8100 (three 3s:
+// six stages), 1 row 84 and 76, 148 rows 96 and 119.
+bool Engine1::row1(unsigned nprop) const {
   for (const auto& s : sets_)
     if (s.data.size() > static_cast<size_t>(ROW1_MAXDS)) return false;
-  return fft_mode_ != 1 && tune_.rfill_mode == 3 && n_ >= 1024 && n_ <= 8192 &&
-         (n_ & (n_ - 1)) == 0 && ninterp_ <= static_cast<unsigned>(ROW1_MAXNI);
+  int f[fft::MIX_STAGES];
+  return fft_mode_ != 1 && tune_.rfill_mode == 3 && n_ <= static_cast<unsigned>(ROW1_MAXN) &&
+         ninterp_ <= static_cast<unsigned>(ROW1_MAXNI) &&
+         (row1_pow2(static_cast<int>(n_)) ||
+          (n_ >= ROW1_MIXMIN && n_ % 2 == 0 && fft::mix_factor(static_cast<int>(n_ / 2), f) > 0 &&
+           static_cast<size_t>(nprop) * D_ <= static_cast<size_t>(sm_count_)));
 }
 
 namespace {
@@ -3448,8 +3494,8 @@ void launch_row1_t(int rows, size_t smem, cudaStream_t st, Args... args) {
 }
 template <int M2, class... Args>
 void launch_row1(bool wide, int rows, size_t smem, cudaStream_t st, Args... args) {
-  if (wide || M2 == ROW1_MAXN / 2) launch_row1_t<M2, 512>(rows, smem, st, args...);
-  else if constexpr (M2 < ROW1_MAXN / 2) launch_row1_t<M2, 256>(rows, smem, st, args...);
+  if (wide || M2 == ROW1_MAXN / 2 || M2 == 0) launch_row1_t<M2, 512>(rows, smem, st, args...);
+  else if constexpr (M2 < ROW1_MAXN / 2 && M2 > 0) launch_row1_t<M2, 256>(rows, smem, st, args...);
 }
 }  // namespace
 
@@ -3489,10 +3535,16 @@ void Engine1::launch_all(unsigned nprop, const float* theta, unsigned npar,
                                           std::log2(10.0), ws_.cnt, ws_.mstatus, d_qu_, d_qs_,
                                           d_qw_, qper_, ws_.bonus, -1);
   mark(1);
-  if (row1()) {
+  if (row1(nprop)) {
     bool several = false;
     for (const auto& bs : h_bsets_) several = several || bs.nds > 1;
-    const Row1Mem mem = row1_mem(n, NI, several);
+    // several datasets to a set: a block each while every block has an SM to
+    // itself (the set's part, done again, costs nothing there): three datasets
+    // of n = 4096 one after the other and apart, 20 rows 66 and 50 us, 49 rows
+    // 70 and 53; two of 70 rows 63 and 55
+    const bool split = several && P * D <= sm_count_;
+    Row1Mem mem = row1_mem(n, NI, several && !split);
+    mem.split = split ? 1 : 0;
     const size_t smem = row1_smem(mem);
     // 512 threads a row while every row has an SM to itself, and at n = 8192,
     // whose rows never share one; else 256, two rows to an SM.  One likelihood
@@ -3502,18 +3554,19 @@ void Engine1::launch_all(unsigned nprop, const float* theta, unsigned npar,
     // 8192, 1 row 49.3 and 53.4, 150 rows 90 and 100, 592 rows 180 and 207.
     const bool wide = P * B <= sm_count_;
 #define POFD_ROW1(M2)                                                                          \
-  launch_row1<M2>(wide, P * B, smem, st, d_bsets_, d_dsets_, B, D, NI, mem, std::log(2.0),           \
+  launch_row1<M2>(wide, P * (split ? D : B), smem, st, d_bsets_, d_dsets_, B, D, NI, mem, std::log(2.0),           \
                   ws_.mstatus, ws_.sigmult, ws_.nodes, d_wn_, d_tw_, ws_.mom, ws_.pbuf,        \
                   ws_.pinfo, prior_, ws_.bonus, logl, status)
     switch (n) {
       case 1024: POFD_ROW1(512); break;
       case 2048: POFD_ROW1(1024); break;
       case 4096: POFD_ROW1(2048); break;
-      default: POFD_ROW1(4096); break;
+      case 8192: POFD_ROW1(4096); break;
+      default: POFD_ROW1(0); break;
     }
 #undef POFD_ROW1
     mark(2);
-    if (B > 1)
+    if (B > 1 || split)
       k_reduce1<<<(P + 127) / 128, 128, 0, st>>>(d_bsets_, B, D, P, ws_.mstatus, ws_.sigmult,
                                                 ws_.pinfo, prior_, ws_.bonus, logl, status);
     mark(3);

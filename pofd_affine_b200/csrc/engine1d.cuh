@@ -217,7 +217,8 @@ class Engine1 {
                    double* x_out, double* r_out);
   void rgrid_host(int bs, const float* theta, unsigned npar, double* out);
   int kernels_per_eval() const {
-    if (row1()) return 1 + 1 + (B_ > 1 ? 1 : 0) + (prior_.needs_bonus() ? 1 : 0);
+    // (one more where few rows of a set with several datasets go a block each)
+    if (row1(1)) return 1 + 1 + (B_ > 1 ? 1 : 0) + (prior_.needs_bonus() ? 1 : 0);
     return (own_fft_ ? (fused_fill() ? 10 : 11) : 8) + (prior_.needs_bonus() ? 1 : 0);
   }
   // the R grid fill runs inside the forward FFT pass A (own FFT, plain passes)
@@ -250,7 +251,7 @@ class Engine1 {
   void fill_bonus(unsigned nprop, float* theta_dev, unsigned npar, cudaStream_t st);
   static constexpr int kNumStages = 10;
   static constexpr size_t kOwnFftMin = 8192;  // automatic four-step FFT from here
-  int num_stages() const { return row1() ? 3 : own_fft_ ? kNumStages - 1 : kNumStages; }
+  int num_stages() const { return row1(prof_rows_) ? 3 : own_fft_ ? kNumStages - 1 : kNumStages; }
   void profile_stages(unsigned nprop, const float* theta, unsigned npar,
                       int reps, double* stage_ms);
   const char* stage_name(int i) const;
@@ -340,7 +341,8 @@ class Engine1 {
   const double2* d_wl_ = nullptr;  // e^{-2 pi i i / m}, i < 128
   const double2* d_wn_ = nullptr;  // e^{-2 pi i k / n}, k <= m
   const double2* d_tw_ = nullptr;  // fft::fft2_twiddles(m) (the single-block kernel)
-  bool row1() const;
+  bool row1(unsigned nprop) const;
+  unsigned prof_rows_ = 1;  // rows of the last profile_stages
   double time_sequence(unsigned nprop, const float* theta, unsigned npar, int reps);
   Tune1 tune_;
   // priors and the knot quadrature of the bonus integrals
