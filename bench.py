@@ -300,8 +300,9 @@ def stage_bytes(stage, P, B, D, n, cuts=None):
     cut-offs of the own-FFT path (noise_cuts), the bins that path skips:
     forward pass B writes only bins with min(k, m - k) <= kc of the beam
     set (the widest of its datasets), the spectrum reads only those pairs
-    and writes, per dataset, only the 256-bin rows the inverse pass A reads,
-    and pass A reads only those rows."""
+    and writes, per dataset, only the 256-bin rows the inverse reads; where
+    those are at most 8 the inverse is one pass over them, else pass A reads
+    them and pass B its rows."""
     nc = n // 2 + 1
     m = n // 2
     row = 16.0 * m  # one complex row of m points
@@ -322,7 +323,8 @@ def stage_bytes(stage, P, B, D, n, cuts=None):
             for kc in kcs:
                 g = float(np.mean(rmin <= kc))
                 spec += P * row * g
-                inv += P * row * (3.0 + g)
+                few = kc < 1024 and (kc >> 8) + 1 + ((kc + 255) >> 8) <= min(8, m // 512)
+                inv += P * row * ((1.0 if few else 3.0) + g)
     # forward pass B alone (pass A fused with the R fill): reads the rows,
     # writes the bins inside the cut-off
     fwdB = 2.0 * row * P * B
@@ -334,12 +336,12 @@ def stage_bytes(stage, P, B, D, n, cuts=None):
     return {
         # own FFT path (n = 2m, m complex per row): passes A and B each read
         # and write the rows; the spectrum reads Z and writes one row per
-        # dataset
+        # dataset; the P(D) reductions are part of the inverse
         "k_fftA1+k_fftB1": fwd,
         "k_fftAR1": row * P * B,                              # write pass A rows
         "k_fftB1": fwdB,
         "k_spectrum1f": spec,
-        "k_fftA1+k_fftB1_inv": inv,
+        "k_fftA1+k_inv1": inv,
         "k_rfill1": 8.0 * n * P * B,                         # write R
         "k_spectrum1": 16.0 * nc * P * B + 16.0 * nc * P * D,  # read R~, write per-dataset spectra
         "k_pscan1": 8.0 * n * P * D,                          # read P(D)
@@ -438,12 +440,13 @@ def cpu_baseline_2d(cfg, seconds, nthreads=None):
 def roofline_2d(L, cfg, thetas, stages, P):
     """Rooflines of the two dominant 2D kernels from the stage times.
     k_rgrid2 (FP64): every active colour term of every main-grid row is
-    evaluated once per column, 25 flops each (the table exp2 21, the
-    squared offset 3, the weighted add 1); the active terms per proposal
+    evaluated once per column, 20 flops each (the offset 2, the table
+    Gaussian 16, the weighted add 2); the active terms per proposal
     are counted by the library for the first proposal and taken for all.
     k_colspec2 (HBM): per proposal it reads the row-transformed R spectrum
-    and writes one column-transformed spectrum per dataset, 16 n (n/2+1)
-    bytes each."""
+    and writes one column-transformed spectrum per dataset, 16 n bytes for
+    each column inside the noise cut-off (min(n/2, ceil(12 n dflux2 / (2 pi
+    sigma2)) + 1) + 1 of them; the widest for the reads)."""
     import ctypes as C
     from pofd_affine_b200._lib import support_lib
     n = cfg["fftsize"]
@@ -457,7 +460,7 @@ def roofline_2d(L, cfg, thetas, stages, P):
     out = {"active_terms_per_proposal": {"main_rows": main, "edge_rows": edge}}
     ms = stages.get("k_rgrid2")
     if ms:
-        flops = 25.0 * main * (n - 1) * P
+        flops = 20.0 * main * (n - 1) * P
         ach = flops / (ms * 1e-3) / 1e12
         tp = read_traffic("k_rgrid2", per_proposal=True)
         out["roofline_rgrid2"] = {
@@ -466,14 +469,18 @@ def roofline_2d(L, cfg, thetas, stages, P):
             "unit": "TFLOP/s", "frac": ach / pk.value,
             "traffic": tp * P if tp else None,
             "peak_source": "measured (pofd_fp64_peak DFMA loop)"}
-    ms = stages.get("k_r0sum2+k_colspec2")
+    ms = stages.get("k_colspec2")
     if ms:
-        nds = len(cfg["maps"])
-        nbytes = 16.0 * n * nc * (1 + nds) * P
+        cols = []
+        for d in range(len(cfg["maps"])):
+            df2 = L.getPD(0, d, thetas[0], setLog=False)[1]["dflux2"]
+            x = 12.0 * n * df2 / (2 * np.pi * cfg["sigmas"][d][1])
+            cols.append(nc if x >= n // 2 else min(nc, int(np.ceil(x)) + 2))
+        nbytes = 16.0 * n * (max(cols) + sum(cols)) * P
         ach = nbytes / (ms * 1e-3) / 1e9
         tp = read_traffic("k_colspec2", per_proposal=True)
         out["roofline_colspec2"] = {
-            "bound": "hbm", "kernel": "k_r0sum2+k_colspec2", "ms_per_launch": ms,
+            "bound": "hbm", "kernel": "k_colspec2", "ms_per_launch": ms,
             "algorithmic_bytes": nbytes, "achieved": ach, "peak": hbm_peak,
             "unit": "GB/s", "frac": ach / hbm_peak,
             "traffic": tp * P if tp else None,

@@ -226,13 +226,15 @@ int pofd_like1_profile(pofd_like1* L, unsigned nprop, const float* theta,
                        unsigned npar, int reps, double* stage_ms,
                        int* nstages);
 const char* pofd_like1_stage_name(const pofd_like1* L, int i);
-/* Transform used by the likelihood.  By default (no mode set) this
- * library's own FP64 four-step FFT, fused with the R-grid fill and the
- * spectrum, runs when the FFT size is a power of two in [8192, 131072] and
- * cuFFT otherwise (at n = 4096 batched cuFFT is the faster one); mode 0
- * runs the own FFT whenever the size is a power of two in [4096, 131072];
- * mode 1 always uses cuFFT.  pofd_like1_fft_info reports whether the own
- * FFT is in use.  The reference uses FFTW (PDFactory.cc:293-338). */
+/* Transform used by the likelihood.  By default (no mode set) a single
+ * block takes each row through everything, its transforms in shared memory,
+ * when the FFT size is a power of two in [1024, 8192], or an even size in
+ * [256, 8192] with no prime factor above 7 and one block per SM is enough;
+ * this library's FP64 four-step FFT, fused with the R-grid fill and the
+ * spectrum, when it is a power of two in [8192, 131072]; cuFFT otherwise.
+ * Mode 0 sets the four-step FFT up from 4096; mode 1 always uses cuFFT.
+ * pofd_like1_fft_info reports whether the four-step FFT is set up.  The
+ * reference uses FFTW (PDFactory.cc:293-338). */
 int pofd_like1_set_fft(pofd_like1* L, int mode);
 int pofd_like1_fft_info(pofd_like1* L, int* own);
 
@@ -363,12 +365,12 @@ const char* pofd_like2_stage_name(int i);
 const char* pofd_like2_stage_name_now(const pofd_like2* L, int i);
 
 /* FFT of the 2D likelihood (the project's own choice; the reference plans
- * FFTW 2D transforms, PDFactoryDouble.cc:727-768): mode 1 (default) runs
- * batched 1D cuFFT transforms along the rows and this library's kernel that
- * transforms the columns, applies exp/shift/noise per bin and transforms the
- * columns back, where n is a power of two in [512, 4096] (else mode 0);
- * mode 0 runs batched 2D cuFFT transforms with the spectrum kernel between
- * them.  fft_info reports whether the fused column path is in use. */
+ * FFTW 2D transforms, PDFactoryDouble.cc:727-768): mode 1 (default) runs this
+ * library's row and column kernels -- rows forward, the columns inside the
+ * noise cut-off forward, exp/shift/noise per bin and back, rows back with the
+ * marginals -- where n is a power of two in [512, 4096] (else mode 0); mode 0
+ * runs batched 2D cuFFT transforms with the spectrum kernel between them.
+ * fft_info reports whether the row and column kernels are in use. */
 int pofd_like2_set_fft(pofd_like2* L, int mode);
 int pofd_like2_fft_info(const pofd_like2* L, int* fused);
 
@@ -383,7 +385,7 @@ int pofd_like2_set_reference_sums(pofd_like2* L, int on);
 /* Autotuner of the 2D launch shapes (the project's own; no counterpart in
  * the reference): times the whole graph-captured launch sequence on nprop
  * host rows (reps replays per candidate, CUDA events) for each knob in turn
- * -- FFT mode (see pofd_like2_set_fft), R-grid rows per block {2, 4, 8},
+ * -- FFT mode (see pofd_like2_set_fft), R-grid rows per block in fours {2, 4, 8},
  * band-1 edge rows per group {4, 8, 16} -- and keeps the fastest.  out5
  * (optional) = {fft_mode, rgrid_rows, edge_rows, best ms, untuned ms}.
  * get/set_tuning read or impose the three knobs in that order.  Results

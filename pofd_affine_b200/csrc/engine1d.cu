@@ -17,10 +17,14 @@
 //   spl   [P][B][2][NI][4]     node spline (y, b, c, d) per interval
 //   rbuf  [P][B][2*nc]         R grid (x dflux), then its D2Z spectrum in place
 //   pbuf  [P][D][2*nc]         per-dataset spectrum, then its Z2D P(D) in place
-//   ppart/pmidx [P][D][nchunk] chunk reductions of the P(D)
+//   tmp   [P][max(B,D)][2*nc]  rows between the passes of the own FFT; spectra
+//                              of few rows on their way to k_inv1
+//   ppart/pmidx                partial reductions of the P(D): [P][D][nchunk]
+//                              of k_pscan1, [P][D][blocks] of k_inv1
 //   pinfo [P][D]               split, normalisation, mean, log-likelihood
 // Each proposal's R and P(D) rows are contiguous so the D2Z/Z2D run as two
-// batched cuFFT calls over P*B and P*D rows.
+// batched cuFFT calls over P*B and P*D rows.  Small grids use nodes, pbuf and
+// pinfo only (k_row1 keeps the rest in shared memory).
 #include "engine1d.cuh"
 
 #include <algorithm>
@@ -3045,10 +3049,11 @@ void Engine1::build_static() {
   d_dsets_ = static_cast<DSet1Dev*>(upload(h_dsets_.data(), D_ * sizeof(DSet1Dev)));
   ntile_ = fill_tiles();
   nchunk_ = (n_ + CHUNK - 1) / CHUNK;
-  // own FFT: n = 2m, m = m1 * 256 with m1 a power of two in [8, 256].  By
-  // default (no FFT mode set) from n = 8192: at n = 4096 batched cuFFT is
-  // ~5 % faster on the B200, above it the own FFT is faster (1.6x at
-  // n = 65536 and 131072); on request (set_fft_mode(0)) from n = 4096.
+  // four-step FFT: n = 2m, m = m1 * 256 with m1 a power of two in [8, 256].
+  // By default (no FFT mode set) from n = 8192 (used there where the
+  // single-block kernel is switched off): against batched cuFFT 5 % slower at
+  // n = 4096, 1.6x faster at n = 65536 and 131072; on request
+  // (set_fft_mode(0)) from n = 4096.
   own_fft_ = (fft_mode_ == 0 || (fft_mode_ < 0 && n_ >= kOwnFftMin)) && n_ >= 4096 && n_ <= 131072 &&
              (n_ & (n_ - 1)) == 0;
   tune_.own_fft = own_fft_ ? 1 : 0;

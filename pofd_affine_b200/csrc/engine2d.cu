@@ -18,8 +18,10 @@
 // T terms per row slot):
 //   rw    [P][B][n + nedge][T][3]  per-row colour terms (c0, a, b)
 //   rbuf  [P][B][n][2nc]           R grid (x dflux1 dflux2), then its 2D
-//                                  spectrum in place
-//   pbuf  [P][D][n][2nc]           per-dataset spectrum, then the P(D)
+//                                  spectrum in place; with the row and column
+//                                  kernels the columns [P][D][nc][n]
+//   pbuf  [P][D][n][2nc]           per-dataset spectrum, then the P(D); with
+//                                  those kernels R at pitch n, then the P(D)
 //   rowpart/colpart                marginal partial sums of the P(D)
 #include "engine2d.cuh"
 
