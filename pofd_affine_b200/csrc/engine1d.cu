@@ -2010,6 +2010,9 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
     red[0][t >> 5] = mn;
     red[1][t >> 5] = var;
   }
+  // read ahead of the barrier: past it the transform's threads, which meet
+  // without the others, write over the grid
+  const double redge = (wrap < n - 1) ? A[Fill1::pad(wrap - 1)] : 0.0;
   __syncthreads();
   mn = red[0][0];
   var = red[1][0];
@@ -2020,7 +2023,7 @@ k_row1(const BSet1Dev* __restrict__ bsets, const DSet1Dev* __restrict__ dsets, i
   }
   if (wrap < n - 1) {
     const double cf = bs.minflux_R;
-    const double prod = 0.5 * cf * A[Fill1::pad(wrap - 1)];
+    const double prod = 0.5 * cf * redge;
     mn -= prod;
     var -= cf * prod;
   }
