@@ -2500,6 +2500,19 @@ void Engine1::give(void* p, bool pinned) {
   else cudaFree(p);
 }
 
+// The single-block kernel's shared memory limit.  It belongs to the kernel,
+// not to an engine: every engine sets the same, the most that any size, node
+// count and number of datasets takes (each region grows with them), so that
+// none lowers it between another thread's set-up and launch.
+template <int M2>
+void row1_attr() {
+  const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  const int sm = static_cast<int>(row1_smem(row1_mem(ROW1_MAXN, ROW1_MAXNI, true)));
+  cuda_check(cudaFuncSetAttribute(k_row1<M2, 512>, dyn, sm), "attr");
+  if constexpr (M2 > 0 && M2 < ROW1_MAXN / 2)
+    cuda_check(cudaFuncSetAttribute(k_row1<M2, 256>, dyn, sm), "attr");
+}
+
 Engine1::Engine1(int device, cudaStream_t stream, BlockPool* pool)
     : device_(device), stream_(stream), pool_(pool) {}
 
@@ -3434,6 +3447,13 @@ void Engine1::reserve(unsigned P) {
   // logL [P] then status [P] in one allocation: one download per call
   ws_.logl = dalloc<double>(P + (P + 1) / 2);
   ws_.status = reinterpret_cast<int*>(ws_.logl + P);
+  switch (n_) {
+    case 1024: row1_attr<512>(); break;
+    case 2048: row1_attr<1024>(); break;
+    case 4096: row1_attr<2048>(); break;
+    case 8192: row1_attr<4096>(); break;
+    default: row1_attr<0>(); break;
+  }
   for (auto k : {k_rnodes1<1>, k_rnodes1<4>})
     cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>((KMAX + 4 * KMAX + 2 * MAXTERMS) * sizeof(double))),
@@ -3494,16 +3514,12 @@ bool Engine1::row1(unsigned nprop) const {
 }
 
 namespace {
-template <int M2, int T, class... Args>
-void launch_row1_t(int rows, size_t smem, cudaStream_t st, Args... args) {
-  cuda_check(cudaFuncSetAttribute(k_row1<M2, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)), "attr");
-  launch_pdl(k_row1<M2, T>, dim3(rows), dim3(T), smem, st, args...);
-}
 template <int M2, class... Args>
 void launch_row1(bool wide, int rows, size_t smem, cudaStream_t st, Args... args) {
-  if (wide || M2 == ROW1_MAXN / 2 || M2 == 0) launch_row1_t<M2, 512>(rows, smem, st, args...);
-  else if constexpr (M2 < ROW1_MAXN / 2 && M2 > 0) launch_row1_t<M2, 256>(rows, smem, st, args...);
+  if (wide || M2 == ROW1_MAXN / 2 || M2 == 0)
+    launch_pdl(k_row1<M2, 512>, dim3(rows), dim3(512), smem, st, args...);
+  else if constexpr (M2 < ROW1_MAXN / 2 && M2 > 0)
+    launch_pdl(k_row1<M2, 256>, dim3(rows), dim3(256), smem, st, args...);
 }
 }  // namespace
 
