@@ -190,8 +190,10 @@ __device__ __forceinline__ double3 row_term(const BSet2Dev& bs, const Model2Dev&
                           sg.logratio[j];
         a = kSqrt32OverLn2 * isigma;
         b = -a * c1;
-        // an infinite or undefined Gaussian makes R undefined
-        if (!isfinite(a) || !isfinite(b)) c0 = __longlong_as_double(0x7ff8000000000000LL);
+        // an infinite offset leaves no source in band 2: the Gaussian is 0 and
+        // the term skipped; a sigma of 0 or an undefined offset makes R undefined
+        if (isinf(c1) && isfinite(c0)) c0 = 0.0;
+        else if (!isfinite(a) || !isfinite(b)) c0 = __longlong_as_double(0x7ff8000000000000LL);
       }
     }
   }
