@@ -214,8 +214,9 @@ int pofd_like1_pd(pofd_like1* L, int beamset, int dataset, const float* theta,
 int pofd_like1_rnodes(pofd_like1* L, int beamset, int negative_side,
                       const float* theta, unsigned npar, double* x_out,
                       double* r_out);
-/* Number of this library's kernels one eval_batch launches (cuFFT's own
- * kernels not counted). */
+/* Number of this library's kernels one eval_batch of the last evaluation's
+ * batch size launches (one row before any; cuFFT's own kernels and the
+ * reduction of the block-per-dataset form not counted). */
 int pofd_like1_kernels_per_eval(const pofd_like1* L, int* nkernels);
 /* Per-stage device time of one launch sequence over nprop proposals
  * (host theta), averaged over reps runs timed with CUDA events between the

@@ -3704,6 +3704,7 @@ void Engine1::enqueue(unsigned nprop, const float* theta_dev, unsigned npar,
   if (!static_ok_ || ws_.P < nprop) reserve(std::max(nprop, ws_.P));
   cuda_check(cudaSetDevice(device_), "cudaSetDevice");
   ensure_plans(nprop);
+  eval_rows_ = nprop;
   if (!st) st = stream_;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cuda_check(cudaStreamIsCapturing(st, &cs), "cudaStreamIsCapturing");
@@ -3813,6 +3814,7 @@ void Engine1::eval_host(unsigned nprop, const float* theta, unsigned npar,
   }
   std::memcpy(ws_.h_theta, theta, static_cast<size_t>(nprop) * npar * sizeof(float));
   ensure_plans(nprop);
+  eval_rows_ = nprop;
   cudaGraphExec_t g = host_graph_for(nprop, npar);
   if (g) {
     cuda_check(cudaGraphLaunch(g, stream_), "graph launch");

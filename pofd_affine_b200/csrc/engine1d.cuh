@@ -216,9 +216,10 @@ class Engine1 {
   void rnodes_host(int bs, int side, const float* theta, unsigned npar,
                    double* x_out, double* r_out);
   void rgrid_host(int bs, const float* theta, unsigned npar, double* out);
+  // of the last evaluation's batch size (one row before any), whose path it
+  // takes; one more where the datasets of few rows go a block each
   int kernels_per_eval() const {
-    // (one more where few rows of a set with several datasets go a block each)
-    if (row1(1)) return 1 + 1 + (B_ > 1 ? 1 : 0) + (prior_.needs_bonus() ? 1 : 0);
+    if (row1(eval_rows_)) return 1 + 1 + (B_ > 1 ? 1 : 0) + (prior_.needs_bonus() ? 1 : 0);
     return (own_fft_ ? (fused_fill() ? 10 : 11) : 8) + (prior_.needs_bonus() ? 1 : 0);
   }
   // the R grid fill runs inside the forward FFT pass A (own FFT, plain passes)
@@ -343,6 +344,7 @@ class Engine1 {
   const double2* d_tw_ = nullptr;  // fft::fft2_twiddles(m) (the single-block kernel)
   bool row1(unsigned nprop) const;
   unsigned prof_rows_ = 1;  // rows of the last profile_stages
+  unsigned eval_rows_ = 1;  // rows of the last evaluation
   double time_sequence(unsigned nprop, const float* theta, unsigned npar, int reps);
   Tune1 tune_;
   // priors and the knot quadrature of the bonus integrals
