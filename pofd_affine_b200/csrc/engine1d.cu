@@ -1484,6 +1484,66 @@ __device__ __forceinline__ double logp_at(const double* __restrict__ p, int n,
   return (v > 0.0) ? log2(v) : dev::kSmallLogVal;
 }
 
+// A normalised P(D) row as the data see it.
+struct Unwrap1 {
+  const double* p;
+  int n, split;
+  double itot, minflux, maxfluxval, idflux;
+
+  __device__ __forceinline__ double at(int j) const { return logp_at(p, n, split, itot, j); }
+  // log2 P at a flux, interpolated; outside the grid its end values (the
+  // unbinned form includes the edge values themselves)
+  template <bool BINNED>
+  __device__ __forceinline__ double at_flux(double f) const {
+    const bool lo = BINNED ? f < minflux : f <= minflux;
+    const bool hi = BINNED ? f > maxfluxval : f >= maxfluxval;
+    const double delt = (f - minflux) * idflux;
+    const int idx = lo ? 0 : (hi ? n - 1 : static_cast<int>(delt));
+    const double t = delt - static_cast<double>(idx);
+    const double a = at(idx), b = at((lo || hi) ? idx : idx + 1);
+    return (lo || hi) ? a : (1.0 - t) * a + t * b;
+  }
+};
+
+// K bins or pixels of a thread, e0, e0 + NTH, ...: their reads and logarithms
+// overlap.  Those past the last are not added.
+template <int K, int NTH, bool BINNED>
+__device__ __forceinline__ void gather_k(const DSet1Dev& ds, const Unwrap1& u, int nnz, int e0,
+                                         double& ll) {
+  double cnt[K], f[K], v[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int e = min(e0 + k * NTH, nnz - 1);
+    if (BINNED) {
+      cnt[k] = ds.nzcnt[e];
+      f[k] = ds.bincent0 + static_cast<double>(ds.nzidx[e]) * ds.bindelta;
+    } else {
+      f[k] = ds.flux[e];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = u.at_flux<BINNED>(f[k]);
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (e0 + k * NTH < nnz) ll += BINNED ? v[k] * cnt[k] : v[k];
+}
+
+// The thread's part of the dataset's log2 likelihood.  A warp whose last bins
+// are fewer than a group takes them one by one.
+template <int NTH, bool BINNED>
+__device__ __forceinline__ double gather1(const DSet1Dev& ds, const Unwrap1& u) {
+  constexpr int U = NTH > 256 ? 2 : 4;
+  const int nnz = ds.nnz, w0 = static_cast<int>(threadIdx.x) & ~31;
+  double ll = 0.0;
+  int e = threadIdx.x;
+  for (; e - static_cast<int>(threadIdx.x) + w0 + (U > 2 ? U - 2 : U - 1) * NTH < nnz; e += U * NTH)
+    gather_k<U, NTH, BINNED>(ds, u, nnz, e, ll);
+#pragma unroll 1
+  for (; e - static_cast<int>(threadIdx.x) + w0 < nnz; e += NTH)
+    gather_k<1, NTH, BINNED>(ds, u, nnz, e, ll);
+  return ll;
+}
+
 // What the split search needs of a row's clipped values.
 struct RowMin1 {
   double peak, minval;  // largest value; smallest inside the search window
@@ -1626,36 +1686,8 @@ __device__ __forceinline__ void finish_row(const BSet1Dev& bs, const DSet1Dev& d
   const double maxflux = minflux + static_cast<double>(n - 1) * dflux;
   const double maxfluxval = maxflux - dflux;
   const double idflux = 1.0 / dflux;
-  // several bins or pixels at a time: their reads, and the logarithms, overlap
-  double ll = 0.0;
-  constexpr int U = NTH > 256 ? 2 : 4;
-  for (int e0 = threadIdx.x; e0 < ds.nnz; e0 += U * NTH) {
-    double cnt[U], cflux[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = min(e0 + u * NTH, ds.nnz - 1);
-      cnt[u] = ds.binned ? ds.nzcnt[e] : 1.0;
-      cflux[u] = ds.binned ? ds.bincent0 + static_cast<double>(ds.nzidx[e]) * ds.bindelta
-                           : ds.flux[e];
-    }
-    double v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      // outside the grid its end values (the unbinned form includes the edge
-      // values themselves)
-      const bool lo = ds.binned ? cflux[u] < minflux : cflux[u] <= minflux;
-      const bool hi = ds.binned ? cflux[u] > maxfluxval : cflux[u] >= maxfluxval;
-      const double delt = (cflux[u] - minflux) * idflux;
-      const int idx = lo ? 0 : (hi ? n - 1 : static_cast<int>(delt));
-      const double t = delt - static_cast<double>(idx);
-      const double a = logp_at(p, n, split, itot, idx);
-      const double b = logp_at(p, n, split, itot, (lo || hi) ? idx : idx + 1);
-      v[u] = (lo || hi) ? a : (1.0 - t) * a + t * b;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (e0 + u * NTH < ds.nnz) ll += ds.binned ? v[u] * cnt[u] : v[u];
-  }
+  const Unwrap1 u1{p, n, split, itot, minflux, maxfluxval, idflux};
+  double ll = ds.binned ? gather1<NTH, true>(ds, u1) : gather1<NTH, false>(ds, u1);
   ll = dev::block_sum<NTH>(ll, shd);
   if (threadIdx.x == 0) {
     info.status = 0;
