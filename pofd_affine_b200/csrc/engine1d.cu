@@ -3523,26 +3523,62 @@ void Engine1::ensure_plans(unsigned nprop) {
 
 // The single-block kernel where the transform may be the library's own (a
 // power of two, or an even size with no prime above 7), the fill is by running
-// products and the row fits a block: at any batch.  One
-// likelihood call (2048 nodes, host to host), this kernel's sequence and the
-// one of eight to nine kernels: n = 4096, 1 row 46.0 and 63.8 us, 148 rows
-// 59.5 and 85.3, 600 rows (a third wave hardly begun) 162 and 188, 2048 rows
-// 424 and 508; n = 1024, 1 row 43.7 and 57.0, 2048 rows 371 and 399; n = 8192
-// (one row to an SM), 1 row 49.7 and 71.2, 148 rows 63 and 98, 600 rows (a
-// fifth wave hardly begun) 207 and 226, 1000 rows 312 and 345.  Mixed sizes
-// while each dataset's row has an SM to itself: n = 6000, 1 row 69 and 75 us,
-// 25 rows 74 and 84, 148 rows 82 and 109, 296 rows 143 and 153; n = 1000, 1 row
-// 47 and 55, 148 rows 61 and 72, but 296 rows 94 and 85; n = 8100 (three 3s:
-// six stages), 1 row 84 and 76, 148 rows 96 and 119.
+// products and the row fits a block.  One likelihood call (2048 nodes, host to
+// host), this kernel's sequence and the one of eight to nine kernels: n = 4096,
+// 1 row 46.0 and 63.8 us, 148 rows 59.5 and 85.3, 600 rows (a third wave hardly
+// begun) 162 and 188, 2048 rows 424 and 508; n = 1024, 1 row 43.7 and 57.0,
+// 2048 rows 371 and 399; n = 8192 (one row to an SM), 1 row 49.7 and 71.2, 148
+// rows 63 and 98, 600 rows (a fifth wave hardly begun) 207 and 226, 1000 rows
+// 312 and 345.  Mixed sizes while each dataset's row has an SM to itself: n =
+// 6000, 1 row 69 and 75 us, 25 rows 74 and 84, 148 rows 82 and 109, 296 rows
+// 143 and 153; n = 1000, 1 row 47 and 55, 148 rows 61 and 72, but 296 rows 94
+// and 85; n = 8100 (three 3s: six stages), 1 row 84 and 76, 148 rows 96 and 119.
+// Powers of two in larger batches by row1_turns.
 bool Engine1::row1(unsigned nprop) const {
   for (const auto& s : sets_)
     if (s.data.size() > static_cast<size_t>(ROW1_MAXDS)) return false;
+  if (fft_mode_ == 1 || tune_.rfill_mode != 3 || n_ > static_cast<unsigned>(ROW1_MAXN) ||
+      ninterp_ > static_cast<unsigned>(ROW1_MAXNI))
+    return false;
+  const bool fits = static_cast<size_t>(nprop) * D_ <= static_cast<size_t>(sm_count_);
+  if (row1_pow2(static_cast<int>(n_))) return fits || row1_turns(nprop);
   int f[fft::MIX_STAGES];
-  return fft_mode_ != 1 && tune_.rfill_mode == 3 && n_ <= static_cast<unsigned>(ROW1_MAXN) &&
-         ninterp_ <= static_cast<unsigned>(ROW1_MAXNI) &&
-         (row1_pow2(static_cast<int>(n_)) ||
-          (n_ >= ROW1_MIXMIN && n_ % 2 == 0 && fft::mix_factor(static_cast<int>(n_ / 2), f) > 0 &&
-           static_cast<size_t>(nprop) * D_ <= static_cast<size_t>(sm_count_)));
+  return fits && n_ >= ROW1_MIXMIN && n_ % 2 == 0 &&
+         fft::mix_factor(static_cast<int>(n_ / 2), f) > 0;
+}
+
+// Past a block per dataset: whether the blocks' turns take less than the
+// separate kernels.  A block takes its set's datasets one after the other, with
+// their bins, and the batch takes whole waves of blocks (one 512-thread block to
+// an SM, then two of 256), while the separate kernels spread rows, datasets and
+// bins over the GPU.  Both estimated in us, less what they share; the constants
+// fit 800 batches of 5 to 2000 rows, 1 to 40 datasets of binned maps or 2000 to
+// 30000 pixels, 1 to 3 sets, n = 1024 to 8192, 2048 nodes, and choose the faster
+// side or one within 2 % of it in 784 of them (the worst 7 % slower).  One call,
+// single-block and separate kernels, us: n = 1024, 20 rows x 8 datasets 95 and
+// 64, 3 x 64 499 and 89, 20 x 40 323 and 98, 300 x 2 113 and 112, 148 x 2 70 and
+// 80, 1000 x 1 203 and 219, 300 rows of 100000 pixels 552 and 487; n = 4096,
+// 300 x 4 167 and 163, 450 x 4 185 and 210, 1000 x 3 329 and 373; n = 8192,
+// 150 x 6 196 and 142, 1000 x 6 691 and 562.
+bool Engine1::row1_turns(unsigned nprop) const {
+  const double x = n_ * 1e-3, sms = sm_count_;
+  const double rows = static_cast<double>(nprop) * B_, drows = static_cast<double>(nprop) * D_;
+  const bool narrow = rows > sms && n_ < static_cast<unsigned>(ROW1_MAXN);
+  double block = 0.0, bins = 0.0, most = 0.0;  // of the longest set; all and most bins, thousands
+  for (const BSet1Dev& bs : h_bsets_) {
+    double k = 0.0;
+    for (int d = bs.ds_begin; d < bs.ds_begin + bs.nds; ++d) {
+      const double e = h_dsets_[d].nnz * 1e-3;
+      k += e;
+      most = std::max(most, e);
+    }
+    bins += k;
+    block = std::max(block, narrow ? 3.22 + 8.04 * bs.nds + 1.22 * k
+                                   : 6.53 + (4.28 + 0.45 * x) * bs.nds + 1.01 * k);
+  }
+  const double turns = std::ceil(rows / (narrow ? 2.0 * sms : sms)) * block;
+  const double gather = std::max(std::ceil(drows / (4.0 * sms)) * bins / D_, most);
+  return turns <= 18.7 + 1.39 * x + 0.0161 * rows + (0.02 + 0.00261 * x) * drows + 1.85 * gather;
 }
 
 namespace {

@@ -343,6 +343,7 @@ class Engine1 {
   const double2* d_wn_ = nullptr;  // e^{-2 pi i k / n}, k <= m
   const double2* d_tw_ = nullptr;  // fft::fft2_twiddles(m) (the single-block kernel)
   bool row1(unsigned nprop) const;
+  bool row1_turns(unsigned nprop) const;
   unsigned prof_rows_ = 1;  // rows of the last profile_stages
   unsigned eval_rows_ = 1;  // rows of the last evaluation
   double time_sequence(unsigned nprop, const float* theta, unsigned npar, int reps);

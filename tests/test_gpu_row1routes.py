@@ -32,3 +32,17 @@ def test_mixed_size_counts_by_batch(gpu_ctx):
     assert L.kernelsPerEval() == 2  # one row
     assert _launches(L, th0, 200) == 8
     assert _launches(L, th0, 100) == 2
+
+
+@pytest.mark.parametrize("n,ndata,npix,rows,launches", [
+    (1024, 64, 0, 2, 2), (1024, 64, 0, 3, 8), (2048, 8, 0, 18, 2), (2048, 8, 0, 20, 8),
+    (4096, 2, 0, 80, 2), (4096, 40, 0, 20, 8), (8192, 40, 0, 20, 10), (1024, 1, 0, 600, 2),
+    (1024, 1, 60000, 148, 2), (1024, 1, 60000, 300, 8), (1024, 2, 30000, 300, 8)])
+def test_serial_work_of_a_block(gpu_ctx, n, ndata, npix, rows, launches):
+    """A block takes the datasets of its row, and their bins, in turn: many of
+    them go to the separate kernels unless each has a block of its own."""
+    L, th0 = _engine(gpu_ctx, n, ndata, 1, npix)
+    assert _launches(L, th0, rows) == launches
+    ll = L.getLogLikeBatch(np.tile(th0, (rows, 1)))[0]
+    L.setFFT(1)
+    assert np.all(np.abs(L.getLogLikeBatch(np.tile(th0, (rows, 1)))[0] - ll) < 1e-7 * (1 + npix * ndata / 4096))
