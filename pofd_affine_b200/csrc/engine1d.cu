@@ -1838,6 +1838,7 @@ __global__ void k_reduce1(const BSet1Dev* __restrict__ bsets, int B, int D,
 constexpr int RU = 3;  // runs per thread whose static data is read ahead
 constexpr int ROW1_MAXN = 8192;
 constexpr unsigned ROW1_MIXMIN = 256;  // below, no measurements
+constexpr unsigned ROW1_MIXLARGE = 7400;  // above, from 32 rows of datasets (row1)
 constexpr int ROW1_MAXNI = 4096;
 constexpr int ROW1_MAXDS = 64;  // datasets per beam set
 
@@ -3532,7 +3533,12 @@ void Engine1::ensure_plans(unsigned nprop) {
 // 312 and 345.  Mixed sizes while each dataset's row has an SM to itself: n =
 // 6000, 1 row 69 and 75 us, 25 rows 74 and 84, 148 rows 82 and 109, 296 rows
 // 143 and 153; n = 1000, 1 row 47 and 55, 148 rows 61 and 72, but 296 rows 94
-// and 85; n = 8100 (three 3s: six stages), 1 row 84 and 76, 148 rows 96 and 119.
+// and 85.  The largest of them not for the smallest batches: the stages of one
+// block grow with the size, cuFFT's launches hardly.  1 row of n = 7056 73 and
+// 74 us, 7290 77 and 77, 7500 79 and 73, 8000 79 and 72, 8100 (seven stages) 89
+// and 76; 40 rows of 8000 83 and 78, 80 rows 86 and 91, 1 row x 32 datasets 85
+// and 92.  A P(D) factory's engine serves a call or two, which cuFFT's plans
+// would be made for: initPD and getPD of n = 8100 0.55 and 2.8 ms.
 // Powers of two in larger batches by row1_turns.
 bool Engine1::row1(unsigned nprop) const {
   for (const auto& s : sets_)
@@ -3544,7 +3550,8 @@ bool Engine1::row1(unsigned nprop) const {
   if (row1_pow2(static_cast<int>(n_))) return fits || row1_turns(nprop);
   int f[fft::MIX_STAGES];
   return fits && n_ >= ROW1_MIXMIN && n_ % 2 == 0 &&
-         fft::mix_factor(static_cast<int>(n_ / 2), f) > 0;
+         fft::mix_factor(static_cast<int>(n_ / 2), f) > 0 &&
+         (n_ <= ROW1_MIXLARGE || static_cast<size_t>(nprop) * D_ >= 32 || pool_);
 }
 
 // Past a block per dataset: whether the blocks' turns take less than the

@@ -37,10 +37,13 @@ def test_mixed_size_counts_by_batch(gpu_ctx):
 @pytest.mark.parametrize("n,ndata,npix,rows,launches", [
     (1024, 64, 0, 2, 2), (1024, 64, 0, 3, 8), (2048, 8, 0, 18, 2), (2048, 8, 0, 20, 8),
     (4096, 2, 0, 80, 2), (4096, 40, 0, 20, 8), (8192, 40, 0, 20, 10), (1024, 1, 0, 600, 2),
-    (1024, 1, 60000, 148, 2), (1024, 1, 60000, 300, 8), (1024, 2, 30000, 300, 8)])
+    (1024, 1, 60000, 148, 2), (1024, 1, 60000, 300, 8), (1024, 2, 30000, 300, 8),
+    (7290, 1, 0, 1, 2), (7500, 2, 0, 3, 8), (8100, 1, 0, 1, 8), (8100, 1, 0, 31, 8),
+    (8100, 1, 0, 32, 2), (8100, 4, 0, 37, 2), (8100, 4, 0, 38, 8)])
 def test_serial_work_of_a_block(gpu_ctx, n, ndata, npix, rows, launches):
     """A block takes the datasets of its row, and their bins, in turn: many of
-    them go to the separate kernels unless each has a block of its own."""
+    them go to the separate kernels unless each has a block of its own.  So do
+    the largest mixed sizes in the smallest batches."""
     L, th0 = _engine(gpu_ctx, n, ndata, 1, npix)
     assert _launches(L, th0, rows) == launches
     ll = L.getLogLikeBatch(np.tile(th0, (rows, 1)))[0]
