@@ -300,6 +300,7 @@ int pofd_pdfactory1_initpd(pofd_pdfactory1* f, unsigned n, double minflux,
       if (std::isnan(static_cast<double>(knotvals[k])))
         throw pofd::Error(POFD_E_INVALID_MODEL, "Invalid model");
     cudaSetDevice(f->ctx->device);
+    f->pool.trim();  // what the engine before did not take
     f->eng.reset();  // its blocks go to the next one
     f->eng.reset(new pofd::Engine1(f->ctx->device, f->ctx->stream, &f->pool));
     f->eng->configure(nknots, knotpos, n, f->ninterp, true, 1);

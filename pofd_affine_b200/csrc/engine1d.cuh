@@ -157,8 +157,10 @@ struct Tune1 {
 // Device and pinned blocks handed from one engine to the next of the same
 // owner (a P(D) factory sets up an engine per call, whose two dozen blocks
 // cost up to 10 ms to map and pin each time).  Bounded by trim(), which frees
-// what the current engine did not take; the rest goes with the pool.  One
-// thread at a time; a block is put back only when its work is done.
+// what the current engine did not take and which the owner calls before each
+// engine gives its blocks back: two engines' blocks at most are held.  The rest
+// goes with the pool.  One thread at a time; a block is put back only when its
+// work is done.
 class BlockPool {
  public:
   BlockPool() = default;
