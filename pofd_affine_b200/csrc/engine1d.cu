@@ -3946,12 +3946,15 @@ void Engine1::rnodes_host(int bs, int side, const float* theta, unsigned npar,
   const Side1Dev& sd = h_bsets_[bs].side[side & 1];
   if (!sd.nodes) throw Error(POFD_E_ARG, "beam has no such side");
   const size_t NI = ninterp_;
-  double* R = dalloc<double>(static_cast<size_t>(B_) * 2 * NI);
+  const size_t nr = static_cast<size_t>(B_) * 2 * NI;
+  double* R = dalloc<double>(nr);
+  // an invalid model has no R: its nodes are 0
+  cudaError_t e = cudaMemsetAsync(R, 0, nr * sizeof(double), stream_);
   k_rnodes1<1><<<dim3(static_cast<unsigned>((NI + 127) / 128), B_ * 2), 128,
               (KMAX + 4 * KMAX + 2 * static_cast<size_t>(maxterms_)) * sizeof(double), stream_>>>(
       d_bsets_, model_, static_cast<int>(B_), static_cast<int>(NI), maxterms_, ws_.theta_in,
       static_cast<int>(npar), std::log2(10.0), ws_.cnt, ws_.mstatus, ws_.sigmult, ws_.nodes, R);
-  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
   if (e == cudaSuccess) e = cudaMemcpy(x_out, sd.x, NI * sizeof(double), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess)
