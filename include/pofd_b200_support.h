@@ -25,6 +25,11 @@ int pofd_fp64_peak(int device, double* tflops);
  * its absolute value). */
 int pofd_exp2_check(int device, int n, double lo, double hi, double* max_rel);
 
+/* The same for the Gaussian of the two-band colour terms, 2^(-t^2 / 64), over
+ * n values of t in [lo, hi): the largest relative difference where |t| < 256,
+ * 1 where it is not within [0, 2^-1022] beyond. */
+int pofd_exp2_gauss_check(int device, int n, double lo, double hi, double* max_rel);
+
 /* The tensor-core kernels' failure path, exercised without a fault: a kernel
  * waits with their bounded mbarrier wait (limit try_wait rounds, 1..2^20) on
  * a barrier of arrival count 1, on which nothing arrives (arrive = 0) or one

@@ -5,6 +5,7 @@
 //                      file carries HBM and BF16 figures only);
 //   * pofd_exp2_check  the table-driven exp2 of the R builders against the
 //                      CUDA library exp2;
+//   * pofd_exp2_gauss_check  the same for the colour terms' Gaussian;
 //   * pofd_wait_check  the tensor-core kernels' bounded mbarrier wait running
 //                      out and reporting it;
 //   * pofd_gauss_*     a multivariate Gaussian target with the batched
@@ -51,6 +52,36 @@ __global__ void k_exp2_check(int n, double lo, double hi, double* __restrict__ o
     const double a = pofd::dev::exp2_tab(x, e2.t);
     const double b = exp2(x);
     const double d = (x < -1022.0) ? fabs(a) : fabs(a - b) / b;
+    worst = fmax(worst, d);
+  }
+  worst = pofd::dev::block_max<256>(worst, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = worst;
+}
+
+// The colour terms' Gaussian 2^(-t^2 / 64) against the library exp2 of the
+// square's leading part, its remainder applied to first order; beyond the cap
+// at |t| = 256 whether it is at most 2^-1022.
+__global__ void k_exp2_gauss_check(int n, double lo, double hi, double* __restrict__ out) {
+  __shared__ pofd::dev::GaussTable gt;
+  __shared__ double sh[32];
+  gt.load();
+  __syncthreads();
+  const double* tab = gt.lane();
+  const pofd::dev::GaussC gc;
+  double worst = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double u = (static_cast<double>(i) + 0.5 + 0.37 * sin(static_cast<double>(i))) /
+                     static_cast<double>(n);
+    const double t = lo + (hi - lo) * u;
+    const double a = pofd::dev::exp2_gauss(t, tab, gc);
+    double d;
+    if (fabs(t) >= 256.0) {
+      d = (a >= 0.0 && a <= 2.2250738585072014e-308) ? 0.0 : 1.0;
+    } else {
+      const double q = t * t, r = fma(t, t, -q);
+      const double b = exp2(-q / 64.0) * (1.0 - r * (0.69314718055994531 / 64.0));
+      d = fabs(a - b) / b;
+    }
     worst = fmax(worst, d);
   }
   worst = pofd::dev::block_max<256>(worst, sh);
@@ -151,13 +182,15 @@ int pofd_fp64_peak(int device, double* tflops) {
   return POFD_OK;
 }
 
-int pofd_exp2_check(int device, int n, double lo, double hi, double* max_rel) {
-  if (!max_rel || n <= 0 || !(lo < hi) || !(hi < 1023.0)) return POFD_E_ARG;
+namespace {
+// The largest of the blocks' results.
+int check_max(int device, void (*kernel)(int, double, double, double*), int n, double lo,
+              double hi, double* max_rel) {
   if (cudaSetDevice(device) != cudaSuccess) return POFD_E_CUDA;
   const int blocks = 592;
   double* d = nullptr;
   if (cudaMalloc(&d, blocks * sizeof(double)) != cudaSuccess) return POFD_E_NOMEM;
-  k_exp2_check<<<blocks, 256>>>(n, lo, hi, d);
+  kernel<<<blocks, 256>>>(n, lo, hi, d);
   double h[blocks];
   const cudaError_t e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
   cudaFree(d);
@@ -166,6 +199,17 @@ int pofd_exp2_check(int device, int n, double lo, double hi, double* max_rel) {
   for (double v : h) w = std::fmax(w, v);
   *max_rel = w;
   return POFD_OK;
+}
+}  // namespace
+
+int pofd_exp2_check(int device, int n, double lo, double hi, double* max_rel) {
+  if (!max_rel || n <= 0 || !(lo < hi) || !(hi < 1023.0)) return POFD_E_ARG;
+  return check_max(device, k_exp2_check, n, lo, hi, max_rel);
+}
+
+int pofd_exp2_gauss_check(int device, int n, double lo, double hi, double* max_rel) {
+  if (!max_rel || n <= 0 || !(lo < hi)) return POFD_E_ARG;
+  return check_max(device, k_exp2_gauss_check, n, lo, hi, max_rel);
 }
 
 int pofd_wait_check(int device, unsigned limit, int arrive, int* timed_out) {
