@@ -421,7 +421,8 @@ class calcLike:
         check(lib().pofd_like1_set_tuning(self.h, k))
 
     def setFFT(self, mode):
-        """0: own FP64 FFT where the size allows (default), 1: cuFFT."""
+        """0: the library's own FP64 FFTs where the size allows (as by default,
+        the four-step one from n = 4096), 1: cuFFT."""
         check(lib().pofd_like1_set_fft(self.h, int(mode)))
 
     def ownFFT(self):

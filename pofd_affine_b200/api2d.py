@@ -321,9 +321,9 @@ class calcLikeDouble:
                 for i in range(ns.value)}
 
     def setFFT(self, mode):
-        """1: 1D cuFFT row transforms around the library's fused column
-        transform + spectrum kernel (default, n a power of two in
-        [512, 4096]); 0: 2D cuFFT transforms with the spectrum kernel between
+        """1: the library's row and column kernels, the spectrum between the
+        columns' transforms (default; where n is a power of two in [512,
+        4096]); 0: 2D cuFFT transforms with the spectrum kernel between
         them."""
         check(lib().pofd_like2_set_fft(self.h, int(mode)))
 

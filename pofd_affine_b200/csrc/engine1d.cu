@@ -13,18 +13,19 @@
 //
 // Layout in HBM (P proposals, B beam sets, D datasets, n FFT size, NI
 // interpolation nodes, nc = n/2+1):
-//   nodes [P][B][2][NI]        R at the nodes (pos/neg side)
+//   nodes [P][B][2][NI]        log2 R at the nodes (pos/neg side)
 //   spl   [P][B][2][NI][4]     node spline (y, b, c, d) per interval
-//   rbuf  [P][B][2*nc]         R grid (x dflux), then its D2Z spectrum in place
-//   pbuf  [P][D][2*nc]         per-dataset spectrum, then its Z2D P(D) in place
+//   rbuf  [P][B][2*nc]         R grid (x dflux; of the own FFT its wrap edge
+//                              only), then its spectrum
+//   pbuf  [P][D][2*nc]         per-dataset spectrum, then the P(D)
 //   tmp   [P][max(B,D)][2*nc]  rows between the passes of the own FFT; spectra
 //                              of few rows on their way to k_inv1
 //   ppart/pmidx                partial reductions of the P(D): [P][D][nchunk]
 //                              of k_pscan1, [P][D][blocks] of k_inv1
 //   pinfo [P][D]               split, normalisation, mean, log-likelihood
-// Each proposal's R and P(D) rows are contiguous so the D2Z/Z2D run as two
-// batched cuFFT calls over P*B and P*D rows.  Small grids use nodes, pbuf and
-// pinfo only (k_row1 keeps the rest in shared memory).
+// Each proposal's R and P(D) rows are contiguous, so that cuFFT's D2Z and Z2D
+// are two batched calls over P*B and P*D rows, in place.  Small grids use nodes,
+// pbuf and pinfo only (k_row1 keeps the rest in shared memory).
 #include "engine1d.cuh"
 
 #include <algorithm>

@@ -1,13 +1,15 @@
 // engine1d.cuh -- batched 1D P(D) likelihood engine (host class).
 //
 // One Engine1 evaluates calcLike::getLogLike (calcLike.cc:884-955) for a
-// batch of proposals in one stream-ordered sequence of launches: model set-up,
-// R at the interpolation nodes, the node spline, the wrapped R grid with its
-// moments, a batched D2Z, the spectrum (exp/shift/noise, one output per
-// dataset), a batched Z2D, the P(D) reduction/split pass and the finishing
-// kernel (split point, normalisation, mean, binned log-likelihood), then the
-// per-proposal sum.  The sequence is captured once per batch size into a CUDA
-// graph and replayed.
+// batch of proposals in one stream-ordered sequence of launches: R at the
+// interpolation nodes (with the model set-up), the node spline, the wrapped R
+// grid with its moments, the forward transform (the library's own or a batched
+// cuFFT D2Z), the spectrum (exp/shift/noise, one output per dataset), the
+// inverse transform with the P(D) reductions (a pass of their own after cuFFT's
+// Z2D) and the finishing kernel (split point, normalisation, mean, binned
+// log-likelihood), then the per-proposal sum; on small grids one kernel after
+// the nodes does all of it.  The sequence is captured once per batch size into
+// a CUDA graph and replayed.
 #ifndef POFD_ENGINE1D_CUH
 #define POFD_ENGINE1D_CUH
 
@@ -113,7 +115,7 @@ struct Workspace1 {
   double* cnt = nullptr;     // [P][4*KMAX] model spline: y, b, c, d per knot
   int* mstatus = nullptr;    // [P] model status
   double* sigmult = nullptr; // [P]
-  double* nodes = nullptr;   // [P][B][2][NI] R at nodes -> log2 R
+  double* nodes = nullptr;   // [P][B][2][NI] log2 R at the nodes
   double* spl = nullptr;     // [P][B][2][NI][4] spline (y,b,c,d) per interval
   double* rbuf = nullptr;    // [P][B][2*(n/2+1)] R grid / spectrum
   double* rpart = nullptr;   // [P][B][ntile][2]
@@ -122,9 +124,12 @@ struct Workspace1 {
   int* kcut_ds = nullptr;    // [P][D] noise cut-off of each dataset's spectrum
   int4* rinfo = nullptr;  // [P][D] status, noise cut-off, split search window
   double* pbuf = nullptr;    // [P][D][2*(n/2+1)] spectrum / P(D)
-  double* tmp = nullptr;     // [P][max(B,D)][2*(n/2+1)] own-FFT pass-A rows
-  double* ppart = nullptr;   // [P][D][nchunk][4] max, sum, wsum, minval
-  int* pmidx = nullptr;      // [P][D][nchunk] argmin index
+  double* tmp = nullptr;     // [P][max(B,D)][2*(n/2+1)] own-FFT pass-A rows, few-row spectra
+  // partial reductions of the P(D) rows: after cuFFT per chunk of 4096 (max,
+  // sum, index-weighted sum, smallest), of k_inv1 per block (16 chunk sums,
+  // max, index-weighted sum, smallest)
+  double* ppart = nullptr;   // [P][D][nchunk][4] or [P][D][blocks][20]
+  int* pmidx = nullptr;      // [P][D][nchunk or blocks] argmin index
   PDInfo1* pinfo = nullptr;  // [P][D]
   double* pdout = nullptr;   // [n] one P(D) for the full-array path
   float* theta_in = nullptr; // [P][npar] staging for host calls

@@ -1003,8 +1003,6 @@ __device__ int split_marginal(const double* data, int n, double dflux,
   return POFD_E_SPLIT_NONE;
 }
 
-// Marginals, split points, normalisation and means of one (proposal,
-// dataset) (PDFactoryDouble.cc:978-1118, PDDouble.cc:142-208, 355-447).
 // The column sums of a P(D) from its nrt partial rows, into the first of them,
 // in their order.  k_psplit2, one block per P(D), took 80 us for 128 partial
 // rows of n = 4096 (4 MB read by one SM), now 54 with this.
@@ -1019,6 +1017,8 @@ k_pcol2(int D, int n, int nrt, const int* __restrict__ mstatus, double* colpart)
   cp[0] = c;
 }
 
+// Marginals, split points, normalisation and means of one (proposal,
+// dataset) (PDFactoryDouble.cc:978-1118, PDDouble.cc:142-208, 355-447).
 __global__ void __launch_bounds__(SNT)
 k_psplit2(const BSet2Dev* __restrict__ bsets,
           const DSet2Dev* __restrict__ dsets, int B, int D, int n, int nc2,

@@ -3,9 +3,10 @@
 // One Engine2 evaluates calcLikeDouble::getLogLike (calcLikeDouble.cc:
 // 1195-1277) for a batch of proposals: model set-up (knot counts, sigma and
 // offset curves), per-row precompute of the log-normal colour terms,
-// the direct n x n R grid with the edge integrals, R moments and shifts, a
-// batched 2D D2Z, the spectrum (exp/shift, Hermitian projection of the
-// self-conjugate columns, one noise product per dataset), a batched 2D Z2D,
+// the direct n x n R grid with the edge integrals, R moments and shifts, the
+// forward transform, the spectrum (exp/shift, Hermitian projection of the
+// self-conjugate columns, one noise product per dataset) and the inverse
+// transform (row and column kernels, or batched 2D cuFFT around the spectrum),
 // marginal sums, split points, normalisation and means, and the bilinear
 // log-likelihood gather.  Captured into a CUDA graph per batch size and
 // pointer set.
